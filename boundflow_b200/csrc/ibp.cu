@@ -5,6 +5,8 @@
 // intersection and the ReLU split clamp.  One CTA owns a 64x64 output tile and
 // keeps two accumulators per output (centre and radius); |W| costs nothing
 // (absolute value is an operand modifier of FFMA).
+#include <cooperative_groups.h>
+
 #include "kernels.cuh"
 
 namespace bf {
@@ -158,6 +160,232 @@ __global__ void __launch_bounds__(256) ibp_linear_kernel(IbpArgs g) {
   }
 }
 
+// bounds of one output from its centre and radius sums: bias, Lp deviation, constraint intersection, split clamp, store
+__device__ __forceinline__ void ibp_finish(const IbpArgs& g, int row, int col, float c, float r) {
+  const float bb = g.bias ? __ldg(g.bias + col) : 0.f;
+  float lo = (c - r) + bb, up = (c + r) + bb;
+  if (g.row_dev) {
+    const float d = __ldg(g.row_dev + col);
+    lo -= d;
+    up += d;
+  }
+  const size_t idx = (size_t)row * g.N + col;
+  bool bad = false;
+  if (g.cons_l) {
+    lo = fmaxf(lo, g.cons_l[idx]);
+    up = fminf(up, g.cons_u[idx]);
+    bad |= lo > up;
+  }
+  if (g.split) {
+    const int s = g.split[(size_t)row * g.split_stride + col];
+    if (s > 0) lo = fmaxf(lo, 0.f);
+    if (s < 0) up = fminf(up, 0.f);
+    bad |= lo > up;
+  }
+  g.out_l[idx] = lo;
+  g.out_u[idx] = up;
+  if (bad && g.infeasible) g.infeasible[row] = 1;
+}
+__device__ __forceinline__ void centre_radius(const IbpArgs& g, float& a, float& b) {
+  if (g.in_mode != BF_IN_LOWER_UPPER) return;
+  if (g.relu_in) { a = fmaxf(a, 0.f); b = fmaxf(b, 0.f); }
+  const float c = (a + b) * 0.5f;
+  b = (b - a) * 0.5f;
+  a = c;
+}
+__device__ __forceinline__ void centre_radius4(const IbpArgs& g, float4& a, float4& b) {
+  centre_radius(g, a.x, b.x); centre_radius(g, a.y, b.y); centre_radius(g, a.z, b.z); centre_radius(g, a.w, b.w);
+}
+
+// Few outputs: 64 x 64 tiles leave most SMs idle and each walks K with one 16-deep slab in flight, so the time is K / 16
+// memory latencies.  Here a tile is 16 rows x 16 CPT columns, one thread per row and CPT columns, a slab 64 deep.  Every sum runs over k
+// in ascending order like the 64 x 64 tiles', so both give the same bits.
+// Shared slabs are [row][k] with a pitch of 68: 128-bit stores and reads without bank conflicts.
+constexpr int QM = 16, QBK = 64, QLD = QBK + 4;
+template <int CPT>
+__global__ void __launch_bounds__(256) ibp_linear_small_kernel(IbpArgs g) {
+  constexpr int QN = 16 * CPT, ROWS = 2 * QM + QN;  // centre, radius, weight rows of a slab
+  __shared__ __align__(16) float smem[2 * ROWS * QLD];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int m0 = blockIdx.x * QM, n0 = blockIdx.y * QN;
+  const int lk = tx * 4;
+  const bool vK = g.vecK != 0;
+  const bool row_ok = m0 + ty < g.B;
+  const float* pa = g.in_a + (size_t)(m0 + ty) * g.K;
+  const float* pb = g.in_b ? g.in_b + (size_t)(m0 + ty) * g.K : nullptr;
+  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 a4, b4, w4[CPT];
+  auto load_slab = [&](int k) {
+    a4 = row_ok ? load4_guard(pa, k + lk, g.K, vK) : z4;
+    b4 = (row_ok && pb) ? load4_guard(pb, k + lk, g.K, vK) : z4;
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) {
+      const int n = n0 + ty + 16 * j;
+      w4[j] = (n < g.N) ? load4_guard(g.W + (size_t)n * g.K, k + lk, g.K, vK) : z4;
+    }
+  };
+  auto store_slab = [&](int stage) {
+    float* s = smem + stage * ROWS * QLD;
+    centre_radius4(g, a4, b4);
+    *reinterpret_cast<float4*>(s + ty * QLD + lk) = a4;
+    *reinterpret_cast<float4*>(s + (QM + ty) * QLD + lk) = b4;
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) *reinterpret_cast<float4*>(s + (2 * QM + ty + 16 * j) * QLD + lk) = w4[j];
+  };
+  float accC[CPT], accR[CPT];
+#pragma unroll
+  for (int j = 0; j < CPT; ++j) accC[j] = accR[j] = 0.f;
+  const int nk = (g.K + QBK - 1) / QBK;
+  load_slab(0);
+  store_slab(0);
+  __syncthreads();
+  for (int kt = 0; kt < nk; ++kt) {
+    if (kt + 1 < nk) load_slab((kt + 1) * QBK);
+    const float* s = smem + (kt & 1) * ROWS * QLD;
+#pragma unroll
+    for (int q = 0; q < QBK; q += 4) {
+      const float4 c = *reinterpret_cast<const float4*>(s + ty * QLD + q);
+      const float4 r = *reinterpret_cast<const float4*>(s + (QM + ty) * QLD + q);
+#pragma unroll
+      for (int j = 0; j < CPT; ++j) {
+        const float4 w = *reinterpret_cast<const float4*>(s + (2 * QM + tx + 16 * j) * QLD + q);
+        accC[j] = fmaf(c.x, w.x, accC[j]); accR[j] = fmaf(r.x, fabsf(w.x), accR[j]);
+        accC[j] = fmaf(c.y, w.y, accC[j]); accR[j] = fmaf(r.y, fabsf(w.y), accR[j]);
+        accC[j] = fmaf(c.z, w.z, accC[j]); accR[j] = fmaf(r.z, fabsf(w.z), accR[j]);
+        accC[j] = fmaf(c.w, w.w, accC[j]); accR[j] = fmaf(r.w, fabsf(w.w), accR[j]);
+      }
+    }
+    if (kt + 1 < nk) store_slab((kt + 1) & 1);
+    __syncthreads();
+  }
+  if (!row_ok) return;
+#pragma unroll
+  for (int j = 0; j < CPT; ++j) {
+    const int col = n0 + tx + 16 * j;
+    if (col < g.N) ibp_finish(g, m0 + ty, col, accC[j], accR[j]);
+  }
+}
+
+// Few outputs and long rows (the layer behind a flatten: K = 4096, 8192): walking K in one CTA is a serial chain whatever the tile.  A tile is
+// 32 x 32, a slab 64 deep (six 128-bit loads in flight per thread), the CTA's four thread groups take 16 of its columns each, and a
+// cluster of up to eight CTAs splits K; partial sums meet in (distributed) shared memory in rank order, without a
+// workspace or atomics.  200 x 4096 x 512: 89 us (64 x 64 tiles: 370), bound by FFMA issue at 224 CTAs; 256 x 1568 x 100: 17 us (144);
+// 16 x 8192 x 10: 26 us (619), bound by the 16 serial slabs of a rank.
+// Shared slabs are [k][row] with rows XOR-ed by ((k >> 2) & 7) << 2: transposed stores conflict two-way, 128-bit reads not at all.
+// Up to IBP_SERIAL_K terms the sums keep their order: bounds of networks of that width feed optimisation loops whose
+// trajectories follow the last bit, and the serial chain costs a few microseconds there.
+constexpr int IBP_SERIAL_K = 1024;
+constexpr int STM = 32, STN = 32, SBK = 64, SSLAB = SBK * 32, SGROUPS = 4;
+__device__ __forceinline__ int swz(int k, int row) { return k * 32 + (row ^ (((k >> 2) & 7) << 2)); }
+
+__global__ void __launch_bounds__(256) ibp_linear_split_kernel(IbpArgs g, int kper) {
+  __shared__ __align__(16) float smem[2 * 3 * SSLAB];
+  static_assert(SGROUPS * 2 * STM * STN + 2 * STM * STN <= 2 * 3 * SSLAB, "the reduction reuses the slabs");
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int tid = threadIdx.x, kg = tid >> 6, tx = tid & 7, ty = (tid & 63) >> 3;
+  const int m0 = blockIdx.x * STM, n0 = blockIdx.y * STN;
+  const int k0 = blockIdx.z * kper, k1 = min(g.K, k0 + kper);
+  const int lrow = tid >> 4, lk = (tid & 15) * 4;
+  const bool vK = g.vecK != 0;
+  float accC[4][4], accR[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) accC[i][j] = accR[i][j] = 0.f;
+
+  float4 creg[2], rreg[2], wreg[2];
+  auto load_slab = [&](int k) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int m = m0 + lrow + 16 * i, n = n0 + lrow + 16 * i;
+      creg[i] = rreg[i] = wreg[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (m < g.B) {
+        creg[i] = load4_guard(g.in_a + (size_t)m * g.K, k + lk, k1, vK);
+        if (g.in_b) rreg[i] = load4_guard(g.in_b + (size_t)m * g.K, k + lk, k1, vK);
+      }
+      if (n < g.N) wreg[i] = load4_guard(g.W + (size_t)n * g.K, k + lk, k1, vK);
+    }
+  };
+  auto store_slab = [&](int stage) {
+    float* cs = smem + stage * 3 * SSLAB;
+    float* rs = cs + SSLAB;
+    float* ws = rs + SSLAB;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float4 a = creg[i], b = rreg[i];
+      centre_radius4(g, a, b);
+      const int r = lrow + 16 * i;
+      cs[swz(lk, r)] = a.x; cs[swz(lk + 1, r)] = a.y; cs[swz(lk + 2, r)] = a.z; cs[swz(lk + 3, r)] = a.w;
+      rs[swz(lk, r)] = b.x; rs[swz(lk + 1, r)] = b.y; rs[swz(lk + 2, r)] = b.z; rs[swz(lk + 3, r)] = b.w;
+      ws[swz(lk, r)] = wreg[i].x; ws[swz(lk + 1, r)] = wreg[i].y; ws[swz(lk + 2, r)] = wreg[i].z; ws[swz(lk + 3, r)] = wreg[i].w;
+    }
+  };
+
+  const int nk = (k1 > k0) ? (k1 - k0 + SBK - 1) / SBK : 0;
+  if (nk > 0) {
+    load_slab(k0);
+    store_slab(0);
+  }
+  __syncthreads();
+  for (int kt = 0; kt < nk; ++kt) {
+    const int stage = kt & 1;
+    if (kt + 1 < nk) load_slab(k0 + (kt + 1) * SBK);
+    const float* cs = smem + stage * 3 * SSLAB;
+    const float* rs = cs + SSLAB;
+    const float* ws = rs + SSLAB;
+#pragma unroll
+    for (int q = 0; q < SBK / SGROUPS; ++q) {
+      const int kk = kg * (SBK / SGROUPS) + q;
+      const float4 c4 = *reinterpret_cast<const float4*>(&cs[swz(kk, ty * 4)]);
+      const float4 r4 = *reinterpret_cast<const float4*>(&rs[swz(kk, ty * 4)]);
+      const float4 w4 = *reinterpret_cast<const float4*>(&ws[swz(kk, tx * 4)]);
+      const float c[4] = {c4.x, c4.y, c4.z, c4.w};
+      const float r[4] = {r4.x, r4.y, r4.z, r4.w};
+      const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          accC[i][j] = fmaf(c[i], w[j], accC[i][j]);
+          accR[i][j] = fmaf(r[i], fabsf(w[j]), accR[i][j]);
+        }
+    }
+    if (kt + 1 < nk) store_slab(stage ^ 1);
+    __syncthreads();
+  }
+
+  // thread groups of the CTA, then ranks of the cluster
+  float* red = smem;                                  // [SGROUPS][2][32][32]
+  float* part = smem + SGROUPS * 2 * STM * STN;       // [2][32][32]
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float* d = red + kg * 2 * STM * STN + (ty * 4 + i) * STN + tx * 4;
+    *reinterpret_cast<float4*>(d) = make_float4(accC[i][0], accC[i][1], accC[i][2], accC[i][3]);
+    *reinterpret_cast<float4*>(d + STM * STN) = make_float4(accR[i][0], accR[i][1], accR[i][2], accR[i][3]);
+  }
+  __syncthreads();
+  for (int e = tid; e < 2 * STM * STN; e += 256) {
+    float t = red[e];
+#pragma unroll
+    for (int q = 1; q < SGROUPS; ++q) t += red[q * 2 * STM * STN + e];
+    part[e] = t;
+  }
+  cluster.sync();
+  const int ranks = gridDim.z;
+  for (int e = blockIdx.z * 256 + tid; e < STM * STN; e += ranks * 256) {
+    const int row = m0 + (e >> 5), col = n0 + (e & 31);
+    if (row >= g.B || col >= g.N) continue;
+    float c = 0.f, r = 0.f;
+    for (int j = 0; j < ranks; ++j) {
+      const float* p = cluster.map_shared_rank(part, j);
+      c += p[e];
+      r += p[STM * STN + e];
+    }
+    ibp_finish(g, row, col, c, r);
+  }
+  cluster.sync();  // the peers read this CTA's shared memory
+}
+
 int launch_ibp_linear(const float* in_a, const float* in_b, int in_mode, int relu_in, const float* W, const float* bias,
                       const int8_t* split, int split_stride, const float* cons_l, const float* cons_u, float* out_l,
                       float* out_u, int* infeasible, int B, int K, int N, const float* row_dev, cudaStream_t stream) {
@@ -168,9 +396,30 @@ int launch_ibp_linear(const float* in_a, const float* in_b, int in_mode, int rel
   g.vecN = (N % 4 == 0);
   const void* nptrs[] = {bias, cons_l, cons_u, out_l, out_u, row_dev};
   for (const void* p : nptrs) if (p && (reinterpret_cast<uintptr_t>(p) & 15u)) g.vecN = 0;
-  dim3 grid(ceil_div(B, IBM), ceil_div(N, IBN));
   timing_begin(T_IBP_LINEAR, stream);
-  ibp_linear_kernel<<<grid, 256, 0, stream>>>(g);
+  const bool few = (long long)ceil_div(B, IBM) * ceil_div(N, IBN) < 148;  // less than one 64 x 64 tile per SM
+  if (few && K <= IBP_SERIAL_K) {
+    const int gx = ceil_div(B, QM);
+    if ((long long)gx * ceil_div(N, 32) < 148) ibp_linear_small_kernel<1><<<dim3(gx, ceil_div(N, 16)), 256, 0, stream>>>(g);
+    else ibp_linear_small_kernel<2><<<dim3(gx, ceil_div(N, 32)), 256, 0, stream>>>(g);
+  } else if (few) {
+    const long long tiles = (long long)ceil_div(B, STM) * ceil_div(N, STN);
+    const int slabs = ceil_div(K, SBK);
+    int ks = 1;
+    while (ks < 8 && tiles * ks < 148 && slabs >= 2 * ks) ks *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ceil_div(B, STM), ceil_div(N, STN), ks);
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = ks;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, ibp_linear_split_kernel, g, ceil_div(slabs, ks) * SBK);
+  } else {
+    ibp_linear_kernel<<<dim3(ceil_div(B, IBM), ceil_div(N, IBN)), 256, 0, stream>>>(g);
+  }
   // weights and bias once, the input interval once, both output bounds once (+ the split bytes)
   timing_end(T_IBP_LINEAR, stream, 4.0 * ((double)K * N + N) + 8.0 * (double)B * (K + N) + (split ? (double)B * N : 0.0),
              4.0 * (double)B * K * N);
