@@ -1,17 +1,15 @@
 // Conv2d layers (NCHW activations, OIHW weights, groups = 1, dilation = 1):
 // interval propagation in centre/radius form and the CROWN backward transformer
 // (ReLU backward + transposed convolution of the coefficient rows).
+#include <cooperative_groups.h>
+
 #include "kernels.cuh"
 
 namespace bf {
 
 // ---------------------------------------------------------------------------
-// IBP conv2d: one thread per output element; weights are warp-uniform loads
-// (a warp covers consecutive output columns of one output channel).
+// Forward convolutions (interval propagation, and plain rows) as implicit GEMMs on FP32 FFMA tiles
 // ---------------------------------------------------------------------------
-struct ConvGeom {
-  int Ci, Hi, Wi, Co, Ho, Wo, kh, kw, sh, sw, ph, pw;
-};
 
 struct IbpConvArgs {
   const float* in_a; const float* in_b; int in_mode; int relu_in;
@@ -22,61 +20,252 @@ struct IbpConvArgs {
   int B, Ci, Hi, Wi, Co, Ho, Wo, kh, kw, sh, sw, ph, pw;
 };
 
-__global__ void __launch_bounds__(256) ibp_conv2d_kernel(IbpConvArgs g) {
-  const long long n_out = (long long)g.Co * g.Ho * g.Wo;
-  const long long total = (long long)g.B * n_out;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
-    const int wo = (int)(idx % g.Wo);
-    const int ho = (int)((idx / g.Wo) % g.Ho);
-    const int co = (int)((idx / ((long long)g.Wo * g.Ho)) % g.Co);
-    const int b = (int)(idx / n_out);
-    float accC = 0.f, accR = 0.f;
-    const int h0 = ho * g.sh - g.ph, w0 = wo * g.sw - g.pw;
-    for (int ci = 0; ci < g.Ci; ++ci) {
-      const float* wa = g.W + ((size_t)co * g.Ci + ci) * g.kh * g.kw;
-      const size_t in_off = ((size_t)b * g.Ci + ci) * g.Hi * g.Wi;
-      for (int r = 0; r < g.kh; ++r) {
-        const int hi = h0 + r;
-        if (hi < 0 || hi >= g.Hi) continue;
-        for (int s = 0; s < g.kw; ++s) {
-          const int wi = w0 + s;
-          if (wi < 0 || wi >= g.Wi) continue;
-          const float w = __ldg(wa + r * g.kw + s);
-          float a = __ldg(g.in_a + in_off + (size_t)hi * g.Wi + wi);
-          float bb = __ldg(g.in_b + in_off + (size_t)hi * g.Wi + wi);
-          float c, rad;
-          if (g.in_mode == BF_IN_LOWER_UPPER) {
-            if (g.relu_in) { a = fmaxf(a, 0.f); bb = fmaxf(bb, 0.f); }
-            c = (a + bb) * 0.5f;
-            rad = (bb - a) * 0.5f;
-          } else {
-            c = a;
-            rad = bb;
-          }
-          accC = fmaf(c, w, accC);
-          accR = fmaf(rad, fabsf(w), accR);
+// A CTA computes TN output channels x TM = 4096 / TN output pixels (pixels of all images in one line), a thread 4 x 4 of them,
+// over slabs of CBK input taps in (channel, kernel row, kernel column) order.  The gather positions of a slab's taps are
+// decoded once per CTA into `tab`, two slabs ahead.  INTERVAL: centre and radius accumulators; otherwise one convolution of
+// plain rows (in_a).  Small grids split K over a cluster of two or four CTAs, whose partial sums meet in distributed
+// shared memory in rank order.
+// Bound by FFMA issue and the slab's shared-memory reads (three 128-bit reads for 32 FMAs): 200 images, 32 -> 32 channels, 4x4 / 2
+// kernel on 32 x 32: 138 us = 24 TFLOP/s (one thread per output, weights and pixels read through L1 for every tap, before: 1.1 ms);
+// plain rows, 432 x 16 x 14 x 14 -> 32, 4x4 / 2: 32 us (164).
+template <int TN>
+struct ConvTile {
+  static constexpr int TM = 4096 / TN, SLAB = (TN == 16) ? 8 : 16;
+};
+
+template <bool INTERVAL, int TN>
+__global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper, int vec) {
+  constexpr int TM = ConvTile<TN>::TM, CBK = ConvTile<TN>::SLAB, ACCS = INTERVAL ? 2 : 1;
+  constexpr int NA = TM * CBK / 256, KSTEP = 256 / TM, WLD = TN + 4, NW = (TN * CBK + 255) / 256;
+  constexpr int STAGE = ACCS * CBK * TM + CBK * WLD, PART = ACCS * TM * TN;
+  __shared__ __align__(16) float smem[2 * STAGE > PART ? 2 * STAGE : PART];
+  __shared__ int4 tab[2][CBK];
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int tid = threadIdx.x, tx = tid % (TM / 4), ty = tid / (TM / 4);
+  const int taps = g.kh * g.kw, K = g.Ci * taps, howo = g.Ho * g.Wo, hw = g.Hi * g.Wi;
+  const long long npix = (long long)g.B * howo;
+  const long long p0 = (long long)blockIdx.x * TM;
+  const int c0 = blockIdx.y * TN;
+  const int k0 = blockIdx.z * kper, k1 = min(K, k0 + kper);
+  const int nk = (k1 > k0) ? (k1 - k0 + CBK - 1) / CBK : 0;
+
+  // this thread's pixel as a loader
+  const long long lp = p0 + tid % TM;
+  const int lk = tid / TM;
+  const bool live = lp < npix;
+  int h0 = 0, w0 = 0;
+  const float *base_a = g.in_a, *base_b = g.in_b;
+  if (live) {
+    const int b = (int)(lp / howo), q = (int)(lp - (long long)b * howo);
+    h0 = (q / g.Wo) * g.sh - g.ph;
+    w0 = (q % g.Wo) * g.sw - g.pw;
+    const long long off = (long long)b * g.Ci * hw;
+    base_a += off;
+    if (INTERVAL) base_b += off;
+  }
+  auto decode = [&](int kt) {  // x: offset of the tap in the image, y / z: kernel row / column (far outside past the end of K)
+    if (tid < CBK) {
+      const int k = k0 + kt * CBK + tid;
+      const int ci = k / taps, t = k - ci * taps, r = t / g.kw, s = t - r * g.kw;
+      tab[kt & 1][tid] = (k < k1) ? make_int4(ci * hw + r * g.Wi + s, r, s, 0) : make_int4(0, 1 << 29, 0, 0);
+    }
+  };
+  const int pix_off = h0 * g.Wi + w0;
+  float ra[NA], rb[INTERVAL ? NA : 1], rw[NW];
+  auto load_slab = [&](int kt) {
+#pragma unroll
+    for (int j = 0; j < NA; ++j) {
+      const int4 t = tab[kt & 1][lk + j * KSTEP];
+      const int hi = h0 + t.y, wi = w0 + t.z;
+      const bool ok = live && (unsigned)hi < (unsigned)g.Hi && (unsigned)wi < (unsigned)g.Wi;
+      ra[j] = ok ? __ldg(base_a + (pix_off + t.x)) : 0.f;
+      if (INTERVAL) rb[j] = ok ? __ldg(base_b + (pix_off + t.x)) : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < NW; ++j) {
+      const int e = tid + j * 256, co = c0 + e / CBK, k = k0 + kt * CBK + e % CBK;
+      rw[j] = (e < TN * CBK && co < g.Co && k < k1) ? __ldg(g.W + (size_t)co * K + k) : 0.f;
+    }
+  };
+  auto store_slab = [&](int stage) {
+    float* as = smem + stage * STAGE;
+    float* ws = as + ACCS * CBK * TM;
+#pragma unroll
+    for (int j = 0; j < NA; ++j) {
+      float a = ra[j];
+      const int at = (lk + j * KSTEP) * TM + tid % TM;
+      if (INTERVAL) {
+        float b = rb[j];
+        if (g.in_mode == BF_IN_LOWER_UPPER) {
+          if (g.relu_in) { a = fmaxf(a, 0.f); b = fmaxf(b, 0.f); }
+          const float c = (a + b) * 0.5f;
+          b = (b - a) * 0.5f;
+          a = c;
+        }
+        as[CBK * TM + at] = b;
+      }
+      as[at] = a;
+    }
+#pragma unroll
+    for (int j = 0; j < NW; ++j) {
+      const int e = tid + j * 256;
+      if (e < TN * CBK) ws[(e % CBK) * WLD + e / CBK] = rw[j];
+    }
+  };
+
+  float accC[4][4], accR[INTERVAL ? 4 : 1][4];  // [channel][pixel]
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      accC[i][j] = 0.f;
+      if (INTERVAL) accR[i][j] = 0.f;
+    }
+  decode(0);
+  decode(1);
+  __syncthreads();
+  if (nk > 0) {
+    load_slab(0);
+    store_slab(0);
+  }
+  __syncthreads();
+  for (int kt = 0; kt < nk; ++kt) {
+    const int stage = kt & 1;
+    if (kt + 1 < nk) load_slab(kt + 1);
+    if (kt + 2 < nk) decode(kt + 2);  // its slot was last read before the previous barrier
+    const float* as = smem + stage * STAGE;
+    const float* ws = as + ACCS * CBK * TM;
+#pragma unroll
+    for (int kk = 0; kk < CBK; ++kk) {
+      const float4 c4 = *reinterpret_cast<const float4*>(as + kk * TM + tx * 4);
+      const float4 w4 = *reinterpret_cast<const float4*>(ws + kk * WLD + ty * 4);
+      float4 r4 = c4;
+      if (INTERVAL) r4 = *reinterpret_cast<const float4*>(as + CBK * TM + kk * TM + tx * 4);
+      const float c[4] = {c4.x, c4.y, c4.z, c4.w}, r[4] = {r4.x, r4.y, r4.z, r4.w}, w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          accC[i][j] = fmaf(c[j], w[i], accC[i][j]);
+          if (INTERVAL) accR[i][j] = fmaf(r[j], fabsf(w[i]), accR[i][j]);
+        }
+    }
+    if (kt + 1 < nk) store_slab(stage ^ 1);
+    __syncthreads();
+  }
+
+  const int ranks = gridDim.z;
+  if (ranks > 1) {
+    const int at = ty * 4 * TM + tx * 4;  // part[acc][channel][pixel]
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      *reinterpret_cast<float4*>(smem + at + i * TM) = make_float4(accC[i][0], accC[i][1], accC[i][2], accC[i][3]);
+      if (INTERVAL) *reinterpret_cast<float4*>(smem + TM * TN + at + i * TM) = make_float4(accR[i][0], accR[i][1], accR[i][2], accR[i][3]);
+    }
+    cluster.sync();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (i % ranks != (int)blockIdx.z) continue;  // rank z finishes channels z, z + ranks, ... of every thread
+      float4 c = make_float4(0.f, 0.f, 0.f, 0.f), r = c;
+      for (int q = 0; q < ranks; ++q) {
+        const float* p = cluster.map_shared_rank(smem, q);
+        const float4 a = *reinterpret_cast<const float4*>(p + at + i * TM);
+        c.x += a.x; c.y += a.y; c.z += a.z; c.w += a.w;
+        if (INTERVAL) {
+          const float4 b = *reinterpret_cast<const float4*>(p + TM * TN + at + i * TM);
+          r.x += b.x; r.y += b.y; r.z += b.z; r.w += b.w;
         }
       }
+      accC[i][0] = c.x; accC[i][1] = c.y; accC[i][2] = c.z; accC[i][3] = c.w;
+      if (INTERVAL) { accR[i][0] = r.x; accR[i][1] = r.y; accR[i][2] = r.z; accR[i][3] = r.w; }
     }
-    const float bias = g.bias ? __ldg(g.bias + co) : 0.f;
-    float lo = (accC - accR) + bias, up = (accC + accR) + bias;
-    const long long j = idx - (long long)b * n_out;
-    bool bad = false;
-    if (g.cons_l) {
-      lo = fmaxf(lo, g.cons_l[idx]);
-      up = fminf(up, g.cons_u[idx]);
-      bad |= lo > up;
-    }
-    if (g.split) {
-      const int s = g.split[(size_t)b * g.split_stride + j];
-      if (s > 0) lo = fmaxf(lo, 0.f);
-      if (s < 0) up = fminf(up, 0.f);
-      bad |= lo > up;
-    }
-    g.out_l[idx] = lo;
-    g.out_u[idx] = up;
-    if (bad && g.infeasible) g.infeasible[b] = 1;
+    cluster.sync();
   }
+
+  const long long pt = p0 + tx * 4;
+  if (pt >= npix) return;
+  int b4[4], q4[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    b4[j] = (int)((pt + j) / howo);
+    q4[j] = (int)((pt + j) - (long long)b4[j] * howo);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int co = c0 + ty * 4 + i;
+    if (co >= g.Co || (ranks > 1 && i % ranks != (int)blockIdx.z)) continue;
+    const float bias = g.bias ? __ldg(g.bias + co) : 0.f;
+    float lo[4], up[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (!INTERVAL) {
+        lo[j] = accC[i][j] + bias;
+        continue;
+      }
+      lo[j] = (accC[i][j] - accR[i][j]) + bias;
+      up[j] = (accC[i][j] + accR[i][j]) + bias;
+      if (pt + j < npix && (g.cons_l || g.split)) {
+        const size_t idx = ((size_t)b4[j] * g.Co + co) * howo + q4[j];
+        bool bad = false;
+        if (g.cons_l) {
+          lo[j] = fmaxf(lo[j], g.cons_l[idx]);
+          up[j] = fminf(up[j], g.cons_u[idx]);
+          bad |= lo[j] > up[j];
+        }
+        if (g.split) {
+          const int s = g.split[(size_t)b4[j] * g.split_stride + (size_t)co * howo + q4[j]];
+          if (s > 0) lo[j] = fmaxf(lo[j], 0.f);
+          if (s < 0) up[j] = fminf(up[j], 0.f);
+          bad |= lo[j] > up[j];
+        }
+        if (bad && g.infeasible) g.infeasible[b4[j]] = 1;
+      }
+    }
+    if (vec) {  // Ho * Wo % 4 == 0: a thread's four pixels lie in one image, and 16-byte aligned outputs
+      const size_t idx = ((size_t)b4[0] * g.Co + co) * howo + q4[0];
+      *reinterpret_cast<float4*>(g.out_l + idx) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+      if (INTERVAL) *reinterpret_cast<float4*>(g.out_u + idx) = make_float4(up[0], up[1], up[2], up[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (pt + j >= npix) continue;
+        const size_t idx = ((size_t)b4[j] * g.Co + co) * howo + q4[j];
+        g.out_l[idx] = lo[j];
+        if (INTERVAL) g.out_u[idx] = up[j];
+      }
+    }
+  }
+}
+
+template <bool INTERVAL, int TN>
+static int launch_conv_tile_n(const IbpConvArgs& g, int vec, cudaStream_t stream) {
+  const long long npix = (long long)g.B * g.Ho * g.Wo;
+  const long long tiles = (npix + ConvTile<TN>::TM - 1) / ConvTile<TN>::TM;
+  const int slabs = ceil_div((long long)g.Ci * g.kh * g.kw, ConvTile<TN>::SLAB), ctas_y = ceil_div(g.Co, TN);
+  BF_REQUIRE(ctas_y <= 65535 && tiles <= 2147483647LL, BF_E_UNSUPPORTED, "conv2d: too many output channels or pixels");
+  int ks = 1;
+  while (ks < 4 && tiles * ctas_y * ks < 148 && slabs >= 4 * ks) ks *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)tiles, ctas_y, ks);
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = ks;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, conv_tile_kernel<INTERVAL, TN>, g, ceil_div(slabs, ks) * ConvTile<TN>::SLAB, vec);
+  BF_CHECK_LAUNCH("conv_tile_kernel");
+  return BF_OK;
+}
+
+// tile width by the output channels: a wider one wastes accumulators on channels that do not exist
+template <bool INTERVAL>
+static int launch_conv_tile(const IbpConvArgs& g, cudaStream_t stream) {
+  int vec = (g.Ho * g.Wo) % 4 == 0 && ((reinterpret_cast<uintptr_t>(g.out_l) | reinterpret_cast<uintptr_t>(g.out_u)) & 15u) == 0;
+  if (g.Co <= 16) return launch_conv_tile_n<INTERVAL, 16>(g, vec, stream);
+  if (g.Co <= 32) return launch_conv_tile_n<INTERVAL, 32>(g, vec, stream);
+  return launch_conv_tile_n<INTERVAL, 64>(g, vec, stream);
 }
 
 int launch_ibp_conv2d(const float* in_a, const float* in_b, int in_mode, int relu_in, const float* W, const float* bias,
@@ -84,59 +273,20 @@ int launch_ibp_conv2d(const float* in_a, const float* in_b, int in_mode, int rel
                       float* out_u, int* infeasible, int B, const bf_layer_desc& L, cudaStream_t stream) {
   IbpConvArgs g{in_a, in_b, in_mode, relu_in, W, bias, split, split_stride, cons_l, cons_u, out_l, out_u, infeasible,
                 B, L.Ci, L.Hi, L.Wi, L.Co, L.Ho, L.Wo, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw};
-  const long long total = (long long)B * L.Co * L.Ho * L.Wo;
-  long long blocks = (total + 255) / 256;
-  if (blocks > 148LL * 32) blocks = 148LL * 32;
   timing_begin(T_IBP_CONV, stream);
-  ibp_conv2d_kernel<<<(int)blocks, 256, 0, stream>>>(g);
+  const int rc = launch_conv_tile<true>(g, stream);
   timing_end(T_IBP_CONV, stream, 4.0 * ((double)L.Co * L.Ci * L.kh * L.kw + L.Co) + 8.0 * (double)B * (L.n_in + L.n_out),
-             4.0 * (double)total * L.Ci * L.kh * L.kw);
-  BF_CHECK_LAUNCH("ibp_conv2d_kernel");
-  return BF_OK;
+             4.0 * (double)B * L.n_out * L.Ci * L.kh * L.kw);
+  return rc;
 }
 
-// ---------------------------------------------------------------------------
-// Forward convolution of rows (the gradient sweep of the alpha optimiser pushes its adjoint
-// points through the layers in forward direction): out[m] = conv2d(in[m], W) + bias, one thread
-// per output element.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) conv_forward_rows_kernel(const float* __restrict__ in, const float* __restrict__ W,
-                                                                const float* __restrict__ bias, float* __restrict__ out,
-                                                                long long total, ConvGeom g) {
-  const long long n_out = (long long)g.Co * g.Ho * g.Wo;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
-    const int wo = (int)(idx % g.Wo);
-    const int ho = (int)((idx / g.Wo) % g.Ho);
-    const int co = (int)((idx / ((long long)g.Wo * g.Ho)) % g.Co);
-    const long long m = idx / n_out;
-    const int h0 = ho * g.sh - g.ph, w0 = wo * g.sw - g.pw;
-    float acc = 0.f;
-    for (int ci = 0; ci < g.Ci; ++ci) {
-      const float* wa = W + ((size_t)co * g.Ci + ci) * g.kh * g.kw;
-      const float* ip = in + ((size_t)m * g.Ci + ci) * g.Hi * g.Wi;
-      for (int r = 0; r < g.kh; ++r) {
-        const int hi = h0 + r;
-        if (hi < 0 || hi >= g.Hi) continue;
-        for (int sc = 0; sc < g.kw; ++sc) {
-          const int wi = w0 + sc;
-          if (wi < 0 || wi >= g.Wi) continue;
-          acc = fmaf(__ldg(ip + (size_t)hi * g.Wi + wi), __ldg(wa + r * g.kw + sc), acc);
-        }
-      }
-    }
-    out[idx] = acc + (bias ? __ldg(bias + co) : 0.f);
-  }
-}
-
+// Forward convolution of rows: out[m] = conv2d(in[m], W) + bias (the gradient sweep of the alpha optimiser pushes its
+// adjoint points through the layers in forward direction).
 int launch_conv_forward_rows(const float* in, const float* W, const float* bias, float* out, int M, const bf_layer_desc& L,
                              cudaStream_t stream) {
-  ConvGeom g{L.Ci, L.Hi, L.Wi, L.Co, L.Ho, L.Wo, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw};
-  const long long total = (long long)M * L.n_out;
-  long long blocks = (total + 255) / 256;
-  if (blocks > 148LL * 32) blocks = 148LL * 32;
-  conv_forward_rows_kernel<<<(int)blocks, 256, 0, stream>>>(in, W, bias, out, total, g);
-  BF_CHECK_LAUNCH("conv_forward_rows_kernel");
-  return BF_OK;
+  IbpConvArgs g{in, nullptr, BF_IN_MID_RAD, 0, W, bias, nullptr, 0, nullptr, nullptr, out, nullptr, nullptr,
+                M, L.Ci, L.Hi, L.Wi, L.Co, L.Ho, L.Wo, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw};
+  return launch_conv_tile<false>(g, stream);
 }
 
 // ---------------------------------------------------------------------------

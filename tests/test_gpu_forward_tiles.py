@@ -1,0 +1,74 @@
+"""Forward interval kernels at the edges of their tiles and dispatch rules, against float64.
+
+Error of a float32 sum of n products in any order: at most n * 2^-24 * sum |c w| (+ the same for the radius), first order.
+"""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    assert torch.cuda.is_available(), "GPU tests need a CUDA device"
+    from boundflow_b200.csrc import build
+
+    build.build()
+    return torch.device("cuda", 0)
+
+
+# 16-row / 16- and 32-column tiles (K <= 1024), K split over a cluster (K > 1024; ragged, unaligned, shorter than eight ranks), 64 x 64 tiles
+@pytest.mark.parametrize("B,K,N", [(1, 1, 1), (16, 63, 16), (17, 64, 17), (37, 1024, 130), (100, 65, 513), (200, 512, 512), (640, 30, 1000), (16, 8192, 10), (1, 1025, 1),
+                                   (33, 1568, 100), (200, 4096, 65), (31, 1031, 33), (513, 2050, 513), (640, 1100, 1000)])
+def test_ibp_linear_tiles(dev, B, K, N):
+    from boundflow_b200 import _lib
+
+    lib = _lib.load()
+    g = torch.Generator("cuda").manual_seed(B + K + N)
+    l = torch.randn(B, K, generator=g, device=dev)
+    u = l + torch.rand(B, K, generator=g, device=dev)
+    W = torch.randn(N, K, generator=g, device=dev)
+    b = torch.randn(N, generator=g, device=dev)
+    split = torch.randint(-1, 2, (B, N), generator=g, device=dev, dtype=torch.int8)
+    out = [torch.full((B, N), float("nan"), device=dev) for _ in range(2)]
+    bad = torch.zeros(B, dtype=torch.int32, device=dev)
+    _lib.check(lib.bf_ibp_linear(l.data_ptr(), u.data_ptr(), _lib.IN_LOWER_UPPER, 1, W.data_ptr(), b.data_ptr(), split.data_ptr(), N, None, None,
+                                 out[0].data_ptr(), out[1].data_ptr(), bad.data_ptr(), B, K, N, None))
+    l64, u64, W64 = l.relu().double(), u.relu().double(), W.double()
+    c, r = (l64 + u64) / 2, (u64 - l64) / 2
+    mid, dev_ = c @ W64.t(), r @ W64.abs().t()
+    lo, up = mid - dev_ + b.double(), mid + dev_ + b.double()
+    lo, up = torch.where(split > 0, lo.clamp(min=0), lo), torch.where(split < 0, up.clamp(max=0), up)
+    tol = (K + 4) * 2.0 ** -24 * (c.abs() @ W64.abs().t() + dev_) + 1e-6
+    assert ((out[0].double() - lo).abs() <= tol).all() and ((out[1].double() - up).abs() <= tol).all()
+    sure = ((lo - up).abs() > 2 * tol).all(dim=1)
+    assert torch.equal(bad[sure].bool(), (lo > up).any(dim=1)[sure])
+
+
+# channel tiles of 16, 32 and 64, ragged pixels and channels, kernels larger than a slab, clusters of 1, 2 and 4 CTAs along K
+@pytest.mark.parametrize("B,Ci,H,W,Co,k,s,p", [(1, 1, 5, 7, 1, 1, 1, 0), (3, 1, 28, 28, 16, 4, 2, 1), (2, 3, 9, 11, 17, 3, 1, 1), (5, 16, 14, 14, 33, 4, 2, 1),
+                                               (64, 8, 16, 16, 32, 3, 2, 1), (300, 3, 16, 15, 20, 5, 1, 2), (7, 64, 8, 8, 70, 4, 2, 1), (40, 40, 13, 13, 64, 3, 1, 0)])
+def test_ibp_conv_tiles(dev, B, Ci, H, W, Co, k, s, p):
+    from boundflow_b200 import _lib
+
+    lib = _lib.load()
+    g = torch.Generator("cuda").manual_seed(B + Ci + Co + k)
+    l = torch.randn(B, Ci, H, W, generator=g, device=dev)
+    u = l + torch.rand(l.shape, generator=g, device=dev)
+    w = torch.randn(Co, Ci, k, k, generator=g, device=dev)
+    b = torch.randn(Co, generator=g, device=dev)
+    conv = lambda x, ww: torch.nn.functional.conv2d(x, ww, None, s, p)
+    l64, u64, w64 = l.relu().double(), u.relu().double(), w.double()
+    c, r = (l64 + u64) / 2, (u64 - l64) / 2
+    mid, dev_ = conv(c, w64) + b.double()[:, None, None], conv(r, w64.abs())
+    split = torch.randint(-1, 2, mid.shape, generator=g, device=dev, dtype=torch.int8)
+    out = [torch.full(mid.shape, float("nan"), device=dev) for _ in range(2)]
+    bad = torch.zeros(B, dtype=torch.int32, device=dev)
+    _lib.check(lib.bf_ibp_conv2d(l.data_ptr(), u.data_ptr(), _lib.IN_LOWER_UPPER, 1, w.data_ptr(), b.data_ptr(), split.data_ptr(), split[0].numel(), None,
+                                 None, out[0].data_ptr(), out[1].data_ptr(), bad.data_ptr(), B, Ci, H, W, Co, k, k, s, s, p, p, None))
+    lo, up = mid - dev_, mid + dev_
+    lo, up = torch.where(split > 0, lo.clamp(min=0), lo), torch.where(split < 0, up.clamp(max=0), up)
+    tol = (Ci * k * k + 4) * 2.0 ** -24 * (conv(c.abs(), w64.abs()) + dev_) + 1e-6
+    assert ((out[0].double() - lo).abs() <= tol).all() and ((out[1].double() - up).abs() <= tol).all()
+    sure = ((lo - up).abs() > 2 * tol).flatten(1).all(dim=1)
+    assert torch.equal(bad[sure].bool(), (lo > up).flatten(1).any(dim=1)[sure])
