@@ -23,11 +23,15 @@ struct IbpConvArgs {
 // A CTA computes TN output channels x TM = 4096 / TN output pixels (pixels of all images in one line), a thread 4 x 4 of them,
 // over slabs of CBK input taps in (channel, kernel row, kernel column) order.  The gather positions of a slab's taps are
 // decoded once per CTA into `tab`, two slabs ahead.  INTERVAL: centre and radius accumulators; otherwise one convolution of
-// plain rows (in_a).  Small grids split K over a cluster of two or four CTAs, whose partial sums meet in distributed
-// shared memory in rank order.
+// plain rows (in_a).  A sum runs over its taps in ascending order; only above CONV_SERIAL_K taps a small grid splits K over a
+// cluster of two or four CTAs, whose partial sums meet in distributed shared memory in rank order.  (Splitting shorter sums
+// too was 10-20 us faster per layer at 16 images, but a pre-activation bound within an ulp of zero then changes sides
+// against the serial sum and takes the relaxation of its ReLU with it.)
 // Bound by FFMA issue and the slab's shared-memory reads (three 128-bit reads for 32 FMAs): 200 images, 32 -> 32 channels, 4x4 / 2
 // kernel on 32 x 32: 138 us = 24 TFLOP/s (one thread per output, weights and pixels read through L1 for every tap, before: 1.1 ms);
 // plain rows, 432 x 16 x 14 x 14 -> 32, 4x4 / 2: 32 us (164).
+constexpr int CONV_SERIAL_K = 1024;
+
 template <int TN>
 struct ConvTile {
   static constexpr int TM = 4096 / TN, SLAB = (TN == 16) ? 8 : 16;
@@ -241,10 +245,10 @@ template <bool INTERVAL, int TN>
 static int launch_conv_tile_n(const IbpConvArgs& g, int vec, cudaStream_t stream) {
   const long long npix = (long long)g.B * g.Ho * g.Wo;
   const long long tiles = (npix + ConvTile<TN>::TM - 1) / ConvTile<TN>::TM;
-  const int slabs = ceil_div((long long)g.Ci * g.kh * g.kw, ConvTile<TN>::SLAB), ctas_y = ceil_div(g.Co, TN);
+  const int K = g.Ci * g.kh * g.kw, slabs = ceil_div(K, ConvTile<TN>::SLAB), ctas_y = ceil_div(g.Co, TN);
   BF_REQUIRE(ctas_y <= 65535 && tiles <= 2147483647LL, BF_E_UNSUPPORTED, "conv2d: too many output channels or pixels");
   int ks = 1;
-  while (ks < 4 && tiles * ctas_y * ks < 148 && slabs >= 4 * ks) ks *= 2;
+  while (K > CONV_SERIAL_K && ks < 4 && tiles * ctas_y * ks < 148 && slabs >= 4 * ks) ks *= 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)tiles, ctas_y, ks);
   cfg.blockDim = dim3(256);
