@@ -15,17 +15,26 @@ struct BwdEpilogue {
   float* out;            // [M,N] or nullptr
   const float* mid;      // [D,N] (only with `partial`)
   const float* rad;      // [D,N]
-  float* partial;        // [M, gridDim.y] concretisation partial sums or nullptr
+  float* partial;        // [M, ntiles] concretisation partial sums or nullptr
   int side;              // BF_SIDE_LOWER: a*mid - |a|*rad ; BF_SIDE_UPPER: a*mid + |a|*rad
+  int ntiles;            // column tiles; 32-row tiles: CTAs of a further column compute the row sums
 };
 
 template <int PRO, int MH, int NH>
 __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_bwd_linear_kernel(GemmArgs g, BwdEpilogue e) {
-  __shared__ __align__(16) float smem[MAINLOOP_SMEM_FLOATS];
+  __shared__ __align__(16) float smem[MH == 0 ? SMALL_SMEM_FLOATS : MAINLOOP_SMEM_FLOATS];
   constexpr int TM = (MH == 0) ? 32 : 64 * MH, MR = (MH == 0) ? 2 : 4 * MH;
   const int m0 = blockIdx.x * TM, n0 = blockIdx.y * (64 * NH);
   float acc[8][8];
-  gemm_mainloop<PRO, false, MH, NH>(g, m0, n0, acc, smem);
+  if constexpr (MH == 0) {
+    if ((int)blockIdx.y == e.ntiles) {
+      prologue_row_sums(g, m0);
+      return;
+    }
+    gemm_small_mainloop<PRO, false>(g, m0, n0, acc, smem);
+  } else {
+    gemm_mainloop<PRO, false, MH, NH>(g, m0, n0, acc, smem);
+  }
 
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const bool vN = g.vecN != 0;
@@ -57,7 +66,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_bwd_linear_kernel(GemmA
       p += __shfl_xor_sync(0xffffffffu, p, 2);
       p += __shfl_xor_sync(0xffffffffu, p, 4);
       p += __shfl_xor_sync(0xffffffffu, p, 8);
-      if (tx == 0 && row_ok) e.partial[(size_t)row * gridDim.y + blockIdx.y] = p;
+      if (tx == 0 && row_ok) e.partial[(size_t)row * e.ntiles + blockIdx.y] = p;
     }
   }
 }
@@ -66,13 +75,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_bwd_linear_kernel(GemmA
 // delta[m] (+)= sum_k A[m,k] * kbias[k].  A store-bound pass, so no tiles: a thread keeps its four
 // columns of W in registers and walks the block's rows, whose K values sit in shared memory.
 constexpr int THIN_KMAX = 16;
-constexpr int THIN_ROWS = 64;
+constexpr int THIN_ROWS = 64;   // rows of a block, at most: a small problem takes fewer (its blocks' rows are a serial chain)
 __global__ void __launch_bounds__(128) crown_bwd_thin_kernel(const float* __restrict__ A, const float* __restrict__ W,
                                                              const float* __restrict__ kbias, float* __restrict__ out,
-                                                             float* __restrict__ delta, int accumulate, int M, int K, int N) {
+                                                             float* __restrict__ delta, int accumulate, int M, int K, int N, int block_rows) {
   __shared__ float a_s[THIN_ROWS * THIN_KMAX];
-  const int m0 = blockIdx.x * THIN_ROWS;
-  const int rows = min(THIN_ROWS, M - m0);
+  const int m0 = blockIdx.x * block_rows;
+  const int rows = min(block_rows, M - m0);
   for (int i = threadIdx.x; i < rows * K; i += blockDim.x) a_s[i] = A[(size_t)m0 * K + i];
   __syncthreads();
   const int cg = blockIdx.y * blockDim.x + threadIdx.x;  // group of four columns
@@ -107,7 +116,7 @@ __global__ void __launch_bounds__(128) crown_bwd_thin_kernel(const float* __rest
 // 128 x 128 tiles leave most of the 148 SMs idle on small problems: below one CTA per SM the kernels switch to 64 x 64 tiles
 bool ffma_small_tiles(int M, int N) { return (long long)ceil_div(M, BM) * ceil_div(N, BN) < 148; }
 // ... and 32 x 64 tiles when even the 64 x 64 tiles give fewer CTAs than SMs
-static bool ffma_quarter_tiles(int M, int N) { return ffma_small_tiles(M, N) && M > 32 && (long long)ceil_div(M, 64) * ceil_div(N, 64) < 148; }
+static bool ffma_quarter_tiles(int M, int N) { return ffma_small_tiles(M, N) && (long long)ceil_div(M, 64) * ceil_div(N, 64) < 148; }
 
 // Measured on B200 (c3: 1152 x 256 x 256 layers, 20 Adam steps): 8.9 ms on these tiles against 9.7 ms on the tcgen05
 // kernels, whose per-launch time of 23-36 us is a serial k-loop on 9-36 CTAs; at 144 rows 6.3 against 7.3 ms.  Beyond one
@@ -120,9 +129,12 @@ int launch_crown_bwd_linear(const float* A, const float* dpos, const float* dneg
                             int K, int N, cudaStream_t stream) {
   if (!dpos && !add && !partial && A_prev && K <= THIN_KMAX && N % 4 == 0 &&
       ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(A_prev)) & 15u) == 0) {
-    dim3 grid(ceil_div(M, THIN_ROWS), ceil_div(N / 4, 128));
+    const int cols = ceil_div(N / 4, 128);
+    int rows = THIN_ROWS;
+    while (rows > 4 && ceil_div(M, rows) * cols < 4 * 148) rows /= 2;
+    dim3 grid(ceil_div(M, rows), cols);
     timing_begin(T_THIN, stream);
-    crown_bwd_thin_kernel<<<grid, 128, 0, stream>>>(A, W, kbias, A_prev, delta, accumulate, M, K, N);
+    crown_bwd_thin_kernel<<<grid, 128, 0, stream>>>(A, W, kbias, A_prev, delta, accumulate, M, K, N, rows);
     timing_end(T_THIN, stream, 4.0 * (double)M * N + 4.0 * (double)M * K + 4.0 * (double)K * N, 2.0 * (double)M * K * N);
     BF_CHECK_LAUNCH("crown_bwd_thin_kernel");
     return BF_OK;
@@ -137,10 +149,10 @@ int launch_crown_bwd_linear(const float* A, const float* dpos, const float* dneg
   for (const void* p : nptrs) if (p && (reinterpret_cast<uintptr_t>(p) & 15u)) g.vecN = 0;
   g.dpos = dpos; g.dneg = dneg; g.epos = epos; g.eneg = eneg; g.add = add; g.kbias = kbias;
   g.delta = delta; g.accumulate = accumulate;
-  BwdEpilogue e{A_prev, mid, rad, partial, side};
+  BwdEpilogue e{A_prev, mid, rad, partial, side, crown_bwd_partial_tiles(N, M)};
   timing_begin(T_BWD, stream);
   if (ffma_quarter_tiles(M, N)) {  // 32 x 64 tiles
-    dim3 grid(ceil_div(M, 32), ceil_div(N, 64));
+    dim3 grid(ceil_div(M, 32), e.ntiles + (delta ? 1 : 0));
     crown_bwd_linear_kernel<PRO_RELU, 0, 1><<<grid, GEMM_THREADS, 0, stream>>>(g, e);
   } else if (ffma_small_tiles(M, N)) {  // 64 x 64 tiles: four times as many CTAs
     dim3 grid(ceil_div(M, 64), ceil_div(N, 64));
@@ -186,7 +198,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_adjoint_linear_kernel(G
   constexpr int TM = (MH == 0) ? 32 : 64 * MH, TN = 64 * NH, MR = (MH == 0) ? 2 : 4 * MH;
   const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
   float acc[8][8];
-  gemm_mainloop<PRO, true, MH, NH>(g, m0, n0, acc, dsmem);
+  if constexpr (MH == 0) gemm_small_mainloop<PRO, true>(g, m0, n0, acc, dsmem);
+  else gemm_mainloop<PRO, true, MH, NH>(g, m0, n0, acc, dsmem);
   // the main loop ends with __syncthreads(): the slabs may now be overwritten by the stage tile
 
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;

@@ -72,3 +72,30 @@ def test_ibp_conv_tiles(dev, B, Ci, H, W, Co, k, s, p):
     assert ((out[0].double() - lo).abs() <= tol).all() and ((out[1].double() - up).abs() <= tol).all()
     sure = ((lo - up).abs() > 2 * tol).flatten(1).all(dim=1)
     assert torch.equal(bad[sure].bool(), (lo > up).flatten(1).any(dim=1)[sure])
+
+
+# 32 x 64 tiles of the CROWN backward step: one row, ragged rows, columns and k, one slab and several, rows of a domain across tiles
+@pytest.mark.parametrize("B,S,K,N", [(1, 1, 20, 30), (1, 9, 64, 64), (3, 11, 65, 61), (37, 9, 130, 257), (128, 9, 256, 256), (5, 40, 513, 100), (64, 9, 100, 784)])
+@pytest.mark.parametrize("side", [0, 1])
+def test_backward_small_tiles(dev, B, S, K, N, side):
+    from boundflow_b200 import _lib
+
+    lib = _lib.load()
+    g = torch.Generator("cuda").manual_seed(B * K + N)
+    A = torch.randn(B, S, K, generator=g, device=dev)
+    au, al, bu = (torch.rand(B, K, generator=g, device=dev) for _ in range(3))
+    W = torch.randn(K, N, generator=g, device=dev)
+    b = torch.randn(K, generator=g, device=dev)
+    out = torch.full((B, S, N), float("nan"), device=dev)
+    delta = torch.full((B, S), 2.0, device=dev)
+    _lib.check(lib.bf_crown_relu_linear_bwd(A.data_ptr(), side, au.data_ptr(), al.data_ptr(), bu.data_ptr(), None, None, W.data_ptr(), b.data_ptr(),
+                                            out.data_ptr(), delta.data_ptr(), 1, B, S, K, N, None))
+    A64, pos = A.double(), A >= 0
+    lo, hi = (al, au) if side == 0 else (au, al)
+    lam = A64 * torch.where(pos, lo.double()[:, None], hi.double()[:, None])
+    icpt = A64 * torch.where(pos == (side == 1), bu.double()[:, None], torch.zeros_like(A64))
+    ref, ref_d = lam @ W.double(), 2.0 + (icpt + lam * b.double()).sum(-1)
+    tol = (K + 2) * 2.0 ** -24 * (lam.abs() @ W.double().abs()) + 1e-6
+    tol_d = (2 * K + 4) * 2.0 ** -24 * (2.0 + (icpt.abs() + (lam * b.double()).abs()).sum(-1))
+    assert ((out.double() - ref).abs() <= tol).all()
+    assert ((delta.double() - ref_d).abs() <= tol_d).all()
