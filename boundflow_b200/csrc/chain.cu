@@ -209,7 +209,7 @@ int launch_ibp_conv2d(const float* in_a, const float* in_b, int in_mode, int rel
                       float* out_u, int* infeasible, int B, const bf_layer_desc& L, cudaStream_t stream);
 int launch_crown_bwd_conv2d(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
                             const float* W, const float* bias, float* A_prev, float* delta, int accumulate, int M, int S,
-                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add = nullptr);
+                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add = nullptr, bool windowed = false);
 size_t crown_bwd_conv2d_scratch_bytes(int M, const bf_layer_desc& L);
 int launch_onehot_conv_rows(int first, const float* W, const float* bias, float* A_prev, float* delta, int M, int S,
                             const bf_layer_desc& L, cudaStream_t stream);
@@ -587,7 +587,7 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
       Lw.ph = 0; Lw.pw = 0;
       Lw.n_out = L.Co * Lw.Ho * Lw.Wo; Lw.n_in = L.Ci * Lw.Hi * Lw.Wi;
       float* dst = ws.buf[toggle];
-      rc = bf::launch_crown_bwd_conv2d(lam, nullptr, nullptr, nullptr, nullptr, L.W, nullptr, dst, nullptr, 1, M, S, Lw, nullptr, stream);
+      rc = bf::launch_crown_bwd_conv2d(lam, nullptr, nullptr, nullptr, nullptr, L.W, nullptr, dst, nullptr, 1, M, S, Lw, nullptr, stream, nullptr, true);
       win.C = L.Ci; win.WH = Lw.Hi; win.WW = Lw.Wi; win.H = L.Hi; win.W = L.Wi;
       win.ty = win.ty * L.sh - L.ph; win.sy *= L.sh;
       win.tx = win.tx * L.sw - L.pw; win.sx *= L.sw;

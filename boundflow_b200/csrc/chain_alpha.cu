@@ -11,7 +11,7 @@ namespace bf {
 
 int launch_crown_bwd_conv2d(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
                             const float* W, const float* bias, float* A_prev, float* delta, int accumulate, int M, int S,
-                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add = nullptr);
+                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add = nullptr, bool windowed = false);
 size_t crown_bwd_conv2d_scratch_bytes(int M, const bf_layer_desc& L);
 int launch_conv_forward_rows(const float* in, const float* W, const float* bias, float* out, int M, const bf_layer_desc& L,
                              cudaStream_t stream);

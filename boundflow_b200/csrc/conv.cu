@@ -3,7 +3,9 @@
 // (ReLU backward + transposed convolution of the coefficient rows).
 #include <cooperative_groups.h>
 
-#include "kernels.cuh"
+#include <stdlib.h>
+
+#include "conv_tc.cuh"
 
 namespace bf {
 
@@ -748,6 +750,16 @@ static int launch_convT_rowseg(const ConvTArgs& g, cudaStream_t stream) {
   return BF_E_UNSUPPORTED;
 }
 
+// Where full coefficient rows take the tensor-core kernel (conv_tc.cu).  From one 128-position tile per SM on: 512 rows of
+// 64 channels 8 x 8 -> 64 channels 16 x 16, 4x4 / 2 (324 tiles): 90 us against 172; 512 rows of 40 channels 9 x 9, 3x3 / 2: 37
+// against 84.  Not for few input channels (1 or 3 channels fill an eighth of the narrowest MMA: 73 against 42 us, 205 against
+// 91) and not for more than nine taps per phase (5x5 / 1: 128 against 120 us; its MMAs are bound by their issue).
+// Windowed rows stay on the FP32 kernels although the tensor cores took a third of their time (64,000 windows, 32 -> 32
+// channels: 0.33 against 1.5 ms): they bound every neuron of the conv layers, millions of values whose last bit differs, and a
+// few of those lie within that bit of zero, where the relaxation of their ReLU changes sides: 2 of 8 networks moved by 6e-5.
+// Full rows bound the neurons of linear layers and the specs, some ten thousand values: no change of sides in 8 networks.
+constexpr int CONV_TC_MIN_TILES = 148, CONV_TC_MIN_CI = 8, CONV_TC_MAX_TAPS = 9;
+
 // scaled coefficients [M, n_out] followed by the per-chunk partial sums of the intercept term [M, chunks]
 static size_t relu_rows_lam_bytes(int M, int n_out) { return ((size_t)M * n_out * sizeof(float) + 255) & ~(size_t)255; }
 size_t crown_bwd_conv2d_scratch_bytes(int M, const bf_layer_desc& L) {
@@ -775,9 +787,40 @@ static int launch_convT(const ConvTArgs& g0, cudaStream_t stream) {
   return BF_OK;
 }
 
+// The tensor-core kernel takes ReLU scaling, row sums and transposed convolution of full rows in one pass.
+// BF_E_UNSUPPORTED: the caller takes the FP32 kernels.
+static int launch_conv_tc_bwd(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg, const float* add,
+                              const float* W, const float* bias, float* A_prev, float* delta, int accumulate, int M, int S,
+                              const bf_layer_desc& L, void* scratch, cudaStream_t stream) {
+  const char* ffma = getenv("BF_B200_FORCE_FFMA");
+  if ((ffma && ffma[0] == '1') || !A_prev || L.Ci < CONV_TC_MIN_CI ||
+      ceil_div(L.kh, L.sh) * ceil_div(L.kw, L.sw) > CONV_TC_MAX_TAPS)
+    return BF_E_UNSUPPORTED;
+  ConvTcProblem c{};
+  c.A = A; c.dpos = dpos; c.dneg = dneg; c.epos = epos; c.eneg = eneg; c.add = dpos ? add : nullptr;
+  c.bias = bias; c.W = W; c.out = A_prev;
+  c.M = M; c.S = S; c.Co = L.Co; c.Ci = L.Ci; c.WH = L.Ho; c.WW = L.Wo; c.Hi = L.Hi; c.Wi = L.Wi;
+  c.kh = L.kh; c.kw = L.kw; c.sh = L.sh; c.sw = L.sw; c.ph = L.ph; c.pw = L.pw;
+  int slots = 0, tiles = 0;
+  if (!conv_tc_supports(c, &slots, &tiles) || tiles < CONV_TC_MIN_TILES) return BF_E_UNSUPPORTED;
+  const bool sums = delta && (dpos || bias || !accumulate);
+  if (sums) {  // the row sums take the place that the scaled coefficients have on the FP32 path
+    if (!scratch || slots > L.Co * L.Ho * L.Wo) return BF_E_UNSUPPORTED;
+    c.partial = static_cast<float*>(scratch);
+  }
+  timing_begin(T_CONV_T, stream);
+  int rc = launch_conv_tc(c, stream);
+  timing_end(T_CONV_T, stream, 4.0 * (double)M * (L.n_out + L.n_in) + 4.0 * (double)L.Co * L.Ci * L.kh * L.kw,
+             2.0 * (double)M * L.n_out * L.Ci * L.kh * L.kw);
+  if (rc == BF_OK && sums) rc = launch_sum_partials(accumulate ? delta : nullptr, c.partial, slots, delta, M, stream);
+  return rc;
+}
+
 int launch_crown_bwd_conv2d(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
                             const float* W, const float* bias, float* A_prev, float* delta, int accumulate, int M, int S,
-                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add = nullptr) {
+                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add = nullptr, bool windowed = false) {
+  const int tc = windowed ? BF_E_UNSUPPORTED : launch_conv_tc_bwd(A, dpos, dneg, epos, eneg, add, W, bias, A_prev, delta, accumulate, M, S, L, scratch, stream);
+  if (tc != BF_E_UNSUPPORTED) return tc;
   const float* lam = A;
   const bool need_pro = (dpos != nullptr) || (bias != nullptr) || (delta != nullptr && !accumulate);
   if (need_pro) {

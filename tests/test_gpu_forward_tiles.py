@@ -99,3 +99,44 @@ def test_backward_small_tiles(dev, B, S, K, N, side):
     tol_d = (2 * K + 4) * 2.0 ** -24 * (2.0 + (icpt.abs() + (lam * b.double()).abs()).sum(-1))
     assert ((out.double() - ref).abs() <= tol).all()
     assert ((delta.double() - ref_d).abs() <= tol_d).all()
+
+
+# tensor-core ReLU + transposed convolution: ragged channels (Co % 16, Ci below a block, several blocks), odd maps, rows that no window reaches
+# ((H + 2p - k) % s != 0), rows shorter and longer than a tile, both sides, with and without a ReLU
+@pytest.mark.parametrize("B,S,Ci,H,W,Co,k,s,p", [(8, 40, 8, 9, 9, 16, 3, 1, 1), (5, 80, 13, 14, 11, 21, 4, 2, 1), (4, 64, 32, 16, 16, 64, 3, 1, 1), (4, 64, 64, 16, 16, 64, 4, 2, 1),
+                                                 (30, 50, 32, 9, 7, 40, 3, 2, 0), (3, 40, 20, 33, 32, 17, 4, 2, 1), (300, 70, 9, 2, 3, 8, 2, 1, 0)])
+@pytest.mark.parametrize("side,relu", [(0, True), (1, True), (0, False)])
+def test_conv_backward_tensor_cores(dev, B, S, Ci, H, W, Co, k, s, p, side, relu):
+    from boundflow_b200 import _lib
+
+    lib = _lib.load()
+    Ho, Wo = (H + 2 * p - k) // s + 1, (W + 2 * p - k) // s + 1
+    g = torch.Generator("cuda").manual_seed(B + Ci + Co)
+    A = torch.randn(B, S, Co, Ho, Wo, generator=g, device=dev)
+    au, al, bu = (torch.rand(B, Co, Ho, Wo, generator=g, device=dev) for _ in range(3))
+    w = torch.randn(Co, Ci, k, k, generator=g, device=dev)
+    b = torch.randn(Co, generator=g, device=dev)
+    out = torch.full((B, S, Ci, H, W), float("nan"), device=dev)
+    delta = torch.full((B, S), 2.0, device=dev)
+    nbytes = lib.bf_crown_relu_conv2d_bwd_scratch_bytes(B, S, Co, Ho, Wo)
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    before = _lib.tc_launch_count()
+    a_u, a_l, b_u = (au.data_ptr(), al.data_ptr(), bu.data_ptr()) if relu else (None, None, None)
+    _lib.check(lib.bf_crown_relu_conv2d_bwd(A.data_ptr(), side, a_u, a_l, b_u, None, w.data_ptr(), b.data_ptr(), out.data_ptr(), delta.data_ptr(), 1,
+                                            scratch.data_ptr(), nbytes, B, S, Ci, H, W, Co, Ho, Wo, k, k, s, s, p, p, None))
+    assert _lib.tc_launch_count() == before + 1
+    lam, icpt = A.double(), torch.zeros_like(A, dtype=torch.float64)
+    if relu:
+        pos = A >= 0
+        lo, hi = (al, au) if side == 0 else (au, al)
+        icpt = lam * torch.where(pos == (side == 1), bu.double()[:, None], icpt)
+        lam = lam * torch.where(pos, lo.double()[:, None], hi.double()[:, None])
+    opad = (H - ((Ho - 1) * s - 2 * p + k), W - ((Wo - 1) * s - 2 * p + k))
+    conv_t = lambda x, ww: torch.nn.functional.conv_transpose2d(x.flatten(0, 1), ww, None, s, p, output_padding=opad).view(out.shape)
+    ref = conv_t(lam, w.double())
+    ref_d = 2.0 + (icpt + lam * b.double()[:, None, None]).sum((2, 3, 4))
+    # operands are exact to 2^-23 each; the sums keep the bound of an FP32 sum of Co k^2 / s^2 products
+    tol = (Co * (k * k) / (s * s) + 8) * 2.0 ** -24 * conv_t(lam.abs(), w.double().abs()) + 1e-6
+    tol_d = (2 * Co * Ho * Wo + 8) * 2.0 ** -24 * (2.0 + (icpt.abs() + (lam * b.double()[:, None, None]).abs()).sum((2, 3, 4)))
+    assert ((out.double() - ref).abs() <= tol).all()
+    assert ((delta.double() - ref_d).abs() <= tol_d).all()
