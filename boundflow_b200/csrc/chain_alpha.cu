@@ -293,17 +293,16 @@ static int alpha_loop(const char* who, const bf_chain* chain, const float* C, co
       if (rc != BF_OK) return rc;
       sc = bf::adam_scalars(t, lr, paired ? BF_REDUCE_SUM : spec_reduce, S);  // row weights already carry 1/S of a paired mean
     }
+    std::vector<bf::StepSegment> seg;
     for (int r = 0; r < R; ++r) {
       const int n = chain->layers[chain->relu_layers[r]].n_in;
-      rc = bf::launch_adam_step(alpha[r], ws.m[r], ws.v[r], ws.grad[r], ws.improve, best_alpha[r], pre_l[r], pre_u[r], ws.sl[r],
-                                sc, last ? 0 : 1, B, n, stream);
-      if (rc != BF_OK) return rc;
-      if (with_beta) {
-        rc = bf::launch_beta_step(beta[r], ws.mb[r], ws.vb[r], ws.gsum[r], splits[r], split_strides ? split_strides[r] : n,
-                                  ws.improve, best_beta[r], ws.addv[r], sc, last ? 0 : 1, B, n, stream);
-        if (rc != BF_OK) return rc;
-      }
+      seg.push_back({alpha[r], ws.m[r], ws.v[r], ws.grad[r], best_alpha[r], ws.sl[r], pre_l[r], pre_u[r], nullptr, 0, n, 0, 0});
+      if (with_beta)
+        seg.push_back({beta[r], ws.mb[r], ws.vb[r], ws.gsum[r], best_beta[r], ws.addv[r], nullptr, nullptr, splits[r],
+                       split_strides ? split_strides[r] : n, n, 1, 0});
     }
+    rc = bf::launch_optimiser_step(seg.data(), (int)seg.size(), ws.improve, sc, last ? 0 : 1, B, stream);
+    if (rc != BF_OK) return rc;
   }
   if (best_upper) {
     // the upper bound of each domain's best iteration = the upper sweep at its best alpha (beta acts on the lower side only)

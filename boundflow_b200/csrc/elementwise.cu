@@ -249,69 +249,101 @@ __device__ __forceinline__ void adam_one(float& a, float& mi, float& vi, float g
   sl = (up <= 0.f) ? 0.f : ((lo >= 0.f) ? 1.f : a);
 }
 
-// grid (B, column chunks): one domain row per blockIdx.x, VEC consecutive columns per thread.
-template <int VEC>
-__global__ void __launch_bounds__(128) adam_step_kernel(float* __restrict__ alpha, float* __restrict__ m, float* __restrict__ v,
-                                                        float* __restrict__ grad, const int* __restrict__ improve,
-                                                        float* __restrict__ best_alpha, const float* __restrict__ pre_l,
-                                                        const float* __restrict__ pre_u, float* __restrict__ slope_l,
-                                                        AdamScalars sc, int do_update, int n) {
+// One optimiser step of all ReLUs' alphas and betas.  grid (B, column chunks, segments): one domain row per blockIdx.x, one
+// parameter tensor per blockIdx.z; a chunk is 512 columns where 16-byte accesses are legal, else 128.  A step of a small loop
+// is bound by its launches: five 256-wide layers took five launches of 5.2 us (alpha) per step.
+__global__ void __launch_bounds__(128) optimiser_step_kernel(StepArgs p, const int* __restrict__ improve, AdamScalars sc, int do_update) {
+  const StepSegment& g = p.seg[blockIdx.z];
   const int b = blockIdx.x;
-  const int j = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
-  if (j >= n) return;
-  const size_t i = (size_t)b * n + j;
-  const bool imp = improve[b] != 0;
-  if (VEC == 4) {
-    float4 a = *reinterpret_cast<const float4*>(alpha + i);
-    if (imp) *reinterpret_cast<float4*>(best_alpha + i) = a;
-    if (!do_update) return;
-    float4 g = *reinterpret_cast<const float4*>(grad + i);
-    float4 mi = *reinterpret_cast<const float4*>(m + i), vi = *reinterpret_cast<const float4*>(v + i);
-    const float4 lo = *reinterpret_cast<const float4*>(pre_l + i), up = *reinterpret_cast<const float4*>(pre_u + i);
+  const int j = (blockIdx.y * blockDim.x + threadIdx.x) * (g.vec ? 4 : 1);
+  if (j >= g.n) return;
+  const size_t i = (size_t)b * g.n + j;
+  const bool imp = improve != nullptr && g.best != nullptr && improve[b] != 0;
+  if (g.beta) {
+    const float s = g.split ? (float)g.split[(size_t)b * g.split_stride + j] : 0.f;
+    float bt = g.x[i];
+    if (imp) g.best[i] = bt;
+    if (do_update) {
+      const float d = g.grad[i] * sc.grad_scale * (-s);
+      g.grad[i] = 0.f;
+      float mi = g.m[i], vi = g.v[i];
+      mi = mi + sc.one_minus_beta1 * (d - mi);
+      vi = vi * sc.beta2 + sc.one_minus_beta2 * d * d;
+      const float denom = sqrtf(vi) / sc.bc2_sqrt + sc.eps;
+      bt = fmaxf(bt - sc.lr_step * (mi / denom), 0.f);
+      g.m[i] = mi;
+      g.v[i] = vi;
+      g.x[i] = bt;
+    }
+    g.out[i] = -bt * s;
+  } else if (g.vec) {
+    float4 a = *reinterpret_cast<const float4*>(g.x + i);
+    const float4 was = a;
+    if (!do_update) {
+      if (imp) *reinterpret_cast<float4*>(g.best + i) = was;
+      return;
+    }
+    const float4 d = *reinterpret_cast<const float4*>(g.grad + i);
+    float4 mi = *reinterpret_cast<const float4*>(g.m + i), vi = *reinterpret_cast<const float4*>(g.v + i);
+    const float4 lo = *reinterpret_cast<const float4*>(g.pre_l + i), up = *reinterpret_cast<const float4*>(g.pre_u + i);
     float4 sl;
-    adam_one(a.x, mi.x, vi.x, g.x * sc.grad_scale, lo.x, up.x, sl.x, sc);
-    adam_one(a.y, mi.y, vi.y, g.y * sc.grad_scale, lo.y, up.y, sl.y, sc);
-    adam_one(a.z, mi.z, vi.z, g.z * sc.grad_scale, lo.z, up.z, sl.z, sc);
-    adam_one(a.w, mi.w, vi.w, g.w * sc.grad_scale, lo.w, up.w, sl.w, sc);
-    *reinterpret_cast<float4*>(grad + i) = make_float4(0.f, 0.f, 0.f, 0.f);
-    *reinterpret_cast<float4*>(m + i) = mi;
-    *reinterpret_cast<float4*>(v + i) = vi;
-    *reinterpret_cast<float4*>(alpha + i) = a;
-    *reinterpret_cast<float4*>(slope_l + i) = sl;
+    adam_one(a.x, mi.x, vi.x, d.x * sc.grad_scale, lo.x, up.x, sl.x, sc);
+    adam_one(a.y, mi.y, vi.y, d.y * sc.grad_scale, lo.y, up.y, sl.y, sc);
+    adam_one(a.z, mi.z, vi.z, d.z * sc.grad_scale, lo.z, up.z, sl.z, sc);
+    adam_one(a.w, mi.w, vi.w, d.w * sc.grad_scale, lo.w, up.w, sl.w, sc);
+    if (imp) *reinterpret_cast<float4*>(g.best + i) = was;
+    *reinterpret_cast<float4*>(g.grad + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4*>(g.m + i) = mi;
+    *reinterpret_cast<float4*>(g.v + i) = vi;
+    *reinterpret_cast<float4*>(g.x + i) = a;
+    *reinterpret_cast<float4*>(g.out + i) = sl;
   } else {
-    float a = alpha[i];
-    if (imp) best_alpha[i] = a;
+    float a = g.x[i];
+    if (imp) g.best[i] = a;
     if (!do_update) return;
-    float mi = m[i], vi = v[i], sl;
-    adam_one(a, mi, vi, grad[i] * sc.grad_scale, pre_l[i], pre_u[i], sl, sc);
-    grad[i] = 0.f;
-    m[i] = mi;
-    v[i] = vi;
-    alpha[i] = a;
-    slope_l[i] = sl;
+    float mi = g.m[i], vi = g.v[i], sl;
+    adam_one(a, mi, vi, g.grad[i] * sc.grad_scale, g.pre_l[i], g.pre_u[i], sl, sc);
+    g.grad[i] = 0.f;
+    g.m[i] = mi;
+    g.v[i] = vi;
+    g.x[i] = a;
+    g.out[i] = sl;
   }
+}
+
+int launch_optimiser_step(const StepSegment* seg, int count, const int* improve, AdamScalars sc, int do_update, int B, cudaStream_t stream) {
+  for (int first = 0; first < count; first += STEP_SEGMENTS) {
+    StepArgs p{};
+    const int here = count - first < STEP_SEGMENTS ? count - first : STEP_SEGMENTS;
+    int chunks = 1;
+    double elements = 0.0;
+    for (int k = 0; k < here; ++k) {
+      StepSegment g = seg[first + k];
+      g.vec = !g.beta && g.n % 4 == 0;
+      const void* ptrs[] = {g.x, g.m, g.v, g.grad, g.best, g.pre_l, g.pre_u, g.out};
+      for (const void* q : ptrs) if (reinterpret_cast<uintptr_t>(q) & 15u) g.vec = 0;
+      const int need = ceil_div(g.vec ? g.n / 4 : g.n, 128);
+      if (need > chunks) chunks = need;
+      elements += (double)B * g.n;
+      p.seg[k] = g;
+    }
+    BF_REQUIRE(chunks <= 65535, BF_E_UNSUPPORTED, "optimiser step: layer too wide");
+    timing_begin(T_ADAM, stream);
+    optimiser_step_kernel<<<dim3(B, chunks, here), 128, 0, stream>>>(p, improve, sc, do_update);
+    // the optimiser's own traffic: read parameter, m, v, grad and write parameter, m, v (28 B per element); the kernel also
+    // reads the pre-activation bounds, clears the gradient and writes the next lower slope and the best-alpha snapshot
+    // (up to 48 B per element in all), which replaces separate relaxation / snapshot passes
+    timing_end(T_ADAM, stream, (do_update ? 28.0 : 8.0) * elements, do_update ? 10.0 * elements : 0.0);
+    BF_CHECK_LAUNCH("optimiser_step_kernel");
+  }
+  return BF_OK;
 }
 
 int launch_adam_step(float* alpha, float* m, float* v, float* grad, const int* improve, float* best_alpha,
                      const float* pre_l, const float* pre_u, float* slope_l, AdamScalars sc, int do_update, int B, int n,
                      cudaStream_t stream) {
-  bool vec = (n % 4 == 0);
-  const void* ptrs[] = {alpha, m, v, grad, best_alpha, pre_l, pre_u, slope_l};
-  for (const void* q : ptrs) if (reinterpret_cast<uintptr_t>(q) & 15u) vec = false;
-  timing_begin(T_ADAM, stream);
-  if (vec) {
-    dim3 grid(B, ceil_div(n / 4, 128));
-    adam_step_kernel<4><<<grid, 128, 0, stream>>>(alpha, m, v, grad, improve, best_alpha, pre_l, pre_u, slope_l, sc, do_update, n);
-  } else {
-    dim3 grid(B, ceil_div(n, 128));
-    adam_step_kernel<1><<<grid, 128, 0, stream>>>(alpha, m, v, grad, improve, best_alpha, pre_l, pre_u, slope_l, sc, do_update, n);
-  }
-  // the optimiser's own traffic: read alpha, m, v, grad and write alpha, m, v (28 B per element); the kernel also
-  // reads the pre-activation bounds, clears the gradient and writes the next lower slope and the best-alpha snapshot
-  // (up to 48 B per element in all), which replaces separate relaxation / snapshot passes
-  timing_end(T_ADAM, stream, (do_update ? 28.0 : 8.0) * (double)B * n, do_update ? 10.0 * (double)B * n : 0.0);
-  BF_CHECK_LAUNCH("adam_step_kernel");
-  return BF_OK;
+  const StepSegment g{alpha, m, v, grad, best_alpha, slope_l, pre_l, pre_u, nullptr, 0, n, 0, 0};
+  return launch_optimiser_step(&g, 1, improve, sc, do_update, B, stream);
 }
 
 __global__ void scale_copy_kernel(const float* __restrict__ src, float scale, float* __restrict__ dst, long long n) {
@@ -677,39 +709,10 @@ namespace bf {
 // gradient of the loss w.r.t. beta_j is grad_scale * (-s_j) * sum_s g[s,j]  (add_j = -beta_j * s_j enters the lower
 // coefficients, d lower / d add_j = g_j); entries without a split never move.  Same Adam recurrences as alpha,
 // projection to beta >= 0.
-__global__ void __launch_bounds__(128) beta_step_kernel(float* __restrict__ beta, float* __restrict__ m, float* __restrict__ v,
-                                                        float* __restrict__ gsum, const int8_t* __restrict__ split,
-                                                        int split_stride, const int* __restrict__ improve,
-                                                        float* __restrict__ best_beta, float* __restrict__ add, AdamScalars sc,
-                                                        int do_update, int n) {
-  const int b = blockIdx.x;
-  const int j = blockIdx.y * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const size_t i = (size_t)b * n + j;
-  const float s = split ? (float)split[(size_t)b * split_stride + j] : 0.f;
-  float bt = beta[i];
-  if (improve != nullptr && best_beta != nullptr && improve[b] != 0) best_beta[i] = bt;
-  if (do_update) {
-    const float g = gsum[i] * sc.grad_scale * (-s);
-    gsum[i] = 0.f;
-    float mi = m[i], vi = v[i];
-    mi = mi + sc.one_minus_beta1 * (g - mi);
-    vi = vi * sc.beta2 + sc.one_minus_beta2 * g * g;
-    const float denom = sqrtf(vi) / sc.bc2_sqrt + sc.eps;
-    bt = fmaxf(bt - sc.lr_step * (mi / denom), 0.f);
-    m[i] = mi;
-    v[i] = vi;
-    beta[i] = bt;
-  }
-  add[i] = -bt * s;
-}
-
 int launch_beta_step(float* beta, float* m, float* v, float* gsum, const int8_t* split, int split_stride, const int* improve,
                      float* best_beta, float* add, AdamScalars sc, int do_update, int B, int n, cudaStream_t stream) {
-  dim3 grid(B, ceil_div(n, 128));
-  beta_step_kernel<<<grid, 128, 0, stream>>>(beta, m, v, gsum, split, split_stride, improve, best_beta, add, sc, do_update, n);
-  BF_CHECK_LAUNCH("beta_step_kernel");
-  return BF_OK;
+  const StepSegment g{beta, m, v, gsum, best_beta, add, nullptr, nullptr, split, split_stride, n, 1, 0};
+  return launch_optimiser_step(&g, 1, improve, sc, do_update, B, stream);
 }
 
 __global__ void fill_kernel(float* __restrict__ dst, float value, int n) {

@@ -81,6 +81,18 @@ struct AdamScalars {
   float one_minus_beta1, one_minus_beta2;
   float grad_scale;   // -1/S (mean) or -1 (sum): d loss / d lower
 };
+// One parameter tensor of an optimiser step: an alpha (out: the next lower slope) or a beta (out: the next split term)
+struct StepSegment {
+  float *x, *m, *v, *grad, *best, *out;
+  const float *pre_l, *pre_u;                 // alpha only
+  const int8_t* split;                        // beta only
+  int split_stride, n, beta, vec;             // vec: set by the launcher
+};
+constexpr int STEP_SEGMENTS = 16;             // per launch
+struct StepArgs {
+  StepSegment seg[STEP_SEGMENTS];
+};
+int launch_optimiser_step(const StepSegment* seg, int count, const int* improve, AdamScalars sc, int do_update, int B, cudaStream_t stream);
 // Snapshot of the best alpha (where improve[b]), Adam update + projection to [0,1], and the
 // lower slope for the next evaluation.  grad is scaled by grad_scale before use and zeroed.
 int launch_adam_step(float* alpha, float* m, float* v, float* grad, const int* improve, float* best_alpha,
