@@ -356,8 +356,10 @@ __device__ __forceinline__ void gemm_small_mainloop(const GemmArgs& g, const int
     if (kt + 1 < nk) load_slab((kt + 1) * SMALL_K);
     const float* as = As + (kt & 1) * SMALL_K * 32;
     const float* bs = Bs + (kt & 1) * SMALL_K * 64;
-#pragma unroll 16
-    for (int kk = 0; kk < SMALL_K; ++kk) {
+    const int left = g.K - kt * SMALL_K;              // the last slab ends with its last 16 columns
+    for (int q = 0; q < SMALL_K && q < left; q += 16)
+#pragma unroll
+    for (int kk = q; kk < q + 16; ++kk) {
       const float2 a = *reinterpret_cast<const float2*>(&as[kk * 32 + ((ty * 2) ^ (((kk >> 2) & 7) << 2))]);
       const float4 b = *reinterpret_cast<const float4*>(&bs[kk * 64 + (B_NT ? ((tx * 4) ^ (((kk >> 2) & 15) << 2)) : tx * 4)]);
       acc[0][0] = fmaf(a.x, b.x, acc[0][0]); acc[0][1] = fmaf(a.x, b.y, acc[0][1]);
