@@ -237,14 +237,27 @@ int launch_scale_rows(float* A, const float* w, long long M, int n, cudaStream_t
 }
 
 // ---- Adam + projection + best-alpha snapshot + next lower slope ---------------
-// One element: torch.optim.Adam (no amsgrad / weight decay): lerp for the first moment,
-// mul+addcmul for the second, sqrt(v)/sqrt(bc2)+eps as denominator, then clamp to [0,1].
-__device__ __forceinline__ void adam_one(float& a, float& mi, float& vi, float g, float lo, float up, float& sl,
-                                         const AdamScalars& sc) {
-  mi = mi + sc.one_minus_beta1 * (g - mi);
-  vi = vi * sc.beta2 + sc.one_minus_beta2 * g * g;
-  const float denom = sqrtf(vi) / sc.bc2_sqrt + sc.eps;
-  a = a - sc.lr_step * (mi / denom);
+// torch.optim.Adam (no amsgrad / weight decay): lerp for the first moment, mul+addcmul for the second,
+// sqrt(v)/sqrt(bc2)+eps as denominator.  The step divides by the root of the element's own second moment, so a last bit here
+// becomes a step of the loop: every rounding is written out and none is left to the compiler's choice of multiply-adds.
+// `d` is the scaled gradient minus the first moment, `g` the scaled gradient; KEEP_V: the decayed second moment is
+// the addend that keeps its product unrounded (otherwise the new square is).  Returns the step.
+template <bool KEEP_V>
+__device__ __forceinline__ float adam_moments(float& mi, float& vi, float g, float d, const AdamScalars& sc) {
+  const float og = __fmul_rn(sc.one_minus_beta2, g);
+  mi = fmaf(sc.one_minus_beta1, d, mi);
+  vi = KEEP_V ? fmaf(vi, sc.beta2, __fmul_rn(og, g)) : fmaf(og, g, __fmul_rn(vi, sc.beta2));
+  const float denom = __fadd_rn(__fdiv_rn(__fsqrt_rn(vi), sc.bc2_sqrt), sc.eps);
+  return __fdiv_rn(mi, denom);
+}
+// One alpha: the step, the projection to [0,1] and the next lower slope.  FUSED: the scaled gradient enters the first moment's
+// difference unrounded.  Columns 4 q + 1 .. 4 q + 3 of rows with 16-byte accesses are of this kind, all others are not: the
+// forms that the recorded trajectories of these loops were computed with.
+template <bool FUSED, bool KEEP_V>
+__device__ __forceinline__ void adam_one(float& a, float& mi, float& vi, float grad, float lo, float up, float& sl, const AdamScalars& sc) {
+  const float g = __fmul_rn(grad, sc.grad_scale);
+  const float d = FUSED ? fmaf(grad, sc.grad_scale, -mi) : __fsub_rn(g, mi);
+  a = fmaf(-sc.lr_step, adam_moments<KEEP_V>(mi, vi, g, d, sc), a);
   a = fminf(fmaxf(a, 0.f), 1.f);
   sl = (up <= 0.f) ? 0.f : ((lo >= 0.f) ? 1.f : a);
 }
@@ -264,13 +277,11 @@ __global__ void __launch_bounds__(128) optimiser_step_kernel(StepArgs p, const i
     float bt = g.x[i];
     if (imp) g.best[i] = bt;
     if (do_update) {
-      const float d = g.grad[i] * sc.grad_scale * (-s);
+      const float d = __fmul_rn(__fmul_rn(g.grad[i], sc.grad_scale), -s);
       g.grad[i] = 0.f;
       float mi = g.m[i], vi = g.v[i];
-      mi = mi + sc.one_minus_beta1 * (d - mi);
-      vi = vi * sc.beta2 + sc.one_minus_beta2 * d * d;
-      const float denom = sqrtf(vi) / sc.bc2_sqrt + sc.eps;
-      bt = fmaxf(bt - sc.lr_step * (mi / denom), 0.f);
+      const float step = adam_moments<true>(mi, vi, d, __fsub_rn(d, mi), sc);
+      bt = fmaxf(fmaf(-sc.lr_step, step, bt), 0.f);
       g.m[i] = mi;
       g.v[i] = vi;
       g.x[i] = bt;
@@ -287,10 +298,10 @@ __global__ void __launch_bounds__(128) optimiser_step_kernel(StepArgs p, const i
     float4 mi = *reinterpret_cast<const float4*>(g.m + i), vi = *reinterpret_cast<const float4*>(g.v + i);
     const float4 lo = *reinterpret_cast<const float4*>(g.pre_l + i), up = *reinterpret_cast<const float4*>(g.pre_u + i);
     float4 sl;
-    adam_one(a.x, mi.x, vi.x, d.x * sc.grad_scale, lo.x, up.x, sl.x, sc);
-    adam_one(a.y, mi.y, vi.y, d.y * sc.grad_scale, lo.y, up.y, sl.y, sc);
-    adam_one(a.z, mi.z, vi.z, d.z * sc.grad_scale, lo.z, up.z, sl.z, sc);
-    adam_one(a.w, mi.w, vi.w, d.w * sc.grad_scale, lo.w, up.w, sl.w, sc);
+    adam_one<false, false>(a.x, mi.x, vi.x, d.x, lo.x, up.x, sl.x, sc);
+    adam_one<true, false>(a.y, mi.y, vi.y, d.y, lo.y, up.y, sl.y, sc);
+    adam_one<true, false>(a.z, mi.z, vi.z, d.z, lo.z, up.z, sl.z, sc);
+    adam_one<true, false>(a.w, mi.w, vi.w, d.w, lo.w, up.w, sl.w, sc);
     if (imp) *reinterpret_cast<float4*>(g.best + i) = was;
     *reinterpret_cast<float4*>(g.grad + i) = make_float4(0.f, 0.f, 0.f, 0.f);
     *reinterpret_cast<float4*>(g.m + i) = mi;
@@ -302,7 +313,7 @@ __global__ void __launch_bounds__(128) optimiser_step_kernel(StepArgs p, const i
     if (imp) g.best[i] = a;
     if (!do_update) return;
     float mi = g.m[i], vi = g.v[i], sl;
-    adam_one(a, mi, vi, g.grad[i] * sc.grad_scale, g.pre_l[i], g.pre_u[i], sl, sc);
+    adam_one<false, true>(a, mi, vi, g.grad[i], g.pre_l[i], g.pre_u[i], sl, sc);
     g.grad[i] = 0.f;
     g.m[i] = mi;
     g.v[i] = vi;
