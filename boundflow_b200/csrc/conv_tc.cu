@@ -6,18 +6,20 @@
 // so a row's coefficient plane, padded with zeros behind each line and behind the plane, becomes one line of positions per
 // coefficient row, and every tap (jy, jx) is the same line read jy * Wp + jx positions earlier.  A GEMM tile is 128
 // consecutive positions x all (phase, input channel) pairs of a block:
-//   * A: the tile's positions and the halo in front of them are scaled, split into hi + lo TF32 and staged ONCE per 16
-//     channels in the unswizzled K-major layout, [4-channel chunk][position][16 bytes]; positions are 16 bytes apart, so
-//     a tap is a descriptor whose start address lies that many positions earlier.  No im2col copy exists.
+//   * A: the tile's positions and the halo in front of them are scaled, split and staged ONCE per 16 channels in the
+//     unswizzled K-major layout, [part][8-channel chunk][position][16 bytes]; positions are 16 bytes apart, so a tap is a
+//     descriptor whose start address lies that many positions earlier.  No im2col copy exists.
 //   * B: the weights of all taps are split and stay in shared memory; the CTAs are persistent.
-// TF32 accumulators truncate: the error of a sum grows with its number of MMA steps, in one direction.  So every tile has
-// several hi*hi accumulators of at most CHUNK_STEPS steps each (half of the steps where there are few: an FP32 sum is more
-// exact there too) and separate ones for the products with a lo part; the epilogue adds them in FP32 and gives back what
-// the truncations took on average (see Plan::give_back).
-// 512 rows of 32 -> 32 channels, 16 x 16 -> 32 x 32, 4x4 / 2: 70 us (ReLU pass + FP32 kernel 172), 64 -> 32 channels 16 x 16, 3x3: 95 us
-// (153); 64 inputs of a CIFAR CNN, 32,768 rows each: 24 ms for layers that took 55.  Error against float64 (2-norm): 1.4e-7
-// and 2.8e-7, the FP32 kernels' 2.0e-7 and 4.2e-7.  Bound by its producers (gathered slopes, splits and stores of about
-// 1 element per clock and SM) and, with one tile's accumulators in tensor memory, by the epilogue that follows its MMAs.
+// An FP32 value is split into three bfloat16 parts of eight bits each, without a remainder: x = x0 + x1 + x2.  Of the nine
+// products all but x1 y2, x2 y1 and x2 y2 are formed (narrow blocks: all nine); those three are below 2^-24 of x y together.
+// Tensor-memory accumulators truncate: the error of a sum grows with its number of MMA steps (16 products each), in one
+// direction, by half a unit in the last place of the running sum per step that adds anything.  So every tile has several
+// accumulators for the leading products x0 y0, of at most CHUNK_STEPS steps where tensor memory has the room, and separate
+// ones for the other products; the epilogue adds them in FP32.  A sum of few non-zero products truncates next to nothing: a
+// row with one non-zero coefficient 1 gives the weights back exactly.
+// Error against float64 (2-norm, random rows): 7e-8 and 1.3e-7 for the two layers below, the FP32 kernels' 2.0e-7 and 4.2e-7.
+// 512 rows without a ReLU, 32 -> 32 channels, 16 x 16 -> 32 x 32, 4x4 / 2: 59 us (FP32 kernel 161); 64 -> 32 channels 16 x 16,
+// 3x3: 71 us (143).  (Two TF32 parts a value, which leave a remainder, and twice as many steps: 63 and 91 us, 2.0e-7 and 4.9e-7.)
 // Warps 0-10 stage A, 11-18 read the accumulators back, 19 issues the MMAs.  Every wait is bounded; on expiry the CTA
 // writes NaN to all rows it owns, so that no bound can be taken from them.
 #include "conv_tc.cuh"
@@ -34,7 +36,8 @@ constexpr int TILE = 128;          // positions of a tile = MMA rows
 constexpr int KC = 16;             // channels of a stage
 constexpr int MAX_STAGES = 4;
 constexpr int SMEM_LIMIT = 221 * 1024;  // dynamic; 5.6 KB of tables are static
-constexpr int CHUNK_STEPS = 12;    // MMA steps (of eight products each) summed in one accumulator, where tensor memory has the room
+constexpr int CHUNK_STEPS = 6;     // MMA steps (of 16 products each) summed in one accumulator, where tensor memory has the room
+constexpr int PARTS = 3;           // bfloat16 parts of an FP32 value
 constexpr int MAX_COLS = 512;
 constexpr int MAX_NB = 128;
 constexpr int MAX_CO = 512;
@@ -58,14 +61,10 @@ struct Div {  // n / d for n < 2^31 by one multiplication (round-up reciprocal: 
 
 struct Plan {  // everything the kernel derives from the geometry, computed on the host
   int JY, JX, Wp, P, halo, npos, pstr, groups;
-  int cib, nblk, NB, merged, nchunk, bufs, ksteps, cpad, stages, slots, tiles, pairs;
+  int cib, nblk, NB, merged, nchunk, bufs, units, cpad, stages, slots, tiles, pairs;
   Div dP, dWp, dS;   // positions per row, per line; rows per domain
   Div dNB, dChunks, dCib, dJX;
   int b_bytes, stage_bytes, smem;
-  // A truncated addition loses half a unit in the last place of the running sum on average, and the running sums of n
-  // steps average two thirds of the last one: measured 0.2-0.35 n 2^-24 of the result (random rows, n additions 4 to 20,
-  // windows to dense planes).
-  float give_back;
 };
 
 struct Args {
@@ -73,16 +72,25 @@ struct Args {
   Plan p;
 };
 
-// stores the 16 bytes of one position and 4-channel chunk (cvt.rna keeps NaN, which the integer rounding would not)
-__device__ __forceinline__ void split_store(float4 v, unsigned char* hi_at, unsigned char* lo_at) {
-  float4 hi, lo;
-  hi.x = tf32_rna(v.x); hi.y = tf32_rna(v.y); hi.z = tf32_rna(v.z); hi.w = tf32_rna(v.w);
-  lo.x = tf32_rna(v.x - hi.x); lo.y = tf32_rna(v.y - hi.y); lo.z = tf32_rna(v.z - hi.z); lo.w = tf32_rna(v.w - hi.w);
-  *reinterpret_cast<float4*>(hi_at) = hi;
-  *reinterpret_cast<float4*>(lo_at) = lo;
+// x = x0 + x1 + x2 for two neighbouring channels (the differences are exact; each part holds the next eight bits)
+__device__ __forceinline__ void split2(float a, float b, uint32_t (&p)[PARTS]) {
+#pragma unroll
+  for (int i = 0; i < PARTS; ++i) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p[i]) : "f"(b), "f"(a));
+    a -= __uint_as_float(p[i] << 16);
+    b -= __uint_as_float(p[i] & 0xffff0000u);
+  }
+}
+// stores the eight channels (16 bytes) of one position in the three images, `part` bytes apart
+__device__ __forceinline__ void split_store(const float (&v)[8], unsigned char* at, size_t part) {
+  uint32_t p[4][PARTS];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) split2(v[2 * q], v[2 * q + 1], p[q]);
+#pragma unroll
+  for (int i = 0; i < PARTS; ++i) *reinterpret_cast<uint4*>(at + i * part) = make_uint4(p[0][i], p[1][i], p[2][i], p[3][i]);
 }
 
-// K-major without swizzle: 8-row x 16-byte core matrices, rows 16 bytes apart, row groups 128 bytes apart (SBO), 4-channel
+// K-major without swizzle: 8-row x 16-byte core matrices, rows 16 bytes apart, row groups 128 bytes apart (SBO), 8-channel
 // chunks `lbo` bytes apart
 __device__ __forceinline__ uint64_t plain_desc(uint32_t saddr, uint32_t lbo) {
   return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | (8ull << 32) | (1ull << 46);
@@ -139,48 +147,45 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
-// The MMAs of one tap and 16 channels (two steps of eight) as one sequence.  a, b: low words of the first descriptors (all
-// share the high word), advanced by plain adds: a_lo from the hi to the lo image, a_k / b_k eight channels on.
+// The MMAs of one tap and 16 channels as one sequence.  a, b: low words of the first descriptors (all share the high word),
+// advanced by plain adds: a_part / b_part from one part's image to the next.
 // MMAs on one accumulator are ordered among themselves only while they have one shape and one address.
-// merged (hi and lo columns side by side): [D | D_lo] += [a_hi; a_lo] * [b_hi | b_lo], four MMAs
-__device__ __forceinline__ void mma_tap_merged(uint32_t d, uint32_t a, uint32_t b, uint32_t high, uint32_t a_lo, uint32_t a_k, uint32_t b_k,
-                                               uint32_t idesc, uint32_t accumulate) {
+// merged (the three parts' columns side by side): [D | D1 | D2] += a0 * [b0 | b1 | b2], [L0 | L1 | L2] += (a1, a2) * [b0 | b1 | b2]
+__device__ __forceinline__ void mma_tap_merged(uint32_t d, uint32_t d_lo, uint32_t a, uint32_t b, uint32_t high, uint32_t a_part, uint32_t idesc,
+                                               uint32_t accumulate, uint32_t accumulate_lo) {
   asm volatile(
-      "{\n\t.reg .pred pacc, pone;\n\t.reg .b32 u, v, w, x;\n\t.reg .b64 da, db;\n\t"
-      "setp.ne.b32 pacc, %8, 0;\n\tsetp.eq.b32 pone, %9, %9;\n\t"
-      "add.u32 u, %1, %4;\n\tadd.u32 v, %1, %5;\n\tadd.u32 w, u, %5;\n\tadd.u32 x, %2, %6;\n\t"
-      "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %7, {%9, %9, %9, %9}, pacc;\n\t"
-      "mov.b64 da, {u, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %7, {%9, %9, %9, %9}, pone;\n\t"
-      "mov.b64 da, {v, %3};\n\tmov.b64 db, {x, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %7, {%9, %9, %9, %9}, pone;\n\t"
-      "mov.b64 da, {w, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %7, {%9, %9, %9, %9}, pone;\n\t}"
-      ::"r"(d), "r"(a), "r"(b), "r"(high), "r"(a_lo), "r"(a_k), "r"(b_k), "r"(idesc), "r"(accumulate), "r"(0u)
+      "{\n\t.reg .pred pacc, plo, pone;\n\t.reg .b32 u, v;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 pacc, %7, 0;\n\tsetp.ne.b32 plo, %8, 0;\n\tsetp.eq.b32 pone, %9, %9;\n\t"
+      "add.u32 u, %2, %5;\n\tadd.u32 v, u, %5;\n\t"
+      "mov.b64 da, {%2, %4};\n\tmov.b64 db, {%3, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %6, {%9, %9, %9, %9}, pacc;\n\t"
+      "mov.b64 da, {u, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %6, {%9, %9, %9, %9}, plo;\n\t"
+      "mov.b64 da, {v, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %6, {%9, %9, %9, %9}, pone;\n\t}"
+      ::"r"(d), "r"(d_lo), "r"(a), "r"(b), "r"(high), "r"(a_part), "r"(idesc), "r"(accumulate), "r"(accumulate_lo), "r"(0u)
       : "memory");
 }
-// D += a_hi * b_hi, D_lo += a_hi * b_lo + a_lo * b_hi, six MMAs
-__device__ __forceinline__ void mma_tap(uint32_t d, uint32_t d_lo, uint32_t a, uint32_t b, uint32_t high, uint32_t a_lo, uint32_t b_lo,
-                                        uint32_t a_k, uint32_t b_k, uint32_t idesc, uint32_t accumulate, uint32_t accumulate_lo) {
+// D += a0 b0, D_lo += a0 b1 + a0 b2 + a1 b0 + a1 b1 + a2 b0, six MMAs
+__device__ __forceinline__ void mma_tap(uint32_t d, uint32_t d_lo, uint32_t a, uint32_t b, uint32_t high, uint32_t a_part, uint32_t b_part,
+                                        uint32_t idesc, uint32_t accumulate, uint32_t accumulate_lo) {
   asm volatile(
-      "{\n\t.reg .pred pacc, plo, pone;\n\t.reg .b32 u, v, w, x, y, z;\n\t.reg .b64 da, db;\n\t"
-      "setp.ne.b32 pacc, %10, 0;\n\tsetp.ne.b32 plo, %11, 0;\n\tsetp.eq.b32 pone, %12, %12;\n\t"
-      "add.u32 u, %2, %5;\n\tadd.u32 v, %2, %7;\n\tadd.u32 w, u, %7;\n\tadd.u32 x, %3, %6;\n\tadd.u32 y, %3, %8;\n\tadd.u32 z, x, %8;\n\t"
+      "{\n\t.reg .pred pacc, plo, pone;\n\t.reg .b32 u, v, x, y;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 pacc, %8, 0;\n\tsetp.ne.b32 plo, %9, 0;\n\tsetp.eq.b32 pone, %10, %10;\n\t"
+      "add.u32 u, %2, %5;\n\tadd.u32 v, u, %5;\n\tadd.u32 x, %3, %6;\n\tadd.u32 y, x, %6;\n\t"
       "mov.b64 da, {%2, %4};\n\tmov.b64 db, {%3, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %9, {%12, %12, %12, %12}, pacc;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %7, {%10, %10, %10, %10}, pacc;\n\t"
       "mov.b64 db, {x, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%1], da, db, %9, {%12, %12, %12, %12}, plo;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %7, {%10, %10, %10, %10}, plo;\n\t"
+      "mov.b64 db, {y, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %7, {%10, %10, %10, %10}, pone;\n\t"
       "mov.b64 da, {u, %4};\n\tmov.b64 db, {%3, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%1], da, db, %9, {%12, %12, %12, %12}, pone;\n\t"
-      "mov.b64 da, {v, %4};\n\tmov.b64 db, {y, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %9, {%12, %12, %12, %12}, pone;\n\t"
-      "mov.b64 db, {z, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%1], da, db, %9, {%12, %12, %12, %12}, pone;\n\t"
-      "mov.b64 da, {w, %4};\n\tmov.b64 db, {y, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%1], da, db, %9, {%12, %12, %12, %12}, pone;\n\t}"
-      ::"r"(d), "r"(d_lo), "r"(a), "r"(b), "r"(high), "r"(a_lo), "r"(b_lo), "r"(a_k), "r"(b_k), "r"(idesc), "r"(accumulate),
-        "r"(accumulate_lo), "r"(0u)
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %7, {%10, %10, %10, %10}, pone;\n\t"
+      "mov.b64 db, {x, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %7, {%10, %10, %10, %10}, pone;\n\t"
+      "mov.b64 da, {v, %4};\n\tmov.b64 db, {%3, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %7, {%10, %10, %10, %10}, pone;\n\t}"
+      ::"r"(d), "r"(d_lo), "r"(a), "r"(b), "r"(high), "r"(a_part), "r"(b_part), "r"(idesc), "r"(accumulate), "r"(accumulate_lo), "r"(0u)
       : "memory");
 }
 
@@ -218,7 +223,7 @@ __device__ __forceinline__ void sum_accumulators(uint32_t at, const int* col, bo
 // Column groups g, g + 1, ... end - 1 (W columns each) of a warp's 32 positions: sums the accumulators and stores; the
 // accumulators are handed back before the last group's stores.
 __device__ __forceinline__ void read_and_store(uint32_t base, int g, int end, int naccs, const int* acc_col, const int2* col_tab, float* out,
-                                               uint32_t ok, bool pairs, float give_back, uint32_t empty_bar) {
+                                               uint32_t ok, bool pairs, uint32_t empty_bar) {
   constexpr int N = 4;  // accumulators in flight
   for (; g < end; ++g) {
     float t[W];
@@ -232,8 +237,6 @@ __device__ __forceinline__ void read_and_store(uint32_t base, int g, int end, in
       __syncwarp();
       if ((threadIdx.x & 31) == 0) mbar_arrive(empty_bar);
     }
-#pragma unroll
-    for (int i = 0; i < W; ++i) t[i] = fmaf(t[i], give_back, t[i]);
     const int4* tab = reinterpret_cast<const int4*>(col_tab + g * W);
     if (pairs) {
 #pragma unroll
@@ -317,36 +320,29 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __grid_consta
     col_tab[n] = (py < c.sh && ci0 + i < c.Ci) ? make_int2((ci0 + i) * c.Hi * c.Wi + py * c.Wi + px, py * c.sw + px) : make_int2(0, 31);
   }
   if (tid < MAX_COLS / 8) {
-    if (p.merged) acc_col[tid] = (tid < p.nchunk) ? tid * 2 * p.NB + p.NB : (tid - p.nchunk) * 2 * p.NB;
-    else acc_col[tid] = (tid == 0) ? p.nchunk * p.NB : (tid - 1) * p.NB;
+    // merged: parts 2, 1 and 0 of the small products' accumulator, parts 2 and 1 of the others, then their leading products
+    if (!p.merged) acc_col[tid] = (tid == 0) ? p.nchunk * p.NB : (tid - 1) * p.NB;
+    else if (tid < PARTS) acc_col[tid] = (p.nchunk * PARTS + PARTS - 1 - tid) * p.NB;
+    else if (tid < PARTS + 2 * p.nchunk) acc_col[tid] = ((tid - PARTS) / 2 * PARTS + 2 - (tid - PARTS) % 2) * p.NB;
+    else acc_col[tid] = (tid - PARTS - 2 * p.nchunk) * PARTS * p.NB;
   }
   for (int co = tid; co < MAX_CO; co += THREADS) bias_s[co] = (c.bias && co < c.Co) ? c.bias[co] : 0.f;
-  // B: [tap][hi, lo][4-channel chunk][column][4]   (merged: hi and lo columns of a chunk side by side)
+  // B: [tap][part][8-channel chunk][column][8]   (merged: [tap][chunk][part][column][8])
   {
-    const int chunks = p.cpad / 4, total = taps * chunks * p.NB;
+    const int chunks = p.cpad / 8, total = taps * chunks * p.NB;
     const size_t step = (size_t)c.Ci * c.kh * c.kw;
-#pragma unroll 2
     for (int e = tid; e < total; e += THREADS) {
       const int tk = p.dNB(e), n = e - tk * p.NB, t = p.dChunks(tk), kc = tk - t * chunks, jy = p.dJX(t);
       int py, i, px;
       column(n, py, i, px);
       const int r = py + c.sh * jy, s = px + c.sw * (t - jy * p.JX);
       const bool in = py < c.sh && ci0 + i < c.Ci && r < c.kh && s < c.kw;
-      const float* w = c.W + (in ? ((size_t)(kc * 4) * c.Ci + ci0 + i) * c.kh * c.kw + r * c.kw + s : 0);
-      float4 v;
-      v.x = ldg_if(w, in && kc * 4 + 0 < c.Co);
-      v.y = ldg_if(w + step, in && kc * 4 + 1 < c.Co);
-      v.z = ldg_if(w + 2 * step, in && kc * 4 + 2 < c.Co);
-      v.w = ldg_if(w + 3 * step, in && kc * 4 + 3 < c.Co);
-      unsigned char *hi, *lo;
-      if (p.merged) {
-        hi = b_sm + ((size_t)tk * 2 * p.NB + n) * 16;
-        lo = hi + p.NB * 16;
-      } else {
-        hi = b_sm + ((size_t)(t * 2 * chunks + kc) * p.NB + n) * 16;
-        lo = hi + (size_t)chunks * p.NB * 16;
-      }
-      split_store(v, hi, lo);
+      const float* w = c.W + (in ? ((size_t)(kc * 8) * c.Ci + ci0 + i) * c.kh * c.kw + r * c.kw + s : 0);
+      float v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = ldg_if(w + q * step, in && kc * 8 + q < c.Co);
+      const size_t part = (size_t)(p.merged ? 1 : chunks) * p.NB * 16;
+      split_store(v, b_sm + ((size_t)(p.merged ? tk * PARTS : t * PARTS * chunks + kc) * p.NB + n) * 16, part);
     }
   }
   fence_proxy_async();
@@ -449,10 +445,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __grid_consta
         const bool opens = p.groups == 2 || (item & 1) == 0, closes = p.groups == 2 || (item & 1) == 1;
         if (opens && !wait_warp(smem_u32(&ctl.a_empty[s]), phase, abort_flag)) { alive = false; break; }
         if (worker) {
-          unsigned char* at = smem + s * p.stage_bytes + (size_t)((ch >> 2) & 3) * p.npos * 16 + pos * 16;
-          split_store(make_float4(lam[0], lam[1], lam[2], lam[3]), at, at + (size_t)4 * p.npos * 16);
-          at += (size_t)p.npos * 16;
-          split_store(make_float4(lam[4], lam[5], lam[6], lam[7]), at, at + (size_t)4 * p.npos * 16);
+          split_store(lam, smem + s * p.stage_bytes + ((ch >> 3) & 1) * p.npos * 16 + pos * 16, (size_t)2 * p.npos * 16);
         }
         if (closes) {
           fence_proxy_async();
@@ -472,7 +465,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __grid_consta
   } else if (warp < MMA_WARP) {
     // ------------------------------------------------------------------ epilogue: thread = position, half of the column groups
     const int q = warp & 3, half = (warp - PROD_WARPS) >> 2;   // a warp may read the tensor-memory lanes of its index mod 4
-    const int naccs = p.merged ? 2 * p.nchunk : p.nchunk + 1;
+    const int naccs = (p.merged ? PARTS : 1) * (p.nchunk + 1);
     const int groups = p.NB / W, from = half ? (groups + 1) / 2 : 0, to = half ? groups : (groups + 1) / 2;
     const uint32_t row = tmem + ((uint32_t)(q * 32) << 16);
     const bool want_delta = c.partial != nullptr && blk == 0;
@@ -509,23 +502,24 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __grid_consta
       const uint32_t base = row + (uint32_t)(buf * (MAX_COLS / 2));
       const uint32_t empty_bar = smem_u32(&ctl.acc_empty[buf]);
       float* out = c.out + off;
-      read_and_store(base, from, to, naccs, acc_col, col_tab, out, ok, p.pairs, p.give_back, empty_bar);
+      read_and_store(base, from, to, naccs, acc_col, col_tab, out, ok, p.pairs, empty_bar);
       if (from >= to && lane == 0) mbar_arrive(empty_bar);
     }
   } else {
     // ------------------------------------------------------------------ MMA issue
     if (elect_one()) {
-      const uint32_t n_mma = p.merged ? 2 * p.NB : p.NB;
-      const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((n_mma >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
+      const uint32_t n_mma = p.merged ? PARTS * p.NB : p.NB;
+      // FP32 accumulators, bfloat16 operands
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((n_mma >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
       const uint32_t a_lbo = (uint32_t)p.npos * 16, b_lbo = n_mma * 16;
-      const int chunks = p.cpad / 4;
-      // descriptor distances: hi to lo image, eight channels, one tap's weights
-      const uint32_t a_lo = (4 * a_lbo) >> 4, a_k = (2 * a_lbo) >> 4, b_k = (2 * b_lbo) >> 4;
-      const uint32_t b_lo = (uint32_t)(chunks * p.NB), b_tap = (uint32_t)(chunks * 2 * p.NB);
+      const int chunks = p.cpad / 8;
+      // descriptor distances: from part to part, 16 channels, one tap's weights
+      const uint32_t a_part = (2 * a_lbo) >> 4, b_k = (2 * b_lbo) >> 4;
+      const uint32_t b_part = (uint32_t)(chunks * p.NB), b_tap = (uint32_t)(chunks * PARTS * p.NB);
       const uint64_t a_desc = plain_desc(smem_u32(smem) + (uint32_t)p.halo * 16, a_lbo), b_desc = plain_desc(smem_u32(b_sm), b_lbo);
       const uint32_t a_first = (uint32_t)a_desc, b_first = (uint32_t)b_desc, high = (uint32_t)(a_desc >> 32);
       const uint32_t a_stage = (uint32_t)(p.stage_bytes >> 4);
-      const int per_chunk = (p.ksteps / 2 + p.nchunk - 1) / p.nchunk;   // taps x 16 channels per accumulator
+      const int per_chunk = (p.units + p.nchunk - 1) / p.nchunk;   // taps x 16 channels per accumulator
       int s = 0, tcount = 0;
       uint32_t phase = 0;
       for (int tile = tile0; tile < p.tiles && alive; tile += tile_step, ++tcount) {
@@ -533,13 +527,13 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __grid_consta
         if (!wait_asleep(smem_u32(&ctl.acc_empty[buf]), ((uint32_t)(tcount / p.bufs) & 1u) ^ 1u, abort_flag)) { alive = false; break; }
         tc_fence_after();
         uint32_t d = tmem + (uint32_t)(buf * (MAX_COLS / 2)) - n_mma;
-        const uint32_t d_lo = tmem + (uint32_t)(buf * (MAX_COLS / 2) + p.nchunk * p.NB);
+        const uint32_t d_lo = tmem + (uint32_t)(buf * (MAX_COLS / 2)) + p.nchunk * n_mma;
         int left = 0;
         uint32_t started = 0;
         for (int kc = 0; kc < kchunks; ++kc) {
           if (!wait_asleep(smem_u32(&ctl.a_full[s]), phase, abort_flag)) { alive = false; break; }
           tc_fence_after();
-          uint32_t ad = a_first + (uint32_t)s * a_stage, bd = b_first + (uint32_t)(2 * kc) * b_k;
+          uint32_t ad = a_first + (uint32_t)s * a_stage, bd = b_first + (uint32_t)kc * b_k;
           int jx = 0;
           for (int t = 0; t < taps; ++t, bd += b_tap) {
             uint32_t acc = 1;
@@ -549,8 +543,8 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __grid_consta
               acc = 0;
             }
             --left;
-            if (p.merged) mma_tap_merged(d, ad, bd, high, a_lo, a_k, b_k, idesc, acc);
-            else mma_tap(d, d_lo, ad, bd, high, a_lo, b_lo, a_k, b_k, idesc, acc, started);
+            if (p.merged) mma_tap_merged(d, d_lo, ad, bd, high, a_part, idesc, acc, started);
+            else mma_tap(d, d_lo, ad, bd, high, a_part, b_part, idesc, acc, started);
             started = 1;
             --ad;                                   // the next tap reads one position earlier, or one line
             if (++jx == p.JX) {
@@ -615,35 +609,32 @@ static bool make_plan(const ConvTcProblem& c, Plan& p) {
   p.slots = (int)((P - 1) / TILE + 2);
   if (p.slots > 32) return false;
   p.cpad = ceil_div(c.Co, KC) * KC;
-  p.ksteps = p.JY * p.JX * p.cpad / 8;
-  p.stage_bytes = ((4 * 2 * p.npos * 16) + 127) / 128 * 128;
+  p.units = p.JY * p.JX * p.cpad / 16;  // MMA steps of a sum
+  p.stage_bytes = ((PARTS * 2 * p.npos * 16) + 127) / 128 * 128;
   const int phases = c.sh * c.sw;
   // input channels per block: as many as the accumulator columns and shared memory hold (each block stages A again)
   for (p.nblk = 1; p.nblk <= 8; ++p.nblk) {
     p.cib = ceil_div(c.Ci, p.nblk);
     while ((phases * p.cib) % 16 != 0) ++p.cib;
     const int NB = phases * p.cib;
-    p.merged = NB <= 32;   // narrow MMAs are bound by their issue: two wider ones instead of three
+    p.merged = NB <= 32;   // narrow MMAs are bound by their issue: three wider ones instead of six
     p.NB = NB;
     if (NB > MAX_NB) continue;
-    p.b_bytes = p.JY * p.JX * p.cpad * NB * 8;
+    p.b_bytes = p.JY * p.JX * p.cpad * NB * 2 * PARTS;
     if (p.b_bytes + 2 * p.stage_bytes > SMEM_LIMIT) continue;
     p.stages = (SMEM_LIMIT - p.b_bytes) / p.stage_bytes;
     if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
     p.smem = p.b_bytes + p.stages * p.stage_bytes;
     // accumulators: as many as the steps ask for; two tiles in tensor memory when they fit side by side
-    const int steps = p.ksteps / 2 < CHUNK_STEPS ? p.ksteps / 2 : CHUNK_STEPS;
-    const int want = ceil_div(p.ksteps, steps);
-    const int one = p.merged ? 2 * NB : NB, extra = p.merged ? 0 : NB;
-    const int room = (MAX_COLS - extra) / one, room2 = (MAX_COLS / 2 - extra) / one;
+    const int want = ceil_div(p.units, p.units / 2 < 1 ? 1 : (p.units / 2 < CHUNK_STEPS ? p.units / 2 : CHUNK_STEPS));
+    const int one = p.merged ? PARTS * NB : NB;
+    const int room = MAX_COLS / one - 1, room2 = MAX_COLS / 2 / one - 1;  // next to the small products'
     p.bufs = (want <= room2) ? 2 : 1;
     const int most = want < room ? want : room;
-    const int units = p.ksteps / 2;  // a tap's 16 channels stay in one accumulator
-    p.nchunk = ceil_div(units, ceil_div(units, most));  // of equal length, all used
-    p.give_back = 0.25f * (float)((p.merged ? 4 : 2) * ceil_div(units, p.nchunk)) / 16777216.f;
+    p.nchunk = ceil_div(p.units, ceil_div(p.units, most));  // of equal length, all used
     p.pairs = c.sw == 2 && c.pw % 2 == 0 && c.Wi % 2 == 0 && (reinterpret_cast<uintptr_t>(c.out) & 7u) == 0;
     p.dNB.set(NB);
-    p.dChunks.set(p.cpad / 4);
+    p.dChunks.set(p.cpad / 8);
     p.dCib.set(p.cib);
     p.dJX.set(p.JX);
     return true;

@@ -1,0 +1,95 @@
+"""The tensor-core ReLU + transposed convolution against float64 and against the FP32 kernels it takes the place of."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    assert torch.cuda.is_available(), "GPU tests need a CUDA device"
+    from boundflow_b200.csrc import build
+
+    build.build()
+    return torch.device("cuda", 0)
+
+
+def _pair(v):
+    return (v, v) if isinstance(v, int) else v
+
+
+def _backward(A, w, stride, padding, H, W, *, b=None, slopes=None, side=0, delta=None, accumulate=1):
+    """bf_crown_relu_conv2d_bwd on rows [B,S,Co,Ho,Wo]: (rows of the input, tensor-core launches)."""
+    from boundflow_b200 import _lib
+
+    lib = _lib.load()
+    (sh, sw), (ph, pw) = _pair(stride), _pair(padding)
+    B, S, Co, Ho, Wo = A.shape
+    Ci, kh, kw = w.shape[1:]
+    out = torch.full((B, S, Ci, H, W), float("nan"), device=A.device)
+    nbytes = lib.bf_crown_relu_conv2d_bwd_scratch_bytes(B, S, Co, Ho, Wo)
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=A.device)
+    au, al, bu = slopes if slopes is not None else (None, None, None)
+    before = _lib.tc_launch_count()
+    _lib.check(lib.bf_crown_relu_conv2d_bwd(_lib.ptr(A), side, _lib.ptr(au), _lib.ptr(al), _lib.ptr(bu), None, _lib.ptr(w), _lib.ptr(b), _lib.ptr(out),
+                                            _lib.ptr(delta), accumulate, _lib.ptr(scratch), nbytes, B, S, Ci, H, W, Co, Ho, Wo, kh, kw, sh, sw, ph, pw, None))
+    return out, _lib.tc_launch_count() - before
+
+
+def _transposed(x, w, stride, padding, H, W):
+    (sh, sw), (ph, pw) = _pair(stride), _pair(padding)
+    Ho, Wo = x.shape[3:]
+    opad = (H - ((Ho - 1) * sh - 2 * ph + w.shape[2]), W - ((Wo - 1) * sw - 2 * pw + w.shape[3]))
+    y = torch.nn.functional.conv_transpose2d(x.flatten(0, 1), w, None, (sh, sw), (ph, pw), output_padding=opad)
+    return y.view(x.shape[0], x.shape[1], w.shape[1], H, W)
+
+
+def _rows(dev, kind, B, S, Co, Ho, Wo, Ci, k, g):
+    kh, kw = _pair(k)
+    A = torch.randn(B, S, Co, Ho, Wo, generator=g, device=dev)
+    w = torch.randn(Co, Ci, kh, kw, generator=g, device=dev)
+    if kind == "identity":
+        A = torch.zeros(B * S, Co * Ho * Wo, device=dev)
+        A[torch.arange(B * S), torch.randint(0, A.shape[1], (B * S,), generator=g, device=dev)] = 1.0
+        A = A.view(B, S, Co, Ho, Wo)
+    elif kind == "integers":
+        A = torch.randint(-9, 10, A.shape, generator=g, device=dev).float()
+        w = torch.randint(-9, 10, w.shape, generator=g, device=dev).float()
+    elif kind == "sparse":
+        A = A * (torch.rand(A.shape, generator=g, device=dev) < 0.03)
+    return A, w
+
+
+# accumulators of one and several parts, one and two tiles in tensor memory, several blocks of input channels, channels that end inside a stage
+GEOMETRIES = [(8, 64, 8, 16, 16, 16, 3, 1, 1), (8, 64, 32, 32, 32, 32, 4, 2, 1), (8, 64, 32, 16, 16, 64, 3, 1, 1), (16, 100, 16, 14, 14, 32, 4, 2, 1),
+              (8, 64, 16, 17, 17, 40, 3, 2, 1), (8, 60, 24, 13, 13, 20, 3, 1, 1), (4, 64, 64, 16, 16, 200, 2, 1, 0)]
+
+
+# products and sums that float32 represents: any order of exact operations gives them back
+@pytest.mark.parametrize("B,S,Ci,H,W,Co,k,s,p", GEOMETRIES)
+@pytest.mark.parametrize("kind", ["identity", "integers"])
+def test_exact_rows_stay_exact(dev, B, S, Ci, H, W, Co, k, s, p, kind):
+    Ho, Wo = (H + 2 * p - k) // s + 1, (W + 2 * p - k) // s + 1
+    g = torch.Generator("cuda").manual_seed(B + Ci + Co)
+    A, w = _rows(dev, kind, B, S, Co, Ho, Wo, Ci, k, g)
+    out, launches = _backward(A, w, s, p, H, W)
+    assert launches == 1
+    assert torch.equal(out.double(), _transposed(A.double(), w.double(), s, p, H, W))
+
+
+# no further from float64 than the FP32 kernels, and without the bias of a systematic scaling: a truncated addition loses half a unit in the
+# last place (2^-24) on average, at most six of them in a row
+@pytest.mark.parametrize("B,S,Ci,H,W,Co,k,s,p", GEOMETRIES)
+@pytest.mark.parametrize("kind", ["dense", "sparse"])
+def test_error_against_fp32_kernels(dev, monkeypatch, B, S, Ci, H, W, Co, k, s, p, kind):
+    Ho, Wo = (H + 2 * p - k) // s + 1, (W + 2 * p - k) // s + 1
+    g = torch.Generator("cuda").manual_seed(B + Ci + Co + 1)
+    A, w = _rows(dev, kind, B, S, Co, Ho, Wo, Ci, k, g)
+    ref = _transposed(A.double(), w.double(), s, p, H, W)
+    out, launches = _backward(A, w, s, p, H, W)
+    monkeypatch.setenv("BF_B200_FORCE_FFMA", "1")
+    fp32, none = _backward(A, w, s, p, H, W)
+    assert (launches, none) == (1, 0)
+    err, err32 = (out.double() - ref), (fp32.double() - ref)
+    assert err.norm() <= err32.norm()
+    assert abs((err * ref.sign()).sum() / ref.abs().sum()) <= 3 * 2.0**-24
