@@ -207,9 +207,6 @@ namespace bf {
 int launch_ibp_conv2d(const float* in_a, const float* in_b, int in_mode, int relu_in, const float* W, const float* bias,
                       const int8_t* split, int split_stride, const float* cons_l, const float* cons_u, float* out_l,
                       float* out_u, int* infeasible, int B, const bf_layer_desc& L, cudaStream_t stream);
-int launch_crown_bwd_conv2d(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
-                            const float* W, const float* bias, float* A_prev, float* delta, int accumulate, int M, int S,
-                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add = nullptr, bool windowed = false);
 size_t crown_bwd_conv2d_scratch_bytes(int M, const bf_layer_desc& L);
 int launch_onehot_conv_rows(int first, const float* W, const float* bias, float* A_prev, float* delta, int M, int S,
                             const bf_layer_desc& L, cudaStream_t stream);
@@ -240,7 +237,13 @@ void refresh_switches(const bf_chain* c) {
   c->sw.tc_auto = !(rows && atoi(rows) > 0);
 }
 
-bool tc_may_run(const bf_chain* c, int M) { return c->status != nullptr && !c->pk_bwd.empty() && !c->sw.force_ffma && M >= c->sw.tc_min_rows; }
+bool tc_may_run(const bf_chain* c, int M) {
+  if (c->status == nullptr || c->sw.force_ffma) return false;
+  if (!c->pk_bwd.empty() && M >= c->sw.tc_min_rows) return true;
+  for (const bf_layer_desc& L : c->layers)
+    if (L.op == BF_OP_CONV2D && conv_rows_on_tensor_cores(M, L)) return true;
+  return false;
+}
 
 static bool adjoint_feature_major(const bf_chain* c, int M, int N) {
   if (c->sw.adjoint_kernel == 1) return false;
@@ -587,7 +590,7 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
       Lw.ph = 0; Lw.pw = 0;
       Lw.n_out = L.Co * Lw.Ho * Lw.Wo; Lw.n_in = L.Ci * Lw.Hi * Lw.Wi;
       float* dst = ws.buf[toggle];
-      rc = bf::launch_crown_bwd_conv2d(lam, nullptr, nullptr, nullptr, nullptr, L.W, nullptr, dst, nullptr, 1, M, S, Lw, nullptr, stream, nullptr, true);
+      rc = bf::launch_crown_bwd_conv2d(lam, nullptr, nullptr, nullptr, nullptr, L.W, nullptr, dst, nullptr, 1, M, S, Lw, nullptr, stream, nullptr, false, nullptr);
       win.C = L.Ci; win.WH = Lw.Hi; win.WW = Lw.Wi; win.H = L.Hi; win.W = L.Wi;
       win.ty = win.ty * L.sh - L.ph; win.sy *= L.sh;
       win.tx = win.tx * L.sw - L.pw; win.sx *= L.sw;
@@ -602,7 +605,7 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
     } else {
       float* dst = ws.buf[toggle];
       rc = bf::launch_crown_bwd_conv2d(curA, dpos, dneg, epos, eneg, L.W, L.bias, dst, ws.cacc, have_c, M, S, L,
-                                       ws.conv_scratch, stream, ad);
+                                       ws.conv_scratch, stream, ad, chain->status != nullptr, chain->status);
       curA = dst;
     }
     if (rc != BF_OK) return rc;

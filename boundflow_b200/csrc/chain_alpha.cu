@@ -9,9 +9,6 @@
 
 namespace bf {
 
-int launch_crown_bwd_conv2d(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
-                            const float* W, const float* bias, float* A_prev, float* delta, int accumulate, int M, int S,
-                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add = nullptr, bool windowed = false);
 size_t crown_bwd_conv2d_scratch_bytes(int M, const bf_layer_desc& L);
 int launch_conv_forward_rows(const float* in, const float* W, const float* bias, float* out, int M, const bf_layer_desc& L,
                              cudaStream_t stream);
@@ -98,7 +95,8 @@ static int alpha_bwd_layer(const bf_chain* c, const AlphaWs& ws, int layer, cons
   const bf_layer_desc& L = c->layers[layer];
   if (L.op == BF_OP_LINEAR)
     return dispatch_bwd(c, layer, A, dpos, dneg, epos, eneg, add, dst, ws.cacc, accumulate, mid, rad, partial, side, M, S, ptiles, stream);
-  return launch_crown_bwd_conv2d(A, dpos, dneg, epos, eneg, L.W, L.bias, dst, ws.cacc, accumulate, M, S, L, ws.conv_scratch, stream, add);
+  return launch_crown_bwd_conv2d(A, dpos, dneg, epos, eneg, L.W, L.bias, dst, ws.cacc, accumulate, M, S, L, ws.conv_scratch, stream, add,
+                                 c->status != nullptr, c->status);
 }
 
 static int alpha_sweep(const bf_chain* c, const AlphaWs& ws, const float* C, int side, bool keep_A0, bool use_add,

@@ -803,22 +803,34 @@ static int launch_convT(const ConvTArgs& g0, cudaStream_t stream) {
   return BF_OK;
 }
 
+static ConvTcProblem conv_tc_geometry(int M, int S, const bf_layer_desc& L) {
+  ConvTcProblem c{};
+  c.M = M; c.S = S; c.Co = L.Co; c.Ci = L.Ci; c.WH = L.Ho; c.WW = L.Wo; c.Hi = L.Hi; c.Wi = L.Wi;
+  c.kh = L.kh; c.kw = L.kw; c.sh = L.sh; c.sw = L.sw; c.ph = L.ph; c.pw = L.pw;
+  return c;
+}
+static bool conv_tc_rule(const ConvTcProblem& c, int* slots) {
+  int tiles = 0;
+  return c.Ci >= CONV_TC_MIN_CI && ceil_div(c.kh, c.sh) * ceil_div(c.kw, c.sw) <= CONV_TC_MAX_TAPS && conv_tc_supports(c, slots, &tiles) &&
+         tiles >= CONV_TC_MIN_TILES;
+}
+bool conv_rows_on_tensor_cores(int M, const bf_layer_desc& L) {
+  int slots = 0;
+  return conv_tc_rule(conv_tc_geometry(M, 1, L), &slots);
+}
+
 // The tensor-core kernel takes ReLU scaling, row sums and transposed convolution of full rows in one pass.
 // BF_E_UNSUPPORTED: the caller takes the FP32 kernels.
 static int launch_conv_tc_bwd(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg, const float* add,
                               const float* W, const float* bias, float* A_prev, float* delta, int accumulate, int M, int S,
-                              const bf_layer_desc& L, void* scratch, cudaStream_t stream) {
+                              const bf_layer_desc& L, void* scratch, int* status, cudaStream_t stream) {
   const char* ffma = getenv("BF_B200_FORCE_FFMA");
-  if ((ffma && ffma[0] == '1') || !A_prev || L.Ci < CONV_TC_MIN_CI ||
-      ceil_div(L.kh, L.sh) * ceil_div(L.kw, L.sw) > CONV_TC_MAX_TAPS)
-    return BF_E_UNSUPPORTED;
-  ConvTcProblem c{};
+  if ((ffma && ffma[0] == '1') || !A_prev) return BF_E_UNSUPPORTED;
+  ConvTcProblem c = conv_tc_geometry(M, S, L);
   c.A = A; c.dpos = dpos; c.dneg = dneg; c.epos = epos; c.eneg = eneg; c.add = dpos ? add : nullptr;
-  c.bias = bias; c.W = W; c.out = A_prev;
-  c.M = M; c.S = S; c.Co = L.Co; c.Ci = L.Ci; c.WH = L.Ho; c.WW = L.Wo; c.Hi = L.Hi; c.Wi = L.Wi;
-  c.kh = L.kh; c.kw = L.kw; c.sh = L.sh; c.sw = L.sw; c.ph = L.ph; c.pw = L.pw;
-  int slots = 0, tiles = 0;
-  if (!conv_tc_supports(c, &slots, &tiles) || tiles < CONV_TC_MIN_TILES) return BF_E_UNSUPPORTED;
+  c.bias = bias; c.W = W; c.out = A_prev; c.status = status;
+  int slots = 0;
+  if (!conv_tc_rule(c, &slots)) return BF_E_UNSUPPORTED;
   const bool sums = delta && (dpos || bias || !accumulate);
   if (sums) {  // the row sums take the place that the scaled coefficients have on the FP32 path
     if (!scratch || slots > L.Co * L.Ho * L.Wo) return BF_E_UNSUPPORTED;
@@ -834,8 +846,9 @@ static int launch_conv_tc_bwd(const float* A, const float* dpos, const float* dn
 
 int launch_crown_bwd_conv2d(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
                             const float* W, const float* bias, float* A_prev, float* delta, int accumulate, int M, int S,
-                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add = nullptr, bool windowed = false) {
-  const int tc = windowed ? BF_E_UNSUPPORTED : launch_conv_tc_bwd(A, dpos, dneg, epos, eneg, add, W, bias, A_prev, delta, accumulate, M, S, L, scratch, stream);
+                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add, bool tensor_cores, int* status) {
+  const int tc = tensor_cores ? launch_conv_tc_bwd(A, dpos, dneg, epos, eneg, add, W, bias, A_prev, delta, accumulate, M, S, L, scratch, status, stream)
+                              : BF_E_UNSUPPORTED;
   if (tc != BF_E_UNSUPPORTED) return tc;
   const float* lam = A;
   const bool need_pro = (dpos != nullptr) || (bias != nullptr) || (delta != nullptr && !accumulate);
@@ -1236,7 +1249,7 @@ extern "C" int bf_crown_relu_conv2d_bwd(const float* A, int side, const float* a
   // (a block then streams a whole coefficient row)
   if (!relu && scratch_bytes < bf_crown_relu_conv2d_bwd_scratch_bytes(B, S, Co, Ho, Wo)) scratch = nullptr;
   return bf::launch_crown_bwd_conv2d(A, dpos, dneg, epos, eneg, W, bias, A_prev, delta, accumulate, B * S, S, L, scratch,
-                                     bf::as_stream(stream));
+                                     bf::as_stream(stream), nullptr, true, nullptr);
 }
 
 // ReLU backward alone (graphs where the ReLU's producer is not a single affine layer, e.g. after an add):

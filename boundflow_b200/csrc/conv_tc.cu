@@ -21,7 +21,7 @@
 // 512 rows without a ReLU, 32 -> 32 channels, 16 x 16 -> 32 x 32, 4x4 / 2: 59 us (FP32 kernel 161); 64 -> 32 channels 16 x 16,
 // 3x3: 71 us (143).  (Two TF32 parts a value, which leave a remainder, and twice as many steps: 63 and 91 us, 2.0e-7 and 4.9e-7.)
 // Warps 0-10 stage A, 11-18 read the accumulators back, 19 issues the MMAs.  Every wait is bounded; on expiry the CTA
-// writes NaN to all rows it owns, so that no bound can be taken from them.
+// writes NaN to all rows it owns and to their sums, so that no bound can be taken from them, and raises the status word.
 #include "conv_tc.cuh"
 #include "tc_primitives.cuh"
 
@@ -580,6 +580,12 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __grid_consta
           if ((ok >> ct.y) & 1u) c.out[off + ct.x] = __int_as_float(0x7fffffff);
         }
       }
+    if (c.partial != nullptr && blk == 0)
+      for (int tile = tile0; tile < p.tiles; tile += tile_step) {
+        const int lo = tile * TILE, hi = min(lo + TILE, c.M * p.P);
+        for (int r = p.dP(lo) + tid; r <= p.dP(hi - 1); r += THREADS) c.partial[(size_t)r * p.slots + tile - r * p.P / TILE] = __int_as_float(0x7fffffff);
+      }
+    if (tid == 0 && c.status) atomicExch(c.status, 1);
   }
   if (warp == MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }

@@ -11,6 +11,7 @@ struct ConvTcProblem {
   const float* W;                                // [Co, Ci, kh, kw]
   float* out;                                    // [M, Ci, Hi, Wi]
   float* partial;                                // [M, slots] sums of a * intercept + lam * bias, or null
+  int* status;                                   // device word, set non-zero when a wait expired (null: the NaN rows are the only sign)
   int M, S, Co, Ci, WH, WW, Hi, Wi, kh, kw, sh, sw, ph, pw;
 };
 

@@ -185,7 +185,9 @@ int bf_crown_relu_linear_bwd_packed(const float* A, int side,
  * bf_crown_relu_conv2d_bwd_scratch_bytes) holds the ReLU-scaled coefficients between the
  * two passes and, for wide layers, partial sums of delta.  Without slopes (no ReLU) it is
  * optional: NULL, or a buffer smaller than bf_crown_relu_conv2d_bwd_scratch_bytes, is simply not
- * used; with slopes a buffer of at least that size is required (BF_E_WORKSPACE otherwise). */
+ * used; with slopes a buffer of at least that size is required (BF_E_WORKSPACE otherwise).
+ * Large row blocks run on the tensor cores (FP32 values as three exact bfloat16 parts).  Every wait of that kernel is
+ * bounded; should one run out, the rows it concerns are NaN in A_prev and in delta. */
 size_t bf_crown_relu_conv2d_bwd_scratch_bytes(int B, int S, int Co, int Ho, int Wo);
 int bf_crown_relu_conv2d_bwd(const float* A, int side,
                              const float* alpha_u, const float* alpha_l,
@@ -343,7 +345,7 @@ int bf_chain_num_relu(const bf_chain* chain);
  * shared-memory image the MMA consumes.  bf_chain_tc_prepare does that packing into a
  * caller-owned device buffer of bf_chain_tc_bytes(chain) bytes (256-byte aligned) that must
  * outlive the chain; without it, or with the environment variable BF_B200_FORCE_FFMA=1, or
- * for tiny problems, the FP32 FFMA kernels are used.  Every wait inside the tensor-core
+ * for tiny problems, the FP32 FFMA kernels are used (for Conv2d layers too).  Every wait inside the tensor-core
  * kernels is bounded; bf_chain_tc_status (synchronous) returns non-zero in *status if a
  * wait ever expired, in which case results of that call are invalid. */
 size_t bf_chain_tc_bytes(const bf_chain* chain);

@@ -93,3 +93,60 @@ def test_error_against_fp32_kernels(dev, monkeypatch, B, S, Ci, H, W, Co, k, s, 
     err, err32 = (out.double() - ref), (fp32.double() - ref)
     assert err.norm() <= err32.norm()
     assert abs((err * ref.sign()).sum() / ref.abs().sum()) <= 3 * 2.0**-24
+
+
+def _network(dev, shape, convs, linears, g):
+    """Chain of convs (channels, kernel, stride, padding) and Linear widths with a ReLU after every layer but the last."""
+    from boundflow_b200.ir import BFTaskModule, BoundTask, TaskKind, TaskOp
+
+    ops, params, cur = [], {}, "input"
+    layers = [("c",) + c for c in convs] + [("f", n) for n in linears]
+    for i, (kind, n, *geo) in enumerate(layers):
+        out = "out" if i + 1 == len(layers) else f"h{i}"
+        if kind == "c":
+            k, s, p = geo
+            params[f"W{i}"] = torch.randn(n, shape[0], k, k, generator=g, device=dev) * (2.0 / (shape[0] * k * k)) ** 0.5
+            ops.append(TaskOp("conv2d", f"conv{i}", [cur, f"W{i}", f"b{i}"], [out], {"stride": (s, s), "padding": (p, p)}))
+            shape = (n, (shape[1] + 2 * p - k) // s + 1, (shape[2] + 2 * p - k) // s + 1)
+        else:
+            if len(shape) == 3:
+                ops.append(TaskOp("flatten", "flatten", [cur], ["flat"], {"start_dim": 1, "end_dim": -1}))
+                cur, shape = "flat", (shape[0] * shape[1] * shape[2],)
+            params[f"W{i}"] = torch.randn(n, shape[0], generator=g, device=dev) * (2.0 / shape[0]) ** 0.5
+            ops.append(TaskOp("linear", f"linear{i}", [cur, f"W{i}", f"b{i}"], [out]))
+            shape = (n,)
+        params[f"b{i}"] = torch.randn(n, generator=g, device=dev) * 0.1
+        cur = out
+        if i + 1 < len(layers):
+            ops.append(TaskOp("relu", f"relu{i}", [cur], [f"r{i}"]))
+            cur = f"r{i}"
+    task = BoundTask(task_id="t0", kind=TaskKind.INTERVAL_IBP, ops=ops, input_values=["input"], output_values=["out"])
+    return BFTaskModule(tasks=[task], entry_task_id="t0", bindings={"params": params})
+
+
+def _box(x, eps):
+    from boundflow_b200.ir import InputSpec
+
+    return InputSpec.box(value_name="input", lower=x - eps, upper=x + eps)
+
+
+# the status word of an expired wait (set here by the host) takes the bounds of a chain whose only tensor-core kernel is the convolution's:
+# 36 rows, too few for the Linear layers' kernels
+def test_expired_wait_takes_the_bounds_of_conv_chains(dev):
+    from boundflow_b200 import _lib
+    from boundflow_b200.crown import adaptive_alpha_from_trace, alpha_crown_from_trace, crown_from_trace, ibp_trace
+
+    g = torch.Generator("cuda").manual_seed(5)
+    module = _network(dev, (3, 32, 32), [(16, 3, 1, 1), (16, 3, 1, 1)], [10], g)
+    trace = ibp_trace(module, _box(torch.rand(4, 3, 32, 32, generator=g, device=dev), 0.01))
+    C = torch.randn(4, 9, 10, generator=g, device=dev)
+    before = _lib.tc_launch_count()
+    assert torch.isfinite(torch.stack(crown_from_trace(trace, C))).all() and _lib.tc_launch_count() == before + 2
+    status = trace.chain._tc_buffer[:4].view(torch.int32)
+    status.fill_(1)
+    try:
+        assert torch.isnan(torch.stack(crown_from_trace(trace, C))).all()
+        lower, upper, _alpha, _last, _metric = alpha_crown_from_trace(trace, C, adaptive_alpha_from_trace(trace), steps=2, lr=0.1, spec_reduce="mean", want_upper=True)
+        assert torch.isnan(lower).all() and torch.isnan(upper).all()
+    finally:
+        status.zero_()
