@@ -530,6 +530,10 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
   bool windowed = false;
   bf::refresh_switches(chain);
   const bool windows_allowed = box && influence == nullptr && !chain->sw.no_windows;
+  // rows that bound the neurons of a conv layer stay on the FP32 kernels in every layer below (see CONV_TC_MIN_TILES in conv.cu)
+  int top = upto_layer - 1;
+  while (top > low && chain->layers[top].op != BF_OP_LINEAR && chain->layers[top].op != BF_OP_CONV2D) --top;
+  const bool neuron_rows = chain->layers[top].op == BF_OP_CONV2D && (C == nullptr || upto_layer < nl);
   for (int i = upto_layer - 1; i >= 0; --i) {
     const bf_layer_desc& L = chain->layers[i];
     if (L.op == BF_OP_FLATTEN) continue;
@@ -605,7 +609,7 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
     } else {
       float* dst = ws.buf[toggle];
       rc = bf::launch_crown_bwd_conv2d(curA, dpos, dneg, epos, eneg, L.W, L.bias, dst, ws.cacc, have_c, M, S, L,
-                                       ws.conv_scratch, stream, ad, chain->status != nullptr, chain->status);
+                                       ws.conv_scratch, stream, ad, chain->status != nullptr && !neuron_rows, chain->status);
       curA = dst;
     }
     if (rc != BF_OK) return rc;

@@ -770,10 +770,11 @@ static int launch_convT_rowseg(const ConvTArgs& g, cudaStream_t stream) {
 // 64 channels 8 x 8 -> 64 channels 16 x 16, 4x4 / 2 (324 tiles): 90 us against 172; 512 rows of 40 channels 9 x 9, 3x3 / 2: 37
 // against 84.  Not for few input channels (1 or 3 channels fill an eighth of the narrowest MMA: 73 against 42 us, 205 against
 // 91) and not for more than nine taps per phase (5x5 / 1: 128 against 120 us; its MMAs are bound by their issue).
-// Windowed rows stay on the FP32 kernels although the tensor cores took a third of their time (64,000 windows, 32 -> 32
-// channels: 0.33 against 1.5 ms): they bound every neuron of the conv layers, millions of values whose last bit differs, and a
-// few of those lie within that bit of zero, where the relaxation of their ReLU changes sides: 2 of 8 networks moved by 6e-5.
-// Full rows bound the neurons of linear layers and the specs, some ten thousand values: no change of sides in 8 networks.
+// Rows that bound the neurons of a conv layer stay on the FP32 kernels, as windows and as full rows (Lp balls, windows that
+// have grown to the map), although the tensor cores took a third of their time (64,000 windows, 32 -> 32 channels: 0.33
+// against 1.5 ms): they are millions of values whose last bit differs, and a few of those lie within that bit of zero, where
+// the relaxation of their ReLU changes sides: 2 of 8 networks moved by 6e-5.  Rows that bound the neurons of Linear layers or
+// the specs are some ten thousand values: no change of sides in 8 networks.
 constexpr int CONV_TC_MIN_TILES = 148, CONV_TC_MIN_CI = 8, CONV_TC_MAX_TAPS = 9;
 
 // scaled coefficients [M, n_out] followed by the per-chunk partial sums of the intercept term [M, chunks]
@@ -1221,11 +1222,10 @@ extern "C" size_t bf_crown_relu_conv2d_bwd_scratch_bytes(int B, int S, int Co, i
   return bf::crown_bwd_conv2d_scratch_bytes(B * S, L);
 }
 
-extern "C" int bf_crown_relu_conv2d_bwd(const float* A, int side, const float* alpha_u, const float* alpha_l,
-                                        const float* beta_u, const float* beta_l, const float* W, const float* bias,
-                                        float* A_prev, float* delta, int accumulate, void* scratch, size_t scratch_bytes,
-                                        int B, int S, int Ci, int Hi, int Wi, int Co, int Ho, int Wo, int kh, int kw, int sh,
-                                        int sw, int ph, int pw, bf_stream_t stream) {
+static int conv2d_bwd(bool tensor_cores, const float* A, int side, const float* alpha_u, const float* alpha_l,
+                      const float* beta_u, const float* beta_l, const float* W, const float* bias, float* A_prev, float* delta,
+                      int accumulate, void* scratch, size_t scratch_bytes, int B, int S, int Ci, int Hi, int Wi, int Co, int Ho,
+                      int Wo, int kh, int kw, int sh, int sw, int ph, int pw, bf_stream_t stream) {
   BF_REQUIRE(A && W, BF_E_INVALID, "bf_crown_relu_conv2d_bwd: A and W must be non-null");
   BF_REQUIRE(B > 0 && S > 0 && Ci > 0 && Co > 0 && Hi > 0 && Wi > 0 && Ho > 0 && Wo > 0 && kh > 0 && kw > 0 && sh > 0 && sw > 0,
              BF_E_INVALID, "bf_crown_relu_conv2d_bwd: bad geometry");
@@ -1249,7 +1249,25 @@ extern "C" int bf_crown_relu_conv2d_bwd(const float* A, int side, const float* a
   // (a block then streams a whole coefficient row)
   if (!relu && scratch_bytes < bf_crown_relu_conv2d_bwd_scratch_bytes(B, S, Co, Ho, Wo)) scratch = nullptr;
   return bf::launch_crown_bwd_conv2d(A, dpos, dneg, epos, eneg, W, bias, A_prev, delta, accumulate, B * S, S, L, scratch,
-                                     bf::as_stream(stream), nullptr, true, nullptr);
+                                     bf::as_stream(stream), nullptr, tensor_cores, nullptr);
+}
+
+extern "C" int bf_crown_relu_conv2d_bwd(const float* A, int side, const float* alpha_u, const float* alpha_l,
+                                        const float* beta_u, const float* beta_l, const float* W, const float* bias,
+                                        float* A_prev, float* delta, int accumulate, void* scratch, size_t scratch_bytes,
+                                        int B, int S, int Ci, int Hi, int Wi, int Co, int Ho, int Wo, int kh, int kw, int sh,
+                                        int sw, int ph, int pw, bf_stream_t stream) {
+  return conv2d_bwd(true, A, side, alpha_u, alpha_l, beta_u, beta_l, W, bias, A_prev, delta, accumulate, scratch, scratch_bytes, B, S,
+                    Ci, Hi, Wi, Co, Ho, Wo, kh, kw, sh, sw, ph, pw, stream);
+}
+
+extern "C" int bf_crown_relu_conv2d_bwd_fp32(const float* A, int side, const float* alpha_u, const float* alpha_l,
+                                             const float* beta_u, const float* beta_l, const float* W, const float* bias,
+                                             float* A_prev, float* delta, int accumulate, void* scratch, size_t scratch_bytes,
+                                             int B, int S, int Ci, int Hi, int Wi, int Co, int Ho, int Wo, int kh, int kw, int sh,
+                                             int sw, int ph, int pw, bf_stream_t stream) {
+  return conv2d_bwd(false, A, side, alpha_u, alpha_l, beta_u, beta_l, W, bias, A_prev, delta, accumulate, scratch, scratch_bytes, B, S,
+                    Ci, Hi, Wi, Co, Ho, Wo, kh, kw, sh, sw, ph, pw, stream);
 }
 
 // ReLU backward alone (graphs where the ReLU's producer is not a single affine layer, e.g. after an add):

@@ -259,6 +259,9 @@ def _sweep(lib, module: Any, tr: DagTrace, params: Dict[str, torch.Tensor], rela
     S = int(C.shape[1])
     s = _stream_ptr(device)
     dynamic = set(tr.lower) - set(params)
+    # rows that bound the neurons of a feature map stay on the FP32 convolutions (bf_b200.h)
+    neurons = len(tr.shape[output_value]) == 3 and (output_value not in task.output_values or S == _numel(tr.shape[output_value]))
+    conv_bwd = lib.bf_crown_relu_conv2d_bwd_fp32 if neurons else lib.bf_crown_relu_conv2d_bwd
     adj: Dict[str, _State] = {output_value: _State(C.clone(), torch.zeros(B, S, device=device))}
 
     def push(name: str, A: torch.Tensor, d: torch.Tensor) -> None:
@@ -294,9 +297,8 @@ def _sweep(lib, module: Any, tr: DagTrace, params: Dict[str, torch.Tensor], rela
             Ap = torch.empty(B, S, Ci * Hi * Wi, device=device)
             nb = int(lib.bf_crown_relu_conv2d_bwd_scratch_bytes(B, S, Co, Ho, Wo))
             scratch = torch.empty(max(nb, 16), dtype=torch.uint8, device=device)
-            _lib.check(lib.bf_crown_relu_conv2d_bwd(_lib.ptr(st.A), side, None, None, None, None, _lib.ptr(W), _lib.ptr(b), _lib.ptr(Ap),
-                                                    _lib.ptr(st.d), 1, _lib.ptr(scratch), scratch.numel(), B, S, Ci, Hi, Wi, Co, Ho, Wo,
-                                                    kh, kw, sth[0], sth[1], pdh[0], pdh[1], s))
+            _lib.check(conv_bwd(_lib.ptr(st.A), side, None, None, None, None, _lib.ptr(W), _lib.ptr(b), _lib.ptr(Ap), _lib.ptr(st.d), 1,
+                                _lib.ptr(scratch), scratch.numel(), B, S, Ci, Hi, Wi, Co, Ho, Wo, kh, kw, sth[0], sth[1], pdh[0], pdh[1], s))
             push(op.inputs[0], Ap, st.d)
         elif t == "relu":
             x = op.inputs[0]

@@ -150,3 +150,28 @@ def test_expired_wait_takes_the_bounds_of_conv_chains(dev):
         assert torch.isnan(lower).all() and torch.isnan(upper).all()
     finally:
         status.zero_()
+
+
+# neurons of conv layers as full rows (a ball that no window represents; windows that outgrow a small map; a graph): the bits of the FP32 kernels
+@pytest.mark.parametrize("case", ["l2", "outgrown", "graph"])
+def test_conv_neuron_rows_stay_on_fp32(dev, monkeypatch, case):
+    from boundflow_b200 import _lib
+    from boundflow_b200.crown import run_crown_ibp_mlp
+    from boundflow_b200.ir import InputSpec, TaskOp
+
+    g = torch.Generator("cuda").manual_seed(6)
+    size = 6 if case == "outgrown" else 16
+    module = _network(dev, (8, size, size), [(16, 3, 1, 1), (16, 3, 1, 1), (16, 3, 1, 1), (16, 3, 1, 1)], [10], g)
+    x = torch.rand(2 if case == "graph" else 4, 8, size, size, generator=g, device=dev)
+    if case == "graph":  # h2 + r0: not a chain any more
+        ops = module.get_entry_task().ops
+        at = next(i for i, o in enumerate(ops) if o.name == "relu2")
+        ops[at] = TaskOp("relu", "relu2", ["s2"], ["r2"])
+        ops.insert(at, TaskOp("add", "add2", ["h2", "r0"], ["s2"]))
+    spec = InputSpec.l2(value_name="input", center=x, eps=0.05) if case == "l2" else _box(x, 0.01)
+    before = _lib.tc_launch_count()
+    got = run_crown_ibp_mlp(module, spec, output_value="h2")
+    assert _lib.tc_launch_count() == before
+    monkeypatch.setenv("BF_B200_FORCE_FFMA", "1")
+    want = run_crown_ibp_mlp(module, spec, output_value="h2")
+    assert torch.equal(got.lower, want.lower) and torch.equal(got.upper, want.upper)
