@@ -3,6 +3,7 @@
 // (ReLU backward + transposed convolution of the coefficient rows).
 #include <cooperative_groups.h>
 
+#include <float.h>
 #include <stdlib.h>
 
 #include "conv_tc.cuh"
@@ -38,6 +39,33 @@ template <int TN>
 struct ConvTile {
   static constexpr int TM = 4096 / TN, SLAB = (TN == 16) ? 8 : 16;
 };
+
+// Sums of one output (pixel of all images, channel) over the taps inside the image: centre, radius
+template <bool INTERVAL>
+__device__ __forceinline__ float2 taps_inside(const IbpConvArgs& g, long long pix, int co) {
+  const int howo = g.Ho * g.Wo, b = (int)(pix / howo), q = (int)(pix - (long long)b * howo);
+  const int h0 = q / g.Wo * g.sh - g.ph, w0 = q % g.Wo * g.sw - g.pw;
+  float2 t = make_float2(0.f, 0.f);
+  for (int ci = 0; ci < g.Ci; ++ci)
+    for (int r = max(0, -h0); r < g.kh && h0 + r < g.Hi; ++r)
+      for (int s = max(0, -w0); s < g.kw && w0 + s < g.Wi; ++s) {
+        const size_t i = (((size_t)b * g.Ci + ci) * g.Hi + h0 + r) * g.Wi + w0 + s;
+        const float w = g.W[(((size_t)co * g.Ci + ci) * g.kh + r) * g.kw + s];
+        float c = g.in_a[i];
+        if (INTERVAL) {
+          float d = g.in_b[i];
+          if (g.in_mode == BF_IN_LOWER_UPPER) {
+            if (g.relu_in) { c = fmaxf(c, 0.f); d = fmaxf(d, 0.f); }
+            const float mid = (c + d) * 0.5f;
+            d = (d - c) * 0.5f;
+            c = mid;
+          }
+          t.y = fmaf(d, fabsf(w), t.y);
+        }
+        t.x = fmaf(c, w, t.x);
+      }
+  return t;
+}
 
 template <bool INTERVAL, int TN>
 __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper, int vec) {
@@ -190,6 +218,30 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
 
   const long long pt = p0 + tx * 4;
   if (pt >= npix) return;
+  // A tap outside the image has multiplied its weight by 0, which is NaN for an infinite weight: sums that are not finite are
+  // formed again from the taps inside.
+  bool finite = true;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      finite &= fabsf(accC[i][j]) <= FLT_MAX;
+      if (INTERVAL) finite &= fabsf(accR[i][j]) <= FLT_MAX;
+    }
+  if (!finite) {
+    for (int e = 0; e < 16; ++e) {
+      const int i = e >> 2, j = e & 3;
+      if (pt + j >= npix || c0 + ty * 4 + i >= g.Co) continue;
+      const float2 t = taps_inside<INTERVAL>(g, pt + j, c0 + ty * 4 + i);
+      smem[e * 256 + tid] = t.x;  // the slabs are read no more; a thread has words of its own
+      if (INTERVAL) smem[4096 + e * 256 + tid] = t.y;
+    }
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      accC[e >> 2][e & 3] = smem[e * 256 + tid];
+      if (INTERVAL) accR[e >> 2][e & 3] = smem[4096 + e * 256 + tid];
+    }
+  }
   int b4[4], q4[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {

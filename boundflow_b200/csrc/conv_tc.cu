@@ -22,6 +22,8 @@
 // 3x3: 71 us (143).  (Two TF32 parts a value, which leave a remainder, and twice as many steps: 63 and 91 us, 2.0e-7 and 4.9e-7.)
 // Warps 0-10 stage A, 11-18 read the accumulators back, 19 issues the MMAs.  Every wait is bounded; on expiry the CTA
 // writes NaN to all rows it owns and to their sums, so that no bound can be taken from them, and raises the status word.
+#include <float.h>
+
 #include "conv_tc.cuh"
 #include "tc_primitives.cuh"
 
@@ -220,11 +222,38 @@ __device__ __forceinline__ void sum_accumulators(uint32_t at, const int* col, bo
   }
 }
 
+// One output on the FP32 units, over the taps that exist.  Splitting an infinity leaves NaN (inf - inf), and a zero that only
+// fills a tile (a tap past the kernel, a channel past Co) times an infinity is NaN too, so outputs that are not finite
+// are formed again from the coefficients and weights they are made of.
+__device__ __forceinline__ float scalar_output(const ConvTcProblem& c, long long at) {
+  const int w = (int)(at % c.Wi), h = (int)(at / c.Wi % c.Hi), ci = (int)(at / ((long long)c.Wi * c.Hi) % c.Ci);
+  const int m = (int)(at / ((long long)c.Wi * c.Hi * c.Ci)), plane = c.WH * c.WW;
+  const float* a = c.A + (size_t)m * c.Co * plane;
+  const size_t dom = (size_t)(m / c.S) * c.Co * plane;
+  float t = 0.f;
+  for (int r = 0; r < c.kh; ++r) {
+    const int u = h + c.ph - r, y = u / c.sh;
+    if (u < 0 || u % c.sh != 0 || y >= c.WH) continue;
+    for (int s = 0; s < c.kw; ++s) {
+      const int v = w + c.pw - s, x = v / c.sw;
+      if (v < 0 || v % c.sw != 0 || x >= c.WW) continue;
+      for (int co = 0; co < c.Co; ++co) {
+        const int i = co * plane + y * c.WW + x;
+        float lam = a[i];
+        if (c.dpos) lam = lam * (lam >= 0.f ? c.dpos : c.dneg)[dom + i] + (c.add ? c.add[dom + i] : 0.f);
+        t = fmaf(lam, c.W[((size_t)co * c.Ci + ci) * c.kh * c.kw + r * c.kw + s], t);
+      }
+    }
+  }
+  return t;
+}
+
 // Column groups g, g + 1, ... end - 1 (W columns each) of a warp's 32 positions: sums the accumulators and stores; the
 // accumulators are handed back before the last group's stores.
-__device__ __forceinline__ void read_and_store(uint32_t base, int g, int end, int naccs, const int* acc_col, const int2* col_tab, float* out,
-                                               uint32_t ok, bool pairs, uint32_t empty_bar) {
+__device__ __forceinline__ void read_and_store(uint32_t base, int g, int end, int naccs, const int* acc_col, const int2* col_tab,
+                                               const ConvTcProblem& c, long long off, uint32_t ok, bool pairs, uint32_t empty_bar) {
   constexpr int N = 4;  // accumulators in flight
+  float* out = c.out + off;
   for (; g < end; ++g) {
     float t[W];
     const uint32_t at = base + (uint32_t)(g * W);
@@ -252,6 +281,16 @@ __device__ __forceinline__ void read_and_store(uint32_t base, int g, int end, in
         stg_if(out + ct.z, t[q + 1], (ok >> ct.w) & 1u);
       }
     }
+    bool finite = true;
+#pragma unroll
+    for (int i = 0; i < W; ++i) finite &= fabsf(t[i]) <= FLT_MAX;
+    if (!finite) {
+      for (int q = g * W; q < (g + 1) * W; ++q) {
+        const int2 ct = col_tab[q];
+        if (((ok >> ct.y) & 1u) && !(fabsf(out[ct.x]) <= FLT_MAX)) out[ct.x] = scalar_output(c, off + ct.x);
+      }
+    }
+    __syncwarp();  // the next tensor-memory loads take the whole warp
   }
 }
 
@@ -501,8 +540,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __grid_consta
       tc_fence_after();
       const uint32_t base = row + (uint32_t)(buf * (MAX_COLS / 2));
       const uint32_t empty_bar = smem_u32(&ctl.acc_empty[buf]);
-      float* out = c.out + off;
-      read_and_store(base, from, to, naccs, acc_col, col_tab, out, ok, p.pairs, empty_bar);
+      read_and_store(base, from, to, naccs, acc_col, col_tab, c, off, ok, p.pairs, empty_bar);
       if (from >= to && lane == 0) mbar_arrive(empty_bar);
     }
   } else {

@@ -175,3 +175,55 @@ def test_conv_neuron_rows_stay_on_fp32(dev, monkeypatch, case):
     monkeypatch.setenv("BF_B200_FORCE_FFMA", "1")
     want = run_crown_ibp_mlp(module, spec, output_value="h2")
     assert torch.equal(got.lower, want.lower) and torch.equal(got.upper, want.upper)
+
+
+# infinities pass as they do through a sum over the taps that exist: rows whose coefficients or weights are infinite, or round to infinity
+@pytest.mark.parametrize("what", ["coefficient", "weight", "largest"])
+@pytest.mark.parametrize("B,S,Ci,H,W,Co,k,s,p", [(8, 64, 16, 17, 17, 20, 3, 2, 1), (8, 64, 32, 16, 16, 30, 3, 1, 1)])
+def test_infinities(dev, B, S, Ci, H, W, Co, k, s, p, what):
+    Ho, Wo = (H + 2 * p - k) // s + 1, (W + 2 * p - k) // s + 1
+    g = torch.Generator("cuda").manual_seed(7)
+    A, w = torch.rand(B, S, Co, Ho, Wo, generator=g, device=dev) + 0.5, torch.rand(Co, Ci, k, k, generator=g, device=dev) + 0.5
+    big = 3.4028234e38 if what == "largest" else float("inf")
+    if what == "weight":
+        w[3, 5, 1, 1] = big
+    else:
+        A[1, 2, 3, 4, 5] = big
+        A[1, 3, 4, 0, 0] = -big
+        w *= 0.25  # the largest number stays in range behind the weight
+    out, launches = _backward(A, w, s, p, H, W)
+    assert launches == 1
+    # every sum is of positive products (and one infinity): in float64, with the infinities in their place
+    ref = _transposed(torch.where(A.isinf(), torch.zeros_like(A), A).double(), torch.where(w.isinf(), torch.zeros_like(w), w).double(), s, p, H, W)
+    reach = _transposed(A.isinf().double() * A.sign(), torch.ones_like(w).double(), s, p, H, W)
+    reach = reach + _transposed(torch.ones_like(A).double(), w.isinf().double(), s, p, H, W)
+    ref = torch.where(reach > 0, torch.full_like(ref, float("inf")), torch.where(reach < 0, torch.full_like(ref, -float("inf")), ref))
+    assert torch.equal(out.isinf(), ref.isinf()) and not out.isnan().any()
+    assert torch.equal(out[ref.isinf()].double(), ref[ref.isinf()])
+    # a sum of n = Co k^2 positive products (one of them minus the largest number): at most (n + 8) 2^-24 of the sum of magnitudes
+    mag = _transposed(torch.where(A.isinf(), torch.zeros_like(A), A).double().abs(), torch.where(w.isinf(), torch.zeros_like(w), w).double(), s, p, H, W)
+    ok = ~ref.isinf()
+    assert ((out.double() - ref)[ok].abs() <= ((Co * k * k + 8) * 2.0**-24 * mag)[ok]).all()
+
+
+@pytest.mark.parametrize("B,Ci,H,W,Co,k,s,p", [(3, 3, 9, 11, 17, 3, 1, 1), (2, 4, 12, 12, 40, 4, 2, 1), (5, 1, 8, 8, 5, 3, 1, 2)])
+def test_infinite_weight_at_the_border_of_forward_convolutions(dev, B, Ci, H, W, Co, k, s, p):
+    from boundflow_b200 import _lib
+
+    lib = _lib.load()
+    Ho, Wo = (H + 2 * p - k) // s + 1, (W + 2 * p - k) // s + 1
+    g = torch.Generator("cuda").manual_seed(8)
+    x = torch.rand(B, Ci, H, W, generator=g, device=dev) + 0.5
+    w = torch.rand(Co, Ci, k, k, generator=g, device=dev)
+    w[1, 0, 0, 0] = float("inf")
+    # channel 1: infinite where kernel position (0, 0) lies inside the image
+    rows, cols = torch.arange(Ho, device=dev) * s - p >= 0, torch.arange(Wo, device=dev) * s - p >= 0
+    hit = torch.zeros(B, Co, Ho, Wo, dtype=torch.bool, device=dev)
+    hit[:, 1] = rows[:, None] & cols[None]
+    out = torch.full((B, Co, Ho, Wo), float("nan"), device=dev)
+    _lib.check(lib.bf_rows_conv2d_fwd(x.data_ptr(), w.data_ptr(), None, out.data_ptr(), B, Ci, H, W, Co, Ho, Wo, k, k, s, s, p, p, None))
+    assert torch.equal(out == float("inf"), hit) and torch.isfinite(out[~hit]).all()
+    lo, up = (torch.full((B, Co, Ho, Wo), float("nan"), device=dev) for _ in range(2))
+    _lib.check(lib.bf_ibp_conv2d(x.data_ptr(), (x * 0).data_ptr(), _lib.IN_MID_RAD, 0, w.abs().data_ptr(), None, None, 0, None, None, lo.data_ptr(), up.data_ptr(),
+                                 None, B, Ci, H, W, Co, k, k, s, s, p, p, None))
+    assert torch.isfinite(lo[~hit]).all() and torch.isfinite(up[~hit]).all()
