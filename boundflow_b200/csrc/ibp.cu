@@ -13,6 +13,15 @@ namespace bf {
 
 constexpr int IBM = 64, IBN = 64, IBK = 16, ILD = 68, ISLAB = IBK * ILD;
 
+// Up to IBP_SERIAL_K terms a sum is one chain over k.  Above (the layer behind a flatten: K = 1568, 4096, 8192) it is four
+// chains, one behind the other, per segment of ibp_segment(K) columns; a segment adds its chains in order, the sum its segments.
+// That is the order of every kernel here, so that an input's bounds are the same bits in every batch.  Widths of hidden layers
+// stay with the single chain: their bounds feed optimisation loops whose trajectories follow the last bit, and cutting it
+// saves a few microseconds there; above it saves most of the time (16 x 8192 x 10: 27 us with eight segments, 113 in one chain).
+constexpr int IBP_SERIAL_K = 1024, IBP_CHAINS = 4;
+static int ibp_segments(int K) { return K <= 2 * IBP_SERIAL_K ? 4 : 8; }
+static int ibp_segment(int K) { return ceil_div(ceil_div(K, 64), ibp_segments(K)) * 64; }
+
 struct IbpArgs {
   const float* in_a; const float* in_b; int in_mode; int relu_in;
   const float* W; const float* bias;
@@ -27,8 +36,11 @@ struct IbpArgs {
 // 784-wide first layer and -7 % on 1024 rows and fewer; four CTAs spill and lose everywhere: occupancy is not the limit.  A 64 x 128 tile (4 x 8 outputs per thread, 1.0 instead of
 // 1.5 shared-memory bytes per FFMA, 128 registers) was measured at 233 against 226 us on 8192 x 512 x 512 (512 CTAs are 1.7
 // waves of 296), 364 against 391 us on the 784-wide layer and 137 against 105 us on a ragged 260-wide one: not kept.
-__global__ void __launch_bounds__(256) ibp_linear_kernel(IbpArgs g) {
+// CHAINS: sums in chains of `chain` slabs (see IBP_SERIAL_K); those of finished segments wait in shared memory.
+template <bool CHAINS>
+__global__ void __launch_bounds__(256) ibp_linear_kernel(IbpArgs g, int chain) {
   __shared__ __align__(16) float smem[2 * 3 * ISLAB];
+  extern __shared__ __align__(16) float seg_smem[];  // CHAINS: segments before this one, [centre, radius][16][thread]
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int m0 = blockIdx.x * IBM, n0 = blockIdx.y * IBN;
   const int lrow = tid >> 2, lkc = (tid & 3) * 4;
@@ -75,6 +87,12 @@ __global__ void __launch_bounds__(256) ibp_linear_kernel(IbpArgs g) {
   };
 
   const int nk = (g.K + IBK - 1) / IBK;
+  int left = chain, chains = IBP_CHAINS;
+  float segment[CHAINS ? 32 : 1];                     // of the segment's finished chains
+  if (CHAINS) {
+#pragma unroll
+    for (int e = 0; e < 32; ++e) segment[e] = seg_smem[e * 256 + tid] = 0.f;
+  }
   load_slab(0);
   store_slab(0);
   __syncthreads();
@@ -100,8 +118,30 @@ __global__ void __launch_bounds__(256) ibp_linear_kernel(IbpArgs g) {
           accR[i][j] = fmaf(r[i], fabsf(w[j]), accR[i][j]);
         }
     }
+    if (CHAINS && (--left == 0 || kt + 1 == nk)) {
+      left = chain;
+      const bool ends = --chains == 0 || kt + 1 == nk;
+      if (ends) chains = IBP_CHAINS;
+#pragma unroll
+      for (int e = 0; e < 32; ++e) {
+        float& acc = e < 16 ? accC[(e & 15) >> 2][e & 3] : accR[(e & 15) >> 2][e & 3];
+        segment[CHAINS ? e : 0] += acc;
+        acc = 0.f;
+        if (ends) {
+          seg_smem[e * 256 + tid] += segment[CHAINS ? e : 0];
+          segment[CHAINS ? e : 0] = 0.f;
+        }
+      }
+    }
     if (kt + 1 < nk) store_slab(stage ^ 1);
     __syncthreads();
+  }
+  if (CHAINS) {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      accC[e >> 2][e & 3] = seg_smem[e * 256 + tid];
+      accR[e >> 2][e & 3] = seg_smem[(16 + e) * 256 + tid];
+    }
   }
 
   const int col = n0 + tx * 4;
@@ -266,26 +306,23 @@ __global__ void __launch_bounds__(256) ibp_linear_small_kernel(IbpArgs g) {
   }
 }
 
-// Few outputs and long rows (the layer behind a flatten: K = 4096, 8192): walking K in one CTA is a serial chain whatever the tile.  A tile is
-// 32 x 32, a slab 64 deep (six 128-bit loads in flight per thread), the CTA's four thread groups take 16 of its columns each, and a
-// cluster of up to eight CTAs splits K; partial sums meet in (distributed) shared memory in rank order, without a
-// workspace or atomics.  200 x 4096 x 512: 89 us (64 x 64 tiles: 370), bound by FFMA issue at 224 CTAs; 256 x 1568 x 100: 17 us (144);
-// 16 x 8192 x 10: 26 us (619), bound by the 16 serial slabs of a rank.
+// Long sums in chains (see IBP_SERIAL_K): a tile is 32 x 32; a CTA takes one segment, each of its four thread groups one chain, 16
+// columns of every chain per slab (six 128-bit loads in flight per thread); the CTAs of a cluster take the segments, whose sums
+// meet in distributed shared memory in rank order, without a workspace or atomics.  Measured, against one chain on 64 x 64
+// tiles: 200 x 4096 x 512: 91 us (320), 256 x 1568 x 100: 17 (124), 16 x 8192 x 10: 27 (541), 600 x 6144 x 249: 162 (476).
 // Shared slabs are [k][row] with rows XOR-ed by ((k >> 2) & 7) << 2: transposed stores conflict two-way, 128-bit reads not at all.
-// Up to IBP_SERIAL_K terms the sums keep their order: bounds of networks of that width feed optimisation loops whose
-// trajectories follow the last bit, and the serial chain costs a few microseconds there.
-constexpr int IBP_SERIAL_K = 1024;
-constexpr int STM = 32, STN = 32, SBK = 64, SSLAB = SBK * 32, SGROUPS = 4;
+constexpr int STM = 32, STN = 32, SBK = 64, SSLAB = SBK * 32, SGROUPS = IBP_CHAINS, SCOLS = SBK / SGROUPS;
 __device__ __forceinline__ int swz(int k, int row) { return k * 32 + (row ^ (((k >> 2) & 7) << 2)); }
 
-__global__ void __launch_bounds__(256) ibp_linear_split_kernel(IbpArgs g, int kper) {
+__global__ void __launch_bounds__(256) ibp_linear_chains_kernel(IbpArgs g, int chain) {  // chain: slabs of a chain
   __shared__ __align__(16) float smem[2 * 3 * SSLAB];
   static_assert(SGROUPS * 2 * STM * STN + 2 * STM * STN <= 2 * 3 * SSLAB, "the reduction reuses the slabs");
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const int tid = threadIdx.x, kg = tid >> 6, tx = tid & 7, ty = (tid & 63) >> 3;
   const int m0 = blockIdx.x * STM, n0 = blockIdx.y * STN;
-  const int k0 = blockIdx.z * kper, k1 = min(g.K, k0 + kper);
+  const int k0 = blockIdx.z * SGROUPS * chain * SCOLS;
   const int lrow = tid >> 4, lk = (tid & 15) * 4;
+  const int column = k0 + lk / SCOLS * chain * SCOLS + lk % SCOLS;  // this thread's in the first slab
   const bool vK = g.vecK != 0;
   float accC[4][4], accR[4][4];
 #pragma unroll
@@ -294,16 +331,17 @@ __global__ void __launch_bounds__(256) ibp_linear_split_kernel(IbpArgs g, int kp
     for (int j = 0; j < 4; ++j) accC[i][j] = accR[i][j] = 0.f;
 
   float4 creg[2], rreg[2], wreg[2];
-  auto load_slab = [&](int k) {
+  auto load_slab = [&](int kt) {
+    const int k = column + kt * SCOLS;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int m = m0 + lrow + 16 * i, n = n0 + lrow + 16 * i;
       creg[i] = rreg[i] = wreg[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (m < g.B) {
-        creg[i] = load4_guard(g.in_a + (size_t)m * g.K, k + lk, k1, vK);
-        if (g.in_b) rreg[i] = load4_guard(g.in_b + (size_t)m * g.K, k + lk, k1, vK);
+        creg[i] = load4_guard(g.in_a + (size_t)m * g.K, k, g.K, vK);
+        if (g.in_b) rreg[i] = load4_guard(g.in_b + (size_t)m * g.K, k, g.K, vK);
       }
-      if (n < g.N) wreg[i] = load4_guard(g.W + (size_t)n * g.K, k + lk, k1, vK);
+      if (n < g.N) wreg[i] = load4_guard(g.W + (size_t)n * g.K, k, g.K, vK);
     }
   };
   auto store_slab = [&](int stage) {
@@ -321,21 +359,21 @@ __global__ void __launch_bounds__(256) ibp_linear_split_kernel(IbpArgs g, int kp
     }
   };
 
-  const int nk = (k1 > k0) ? (k1 - k0 + SBK - 1) / SBK : 0;
+  const int nk = max(0, min(chain, (g.K - k0 + SCOLS - 1) / SCOLS));
   if (nk > 0) {
-    load_slab(k0);
+    load_slab(0);
     store_slab(0);
   }
   __syncthreads();
   for (int kt = 0; kt < nk; ++kt) {
     const int stage = kt & 1;
-    if (kt + 1 < nk) load_slab(k0 + (kt + 1) * SBK);
+    if (kt + 1 < nk) load_slab(kt + 1);
     const float* cs = smem + stage * 3 * SSLAB;
     const float* rs = cs + SSLAB;
     const float* ws = rs + SSLAB;
 #pragma unroll
-    for (int q = 0; q < SBK / SGROUPS; ++q) {
-      const int kk = kg * (SBK / SGROUPS) + q;
+    for (int q = 0; q < SCOLS; ++q) {
+      const int kk = kg * SCOLS + q;
       const float4 c4 = *reinterpret_cast<const float4*>(&cs[swz(kk, ty * 4)]);
       const float4 r4 = *reinterpret_cast<const float4*>(&rs[swz(kk, ty * 4)]);
       const float4 w4 = *reinterpret_cast<const float4*>(&ws[swz(kk, tx * 4)]);
@@ -354,7 +392,7 @@ __global__ void __launch_bounds__(256) ibp_linear_split_kernel(IbpArgs g, int kp
     __syncthreads();
   }
 
-  // thread groups of the CTA, then ranks of the cluster
+  // chains of the segment, then segments
   float* red = smem;                                  // [SGROUPS][2][32][32]
   float* part = smem + SGROUPS * 2 * STM * STN;       // [2][32][32]
 #pragma unroll
@@ -397,32 +435,40 @@ int launch_ibp_linear(const float* in_a, const float* in_b, int in_mode, int rel
   const void* nptrs[] = {bias, cons_l, cons_u, out_l, out_u, row_dev};
   for (const void* p : nptrs) if (p && (reinterpret_cast<uintptr_t>(p) & 15u)) g.vecN = 0;
   timing_begin(T_IBP_LINEAR, stream);
-  const bool few = (long long)ceil_div(B, IBM) * ceil_div(N, IBN) < 148;  // less than one 64 x 64 tile per SM
-  if (few && K <= IBP_SERIAL_K) {
+  // Above IBP_SERIAL_K one tile per SM: 1000 x 8192 x 300
+  // (80 tiles) 416 us on 32 x 32 tiles, 742 on 64 x 64; 1000 x 4096 x 512 (128) 349 and 320; 2300 x 2048 x 512 (288) 365 and 254.
+  const long long tiles = (long long)ceil_div(B, IBM) * ceil_div(N, IBN);
+  const dim3 grid(ceil_div(B, IBM), ceil_div(N, IBN));
+  int rc = BF_OK;
+  if (K <= IBP_SERIAL_K) {
     const int gx = ceil_div(B, QM);
-    if ((long long)gx * ceil_div(N, 32) < 148) ibp_linear_small_kernel<1><<<dim3(gx, ceil_div(N, 16)), 256, 0, stream>>>(g);
+    if (tiles >= 148) ibp_linear_kernel<false><<<grid, 256, 0, stream>>>(g, 0);
+    else if ((long long)gx * ceil_div(N, 32) < 148) ibp_linear_small_kernel<1><<<dim3(gx, ceil_div(N, 16)), 256, 0, stream>>>(g);
     else ibp_linear_small_kernel<2><<<dim3(gx, ceil_div(N, 32)), 256, 0, stream>>>(g);
-  } else if (few) {
-    const long long tiles = (long long)ceil_div(B, STM) * ceil_div(N, STN);
-    const int slabs = ceil_div(K, SBK);
-    int ks = 1;
-    while (ks < 8 && tiles * ks < 148 && slabs >= 2 * ks) ks *= 2;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ceil_div(B, STM), ceil_div(N, STN), ks);
-    cfg.blockDim = dim3(256);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = ks;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, ibp_linear_split_kernel, g, ceil_div(slabs, ks) * SBK);
   } else {
-    ibp_linear_kernel<<<dim3(ceil_div(B, IBM), ceil_div(N, IBN)), 256, 0, stream>>>(g);
+    const int chain = ibp_segment(K) / (IBP_CHAINS * IBK);
+    if (tiles < 148) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(ceil_div(B, STM), ceil_div(N, STN), ibp_segments(K));
+      cfg.blockDim = dim3(256);
+      cfg.stream = stream;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = ibp_segments(K);
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      cudaLaunchKernelEx(&cfg, ibp_linear_chains_kernel, g, chain);
+    } else {
+      constexpr int bytes = 32 * 256 * sizeof(float);
+      static SmemOptIn opt_in;
+      rc = ensure_dynamic_smem(ibp_linear_kernel<true>, bytes, opt_in, "ibp_linear_kernel");
+      if (rc == BF_OK) ibp_linear_kernel<true><<<grid, 256, bytes, stream>>>(g, chain);
+    }
   }
   // weights and bias once, the input interval once, both output bounds once (+ the split bytes)
   timing_end(T_IBP_LINEAR, stream, 4.0 * ((double)K * N + N) + 8.0 * (double)B * (K + N) + (split ? (double)B * N : 0.0),
              4.0 * (double)B * K * N);
+  if (rc != BF_OK) return rc;
   BF_CHECK_LAUNCH("ibp_linear_kernel");
   return BF_OK;
 }

@@ -140,3 +140,26 @@ def test_conv_backward_tensor_cores(dev, B, S, Ci, H, W, Co, k, s, p, side, relu
     tol_d = (2 * Co * Ho * Wo + 8) * 2.0 ** -24 * (2.0 + (icpt.abs() + (lam * b.double()[:, None, None]).abs()).sum((2, 3, 4)))
     assert ((out.double() - ref).abs() <= tol).all()
     assert ((delta.double() - ref_d).abs() <= tol_d).all()
+
+
+# an input's interval bounds are the same bits in every batch: all kernels behind one layer sum in one order (also above 1024 terms)
+@pytest.mark.parametrize("K,N", [(700, 33), (1025, 1), (1568, 100), (4096, 65)])
+def test_ibp_linear_bits_do_not_depend_on_the_batch(dev, K, N):
+    from boundflow_b200 import _lib
+
+    lib = _lib.load()
+    g = torch.Generator("cuda").manual_seed(K + N)
+    most = 148 * 64  # a 64 x 64 tile per SM
+    l = torch.randn(most, K, generator=g, device=dev)
+    u = l + torch.rand(most, K, generator=g, device=dev)
+    W = torch.randn(N, K, generator=g, device=dev)
+
+    def bounds(rows):
+        out = [torch.full((rows, N), float("nan"), device=dev) for _ in range(2)]
+        _lib.check(lib.bf_ibp_linear(l.data_ptr(), u.data_ptr(), _lib.IN_LOWER_UPPER, 1, W.data_ptr(), None, None, 0, None, None, out[0].data_ptr(),
+                                     out[1].data_ptr(), None, rows, K, N, None))
+        return torch.stack(out)
+
+    whole = bounds(most)
+    for rows in (1, 17, 200):
+        assert torch.equal(bounds(rows), whole[:, :rows])
