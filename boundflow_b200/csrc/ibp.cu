@@ -435,14 +435,15 @@ int launch_ibp_linear(const float* in_a, const float* in_b, int in_mode, int rel
   const void* nptrs[] = {bias, cons_l, cons_u, out_l, out_u, row_dev};
   for (const void* p : nptrs) if (p && (reinterpret_cast<uintptr_t>(p) & 15u)) g.vecN = 0;
   timing_begin(T_IBP_LINEAR, stream);
-  // Above IBP_SERIAL_K one tile per SM: 1000 x 8192 x 300
+  // Measured around the lines (64 x 64 tiles; K = 100 to 1024): the small kernel takes 0.8 of the other's time at 64 tiles, 1.2 at
+  // 95 (512 wide: 35 and 50 against 44 us).  Above IBP_SERIAL_K one tile per SM: 1000 x 8192 x 300
   // (80 tiles) 416 us on 32 x 32 tiles, 742 on 64 x 64; 1000 x 4096 x 512 (128) 349 and 320; 2300 x 2048 x 512 (288) 365 and 254.
   const long long tiles = (long long)ceil_div(B, IBM) * ceil_div(N, IBN);
   const dim3 grid(ceil_div(B, IBM), ceil_div(N, IBN));
   int rc = BF_OK;
   if (K <= IBP_SERIAL_K) {
     const int gx = ceil_div(B, QM);
-    if (tiles >= 148) ibp_linear_kernel<false><<<grid, 256, 0, stream>>>(g, 0);
+    if (2 * tiles > 148) ibp_linear_kernel<false><<<grid, 256, 0, stream>>>(g, 0);
     else if ((long long)gx * ceil_div(N, 32) < 148) ibp_linear_small_kernel<1><<<dim3(gx, ceil_div(N, 16)), 256, 0, stream>>>(g);
     else ibp_linear_small_kernel<2><<<dim3(gx, ceil_div(N, 32)), 256, 0, stream>>>(g);
   } else {
