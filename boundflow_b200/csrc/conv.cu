@@ -26,14 +26,15 @@ struct IbpConvArgs {
 // A CTA computes TN output channels x TM = 4096 / TN output pixels (pixels of all images in one line), a thread 4 x 4 of them,
 // over slabs of CBK input taps in (channel, kernel row, kernel column) order.  The gather positions of a slab's taps are
 // decoded once per CTA into `tab`, two slabs ahead.  INTERVAL: centre and radius accumulators; otherwise one convolution of
-// plain rows (in_a).  A sum runs over its taps in ascending order; only above CONV_SERIAL_K taps a small grid splits K over a
-// cluster of two or four CTAs, whose partial sums meet in distributed shared memory in rank order.  (Splitting shorter sums
-// too was 10-20 us faster per layer at 16 images, but a pre-activation bound within an ulp of zero then changes sides
+// plain rows (in_a).  A sum runs over its taps in ascending order; above CONV_SERIAL_K taps it is cut in four, whatever the
+// batch (so that an image's bounds are the same bits in every one), and a cluster of four CTAs takes the parts, which meet in
+// distributed shared memory in rank order: 16 images, 128 -> 128 channels, 3x3 on 8 x 8: 31 us, in one part 113.  (Cutting shorter
+// sums too was 10-20 us faster per layer at 16 images, but a pre-activation bound within an ulp of zero then changes sides
 // against the serial sum and takes the relaxation of its ReLU with it.)
 // Bound by FFMA issue and the slab's shared-memory reads (three 128-bit reads for 32 FMAs): 200 images, 32 -> 32 channels, 4x4 / 2
 // kernel on 32 x 32: 138 us = 24 TFLOP/s (one thread per output, weights and pixels read through L1 for every tap, before: 1.1 ms);
 // plain rows, 432 x 16 x 14 x 14 -> 32, 4x4 / 2: 32 us (164).
-constexpr int CONV_SERIAL_K = 1024;
+constexpr int CONV_SERIAL_K = 1024, CONV_PARTS = 4;
 
 template <int TN>
 struct ConvTile {
@@ -189,7 +190,7 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
   }
 
   const int ranks = gridDim.z;
-  if (ranks > 1) {
+  if (ranks > 1) {  // four: rank z finishes channel z of every thread
     const int at = ty * 4 * TM + tx * 4;  // part[acc][channel][pixel]
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -301,8 +302,7 @@ static int launch_conv_tile_n(const IbpConvArgs& g, int vec, cudaStream_t stream
   const long long tiles = (npix + ConvTile<TN>::TM - 1) / ConvTile<TN>::TM;
   const int K = g.Ci * g.kh * g.kw, slabs = ceil_div(K, ConvTile<TN>::SLAB), ctas_y = ceil_div(g.Co, TN);
   BF_REQUIRE(ctas_y <= 65535 && tiles <= 2147483647LL, BF_E_UNSUPPORTED, "conv2d: too many output channels or pixels");
-  int ks = 1;
-  while (K > CONV_SERIAL_K && ks < 4 && tiles * ctas_y * ks < 148 && slabs >= 4 * ks) ks *= 2;
+  const int ks = K > CONV_SERIAL_K ? CONV_PARTS : 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)tiles, ctas_y, ks);
   cfg.blockDim = dim3(256);

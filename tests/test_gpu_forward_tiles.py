@@ -163,3 +163,35 @@ def test_ibp_linear_bits_do_not_depend_on_the_batch(dev, K, N):
     whole = bounds(most)
     for rows in (1, 17, 200):
         assert torch.equal(bounds(rows), whole[:, :rows])
+
+
+# the same of convolutions, of intervals and of plain rows; all three channel-tile widths above 1024 terms, ragged pixels, several images in a tile
+@pytest.mark.parametrize("Ci,H,W,Co,k,s,p", [(65, 7, 6, 16, 4, 1, 1), (130, 5, 9, 30, 3, 2, 1), (65, 9, 9, 70, 4, 2, 0), (12, 9, 8, 17, 3, 1, 1)])
+def test_forward_conv_bits_do_not_depend_on_the_batch(dev, Ci, H, W, Co, k, s, p):
+    from boundflow_b200 import _lib
+
+    lib = _lib.load()
+    Ho, Wo = (H + 2 * p - k) // s + 1, (W + 2 * p - k) // s + 1
+    g = torch.Generator("cuda").manual_seed(Ci + Co)
+    most = 2000
+    x = torch.randn(most, Ci, H, W, generator=g, device=dev)
+    r = torch.rand(most, Ci, H, W, generator=g, device=dev)
+    w = torch.randn(Co, Ci, k, k, generator=g, device=dev)
+    b = torch.randn(Co, generator=g, device=dev)
+
+    def run(B):
+        lo, up, y = (torch.full((B, Co, Ho, Wo), float("nan"), device=dev) for _ in range(3))
+        _lib.check(lib.bf_ibp_conv2d(x.data_ptr(), r.data_ptr(), _lib.IN_MID_RAD, 0, w.data_ptr(), b.data_ptr(), None, 0, None, None, lo.data_ptr(), up.data_ptr(),
+                                     None, B, Ci, H, W, Co, k, k, s, s, p, p, None))
+        _lib.check(lib.bf_rows_conv2d_fwd(x.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), B, Ci, H, W, Co, Ho, Wo, k, k, s, s, p, p, None))
+        return lo, up, y
+
+    whole = run(most)
+    for B in (1, 7):
+        assert all(torch.equal(part, full[:B]) for part, full in zip(run(B), whole))
+    # against float64: n products and sums, in any order
+    conv = lambda a, ww: torch.nn.functional.conv2d(a[:7].double(), ww.double(), None, s, p)
+    tol = (Ci * k * k + 4) * 2.0**-24 * (conv(x.abs(), w.abs()) + conv(r, w.abs())) + 1e-6
+    bias = b.double()[:, None, None]
+    for got, ref in zip(whole, (conv(x, w) - conv(r, w.abs()), conv(x, w) + conv(r, w.abs()), conv(x, w))):
+        assert ((got[:7].double() - (ref + bias)).abs() <= tol).all()
