@@ -565,9 +565,8 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// RT = 2 (8-pixel segments): a thread owns two image rows that meet the same kernel rows (stride 1: half a block apart, so that
-// the lanes' tile rows stay consecutive and their reads free of bank conflicts), and each weight read feeds twice the multiply-adds.
-// Same order of sums.  Windows of a CIFAR CNN (64 images): 244 -> 240 ms for the whole query.
+// RT = 2 (8-pixel segments): a thread owns two image rows that meet the same kernel rows, and each weight read feeds twice the
+// multiply-adds.  Same order of sums.
 template <int KS, int ST, int PD, int TCI, bool VEC, int TWP, int RT>
 __global__ void __launch_bounds__(256, (TCI > 1 && TWP * RT > 8 ? 2 : 3)) conv_transpose_rowseg_kernel(RowSegArgs a) {
   using G = RowSeg<KS, ST, PD, VEC, TWP>;
@@ -596,8 +595,7 @@ __global__ void __launch_bounds__(256, (TCI > 1 && TWP * RT > 8 ? 2 : 3)) conv_t
   const int seg = threadIdx.x & ((1 << nsegl) - 1);
   const int cig = threadIdx.x >> nsegl;
   const int hrow = seg & ((1 << hrowl) - 1);
-  const int hi = h0 + (RT == 1 || ST == 1 ? hrow : hrow / ST * (2 * ST) + hrow % ST);  // lanes of a warp: consecutive image rows (pairs of rows)
-  const int row_gap = (ST == 1) ? 1 << hrowl : ST;        // image rows between a thread's two rows
+  const int hi = h0 + (RT == 1 ? hrow : hrow / ST * (2 * ST) + hrow % ST);  // lanes of a warp: consecutive image rows (pairs of rows)
   const int colseg = (seg >> hrowl) & (sx - 1);
   const int mr = seg >> (a.sxl + hrowl);
   const int ho_lo = h0 / ST - G::C0;
@@ -698,7 +696,7 @@ __global__ void __launch_bounds__(256, (TCI > 1 && TWP * RT > 8 ? 2 : 3)) conv_t
           }
 #pragma unroll
           for (int rt = 0; rt < RT; ++rt) {
-            const float4* lp = reinterpret_cast<const float4*>(lam_co + (rt * (row_gap / ST) - jr) * NLT);
+            const float4* lp = reinterpret_cast<const float4*>(lam_co + (rt - jr) * NLT);
             float L[G::NL];
 #pragma unroll
             for (int q = G::Q0; q < G::NL / 4; ++q) {
@@ -725,12 +723,12 @@ __global__ void __launch_bounds__(256, (TCI > 1 && TWP * RT > 8 ? 2 : 3)) conv_t
   const int wleft = g.Wi - (w0 + colseg * G::TW);
 #pragma unroll
   for (int rt = 0; rt < RT; ++rt) {
-    if (hi + rt * row_gap >= g.Hi) break;
+    if (hi + rt * ST >= g.Hi) break;
 #pragma unroll
     for (int c = 0; c < TCI; ++c) {
       const int ci = ci0 + cig * TCI + c;
       if (ci >= g.Ci) break;
-      float* op = g.out + (((size_t)(m0 + mr) * g.Ci + ci) * g.Hi + hi + rt * row_gap) * g.Wi + w0 + colseg * G::TW;
+      float* op = g.out + (((size_t)(m0 + mr) * g.Ci + ci) * g.Hi + hi + rt * ST) * g.Wi + w0 + colseg * G::TW;
       if (wleft >= G::TW && (reinterpret_cast<uintptr_t>(op) & 15u) == 0) {
 #pragma unroll
         for (int q = 0; q < G::TW / 4; ++q)
@@ -799,7 +797,13 @@ static int launch_rowseg(const ConvTArgs& g, cudaStream_t stream) {
   if (g.Ci <= 2) return vec ? launch_rowseg_tci<KS, ST, PD, 1, true, 16>(g, stream) : launch_rowseg_tci<KS, ST, PD, 1, false, 16>(g, stream);
   // 8-pixel segments when they waste fewer lanes than 16-pixel ones (narrow windows of the windowed sweeps)
   const bool narrow = ((g.Wi + 7) / 8) * 8 < ((g.Wi + 15) / 16) * 16;
-  if (narrow && g.Hi >= 2 * ST) return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 8, 2>(g, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 8, 2>(g, stream);
+  if constexpr (KS == 4) {
+    // Two image rows per thread, measured against one over seven kernels, 8 to 64 channels and 4 to 24 rows: faster for 4x4 / 2
+    // kernels on five to eight rows from 24 -> 32 channels on (1.03 to 1.18 of the speed), elsewhere mostly slower (4x4 / 2 on 17 to
+    // 24 rows 0.90 to 0.98, 3x3 / 1 0.66 to 1.02, 5x5 / 1 0.8 to 1.05), and with few channels its tile can outgrow shared memory.
+    if (narrow && g.Ci >= 24 && g.Co >= 32 && g.Hi >= 5 && g.Hi <= 8)
+      return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 8, 2>(g, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 8, 2>(g, stream);
+  }
   if (narrow) return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 8>(g, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 8>(g, stream);
   return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 16>(g, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 16>(g, stream);
 }
