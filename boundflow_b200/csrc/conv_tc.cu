@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __grid_consta
 }
 
 static bool make_plan(const ConvTcProblem& c, Plan& p) {
-  if (c.Co > MAX_CO || c.sh * c.sw > 16) return false;
+  if (c.Co > MAX_CO || c.sh * c.sw > 16 || c.ph < 0 || c.pw < 0) return false;  // a negative padding leaves input rows that no position stands for
   p.JY = ceil_div(c.kh, c.sh);
   p.JX = ceil_div(c.kw, c.sw);
   // lines and columns of positions: all outputs, and at least JY - 1 / JX - 1 zero ones behind the plane

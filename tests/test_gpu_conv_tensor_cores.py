@@ -227,3 +227,13 @@ def test_infinite_weight_at_the_border_of_forward_convolutions(dev, B, Ci, H, W,
     _lib.check(lib.bf_ibp_conv2d(x.data_ptr(), (x * 0).data_ptr(), _lib.IN_MID_RAD, 0, w.abs().data_ptr(), None, None, 0, None, None, lo.data_ptr(), up.data_ptr(),
                                  None, B, Ci, H, W, Co, k, k, s, s, p, p, None))
     assert torch.isfinite(lo[~hit]).all() and torch.isfinite(up[~hit]).all()
+
+
+# a negative padding (a cropped input) reaches no output near the border: zeros there, from the FP32 kernels
+def test_negative_padding(dev):
+    B, S, Ci, H, W, Co, k = 8, 64, 16, 16, 17, 24, 3
+    g = torch.Generator("cuda").manual_seed(11)
+    A, w = _rows(dev, "integers", B, S, Co, H - 4, W - 4, Ci, k, g)
+    out, _ = _backward(A, w, 1, -1, H, W)
+    want = torch.nn.functional.pad(_transposed(A.double(), w.double(), 1, 0, H - 2, W - 2), (1, 1, 1, 1))
+    assert torch.equal(out.double(), want)
