@@ -748,8 +748,9 @@ static int ilog2_ceil(int v) {
   return l;
 }
 
+// us: only the time that the launch is expected to take, without its start (nothing is launched)
 template <int KS, int ST, int PD, int TCI, bool VEC, int TWP, int RT = 1>
-static int launch_rowseg_tci(const ConvTArgs& g, cudaStream_t stream) {
+static int launch_rowseg_tci(const ConvTArgs& g, double* us, cudaStream_t stream) {
   using G = RowSeg<KS, ST, PD, VEC, TWP>;
   RowSegArgs a{};
   a.c = g;
@@ -782,19 +783,29 @@ static int launch_rowseg_tci(const ConvTArgs& g, cudaStream_t stream) {
   const size_t lam_words = (size_t)(1 << a.mrl) * cc * G::tile_h(1 << a.thl) * nlt;
   const size_t w_words = ((size_t)cc * KS * (KS * cib + 4) + 3) & ~(size_t)3;
   const size_t smem = 2 * (lam_words + w_words) * sizeof(float) + (size_t)(1 << a.mrl) * cc * G::tile_h(1 << a.thl) * sizeof(int);
-  static SmemOptIn opt_in;
-  if (int rc = ensure_dynamic_smem(conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT>, 110 * 1024, opt_in, "conv_transpose_rowseg_kernel")) return rc;
   dim3 grid(ceil_div(g.M, 1 << a.mrl), a.tiles_x * a.tiles_y, ceil_div(g.Ci, cib));
   if (grid.y > 65535 || grid.z > 65535) return BF_E_UNSUPPORTED;
+  if (us) {
+    // multiply-adds of a block at a rate per kernel shape, and its chunks; blocks share an SM up to its shared memory
+    const double blocks = (double)grid.x * grid.y * grid.z / 148.0;
+    double room = (TCI > 1 && TWP * RT > 8) ? 2 : 3;
+    if (room > 227 * 1024 / (double)(smem + 1024)) room = (double)(int)(227 * 1024 / (smem + 1024));
+    const double waves = blocks > room ? blocks / room : 1.0, side = blocks > room ? room : (blocks > 1.0 ? blocks : 1.0);
+    const double rate = KS == 5 ? 1.17e-3 : (KS == 4 ? 2.4e-3 : (ST == 1 ? 1.67e-3 : 3.3e-3));
+    *us = waves * (side * rate * g.Co * KS * KS * TCI * TWP * RT / (ST * ST) + 0.4 * g.Co / cc) * (TWP == 8 ? 1.35 : 1.0);
+    return BF_OK;
+  }
+  static SmemOptIn opt_in;
+  if (int rc = ensure_dynamic_smem(conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT>, 110 * 1024, opt_in, "conv_transpose_rowseg_kernel")) return rc;
   conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT><<<grid, 256, smem, stream>>>(a);
   BF_CHECK_LAUNCH("conv_transpose_rowseg_kernel");
   return BF_OK;
 }
 
 template <int KS, int ST, int PD>
-static int launch_rowseg(const ConvTArgs& g, cudaStream_t stream) {
+static int launch_rowseg(const ConvTArgs& g, double* us, cudaStream_t stream) {
   const bool vec = (g.Wo % 4 == 0) && ((reinterpret_cast<uintptr_t>(g.Lam) & 15u) == 0);
-  if (g.Ci <= 2) return vec ? launch_rowseg_tci<KS, ST, PD, 1, true, 16>(g, stream) : launch_rowseg_tci<KS, ST, PD, 1, false, 16>(g, stream);
+  if (g.Ci <= 2) return vec ? launch_rowseg_tci<KS, ST, PD, 1, true, 16>(g, us, stream) : launch_rowseg_tci<KS, ST, PD, 1, false, 16>(g, us, stream);
   // 8-pixel segments when they waste fewer lanes than 16-pixel ones (narrow windows of the windowed sweeps)
   const bool narrow = ((g.Wi + 7) / 8) * 8 < ((g.Wi + 15) / 16) * 16;
   if constexpr (KS == 4) {
@@ -802,30 +813,34 @@ static int launch_rowseg(const ConvTArgs& g, cudaStream_t stream) {
     // kernels on five to eight rows from 24 -> 32 channels on (1.03 to 1.18 of the speed), elsewhere mostly slower (4x4 / 2 on 17 to
     // 24 rows 0.90 to 0.98, 3x3 / 1 0.66 to 1.02, 5x5 / 1 0.8 to 1.05), and with few channels its tile can outgrow shared memory.
     if (narrow && g.Ci >= 24 && g.Co >= 32 && g.Hi >= 5 && g.Hi <= 8)
-      return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 8, 2>(g, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 8, 2>(g, stream);
+      return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 8, 2>(g, us, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 8, 2>(g, us, stream);
   }
-  if (narrow) return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 8>(g, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 8>(g, stream);
-  return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 16>(g, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 16>(g, stream);
+  if (narrow) return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 8>(g, us, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 8>(g, us, stream);
+  return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 16>(g, us, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 16>(g, us, stream);
 }
 
 // Row-segment kernel for the geometries it is instantiated for; BF_E_UNSUPPORTED otherwise.
-static int launch_convT_rowseg(const ConvTArgs& g, cudaStream_t stream) {
+static int launch_convT_rowseg(const ConvTArgs& g, double* us, cudaStream_t stream) {
   if (g.kh != g.kw || g.sh != g.sw || g.ph != g.pw) return BF_E_UNSUPPORTED;
-  if (g.kh == 3 && g.sh == 1 && g.ph == 1) return launch_rowseg<3, 1, 1>(g, stream);
-  if (g.kh == 4 && g.sh == 2 && g.ph == 1) return launch_rowseg<4, 2, 1>(g, stream);
-  if (g.kh == 3 && g.sh == 2 && g.ph == 1) return launch_rowseg<3, 2, 1>(g, stream);
+  if (g.kh == 3 && g.sh == 1 && g.ph == 1) return launch_rowseg<3, 1, 1>(g, us, stream);
+  if (g.kh == 4 && g.sh == 2 && g.ph == 1) return launch_rowseg<4, 2, 1>(g, us, stream);
+  if (g.kh == 3 && g.sh == 2 && g.ph == 1) return launch_rowseg<3, 2, 1>(g, us, stream);
   // zero padding: the windowed sweeps below run every transposed convolution in window coordinates
-  if (g.kh == 3 && g.sh == 1 && g.ph == 0) return launch_rowseg<3, 1, 0>(g, stream);
-  if (g.kh == 4 && g.sh == 2 && g.ph == 0) return launch_rowseg<4, 2, 0>(g, stream);
-  if (g.kh == 3 && g.sh == 2 && g.ph == 0) return launch_rowseg<3, 2, 0>(g, stream);
-  if (g.kh == 5 && g.sh == 1 && g.ph == 2) return launch_rowseg<5, 1, 2>(g, stream);
+  if (g.kh == 3 && g.sh == 1 && g.ph == 0) return launch_rowseg<3, 1, 0>(g, us, stream);
+  if (g.kh == 4 && g.sh == 2 && g.ph == 0) return launch_rowseg<4, 2, 0>(g, us, stream);
+  if (g.kh == 3 && g.sh == 2 && g.ph == 0) return launch_rowseg<3, 2, 0>(g, us, stream);
+  if (g.kh == 5 && g.sh == 1 && g.ph == 2) return launch_rowseg<5, 1, 2>(g, us, stream);
   return BF_E_UNSUPPORTED;
 }
 
-// Where full coefficient rows take the tensor-core kernel (conv_tc.cu).  From one 128-position tile per SM on: 512 rows of
-// 64 channels 8 x 8 -> 64 channels 16 x 16, 4x4 / 2 (324 tiles): 90 us against 172; 512 rows of 40 channels 9 x 9, 3x3 / 2: 37
-// against 84.  Not for few input channels (1 or 3 channels fill an eighth of the narrowest MMA: 73 against 42 us, 205 against
-// 91) and not for more than nine taps per phase (5x5 / 1: 128 against 120 us; its MMAs are bound by their issue).
+// Where full coefficient rows take the tensor-core kernel (conv_tc.cu): from one 128-position tile per SM on, and where the
+// expected time (conv_tc_supports) is below that of the ReLU pass and the FP32 kernel.  Of 2791 layers of 148 tiles and more (1x1 to
+// 5x5 kernels, 8 to 256 channels, 7 to 32 pixels) it takes 2211, 33 of them at less than 0.9 of the FP32 speed (worst 0.72), and leaves
+// 44 that would gain 1.3 and more.  (All layers of 148 tiles, 8 channels and up to 9 taps: 266 below 0.9, worst 0.39, namely 8 to 16
+// input channels at stride 1, 8 output channels, and weights of so many blocks that the rows are staged four and eight times.)
+// Kernels without a row-segment form take it unless a staged element feeds few multiply-adds: 1x1 / 1 from 32 -> 32 channels on (0.9 to
+// 1.4 of the gather kernel's speed; 16 -> 32: 0.7 to 1.1), 2x2 / 1 from 8 -> 32 or 16 -> 16 (0.8 to 1.6), strided ones from 12 -> 32 at
+// 1x1 (0.8 to 1.8) and 12 -> 8 at 2x2 (0.8 to 2.0).
 // Rows that bound the neurons of a conv layer stay on the FP32 kernels, as windows and as full rows (Lp balls, windows that
 // have grown to the map), although the tensor cores took a third of their time (64,000 windows, 32 -> 32 channels: 0.33
 // against 1.5 ms): they are millions of values whose last bit differs, and a few of those lie within that bit of zero, where
@@ -868,8 +883,15 @@ static ConvTcProblem conv_tc_geometry(int M, int S, const bf_layer_desc& L) {
 }
 static bool conv_tc_rule(const ConvTcProblem& c, int* slots) {
   int tiles = 0;
-  return c.Ci >= CONV_TC_MIN_CI && ceil_div(c.kh, c.sh) * ceil_div(c.kw, c.sw) <= CONV_TC_MAX_TAPS && conv_tc_supports(c, slots, &tiles) &&
-         tiles >= CONV_TC_MIN_TILES;
+  double tc = 0.0, fp32 = 0.0;
+  const int taps = ceil_div(c.kh, c.sh) * ceil_div(c.kw, c.sw);
+  if (c.Ci < CONV_TC_MIN_CI || taps > CONV_TC_MAX_TAPS || !conv_tc_supports(c, slots, &tiles, &tc) || tiles < CONV_TC_MIN_TILES) return false;
+  ConvTArgs g{nullptr, nullptr, nullptr, c.M, c.Ci, c.Hi, c.Wi, c.Co, c.WH, c.WW, c.kh, c.kw, c.sh, c.sw, c.ph, c.pw, 0};
+  if (launch_convT_rowseg(g, &fp32, nullptr) != BF_OK) {
+    const int npix = c.Hi * c.Wi, idle = npix < 32 ? 32 : npix;  // the gather kernel's threads of a small map
+    return (long long)c.kh * c.kw * c.Ci * (c.Co < 32 ? c.Co : 32) * idle / npix >= (c.sh * c.sw > 1 ? 384 : 1024);
+  }
+  return tc < fp32 + 13.0 + 2.5e-6 * c.M * c.Co * c.WH * c.WW;  // and the ReLU pass
 }
 bool conv_rows_on_tensor_cores(int M, const bf_layer_desc& L) {
   int slots = 0;
@@ -940,7 +962,7 @@ int launch_crown_bwd_conv2d(const float* A, const float* dpos, const float* dneg
   const double conv_bytes = 4.0 * (double)M * (L.n_out + L.n_in) + 4.0 * (double)L.Co * L.Ci * L.kh * L.kw;
   const double conv_flops = 2.0 * (double)M * L.n_out * L.Ci * L.kh * L.kw;
   timing_begin(T_CONV_T, stream);
-  int rc = gather_only ? BF_E_UNSUPPORTED : launch_convT_rowseg(g, stream);
+  int rc = gather_only ? BF_E_UNSUPPORTED : launch_convT_rowseg(g, nullptr, stream);
   if (rc == BF_E_UNSUPPORTED) {
     if (L.Ci <= 4) rc = launch_convT<4>(g, stream);
     else if (L.Ci <= 16) rc = launch_convT<16>(g, stream);

@@ -688,11 +688,19 @@ static bool make_plan(const ConvTcProblem& c, Plan& p) {
 
 }  // namespace ctc
 
-bool conv_tc_supports(const ConvTcProblem& c, int* slots, int* tiles) {
+bool conv_tc_supports(const ConvTcProblem& c, int* slots, int* tiles, double* us) {
   ctc::Plan p{};
   if (!ctc::make_plan(c, p)) return false;
   *slots = p.slots;
   *tiles = p.tiles;
+  // launch and set-up, splitting the weights, and per tile of a CTA: hand-over, staging (two passes where the halo takes all
+  // producers), read-back, MMAs.  Fitted to 3279 layers (1x1 to 7x7 kernels, 8 to 256 channels, 7 to 32 pixels, 160 to 2400
+  // tiles): 7 % from the measured time in the 2-norm, 15 % at the 95th percentile.
+  const int per = p.tiles < 148 / p.nblk ? p.tiles : 148 / p.nblk;
+  const double split = 1.0 * p.JY * p.JX * p.cpad / 8 * p.NB / ctc::THREADS;
+  const double stage = 1.25 * p.cpad / ctc::KC * (p.groups == 2 ? 1 : 2), read = 0.207 * p.NB / ctc::W;
+  const double mma = p.units * ((p.merged ? 0.012 : 0.008) + 0.00133 * p.NB);
+  *us = 14.2 + split + ceil_div(p.tiles, per) * (0.91 + stage + read + mma);
   return true;
 }
 

@@ -15,8 +15,9 @@ struct ConvTcProblem {
   int M, S, Co, Ci, WH, WW, Hi, Wi, kh, kw, sh, sw, ph, pw;
 };
 
-// false: this geometry stays on the FP32 kernels.  slots: partial sums per row, tiles: 128-position tiles of the problem.
-bool conv_tc_supports(const ConvTcProblem& c, int* slots, int* tiles);
+// false: this geometry stays on the FP32 kernels.  slots: partial sums per row, tiles: 128-position tiles of the problem,
+// us: the time the kernel is expected to take.
+bool conv_tc_supports(const ConvTcProblem& c, int* slots, int* tiles, double* us);
 int launch_conv_tc(const ConvTcProblem& c, cudaStream_t stream);
 
 }  // namespace bf

@@ -61,7 +61,7 @@ def _rows(dev, kind, B, S, Co, Ho, Wo, Ci, k, g):
 
 
 # accumulators of one and several parts, one and two tiles in tensor memory, several blocks of input channels, channels that end inside a stage
-GEOMETRIES = [(8, 64, 8, 16, 16, 16, 3, 1, 1), (8, 64, 32, 32, 32, 32, 4, 2, 1), (8, 64, 32, 16, 16, 64, 3, 1, 1), (16, 100, 16, 14, 14, 32, 4, 2, 1),
+GEOMETRIES = [(8, 40, 8, 9, 9, 16, 3, 1, 1), (8, 64, 32, 32, 32, 32, 4, 2, 1), (8, 64, 32, 16, 16, 64, 3, 1, 1), (16, 100, 16, 14, 14, 32, 4, 2, 1),
               (8, 64, 16, 17, 17, 40, 3, 2, 1), (8, 60, 24, 13, 13, 20, 3, 1, 1), (4, 64, 64, 16, 16, 200, 2, 1, 0)]
 
 
@@ -237,3 +237,17 @@ def test_negative_padding(dev):
     out, _ = _backward(A, w, 1, -1, H, W)
     want = torch.nn.functional.pad(_transposed(A.double(), w.double(), 1, 0, H - 2, W - 2), (1, 1, 1, 1))
     assert torch.equal(out.double(), want)
+
+
+# the dispatch's two sides: layers that were measured faster on the tensor cores, and slower
+@pytest.mark.parametrize("M,Ci,H,Co,k,s,p,takes", [(512, 32, 32, 32, 4, 2, 1, 1), (512, 32, 16, 64, 3, 1, 1, 1), (512, 32, 8, 64, 2, 1, 0, 1), (40, 32, 8, 64, 3, 1, 1, 0),
+                                                   (945, 8, 16, 16, 3, 1, 1, 0), (261, 16, 32, 16, 3, 1, 1, 0), (261, 128, 32, 128, 3, 1, 1, 0), (1197, 8, 16, 16, 1, 1, 0, 0),
+                                                   (1062, 8, 32, 8, 4, 2, 1, 0), (512, 4, 32, 32, 4, 2, 1, 0), (300, 16, 16, 32, 5, 1, 2, 0)])
+def test_dispatch(dev, M, Ci, H, Co, k, s, p, takes):
+    Ho = (H + 2 * p - k) // s + 1
+    g = torch.Generator("cuda").manual_seed(12)
+    A, w = _rows(dev, "integers", M, 1, Co, Ho, Ho, Ci, k, g)
+    out, launches = _backward(A, w, s, p, H, H)
+    assert launches == takes
+    # whole numbers below 2^24: both kernels are exact
+    assert torch.equal(out[:16].double(), _transposed(A[:16].double(), w.double(), s, p, H, H))
