@@ -251,3 +251,71 @@ def test_dispatch(dev, M, Ci, H, Co, k, s, p, takes):
     assert launches == takes
     # whole numbers below 2^24: both kernels are exact
     assert torch.equal(out[:16].double(), _transposed(A[:16].double(), w.double(), s, p, H, H))
+
+
+# kernels of one tap and of unequal sides, strides and paddings; with and without bias, row sums, a value to add them to, slopes
+@pytest.mark.parametrize("B,S,Ci,H,W,Co,k,s,p", [(8, 40, 48, 12, 13, 24, (1, 1), (1, 1), (0, 0)), (8, 40, 16, 15, 14, 32, (3, 2), (2, 1), (1, 0)),
+                                                 (8, 40, 32, 14, 15, 20, (2, 3), (1, 2), (0, 1)), (6, 50, 16, 16, 16, 32, (2, 2), (2, 2), (0, 0))])
+@pytest.mark.parametrize("relu,bias,sums,accumulate", [(True, True, True, 0), (False, True, True, 0), (True, False, True, 1), (True, False, True, 0),
+                                                       (False, False, True, 0), (False, False, True, 1), (True, True, False, 1)])
+def test_forms_of_the_call(dev, B, S, Ci, H, W, Co, k, s, p, relu, bias, sums, accumulate):
+    Ho, Wo = (H + 2 * p[0] - k[0]) // s[0] + 1, (W + 2 * p[1] - k[1]) // s[1] + 1
+    g = torch.Generator("cuda").manual_seed(9)
+    A, w = _rows(dev, "dense", B, S, Co, Ho, Wo, Ci, k, g)
+    b = torch.randn(Co, generator=g, device=dev) if bias else None
+    slopes = tuple(torch.rand(B, Co, Ho, Wo, generator=g, device=dev) for _ in range(3)) if relu else None
+    delta = torch.full((B, S), 2.0, device=dev) if sums else None
+    out, launches = _backward(A, w, s, p, H, W, b=b, slopes=slopes, side=1, delta=delta, accumulate=accumulate)
+    assert launches == 1
+    lam, icpt = A.double(), torch.zeros_like(A, dtype=torch.float64)
+    if relu:
+        au, al, bu = (t.double()[:, None] for t in slopes)
+        icpt = torch.where(A >= 0, lam * bu, icpt)
+        lam = lam * torch.where(A >= 0, au, al)
+    # operands are exact; the sums keep the bound of an FP32 sum of Co k^2 / s^2 products
+    tol = (Co * k[0] * k[1] / (s[0] * s[1]) + 8) * 2.0**-24 * _transposed(lam.abs(), w.double().abs(), s, p, H, W) + 1e-6
+    assert ((out.double() - _transposed(lam, w.double(), s, p, H, W)).abs() <= tol).all()
+    if sums:
+        term = lam * (b.double()[:, None, None] if bias else 0.0)
+        start = 2.0 if accumulate else 0.0
+        tol = (2 * Co * Ho * Wo + 8) * 2.0**-24 * (start + (icpt.abs() + term.abs()).sum((2, 3, 4)))
+        assert ((delta.double() - (start + (icpt + term).sum((2, 3, 4)))).abs() <= tol).all()
+
+
+# the term behind a conv ReLU (beta-CROWN's splits enter there) in the tensor-core kernel, against float64
+def test_term_behind_a_conv_relu(dev):
+    from boundflow_b200 import _lib
+    from boundflow_b200.crown import crown_from_trace, ibp_trace
+
+    g = torch.Generator("cuda").manual_seed(10)
+    module = _network(dev, (3, 32, 32), [(16, 3, 1, 1), (32, 3, 1, 1)], [10], g)
+    trace = ibp_trace(module, _box(torch.rand(4, 3, 32, 32, generator=g, device=dev), 0.01))
+    C = torch.randn(4, 9, 10, generator=g, device=dev)
+    add = torch.randn(4, 32 * 32 * 32, generator=g, device=dev)
+    before = _lib.tc_launch_count()
+    got, _ = crown_from_trace(trace, C, sides=(_lib.SIDE_LOWER,), relu_pre_add_coeff_l={"h1": add})
+    assert _lib.tc_launch_count() == before + 1
+    P = {n: t.double() for n, t in module.bindings["params"].items()}
+
+    def relu_back(A, r):
+        l, u = trace.pre_l[r].double()[:, None], trace.pre_u[r].double()[:, None]
+        off, on = u <= 0, l >= 0
+        up = torch.where(off, 0.0, torch.where(on, 1.0, u / (u - l)))
+        shift = torch.where(off | on, 0.0, -u * l / (u - l))
+        low = on.double()
+        return torch.where(A >= 0, A * low, A * up), torch.where(A >= 0, 0.0, A * shift).sum(-1)
+
+    def conv_back(A, name, co):
+        return torch.nn.functional.conv_transpose2d(A.view(36, co, 32, 32), P["W" + name], None, 1, 1).view(4, 9, -1), A.view(4, 9, co, -1).sum(-1) @ P["b" + name]
+
+    def bound(add, A=C.double()):
+        A, c = A @ P["W2"], A @ P["b2"]
+        A, d = relu_back(A, 1)
+        A, e = conv_back(A + add, "1", 32)
+        A, f = relu_back(A, 0)
+        A, h = conv_back(A, "0", 16)
+        return c + d + e + f + h + (A * trace.mid.double()[:, None]).sum(-1) - (A.abs() * trace.rad.double()[:, None]).sum(-1)
+
+    want = bound(add.double()[:, None])
+    # three layers of float32 sums: 2-norm error of a few 2^-24, against a term that is most of the bound
+    assert (got.double() - want).norm() <= 64 * 2.0**-24 * want.norm() <= 1e-3 * (bound(0.0) - want).norm()

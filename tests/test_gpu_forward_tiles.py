@@ -45,7 +45,7 @@ def test_ibp_linear_tiles(dev, B, K, N):
     assert torch.equal(bad[sure].bool(), (lo > up).any(dim=1)[sure])
 
 
-# channel tiles of 16, 32 and 64, ragged pixels and channels, kernels larger than a slab, clusters of 1, 2 and 4 CTAs along K
+# channel tiles of 16, 32 and 64, ragged pixels and channels, kernels larger than a slab (clusters along K: below, above 1024 taps)
 @pytest.mark.parametrize("B,Ci,H,W,Co,k,s,p", [(1, 1, 5, 7, 1, 1, 1, 0), (3, 1, 28, 28, 16, 4, 2, 1), (2, 3, 9, 11, 17, 3, 1, 1), (5, 16, 14, 14, 33, 4, 2, 1),
                                                (64, 8, 16, 16, 32, 3, 2, 1), (300, 3, 16, 15, 20, 5, 1, 2), (7, 64, 8, 8, 70, 4, 2, 1), (40, 40, 13, 13, 64, 3, 1, 0)])
 def test_ibp_conv_tiles(dev, B, Ci, H, W, Co, k, s, p):
@@ -135,7 +135,7 @@ def test_conv_backward_tensor_cores(dev, B, S, Ci, H, W, Co, k, s, p, side, relu
     conv_t = lambda x, ww: torch.nn.functional.conv_transpose2d(x.flatten(0, 1), ww, None, s, p, output_padding=opad).view(out.shape)
     ref = conv_t(lam, w.double())
     ref_d = 2.0 + (icpt + lam * b.double()[:, None, None]).sum((2, 3, 4))
-    # operands are exact to 2^-23 each; the sums keep the bound of an FP32 sum of Co k^2 / s^2 products
+    # operands are exact; the sums keep the bound of an FP32 sum of Co k^2 / s^2 products
     tol = (Co * (k * k) / (s * s) + 8) * 2.0 ** -24 * conv_t(lam.abs(), w.double().abs()) + 1e-6
     tol_d = (2 * Co * Ho * Wo + 8) * 2.0 ** -24 * (2.0 + (icpt.abs() + (lam * b.double()[:, None, None]).abs()).sum((2, 3, 4)))
     assert ((out.double() - ref).abs() <= tol).all()
