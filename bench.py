@@ -349,7 +349,7 @@ def kernel_rooflines(dev, peaks):
         ol, ou = torch.empty(Bq, Co * Ho * Ho, device=dev), torch.empty(Bq, Co * Ho * Ho, device=dev)
         s = timed(lambda: _lib.check(lib.bf_ibp_conv2d(lo.data_ptr(), up.data_ptr(), _lib.IN_LOWER_UPPER, 0, Wc.data_ptr(), bc.data_ptr(), None, 0, None, None,
                                                        ol.data_ptr(), ou.data_ptr(), None, Bq, Ci, Hi, Hi, Co, k, k, stv, stv, pd, pd, st)), 10, True)
-        out[f"ibp_conv2d_kernel_{tag}"] = hbm_roofline("ibp_conv2d_kernel", s["ibp_conv2d_kernel"], peaks, "L2 flushed between launches")
+        out[f"conv_tile_kernel_{tag}"] = hbm_roofline("conv_tile_kernel", s["conv_tile_kernel"], peaks, "L2 flushed between launches")
     return out
 
 
@@ -704,7 +704,7 @@ def main():
         },
         # HBM-bound kernels: inside the timed c4 step (live event pairs), and single kernels at the configurations' sizes
         "roofline_hbm": {
-            "in_step": {n: hbm_roofline(n, slots[n], peaks) for n in ("crown_bwd_thin_kernel", "adam_step_kernel", "ibp_linear_kernel") if n in slots},
+            "in_step": {n: hbm_roofline(n, slots[n], peaks) for n in ("crown_bwd_thin_kernel", "optimiser_step_kernel", "ibp_linear_kernel") if n in slots},
             "single_kernels": kernels,
         },
         "kernel_share_of_step": {n: r["ms"] / ms_res for n, r in slots.items()},

@@ -70,8 +70,8 @@ void timing_end(int slot, cudaStream_t stream, double bytes, double flops) {
 }
 
 static const char* const g_timing_names[T_SLOTS] = {
-    "crown_bwd_contraction", "crown_adjoint_contraction", "crown_bwd_thin_kernel", "ibp_linear_kernel", "ibp_conv2d_kernel",
-    "adam_step_kernel", "concretize_kernel", "relu_bwd_window_kernel", "conv_transpose_kernel", "relu_bwd_rows_kernel"};
+    "crown_bwd_contraction", "crown_adjoint_contraction", "crown_bwd_thin_kernel", "ibp_linear_kernel", "conv_tile_kernel",
+    "optimiser_step_kernel", "concretize_kernel", "relu_bwd_window_kernel", "conv_transpose_kernel", "relu_bwd_rows_kernel"};
 
 }  // namespace bf
 

@@ -251,8 +251,8 @@ __device__ __forceinline__ void gemm_mainloop(const GemmArgs& g, const int m0, c
 }
 
 // Main loop for 32 x 64 tiles (2 x 4 outputs per thread, rows / columns as tile_row<0> and tile_col) with 64-deep slabs: a
-// problem with less than one 128 x 128 tile per SM is bound by the latency of its slabs, so a quarter of them, with six to
-// fourteen 128-bit loads of a thread in flight, takes a quarter of the time.  Every sum runs over k in ascending order as
+// problem with less than one 64 x 64 tile per SM is bound by the latency of its slabs, so it takes a quarter of them, with six to
+// fourteen 128-bit loads of a thread in flight (1152 x 256 x 256: 20 -> 14 us).  Every sum runs over k in ascending order as
 // above.  Row sums are left to prologue_row_sums (CTAs of their own).  On alpha-CROWN loops with ten specs, against 16-deep slabs:
 // 128 inputs, five 256-wide layers, 20 steps 5.64 -> 5.06 ms; 37 nodes, four 512-wide layers, 10 steps 3.69 -> 3.29 ms.
 // Transposed operands are XOR-swizzled in groups of four rows / columns: stores conflict two-way, reads not at all.
