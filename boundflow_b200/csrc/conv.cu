@@ -31,7 +31,8 @@ struct IbpConvArgs {
 // distributed shared memory in rank order: 16 images, 128 -> 128 channels, 3x3 on 8 x 8: 31 us, in one part 113.  (Cutting shorter
 // sums too was 10-20 us faster per layer at 16 images, but a pre-activation bound within an ulp of zero then changes sides
 // against the serial sum and takes the relaxation of its ReLU with it.)
-// Bound by FFMA issue and the slab's shared-memory reads (three 128-bit reads for 32 FMAs): 200 images, 32 -> 32 channels, 4x4 / 2
+// Bound by FFMA issue and the slab's shared-memory reads (three 128-bit reads for 32 FMAs; issue slots 66 %, shared memory 51 %, FMA
+// pipe 44 % busy): 200 images, 32 -> 32 channels, 4x4 / 2
 // kernel on 32 x 32: 138 us = 24 TFLOP/s (one thread per output, weights and pixels read through L1 for every tap, before: 1.1 ms);
 // plain rows, 432 x 16 x 14 x 14 -> 32, 4x4 / 2: 32 us (164).
 constexpr int CONV_SERIAL_K = 1024, CONV_PARTS = 4;

@@ -19,7 +19,9 @@
 // row with one non-zero coefficient 1 gives the weights back exactly.
 // Error against float64 (2-norm, random rows): 7e-8 and 1.3e-7 for the two layers below, the FP32 kernels' 2.0e-7 and 4.2e-7.
 // 512 rows without a ReLU, 32 -> 32 channels, 16 x 16 -> 32 x 32, 4x4 / 2: 59 us (FP32 kernel 161); 64 -> 32 channels 16 x 16,
-// 3x3: 71 us (143).  (Two TF32 parts a value, which leave a remainder, and twice as many steps: 63 and 91 us, 2.0e-7 and 4.9e-7.)
+// 3x3: 71 us (143); with one 70 and 89 us (ReLU pass and FP32 kernel 170 and 153).  (Two TF32 parts a value, which leave a remainder,
+// and twice as many steps: 63 and 91 us without a ReLU, 2.0e-7 and 4.9e-7.)  Bound by the instructions of its producers and of the
+// read-back: issue slots 56 and 65 % busy at 31 % of the warps, tensor pipe 23 and 34 %, DRAM 11 and 6 %.
 // Warps 0-10 stage A, 11-18 read the accumulators back, 19 issues the MMAs.  Every wait is bounded; on expiry the CTA
 // writes NaN to all rows it owns and to their sums, so that no bound can be taken from them, and raises the status word.
 #include <float.h>

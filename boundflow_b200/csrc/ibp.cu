@@ -310,6 +310,7 @@ __global__ void __launch_bounds__(256) ibp_linear_small_kernel(IbpArgs g) {
 // columns of every chain per slab (six 128-bit loads in flight per thread); the CTAs of a cluster take the segments, whose sums
 // meet in distributed shared memory in rank order, without a workspace or atomics.  Measured, against one chain on 64 x 64
 // tiles: 200 x 4096 x 512: 91 us (320), 256 x 1568 x 100: 17 (124), 16 x 8192 x 10: 27 (541), 600 x 6144 x 249: 162 (476).
+// Issue slots 61 %, shared memory 40 %, FMA pipe 38 % busy on the first.
 // Shared slabs are [k][row] with rows XOR-ed by ((k >> 2) & 7) << 2: transposed stores conflict two-way, 128-bit reads not at all.
 constexpr int STM = 32, STN = 32, SBK = 64, SSLAB = SBK * 32, SGROUPS = IBP_CHAINS, SCOLS = SBK / SGROUPS;
 __device__ __forceinline__ int swz(int k, int row) { return k * 32 + (row ^ (((k >> 2) & 7) << 2)); }
