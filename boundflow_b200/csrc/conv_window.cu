@@ -1,0 +1,249 @@
+// Transposed convolution of narrow windows of coefficient rows (the identity-row sweeps on conv layers): no padding, square
+// windows, kernels and strides, lanes = coefficient rows.
+#include "common.cuh"
+#include "kernels.cuh"
+
+namespace bf {
+
+// A row's window is WW x WW pixels of Co channels, its result OW x OW pixels (OW = (WW - 1) * ST + KS) of Ci channels.  Every
+// row has the same geometry, so a warp takes 32 rows, a lane one of them: the window values are 16-byte words per lane, the
+// weights are the same for the whole warp, and every tap that exists is a compile-time index, so no work is done for the zeros
+// around a window (gathered from a padded tile, 3 x 3 -> 8 x 8 pixels of a 4x4 / 2 kernel is 256 multiply-adds per channel pair
+// for 144 that exist).  A thread holds a band of TH image rows of TCI input channels (up to 72 sums, so that 16 warps share an SM):
+// per output channel it reads its KS * KS * TCI weights once and its part of the window row by row, about one shared-memory word
+// per six multiply-adds.  Window rows come in descending, kernel columns in ascending order: for each sum that is channel,
+// kernel row, kernel column ascending, the order of conv_transpose_rowseg_kernel, whose bits it returns.
+// Blocks stay: a block keeps the weights of its channel groups and walks tiles of 32 * R rows, whose windows come in chunks of
+// cc output channels with 16-byte cp.async (4-byte copies took eight clocks of the SM for 128 bytes and bound the kernel), one
+// chunk ahead.  Results leave through a 32 x 33 tile per warp, 128 bytes of a row at a time.
+struct ConvWindowArgs {
+  const float* Lam;  // [M, Co, WW, WW]
+  const float* W;    // [Co, Ci, KS, KS]
+  float* out;        // [M, Ci, OW, OW]
+  int M, Co, Ci;
+  int cgb;           // channel groups (of TCI) per block
+  int R;             // groups of 32 rows per block
+  int cc;            // output channels per chunk, a multiple of ConvWindow::CU
+  int lprl;          // log2 of the lanes that copy one row's chunk
+};
+
+constexpr int CONV_WINDOW_SUMS = 72;
+
+template <int KS, int ST, int WW>
+struct ConvWindow {
+  static constexpr int OW = (WW - 1) * ST + KS;
+  static constexpr int TH0 = (CONV_WINDOW_SUMS / OW) / ST * ST;                  // whole image rows that fit
+  static constexpr bool FULL = OW * OW <= CONV_WINDOW_SUMS;
+  static constexpr int NB0 = FULL ? 1 : (OW + TH0 - 1) / TH0;
+  static constexpr int TH = FULL ? OW : ((OW + NB0 - 1) / NB0 + ST - 1) / ST * ST;
+  static constexpr int NB = (OW + TH - 1) / TH;                                  // bands of TH image rows
+  static constexpr int TCI = FULL ? (CONV_WINDOW_SUMS / (OW * OW) > 4 ? 4 : CONV_WINDOW_SUMS / (OW * OW)) : 1;
+  static constexpr int CU = WW % 2 ? 4 : 1;                                      // channels whose windows end on 16 bytes
+  static constexpr int WARPS = NB > 2 ? 12 : 8, BLOCKS = NB > 2 ? 1 : 2;         // three channels of four bands in one block
+};
+
+// One output channel (number U of CU) of a band: acc += window * weights.  lam: the channels' windows, in 16-byte words.
+template <int KS, int ST, int WW, int TCI, int BAND, int U>
+__device__ __forceinline__ void window_band(const float4* lam, const float* w, float (&acc)[TCI][ConvWindow<KS, ST, WW>::TH][ConvWindow<KS, ST, WW>::OW]) {
+  using G = ConvWindow<KS, ST, WW>;
+  constexpr int H0 = BAND * G::TH;
+  constexpr int HI = (H0 + G::TH - 1) / ST < WW - 1 ? (H0 + G::TH - 1) / ST : WW - 1;
+  constexpr int LO = H0 > KS - 1 ? (H0 - KS + ST) / ST : 0;   // window rows LO to HI reach the band
+  float l[G::CU * WW * WW + 4];
+#pragma unroll
+  for (int iy = HI; iy >= LO; --iy) {
+    const int first = U * WW * WW + iy * WW, last = first + WW - 1;
+#pragma unroll
+    for (int k = first / 4; k <= last / 4; ++k) {
+      if (iy < HI && k == (last + 1) / 4) continue;  // came with the row below
+      const float4 t = lam[k];
+      l[4 * k] = t.x; l[4 * k + 1] = t.y; l[4 * k + 2] = t.z; l[4 * k + 3] = t.w;
+    }
+#pragma unroll
+    for (int r = 0; r < KS; ++r) {
+      const int oy = iy * ST + r - H0;
+      if (oy < 0 || oy >= G::TH) continue;
+#pragma unroll
+      for (int s = 0; s < KS; ++s)
+#pragma unroll
+        for (int x = 0; x < WW; ++x)
+#pragma unroll
+          for (int c = 0; c < TCI; ++c) acc[c][oy][x * ST + s] = fmaf(l[first + x], w[(r * KS + s) * TCI + c], acc[c][oy][x * ST + s]);
+    }
+  }
+}
+
+template <int KS, int ST, int WW, int TCI, int BAND, int U>
+__device__ __forceinline__ void window_channels(const float4* lam, const float4* wp, int w_step,
+                                                float (&acc)[TCI][ConvWindow<KS, ST, WW>::TH][ConvWindow<KS, ST, WW>::OW]) {
+  constexpr int NWP = (KS * KS * TCI + 3) / 4 * 4;
+  float w[NWP];
+#pragma unroll
+  for (int k = 0; k < NWP / 4; ++k) {
+    const float4 t = wp[k];
+    w[4 * k] = t.x; w[4 * k + 1] = t.y; w[4 * k + 2] = t.z; w[4 * k + 3] = t.w;
+  }
+  window_band<KS, ST, WW, TCI, BAND, U>(lam, w, acc);
+  if constexpr (U + 1 < ConvWindow<KS, ST, WW>::CU) window_channels<KS, ST, WW, TCI, BAND, U + 1>(lam, wp + w_step, w_step, acc);
+}
+
+// ncc channels of a chunk for the warp's band
+template <int KS, int ST, int WW, int TCI, int BAND>
+__device__ __forceinline__ void window_chunk(int band, const float4* lam, const float4* wp, int w_step, int ncc,
+                                             float (&acc)[TCI][ConvWindow<KS, ST, WW>::TH][ConvWindow<KS, ST, WW>::OW]) {
+  using G = ConvWindow<KS, ST, WW>;
+  if (band == BAND) {
+#pragma unroll 1
+    for (int co = 0; co < ncc; co += G::CU, lam += G::CU * WW * WW / 4, wp += G::CU * w_step)
+      window_channels<KS, ST, WW, TCI, BAND, 0>(lam, wp, w_step, acc);
+  } else if constexpr (BAND + 1 < G::NB) {
+    window_chunk<KS, ST, WW, TCI, BAND + 1>(band, lam, wp, w_step, ncc, acc);
+  }
+}
+
+template <int KS, int ST, int WW, int TCI>
+__global__ void __launch_bounds__(32 * ConvWindow<KS, ST, WW>::WARPS, ConvWindow<KS, ST, WW>::BLOCKS) conv_window_kernel(ConvWindowArgs a) {
+  using G = ConvWindow<KS, ST, WW>;
+  constexpr int OW = G::OW, TH = G::TH, NB = G::NB, PLANE = WW * WW;
+  constexpr int NW = KS * KS * TCI, NWP = (NW + 3) / 4 * 4;
+  constexpr int N = TCI * TH * OW;
+  static_assert(NB == 1 || (TCI == 1 && TH % ST == 0), "bands start at a window row");
+  extern __shared__ __align__(16) float cw_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int combos = a.cgb * NB, rg = warp / combos, q = warp - rg * combos;
+  const int cgl = q / NB, band = (q % NB + cgl + rg) % NB;        // bands of unequal work meet different schedulers
+  const int pitch4 = (a.cc * PLANE / 4) | 1, buf4 = 32 * a.R * pitch4;
+  float* wS = cw_smem;                                            // [Co][cgb][NWP]: kernel row, kernel column, channel
+  float4* lamS = reinterpret_cast<float4*>(wS + a.Co * a.cgb * NWP);  // two buffers [32 * R][pitch4]
+  float* epi = reinterpret_cast<float*>(lamS + 2 * buf4) + warp * (32 * 33);
+  const int cg0 = blockIdx.y * a.cgb, ci0 = (cg0 + cgl) * TCI;
+
+  for (int e = threadIdx.x; e < a.Co * a.cgb * NWP; e += blockDim.x) {
+    const int k = e % NWP, g = e / NWP, co = g / a.cgb, ci = (cg0 + g - co * a.cgb) * TCI + k % TCI;
+    wS[e] = (k < NW && ci < a.Ci) ? __ldg(a.W + ((size_t)co * a.Ci + ci) * (KS * KS) + k / TCI) : 0.f;
+  }
+
+  const int rows = 32 * a.R, nch = (a.Co + a.cc - 1) / a.cc;
+  const size_t row4 = (size_t)a.Co * PLANE / 4;
+  const int lpr = 1 << a.lprl, sub = threadIdx.x & (lpr - 1), row0 = threadIdx.x >> a.lprl, row_step = blockDim.x >> a.lprl;
+  auto stage = [&](int buf, int m0, int co0) {
+    const int n4 = min(a.cc, a.Co - co0) * PLANE / 4;
+    const float4* base = reinterpret_cast<const float4*>(a.Lam) + co0 * PLANE / 4;
+    for (int i = row0; i < rows; i += row_step) {
+      const float4* src = base + (size_t)min(m0 + i, a.M - 1) * row4;
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(lamS + buf * buf4 + i * pitch4);
+      for (int e = sub; e < n4; e += lpr) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * e), "l"(src + e) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  const int tiles = (a.M + rows - 1) / rows;
+  int tile = blockIdx.x, ch = 0, buf = 0;
+  if (tile < tiles) stage(0, tile * rows, 0);
+  float acc[TCI][TH][OW];
+#pragma unroll
+  for (int k = 0; k < N; ++k) acc[k / (TH * OW)][k / OW % TH][k % OW] = 0.f;
+  while (tile < tiles) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                       // this chunk is there, and nobody reads the other buffer any more
+    int next_tile = tile, next_ch = ch + 1;
+    if (next_ch == nch) { next_ch = 0; next_tile += gridDim.x; }
+    if (next_tile < tiles) stage(buf ^ 1, next_tile * rows, next_ch * a.cc);
+    window_chunk<KS, ST, WW, TCI, 0>(band, lamS + buf * buf4 + (rg * 32 + lane) * pitch4,
+                                     reinterpret_cast<const float4*>(wS) + (ch * a.cc * a.cgb + cgl) * (NWP / 4), a.cgb * (NWP / 4),
+                                     min(a.cc, a.Co - ch * a.cc), acc);
+    if (next_ch == 0) {
+      const int m0 = tile * rows + rg * 32, mrows = min(32, a.M - m0);
+      const int h0 = band * TH;
+      const int valid = G::FULL ? max(0, min(TCI, a.Ci - ci0)) * OW * OW : (ci0 < a.Ci ? min(TH, OW - h0) * OW : 0);
+      const size_t m_step = (size_t)a.Ci * OW * OW;
+      float* out = a.out + (size_t)m0 * m_step + ((size_t)ci0 * OW + h0) * OW + lane;
+#pragma unroll
+      for (int k0 = 0; k0 < N; k0 += 32) {
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (k0 + j < N) epi[lane * 33 + j] = acc[(k0 + j) / (TH * OW)][(k0 + j) / OW % TH][(k0 + j) % OW];
+        __syncwarp();
+        if (k0 + lane < valid) {
+#pragma unroll 8
+          for (int i = 0; i < mrows; ++i) out[(size_t)i * m_step + k0] = epi[i * 33 + lane];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < N; ++k) acc[k / (TH * OW)][k / OW % TH][k % OW] = 0.f;
+    }
+    tile = next_tile;
+    ch = next_ch;
+    buf ^= 1;
+  }
+}
+
+template <int KS, int ST, int WW, int TCI>
+static int launch_window(ConvWindowArgs a, cudaStream_t stream) {
+  using G = ConvWindow<KS, ST, WW>;
+  constexpr int NWP = (KS * KS * TCI + 3) / 4 * 4, LIMIT = (G::BLOCKS == 1 ? 224 : 112) * 1024, EPI = 32 * 33 * 4, PLANE = WW * WW;
+  const int ncg = ceil_div(a.Ci, TCI);
+  // channel groups per block: the choice that leaves the fewest idle, and of those the largest
+  double best = 0.0;
+  int gy = 0;
+  for (int c = G::WARPS / G::NB; c >= 1; --c) {
+    if (c > ncg) continue;
+    const int r = G::WARPS / (c * G::NB), y = ceil_div(ncg, c);
+    const double used = (double)ncg / (y * c);
+    const long long left = LIMIT - (long long)a.Co * c * NWP * 4 - c * G::NB * r * EPI;
+    const long long room = left / (2 * 32 * r * 16) - 1;                  // 16-byte words of a row's chunk
+    if (room < G::CU * PLANE / 4 || used <= best + 1e-9) continue;
+    long long cc = room * 4 / PLANE, want = 24 * 1024 / (32 * r * 4 * PLANE);
+    if (want < G::CU) want = G::CU;
+    if (cc > want) cc = want;
+    if (cc > 16) cc = 16;
+    if (cc > a.Co) cc = a.Co;
+    best = used;
+    a.cgb = c; a.R = r; a.cc = (int)cc / G::CU * G::CU; gy = y;
+  }
+  if (gy == 0 || gy > 65535) return BF_E_UNSUPPORTED;  // weights beyond an SM's shared memory
+  const int threads = 32 * a.cgb * G::NB * a.R;
+  a.lprl = 0;
+  while (a.lprl < 5 && (1 << a.lprl) < a.cc * PLANE / 4) ++a.lprl;
+  const size_t smem = (size_t)a.Co * a.cgb * NWP * 4 + 2 * (size_t)32 * a.R * ((a.cc * PLANE / 4) | 1) * 16 + threads / 32 * EPI;
+  const int tiles = ceil_div(a.M, 32 * a.R);
+  int gx = G::BLOCKS * 148 / gy;
+  if (gx > tiles) gx = tiles;
+  if (gx < 1) gx = 1;
+  static SmemOptIn opt_in;
+  if (int rc = ensure_dynamic_smem(conv_window_kernel<KS, ST, WW, TCI>, LIMIT, opt_in, "conv_window_kernel")) return rc;
+  conv_window_kernel<KS, ST, WW, TCI><<<dim3(gx, gy), threads, smem, stream>>>(a);
+  BF_CHECK_LAUNCH("conv_window_kernel");
+  return BF_OK;
+}
+
+template <int KS, int ST, int WW, int MAXW>
+static int launch_window_side(const ConvWindowArgs& a, int ww, cudaStream_t stream) {
+  if constexpr (WW > MAXW) {
+    return BF_E_UNSUPPORTED;
+  } else {
+    if (ww != WW) return launch_window_side<KS, ST, WW + 1, MAXW>(a, ww, stream);
+    if constexpr (WW % 2 == 0 || WW <= 7) {
+      constexpr int TCI = ConvWindow<KS, ST, WW>::TCI;
+      if (a.Co % ConvWindow<KS, ST, WW>::CU != 0) return BF_E_UNSUPPORTED;
+      // single channels where groups would be mostly padding (three channels in groups of four or two)
+      if (TCI > 1 && 5 * (ceil_div(a.Ci, TCI) * TCI) > 6 * a.Ci) return launch_window<KS, ST, WW, 1>(a, stream);
+      return launch_window<KS, ST, WW, TCI>(a, stream);
+    }
+    return BF_E_UNSUPPORTED;
+  }
+}
+
+// Transposed convolution without padding of M rows of WH x WW windows; BF_E_UNSUPPORTED for geometries without an instance.
+int launch_conv_window(const float* Lam, const float* W, float* out, int M, int Ci, int Co, int WH, int WW, int kh, int kw, int sh, int sw,
+                       cudaStream_t stream) {
+  if (WH != WW || kh != kw || sh != sw || (reinterpret_cast<uintptr_t>(Lam) & 15u) != 0) return BF_E_UNSUPPORTED;
+  const ConvWindowArgs a{Lam, W, out, M, Co, Ci, 0, 0, 0, 0};
+  if (kh == 3 && sh == 1) return launch_window_side<3, 1, 2, 14>(a, WW, stream);
+  if (kh == 4 && sh == 2) return launch_window_side<4, 2, 2, 7>(a, WW, stream);
+  if (kh == 3 && sh == 2) return launch_window_side<3, 2, 2, 7>(a, WW, stream);
+  return BF_E_UNSUPPORTED;
+}
+
+}  // namespace bf
