@@ -1,5 +1,7 @@
 // Transposed convolution of narrow windows of coefficient rows (the identity-row sweeps on conv layers): no padding, square
 // windows, kernels and strides, lanes = coefficient rows.
+#include <math.h>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -16,6 +18,11 @@ namespace bf {
 // Blocks stay: a block keeps the weights of its channel groups and walks tiles of 32 * R rows, whose windows come in chunks of
 // cc output channels with 16-byte cp.async (4-byte copies took eight clocks of the SM for 128 bytes and bound the kernel), one
 // chunk ahead.  Results leave through a 32 x 33 tile per warp, 128 bytes of a row at a time.
+// Bound by FFMA issue next to the shared-memory reads where a block's channels are many (20 to 23 of 31 T multiply-adds/s that
+// the chip reaches), by the chunks' copies and the results' stores with one to three channels.  65,536 rows, against the
+// row-segment kernels: 32 -> 32 channels, 3 x 3 -> 8 x 8 of 4x4 / 2: 1293 -> 472 us; 64 -> 32, 4 x 4 -> 6 x 6 of 3x3: 3674 -> 841;
+// 32 -> 32, 6 x 6 -> 14 x 14 of 4x4 / 2: 5490 -> 2515; 32 -> 3, 8 x 8 -> 10 x 10 of 3x3: 1124 -> 218; 32 -> 1, 4 x 4 -> 10 x 10 of
+// 4x4 / 2: 223 -> 60.  64 rows: 0.9 (7 x 7, 4x4 / 2) to 3.8 of the speed, so no line in the rows.
 struct ConvWindowArgs {
   const float* Lam;  // [M, Co, WW, WW]
   const float* W;    // [Co, Ci, KS, KS]
@@ -184,17 +191,19 @@ static int launch_window(ConvWindowArgs a, cudaStream_t stream) {
   using G = ConvWindow<KS, ST, WW>;
   constexpr int NWP = (KS * KS * TCI + 3) / 4 * 4, LIMIT = (G::BLOCKS == 1 ? 224 : 112) * 1024, EPI = 32 * 33 * 4, PLANE = WW * WW;
   const int ncg = ceil_div(a.Ci, TCI);
-  // channel groups per block: the choice that leaves the fewest idle, and of those the largest
+  // channel groups per block: few of them idle, few blocks that read the same rows, and no idle warps where a block has an SM
   double best = 0.0;
   int gy = 0;
   for (int c = G::WARPS / G::NB; c >= 1; --c) {
     if (c > ncg) continue;
-    const int r = G::WARPS / (c * G::NB), y = ceil_div(ncg, c);
-    const double used = (double)ncg / (y * c);
+    const int y = ceil_div(ncg, c);
+    int r = G::WARPS / (c * G::NB);
+    const double used = (double)ncg / (y * c) / (1.0 + 0.1 * y) * (G::BLOCKS == 1 ? sqrt((double)(c * G::NB * r) / G::WARPS) : 1.0);
+    while (r > 1 && (long long)ceil_div(a.M, 32 * r) * y < 148) --r;      // few rows: more blocks with longer chunks
     const long long left = LIMIT - (long long)a.Co * c * NWP * 4 - c * G::NB * r * EPI;
     const long long room = left / (2 * 32 * r * 16) - 1;                  // 16-byte words of a row's chunk
     if (room < G::CU * PLANE / 4 || used <= best + 1e-9) continue;
-    long long cc = room * 4 / PLANE, want = 24 * 1024 / (32 * r * 4 * PLANE);
+    long long cc = room * 4 / PLANE, want = (G::BLOCKS == 1 ? 40 : 24) * 1024 / (32 * r * 4 * PLANE);
     if (want < G::CU) want = G::CU;
     if (cc > want) cc = want;
     if (cc > 16) cc = 16;
