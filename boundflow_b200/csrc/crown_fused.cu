@@ -17,10 +17,8 @@
 
 namespace bf {
 
-constexpr int FS_ROWS = 32, FS_COLS = 64, FS_K = 32, FS_STAGES = 6, FS_LAG = 4;
+constexpr int FS_ROWS = 32, FS_COLS = 64, FS_K = 32, FS_STAGES = 3, FS_COMPUTE = 128;
 constexpr int FS_KP = FS_K + 4;  // adjoint: pitch of a weight row's slab
-// Threads of a CTA: 128 compute, 64 copy weights, 64 form the row sums (backward) or the points at the input (adjoint).
-constexpr int FS_COMPUTE = 128, FS_COPY = 64, FS_THREADS = 256;
 
 __device__ __forceinline__ void fs_copy16(float* dst, const float* src, bool ok) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
@@ -28,116 +26,84 @@ __device__ __forceinline__ void fs_copy16(float* dst, const float* src, bool ok)
 __device__ __forceinline__ void fs_copy4(float* dst, const float* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 4 : 0) : "memory");
 }
-// Named barriers: 1 + s: slab s is there; 1 + FS_STAGES + s: slab s has been read; the last one: the computing warps alone.
-__device__ __forceinline__ void fs_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
-__device__ __forceinline__ void fs_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
-__device__ __forceinline__ void fs_bar() { asm volatile("bar.sync 15, 128;" ::: "memory"); }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void fs_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void fs_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void fs_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }  // the computing warps
 
-// The copying warps: the slabs of all layers and tiles of this CTA in the order in which they are used, up to FS_STAGES ahead of the
-// computing warps and FS_LAG in flight.  Their part in the layers' cluster barriers is taken as late as the
-// ring allows, so that the first slabs of a layer arrive while the one above is computed: before they wait for the place of slab i - FS_STAGES, of layer
-// l, they have arrived at every barrier up to the one that ends layer l.  What they wait for there needs slabs before i - FS_STAGES
-// only, which have been announced (FS_LAG < FS_STAGES).  ring_threads(i): threads that take part in the barriers of slab i.
-template <typename Args, typename Ring, typename Copy>
-__device__ __forceinline__ void fs_copy_weights(const Args& a, int ranks, int rank, Ring&& ring_threads, Copy&& copy) {
-  int i = 0, arrived = 0;
-  int layer_of[FS_STAGES];                                    // layers of the last FS_STAGES slabs
-#pragma unroll
-  for (int s = 0; s < FS_STAGES; ++s) layer_of[s] = 0;
-  auto arrive_until = [&](int phases) {
-    while (arrived < phases) {
-      if (arrived > 0) cluster_wait();
-      cluster_arrive();
-      ++arrived;
-    }
-  };
-  arrive_until(1);
-  for (int l = 0; l < a.layers; ++l) {
-    for (int tile = rank; tile * FS_COLS < a.L[l].N; tile += ranks) {
-      for (int k0 = 0; k0 < a.L[l].K; k0 += FS_K, ++i) {
-        const int s = i % FS_STAGES;
-        if (i >= FS_STAGES) {
-          int before = 0;
-#pragma unroll
-          for (int q = 0; q < FS_STAGES; ++q) before = (q == s) ? layer_of[q] : before;
-          arrive_until(before + 1);
-          fs_sync(1 + FS_STAGES + s, ring_threads(i));
-        }
-#pragma unroll
-        for (int q = 0; q < FS_STAGES; ++q) layer_of[q] = (q == s) ? l : layer_of[q];
-        copy(a.L[l], tile * FS_COLS, k0, s);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (i >= FS_LAG) {
-          asm volatile("cp.async.wait_group %0;" ::"n"(FS_LAG) : "memory");
-          fs_arrive(1 + (i - FS_LAG) % FS_STAGES, ring_threads(i - FS_LAG));
-        }
-      }
-    }
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  for (int j = max(0, i - FS_LAG); j < i; ++j) fs_arrive(1 + j % FS_STAGES, ring_threads(j));
-  arrive_until(a.layers);
-  cluster_wait();
-}
+// position in the stream of weight slabs: layer, tile of this CTA, slab
+struct FsCursor {
+  int layer, tile, k0;
+};
 
 // ---------------------------------------------------------------------------
 // backward sweep
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(FS_THREADS, 1) crown_fused_bwd_kernel(FusedSweepArgs a) {
+__device__ __forceinline__ void fs_advance(const FusedSweepArgs& a, FsCursor& c, int ranks, int rank) {
+  while (c.layer < a.layers) {
+    const FusedSweepLayer& L = a.L[c.layer];
+    if (c.tile * FS_COLS < L.N && c.k0 < L.K) return;
+    if (c.tile * FS_COLS < L.N) { c.tile += ranks; c.k0 = 0; }
+    if (c.tile * FS_COLS >= L.N) { ++c.layer; c.tile = rank; c.k0 = 0; }
+  }
+}
+
+__global__ void __launch_bounds__(256, 2) crown_fused_bwd_kernel(FusedSweepArgs a) {
   extern __shared__ __align__(16) float fs_smem[];
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int m0 = (int)(blockIdx.x / ranks) * FS_ROWS;
-  float* const As0 = fs_smem;                               // [k][row], coefficients after the ReLU scaling, of even and odd layers
-  float* const As1 = fs_smem + a.kmax * FS_ROWS;
+  float* As[2] = {fs_smem, fs_smem + a.kmax * FS_ROWS};     // [k][row], coefficients after the ReLU scaling
   float* Bs = fs_smem + 2 * a.kmax * FS_ROWS;               // [stage][k][column]
   float* pbuf = Bs + FS_STAGES * FS_K * FS_COLS;            // [row]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int RING = FS_COMPUTE + FS_COPY;
+  const bool computing = tid < FS_COMPUTE;
 
   // spec rows
-  for (int k = warp; k < a.L[0].K; k += FS_THREADS / 32) As0[k * FS_ROWS + lane] = (m0 + lane < a.M) ? a.C[(size_t)(m0 + lane) * a.L[0].K + k] : 0.f;
-  cluster.sync();  // every CTA of the cluster runs, and its spec rows are in place
+  for (int k = warp; k < a.L[0].K; k += 8) As[0][k * FS_ROWS + lane] = (m0 + lane < a.M) ? a.C[(size_t)(m0 + lane) * a.L[0].K + k] : 0.f;
 
-  if (tid >= FS_COMPUTE && tid < FS_COMPUTE + FS_COPY) {
-    const int t = tid - FS_COMPUTE;
-    fs_copy_weights(a, ranks, rank, [](int) { return RING; }, [&](const FusedSweepLayer& L, int n0, int k0, int s) {
-      float* dst = Bs + s * (FS_K * FS_COLS);
+  FsCursor next{0, rank, 0};
+  int fetched = 0, used = 0;
+  auto fetch = [&]() {
+    fs_advance(a, next, ranks, rank);
+    if (next.layer < a.layers) {
+      const FusedSweepLayer& L = a.L[next.layer];
+      float* dst = Bs + fetched % FS_STAGES * (FS_K * FS_COLS);
+      const int n0 = next.tile * FS_COLS;
       if (L.vec) {
-        const int c = t % (FS_COLS / 4) * 4;
-        const bool in = n0 + c < L.N;
-        const float* src = L.W + (size_t)(k0 + t / (FS_COLS / 4)) * L.N + n0 + c;
 #pragma unroll
-        for (int kk = t / (FS_COLS / 4); kk < FS_K; kk += FS_COPY / (FS_COLS / 4), src += (size_t)(FS_COPY / (FS_COLS / 4)) * L.N) {
-          const bool ok = in && k0 + kk < L.K;
-          fs_copy16(dst + kk * FS_COLS + c, ok ? src : L.W, ok);
+        for (int j = 0; j < FS_K * FS_COLS / 4 / FS_COMPUTE; ++j) {
+          const int e = tid + j * FS_COMPUTE, kk = e / (FS_COLS / 4), c = e % (FS_COLS / 4) * 4;
+          const bool ok = next.k0 + kk < L.K && n0 + c < L.N;
+          fs_copy16(dst + kk * FS_COLS + c, ok ? L.W + (size_t)(next.k0 + kk) * L.N + n0 + c : L.W, ok);
         }
       } else {
-        const bool in = n0 + t < L.N;
-        const float* src = L.W + (size_t)k0 * L.N + n0 + t;
-#pragma unroll 8
-        for (int kk = 0; kk < FS_K; ++kk, src += L.N) {
-          const bool ok = in && k0 + kk < L.K;
-          fs_copy4(dst + kk * FS_COLS + t, ok ? src : L.W, ok);
+#pragma unroll 4
+        for (int j = 0; j < FS_K * FS_COLS / FS_COMPUTE; ++j) {
+          const int e = tid + j * FS_COMPUTE, kk = e / FS_COLS, c = e % FS_COLS;
+          const bool ok = next.k0 + kk < L.K && n0 + c < L.N;
+          fs_copy4(dst + kk * FS_COLS + c, ok ? L.W + (size_t)(next.k0 + kk) * L.N + n0 + c : L.W, ok);
         }
       }
-    });
-    return;
-  }
+      next.k0 += FS_K;
+    }
+    ++fetched;
+    fs_commit();
+  };
+  if (computing)
+    for (int i = 0; i < FS_STAGES - 1; ++i) fetch();
+  cluster.sync();  // every CTA of the cluster runs, and its spec rows are in place
 
   // computing warps: rows r0 .. r0 + 3, columns c0 .. c0 + 3 of a tile
   const int tx = lane & 7, ty = lane >> 3;
   const int r0 = (warp >> 1) * 16 + ty * 4, c0 = (warp & 1) * 32 + tx * 4;
   const float sgn = (a.side == BF_SIDE_LOWER) ? -1.f : 1.f;
-  float delta[2] = {0.f, 0.f};  // row-sum warps of the last rank
-  int used = 0;
+  float delta = 0.f;  // row-sum warps of the last rank
   for (int l = 0; l < a.layers; ++l) {
     const FusedSweepLayer& L = a.L[l];
     const bool last = l + 1 == a.layers;
-    if (tid < FS_COMPUTE) {
-      const float* A = (l & 1) ? As1 : As0;
+    if (computing) {
+      const float* A = As[l & 1];
       for (int tile = rank; tile * FS_COLS < L.N; tile += ranks) {
         const int col = tile * FS_COLS + c0;
         // what the epilogue needs: the next layer's slopes and split terms, or the input box
@@ -162,10 +128,11 @@ __global__ void __launch_bounds__(FS_THREADS, 1) crown_fused_bwd_kernel(FusedSwe
 #pragma unroll
           for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
         for (int k0 = 0; k0 < L.K; k0 += FS_K, ++used) {
-          const int stage = used % FS_STAGES;
-          fs_sync(1 + stage, RING);
+          fs_wait<FS_STAGES - 2>();
+          fs_bar();                                   // this slab is there, and nobody reads the one before it any more
+          fetch();
           const float* as = A + k0 * FS_ROWS + r0;
-          const float* bs = Bs + stage * (FS_K * FS_COLS) + c0;
+          const float* bs = Bs + used % FS_STAGES * (FS_K * FS_COLS) + c0;
           const int left = min(FS_K, L.K - k0);
           auto step = [&](int kk) {
             const float4 p = *reinterpret_cast<const float4*>(as + kk * FS_ROWS);
@@ -183,7 +150,6 @@ __global__ void __launch_bounds__(FS_THREADS, 1) crown_fused_bwd_kernel(FusedSwe
 #pragma unroll 1
             for (int kk = 0; kk < left; ++kk) step(kk);
           }
-          fs_arrive(1 + FS_STAGES + stage, RING);
         }
         // raw coefficients
         if (L.out && col < L.N) {
@@ -199,7 +165,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) crown_fused_bwd_kernel(FusedSwe
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(acc[i][j], acc[i][j] >= 0.f ? xs[j] : ys[j], zs[j]);
           }
-          float* to = ((l & 1) ? As0 : As1) + r0;
+          float* to = As[(l + 1) & 1] + r0;
           for (int q = 0; q < ranks; ++q) {
             float* p = cluster.map_shared_rank(to, (rank + q) % ranks);
 #pragma unroll
@@ -232,179 +198,156 @@ __global__ void __launch_bounds__(FS_THREADS, 1) crown_fused_bwd_kernel(FusedSwe
         }
       }
     } else if (rank == ranks - 1) {
-      // row sums of this layer's prologue: four threads per row (gemm_mainloop's order), two rows per thread
-      const int t = tid - FS_COMPUTE - FS_COPY, lkc = (t & 3) * 4;
-      const bool thin = l == 0 && a.thin_top;
-      float r[2] = {0.f, 0.f};
-      if (thin) {
-        for (int h = 0; h < 2; ++h) {
-          const int row = m0 + (t >> 2) + 16 * h;
-          if (row < a.M && lkc == 0 && L.kbias)
-            for (int k = 0; k < L.K; ++k) r[h] = fmaf(a.C[(size_t)row * L.K + k], __ldg(L.kbias + k), r[h]);
-        }
-      } else {
-        constexpr int U = 4;
-        const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float* base = l == 0 ? a.C : a.L[l - 1].out;
-        for (int k0 = lkc; k0 < L.K; k0 += 16 * U) {
-          float4 v[2][U], kb[U], dp[2][U], dn[2][U], ep[2][U], en[2][U], ad[2][U];
+      // row sums of this layer's prologue: four threads per row (gemm_mainloop's order)
+      const int t = tid - FS_COMPUTE, row = m0 + (t >> 2), lkc = (t & 3) * 4;
+      if (row < a.M) {
+        const float* pa = (l == 0) ? a.C + (size_t)row * L.K : a.L[l - 1].out + (size_t)row * L.K;
+        const size_t off = (size_t)(row / a.S) * L.K;
+        float r = 0.f;
+        if (l == 0 && a.thin_top) {
+          if (lkc == 0 && L.kbias)
+            for (int k = 0; k < L.K; ++k) r = fmaf(pa[k], __ldg(L.kbias + k), r);
+        } else {
+          constexpr int U = 4;
+          const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int k0 = lkc; k0 < L.K; k0 += 16 * U) {
+            float4 v[U], kb[U], dp[U], dn[U], ep[U], en[U], ad[U];
 #pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const int k = k0 + 16 * u;
-            kb[u] = (L.kbias && k < L.K) ? load4_guard(L.kbias, k, L.K, L.veck) : z4;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int row = m0 + (t >> 2) + 16 * h;
-              v[h][u] = dp[h][u] = dn[h][u] = ep[h][u] = en[h][u] = ad[h][u] = z4;
-              if (k < L.K && row < a.M) {
-                v[h][u] = load4_plain(base + (size_t)row * L.K, k, L.K, L.veck);  // written by other CTAs of the cluster during this launch
+            for (int u = 0; u < U; ++u) {
+              const int k = k0 + 16 * u;
+              v[u] = kb[u] = dp[u] = dn[u] = ep[u] = en[u] = ad[u] = z4;
+              if (k < L.K) {
+                v[u] = load4_plain(pa, k, L.K, L.veck);  // written by other CTAs of the cluster during this launch
+                if (L.kbias) kb[u] = load4_guard(L.kbias, k, L.K, L.veck);
                 if (L.dpos) {
-                  const size_t off = (size_t)(row / a.S) * L.K;
-                  dp[h][u] = load4_guard(L.dpos + off, k, L.K, L.veck);
-                  dn[h][u] = load4_guard(L.dneg + off, k, L.K, L.veck);
-                  if (L.epos) ep[h][u] = load4_guard(L.epos + off, k, L.K, L.veck);
-                  if (L.eneg) en[h][u] = load4_guard(L.eneg + off, k, L.K, L.veck);
-                  if (L.add) ad[h][u] = load4_guard(L.add + off, k, L.K, L.veck);
+                  dp[u] = load4_guard(L.dpos + off, k, L.K, L.veck);
+                  dn[u] = load4_guard(L.dneg + off, k, L.K, L.veck);
+                  if (L.epos) ep[u] = load4_guard(L.epos + off, k, L.K, L.veck);
+                  if (L.eneg) en[u] = load4_guard(L.eneg + off, k, L.K, L.veck);
+                  if (L.add) ad[u] = load4_guard(L.add + off, k, L.K, L.veck);
                 }
               }
             }
-          }
 #pragma unroll
-          for (int u = 0; u < U; ++u) {
-            if (k0 + 16 * u >= L.K) break;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            for (int u = 0; u < U; ++u) {
+              if (k0 + 16 * u >= L.K) break;
               if (L.dpos) {
 #define BF_ROW_SUM(c)                                                          \
   {                                                                            \
-    const bool sel = v[h][u].c >= 0.f;                                         \
-    const float lam = v[h][u].c * (sel ? dp[h][u].c : dn[h][u].c) + ad[h][u].c; \
-    r[h] += v[h][u].c * (sel ? ep[h][u].c : en[h][u].c);                       \
-    r[h] = fmaf(lam, kb[u].c, r[h]);                                           \
+    const bool sel = v[u].c >= 0.f;                                            \
+    const float lam = v[u].c * (sel ? dp[u].c : dn[u].c) + ad[u].c;            \
+    r += v[u].c * (sel ? ep[u].c : en[u].c);                                   \
+    r = fmaf(lam, kb[u].c, r);                                                 \
   }
                 BF_ROW_SUM(x) BF_ROW_SUM(y) BF_ROW_SUM(z) BF_ROW_SUM(w)
 #undef BF_ROW_SUM
               } else {
-                r[h] += v[h][u].x * kb[u].x + v[h][u].y * kb[u].y + v[h][u].z * kb[u].z + v[h][u].w * kb[u].w;
+                r += v[u].x * kb[u].x + v[u].y * kb[u].y + v[u].z * kb[u].z + v[u].w * kb[u].w;
               }
             }
           }
         }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          r[h] += __shfl_xor_sync(0xffffffffu, r[h], 1);
-          r[h] += __shfl_xor_sync(0xffffffffu, r[h], 2);
+        const unsigned quad = 0xfu << (lane & ~3);
+        if (!(l == 0 && a.thin_top)) {
+          r += __shfl_xor_sync(quad, r, 1);
+          r += __shfl_xor_sync(quad, r, 2);
         }
-      }
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int row = m0 + (t >> 2) + 16 * h;
-        delta[h] = (l == 0) ? r[h] : delta[h] + r[h];
-        if (last && lkc == 0 && row < a.M) a.delta[row] = delta[h];
+        delta = (l == 0) ? r : delta + r;
+        if (last && lkc == 0) a.delta[row] = delta;
       }
     }
-    __syncwarp();
-    cluster_arrive();
-    cluster_wait();  // the next layer's coefficients are complete in every CTA; nobody leaves before the others' last stores to it
+    cluster.sync();  // the next layer's coefficients are complete in every CTA; nobody leaves before the others' last stores to it
   }
 }
 
 // ---------------------------------------------------------------------------
 // adjoint (gradient) sweep
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(FS_THREADS, 1) crown_fused_adjoint_kernel(FusedAdjointArgs a) {
+__device__ __forceinline__ void fs_advance(const FusedAdjointArgs& a, FsCursor& c, int ranks, int rank) {
+  while (c.layer < a.layers) {
+    const FusedAdjointLayer& L = a.L[c.layer];
+    if (c.tile * FS_COLS < L.N && c.k0 < L.K) return;
+    if (c.tile * FS_COLS < L.N) { c.tile += ranks; c.k0 = 0; }
+    if (c.tile * FS_COLS >= L.N) { ++c.layer; c.tile = rank; c.k0 = 0; }
+  }
+}
+
+__global__ void __launch_bounds__(FS_COMPUTE, 2) crown_fused_adjoint_kernel(FusedAdjointArgs a) {
   extern __shared__ __align__(16) float fs_smem[];
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int m0 = (int)(blockIdx.x / ranks) * FS_ROWS;
-  float* const As0 = fs_smem;                                // [k][row], adjoint points after even and odd layers
-  float* const As1 = fs_smem + a.kmax * FS_ROWS;
+  float* As[2] = {fs_smem, fs_smem + a.kmax * FS_ROWS};      // [k][row], adjoint points between layers
   float* Bs = fs_smem + 2 * a.kmax * FS_ROWS;                // [stage][column][FS_KP]
-  float* A0s = Bs + FS_STAGES * FS_COLS * FS_KP;             // [stage][k][row], slabs of the points at the network input
-  float* red = A0s + FS_STAGES * FS_K * FS_ROWS;             // [row][FS_COLS + 1]
+  float* A0s = Bs + FS_STAGES * FS_COLS * FS_KP;             // [2][k][row], slabs of the points at the network input
+  float* red = A0s + 2 * FS_K * FS_ROWS;                     // [row][FS_COLS + 1]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // the warps that form the points at the input take part in the slabs of the first layer
-  const int first_slabs = (a.L[0].N > rank * FS_COLS ? (a.L[0].N - rank * FS_COLS + ranks * FS_COLS - 1) / (ranks * FS_COLS) : 0) * ((a.L[0].K + FS_K - 1) / FS_K);
-  auto ring = [first_slabs](int i) { return i < first_slabs ? FS_THREADS : FS_COMPUTE + FS_COPY; };
-  cluster.sync();  // every CTA of the cluster runs
 
-  if (tid >= FS_COMPUTE && tid < FS_COMPUTE + FS_COPY) {
-    const int t = tid - FS_COMPUTE;
-    fs_copy_weights(a, ranks, rank, ring, [&](const FusedAdjointLayer& L, int n0, int k0, int s) {
-      float* dst = Bs + s * (FS_COLS * FS_KP);
+  FsCursor next{0, rank, 0};
+  int fetched = 0, used = 0;
+  auto fetch = [&]() {
+    fs_advance(a, next, ranks, rank);
+    if (next.layer < a.layers) {
+      const FusedAdjointLayer& L = a.L[next.layer];
+      float* dst = Bs + fetched % FS_STAGES * (FS_COLS * FS_KP);
+      const int n0 = next.tile * FS_COLS;
       if (L.veck) {
-        const int kk = t % (FS_K / 4) * 4;
-        const bool in = k0 + kk < L.K;
-        const float* src = L.W + (size_t)(n0 + t / (FS_K / 4)) * L.K + k0 + kk;
 #pragma unroll
-        for (int c = t / (FS_K / 4); c < FS_COLS; c += FS_COPY / (FS_K / 4), src += (size_t)(FS_COPY / (FS_K / 4)) * L.K) {
-          const bool ok = in && n0 + c < L.N;
-          fs_copy16(dst + c * FS_KP + kk, ok ? src : L.W, ok);
+        for (int j = 0; j < FS_K * FS_COLS / 4 / FS_COMPUTE; ++j) {
+          const int e = tid + j * FS_COMPUTE, c = e / (FS_K / 4), kk = e % (FS_K / 4) * 4;
+          const bool ok = next.k0 + kk < L.K && n0 + c < L.N;
+          fs_copy16(dst + c * FS_KP + kk, ok ? L.W + (size_t)(n0 + c) * L.K + next.k0 + kk : L.W, ok);
         }
       } else {
-        const int kk = t % FS_K;
-        const bool in = k0 + kk < L.K;
-        const float* src = L.W + (size_t)(n0 + t / FS_K) * L.K + k0 + kk;
-#pragma unroll 8
-        for (int c = t / FS_K; c < FS_COLS; c += FS_COPY / FS_K, src += (size_t)(FS_COPY / FS_K) * L.K) {
-          const bool ok = in && n0 + c < L.N;
-          fs_copy4(dst + c * FS_KP + kk, ok ? src : L.W, ok);
+#pragma unroll 4
+        for (int j = 0; j < FS_K * FS_COLS / FS_COMPUTE; ++j) {
+          const int e = tid + j * FS_COMPUTE, c = e / FS_K, kk = e % FS_K;
+          const bool ok = next.k0 + kk < L.K && n0 + c < L.N;
+          fs_copy4(dst + c * FS_KP + kk, ok ? L.W + (size_t)(n0 + c) * L.K + next.k0 + kk : L.W, ok);
         }
       }
-    });
-    return;
-  }
+      next.k0 += FS_K;
+    }
+    ++fetched;
+    fs_commit();
+  };
+  for (int i = 0; i < FS_STAGES - 1; ++i) fetch();
 
-  if (tid >= FS_COMPUTE + FS_COPY) {
-    // points at the network input: lane = row, a warp 16 of the slab's k; the next slab's values in registers meanwhile
-    const int arow = m0 + lane, kw = (warp - 6) * 16, K = a.L[0].K;
-    const size_t off = (size_t)((arow < a.M ? arow : 0) / a.S) * K;
-    float4 ha[4], hm[4], hr[4];
-    auto load_h0 = [&](int k0) {
+  // points at the network input, one slab ahead in registers: row = lane, k = 8 * warp .. + 7
+  const int arow = m0 + lane;
+  float4 ha[2], hm[2], hr[2];
+  auto load_h0 = [&](int k0) {
+    const int K = a.L[0].K;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int k = k0 + kw + i * 4;
-        ha[i] = hm[i] = hr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (arow < a.M && k < K) {
-          ha[i] = load4_guard(a.A0 + (size_t)arow * K, k, K, a.L[0].veck);
-          if (a.mid) {
-            hm[i] = load4_guard(a.mid + off, k, K, a.L[0].veck);
-            hr[i] = load4_guard(a.rad + off, k, K, a.L[0].veck);
-          }
+    for (int i = 0; i < 2; ++i) {
+      const int k = k0 + warp * 8 + i * 4;
+      ha[i] = hm[i] = hr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (arow < a.M && k < K) {
+        ha[i] = load4_guard(a.A0 + (size_t)arow * K, k, K, a.L[0].veck);
+        if (a.mid) {
+          const size_t off = (size_t)(arow / a.S) * K;
+          hm[i] = load4_guard(a.mid + off, k, K, a.L[0].veck);
+          hr[i] = load4_guard(a.rad + off, k, K, a.L[0].veck);
         }
-      }
-    };
-    int i = 0;
-    for (int tile = rank; tile * FS_COLS < a.L[0].N; tile += ranks) {
-      load_h0(0);
-      for (int k0 = 0; k0 < K; k0 += FS_K, ++i) {
-        const int s = i % FS_STAGES;
-        if (i >= FS_STAGES) fs_sync(1 + FS_STAGES + s, FS_THREADS);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float4 v = ha[q];
-          if (a.mid) {
-            v.x = hm[q].x - sgnf(v.x) * hr[q].x;
-            v.y = hm[q].y - sgnf(v.y) * hr[q].y;
-            v.z = hm[q].z - sgnf(v.z) * hr[q].z;
-            v.w = hm[q].w - sgnf(v.w) * hr[q].w;
-          }
-          float* d = A0s + s * (FS_K * FS_ROWS) + (kw + q * 4) * FS_ROWS + lane;
-          d[0] = v.x; d[FS_ROWS] = v.y; d[2 * FS_ROWS] = v.z; d[3 * FS_ROWS] = v.w;
-        }
-        if (k0 + FS_K < K) load_h0(k0 + FS_K);
-        fs_arrive(1 + s, FS_THREADS);
       }
     }
-    for (int l = 0; l < a.layers; ++l) {
-      __syncwarp();
-      cluster_arrive();
-      cluster_wait();
+  };
+  auto store_h0 = [&](float* to) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float4 v = ha[i];
+      if (a.mid) {
+        v.x = hm[i].x - sgnf(v.x) * hr[i].x;
+        v.y = hm[i].y - sgnf(v.y) * hr[i].y;
+        v.z = hm[i].z - sgnf(v.z) * hr[i].z;
+        v.w = hm[i].w - sgnf(v.w) * hr[i].w;
+      }
+      float* d = to + (warp * 8 + i * 4) * FS_ROWS + lane;
+      d[0] = v.x; d[FS_ROWS] = v.y; d[2 * FS_ROWS] = v.z; d[3 * FS_ROWS] = v.w;
     }
-    return;
-  }
+  };
+  cluster.sync();  // every CTA of the cluster runs
 
-  int used = 0;
   const int tx = lane & 7, ty = lane >> 3;
   const int r0 = (warp >> 1) * 16 + ty * 4, c0 = (warp & 1) * 32 + tx;  // columns c0, c0 + 8, + 16, + 24
   for (int l = 0; l < a.layers; ++l) {
@@ -435,11 +378,15 @@ __global__ void __launch_bounds__(FS_THREADS, 1) crown_fused_adjoint_kernel(Fuse
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+      if (l == 0) load_h0(0);
       for (int k0 = 0; k0 < L.K; k0 += FS_K, ++used) {
-        const int stage = used % FS_STAGES;
-        fs_sync(1 + stage, ring(used));
-        const float* as = (l == 0 ? A0s + stage * (FS_K * FS_ROWS) : ((l & 1) ? As1 : As0) + k0 * FS_ROWS) + r0;
-        const float* bs = Bs + stage * (FS_COLS * FS_KP) + c0 * FS_KP;
+        if (l == 0) store_h0(A0s + (k0 / FS_K & 1) * (FS_K * FS_ROWS));
+        fs_wait<FS_STAGES - 2>();
+        __syncthreads();                              // this slab is there, and nobody reads the one before it any more
+        fetch();
+        if (l == 0 && k0 + FS_K < L.K) load_h0(k0 + FS_K);
+        const float* as = (l == 0 ? A0s + (k0 / FS_K & 1) * (FS_K * FS_ROWS) : As[l & 1] + k0 * FS_ROWS) + r0;
+        const float* bs = Bs + used % FS_STAGES * (FS_COLS * FS_KP) + c0 * FS_KP;
         const int left = min(FS_K, L.K - k0);
         auto step = [&](int kk) {                     // four terms; past the end of K both operands are zero
           float av[4][4], bv[4][4];
@@ -464,9 +411,8 @@ __global__ void __launch_bounds__(FS_THREADS, 1) crown_fused_adjoint_kernel(Fuse
 #pragma unroll 1
           for (int kk = 0; kk < left; kk += 4) step(kk);
         }
-        fs_arrive(1 + FS_STAGES + stage, ring(used + FS_STAGES));
       }
-      fs_bar();                                       // `red` of the tile before is read
+      __syncthreads();                                // `red` of the tile before is read, A0s too
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int col = n0 + c0 + 8 * j;
@@ -481,7 +427,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) crown_fused_adjoint_kernel(Fuse
         }
       }
       if (l + 1 < a.layers) {
-        float* to = ((l & 1) ? As0 : As1) + r0;
+        float* to = As[(l + 1) & 1] + r0;
         const int np = (L.N + 3) & ~3;                // columns past the end carry zeros
         for (int q = 0; q < ranks; ++q) {
           float* p = cluster.map_shared_rank(to, (rank + q) % ranks);
@@ -497,7 +443,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) crown_fused_adjoint_kernel(Fuse
       const int m_end = min(m0 + FS_ROWS, a.M), d_first = m0 / a.S, d_last = (m_end - 1) / a.S;
       const int c = tid % FS_COLS, half = tid / FS_COLS, col = n0 + c;
       auto reduce = [&](float* to) {
-        fs_bar();
+        __syncthreads();
         for (int d = d_first + half; d <= d_last; d += FS_COMPUTE / FS_COLS) {
           const int lo = max(d * a.S, m0) - m0, hi = min((d + 1) * a.S, m_end) - m0;
           float s = 0.f;
@@ -507,7 +453,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) crown_fused_adjoint_kernel(Fuse
       };
       reduce(L.grad);
       if (L.gsum) {
-        fs_bar();
+        __syncthreads();
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float w = (a.gw && m0 + r0 + i < a.M) ? __ldg(a.gw + m0 + r0 + i) : 1.f;
@@ -517,8 +463,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) crown_fused_adjoint_kernel(Fuse
         reduce(L.gsum);
       }
     }
-    cluster_arrive();
-    cluster_wait();
+    cluster.sync();
   }
 }
 
@@ -527,25 +472,26 @@ __global__ void __launch_bounds__(FS_THREADS, 1) crown_fused_adjoint_kernel(Fuse
 // ---------------------------------------------------------------------------
 static size_t fused_bwd_smem(int kmax) { return ((size_t)2 * kmax * FS_ROWS + FS_STAGES * FS_K * FS_COLS + FS_ROWS) * sizeof(float); }
 static size_t fused_adjoint_smem(int kmax) {
-  return ((size_t)2 * kmax * FS_ROWS + FS_STAGES * (FS_COLS * FS_KP + FS_K * FS_ROWS) + FS_ROWS * (FS_COLS + 1)) * sizeof(float);
+  return ((size_t)2 * kmax * FS_ROWS + FS_STAGES * FS_COLS * FS_KP + 2 * FS_K * FS_ROWS + FS_ROWS * (FS_COLS + 1)) * sizeof(float);
 }
 constexpr int FUSED_SMEM = 220 * 1024;
 
-// Clusters of 2^csl CTAs that run at once, one CTA per SM (a property of the device)
+// Clusters of cs CTAs that run at once, for kernels of up to HALF_SM or FUSED_SMEM bytes of shared memory (a property of the device)
+constexpr size_t HALF_SM = 112 * 1024;
 struct ClusterRoom {
-  std::atomic<int> active[MAX_DEVICES][4];  // [device][csl], plus one; 0: not asked yet
+  std::atomic<int> active[MAX_DEVICES][2][4];  // [device][half an SM or more][log2 cs], plus one; 0: not asked yet
 };
 template <typename Kernel>
-static int clusters_at_once(Kernel kernel, int csl, ClusterRoom& room) {
+static int clusters_at_once(Kernel kernel, int threads, size_t smem, int csl, ClusterRoom& room) {
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return 0;
-  std::atomic<int>& slot = room.active[dev][csl];
+  std::atomic<int>& slot = room.active[dev][smem > HALF_SM][csl];
   int known = slot.load(std::memory_order_relaxed);
   if (known == 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(148 << csl);
-    cfg.blockDim = dim3(FS_THREADS);
-    cfg.dynamicSmemBytes = FUSED_SMEM;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem > HALF_SM ? FUSED_SMEM : HALF_SM;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1 << csl; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
@@ -561,18 +507,18 @@ static int clusters_at_once(Kernel kernel, int csl, ClusterRoom& room) {
 
 // CTAs per cluster for M rows: as many as have a tile in the widest layer, and as let every cluster run at once (0: none do)
 template <typename Kernel>
-static int fused_cluster(Kernel kernel, int M, int widest, ClusterRoom& room) {
+static int fused_cluster(Kernel kernel, int threads, size_t smem, int M, int widest, ClusterRoom& room) {
   const int clusters = ceil_div(M, FS_ROWS), tiles = ceil_div(widest, FS_COLS);
   for (int csl = 3; csl >= 1; --csl)
-    if ((1 << (csl - 1)) < tiles && clusters <= clusters_at_once(kernel, csl, room)) return 1 << csl;
+    if ((1 << (csl - 1)) < tiles && clusters <= clusters_at_once(kernel, threads, smem, csl, room)) return 1 << csl;
   return 0;
 }
 
 template <typename Kernel, typename Args>
-static int fused_launch(Kernel kernel, const Args& a, size_t smem, int cs, cudaStream_t stream, const char* name) {
+static int fused_launch(Kernel kernel, const Args& a, int threads, size_t smem, int cs, cudaStream_t stream, const char* name) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ceil_div(a.M, FS_ROWS) * cs);
-  cfg.blockDim = dim3(FS_THREADS);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -612,10 +558,10 @@ int launch_crown_fused_bwd(FusedSweepArgs a, cudaStream_t stream) {
   static SmemOptIn opt_in;
   static ClusterRoom room;
   if (int rc = ensure_dynamic_smem(crown_fused_bwd_kernel, FUSED_SMEM, opt_in, "crown_fused_bwd_kernel")) return rc;
-  const int cs = fused_cluster(crown_fused_bwd_kernel, a.M, widest, room);
+  const int cs = fused_cluster(crown_fused_bwd_kernel, 256, smem, a.M, widest, room);
   if (cs == 0) return BF_E_UNSUPPORTED;
   timing_begin(T_BWD, stream);
-  const int rc = fused_launch(crown_fused_bwd_kernel, a, smem, cs, stream, "crown_fused_bwd_kernel");
+  const int rc = fused_launch(crown_fused_bwd_kernel, a, 256, smem, cs, stream, "crown_fused_bwd_kernel");
   timing_end(T_BWD, stream, bytes, flops);
   return rc;
 }
@@ -639,10 +585,10 @@ int launch_crown_fused_adjoint(FusedAdjointArgs a, cudaStream_t stream) {
   static SmemOptIn opt_in;
   static ClusterRoom room;
   if (int rc = ensure_dynamic_smem(crown_fused_adjoint_kernel, FUSED_SMEM, opt_in, "crown_fused_adjoint_kernel")) return rc;
-  const int cs = fused_cluster(crown_fused_adjoint_kernel, a.M, widest, room);
+  const int cs = fused_cluster(crown_fused_adjoint_kernel, FS_COMPUTE, smem, a.M, widest, room);
   if (cs == 0) return BF_E_UNSUPPORTED;
   timing_begin(T_ADJ, stream);
-  const int rc = fused_launch(crown_fused_adjoint_kernel, a, smem, cs, stream, "crown_fused_adjoint_kernel");
+  const int rc = fused_launch(crown_fused_adjoint_kernel, a, FS_COMPUTE, smem, cs, stream, "crown_fused_adjoint_kernel");
   timing_end(T_ADJ, stream, bytes, flops);
   return rc;
 }
