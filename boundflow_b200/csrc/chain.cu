@@ -286,37 +286,6 @@ int dispatch_bwd(const bf_chain* c, int layer, const float* A, const float* dpos
                                  M, S, K, N, stream);
 }
 
-int dispatch_bwd_fused(const bf_chain* c, const float* C, const LinearStep* steps, int count, float* delta, const float* mid, const float* rad,
-                       float* partial, int side, int M, int S, int* ptiles, int* done, cudaStream_t stream) {
-  *done = 0;
-  FusedSweepArgs a{};
-  int n = 0;
-  for (; n < count && n < FUSED_LAYERS; ++n) {
-    const bf_layer_desc& L = c->layers[steps[n].layer];
-    const int K = L.n_out, N = L.n_in;
-    if (tc_weights(c, steps[n].layer, false, M, K, N) || (n + 1 == count && partial && !ffma_small_tiles(M, N))) break;
-    const LinearStep& t = steps[n];
-    a.L[n] = FusedSweepLayer{L.W, L.bias, t.dpos, t.dneg, t.epos, t.eneg, t.add, t.out, K, N, 0, 0};
-  }
-  if (n < 2) return BF_OK;
-  const bool whole = n == count;
-  a.layers = n; a.M = M; a.S = S; a.side = side; a.C = C; a.delta = delta;
-  a.thin_top = crown_bwd_is_thin(a.L[0].W, a.L[0].out, a.L[0].K, a.L[0].N) && !a.L[0].dpos && !a.L[0].add;
-  if (whole && partial) {
-    a.mid = mid; a.rad = rad; a.partial = partial;
-    a.ptiles = ceil_div(a.L[n - 1].N, 64);
-  }
-  const int rc = launch_crown_fused_bwd(a, stream);
-  if (rc == BF_E_UNSUPPORTED) return BF_OK;
-  if (rc == BF_OK) *done = n;
-  if (whole && ptiles) *ptiles = a.ptiles;
-  return rc;
-}
-
-bool adjoint_on_ffma(const bf_chain* c, int layer, int M) {
-  return tc_weights(c, layer, true, M, c->layers[layer].n_in, c->layers[layer].n_out) == nullptr;
-}
-
 int dispatch_adjoint(const bf_chain* c, int layer, const float* Hprev, int first_layer, const float* mid,
                             const float* rad, const float* Ahat, const float* dpos, const float* dneg, const float* epos,
                             const float* eneg, const float* pre_l, const float* pre_u, float* hout, float* grad, float* gsum,
@@ -565,45 +534,7 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
   int top = upto_layer - 1;
   while (top > low && chain->layers[top].op != BF_OP_LINEAR && chain->layers[top].op != BF_OP_CONV2D) --top;
   const bool neuron_rows = chain->layers[top].op == BF_OP_CONV2D && (C == nullptr || upto_layer < nl);
-  int start = upto_layer - 1;
-  if (C && !influence) {
-    // Linear layers from the spec rows down, as far as they are alone
-    bf::LinearStep steps[bf::FUSED_LAYERS];
-    int count = 0, relu = -1, flip = 0;
-    for (int i = start; i >= 0 && count < bf::FUSED_LAYERS; --i) {
-      const bf_layer_desc& L = chain->layers[i];
-      if (L.op == BF_OP_FLATTEN) continue;
-      if (L.op == BF_OP_RELU) {
-        if (relu >= 0) break;
-        relu = bf::relu_index_of(chain, i);
-        if (!(alpha_u && beta_u && alpha_l && alpha_u[relu] && beta_u[relu] && alpha_l[relu])) break;
-        continue;
-      }
-      if (L.op != BF_OP_LINEAR) break;
-      bf::LinearStep t{i, nullptr, nullptr, nullptr, nullptr, nullptr, (box && i == low) ? nullptr : ws.buf[flip]};
-      if (relu >= 0) {
-        if (side == BF_SIDE_LOWER) { t.dpos = alpha_l[relu]; t.dneg = alpha_u[relu]; t.eneg = beta_u[relu]; }
-        else { t.dpos = alpha_u[relu]; t.dneg = alpha_l[relu]; t.epos = beta_u[relu]; }
-        t.add = add ? add[relu] : nullptr;
-      }
-      steps[count++] = t;
-      relu = -1;
-      flip ^= 1;
-    }
-    const bool to_input = count > 0 && steps[count - 1].layer == low;
-    int done = 0;
-    const int rc = bf::dispatch_bwd_fused(chain, C, steps, count, ws.cacc, mid, rad, (box && to_input) ? ws.partial : nullptr, side, M, S, &ptiles,
-                                          &done, stream);
-    if (rc != BF_OK) return rc;
-    if (done) {
-      curA = steps[done - 1].out;
-      fused_concretize = box && steps[done - 1].layer == low;
-      start = steps[done - 1].layer - 1;
-      toggle = done & 1;
-      have_c = 1;
-    }
-  }
-  for (int i = start; i >= 0; --i) {
+  for (int i = upto_layer - 1; i >= 0; --i) {
     const bf_layer_desc& L = chain->layers[i];
     if (L.op == BF_OP_FLATTEN) continue;
     if (L.op == BF_OP_RELU) {

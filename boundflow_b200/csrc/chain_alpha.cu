@@ -116,27 +116,10 @@ static int alpha_sweep(const bf_chain* c, const AlphaWs& ws, const float* C, int
                          rad, fused ? ws.partial : nullptr, side, M, S, &ptiles, stream);
     if (rc != BF_OK) return rc;
   } else {
-    // Linear layers from the spec rows down that share one launch
-    LinearStep steps[FUSED_LAYERS];
-    int count = 0, done = 0;
-    for (int r = R; r >= 0 && count < FUSED_LAYERS && c->layers[c->affine_layers[r]].op == BF_OP_LINEAR; --r) {
-      LinearStep t{c->affine_layers[r], nullptr, nullptr, nullptr, nullptr, nullptr, r > 0 ? ws.Ahat[r - 1] : (keep_A0 ? ws.A0 : nullptr)};
-      if (r < R) {
-        if (side == BF_SIDE_LOWER) { t.dpos = ws.sl[r]; t.dneg = ws.au[r]; t.eneg = ws.bu[r]; }
-        else { t.dpos = ws.au[r]; t.dneg = ws.sl[r]; t.epos = ws.bu[r]; }
-        t.add = (use_add && side == BF_SIDE_LOWER) ? ws.addv[r] : nullptr;
-      }
-      steps[count++] = t;
-    }
-    rc = dispatch_bwd_fused(c, C, steps, count, ws.cacc, mid, rad, (fused && count == R + 1) ? ws.partial : nullptr, side, M, S, &ptiles, &done, stream);
+    rc = alpha_bwd_layer(c, ws, c->affine_layers[R], C, nullptr, nullptr, nullptr, nullptr, nullptr, ws.Ahat[R - 1], 0, nullptr,
+                         nullptr, nullptr, side, M, S, nullptr, stream);
     if (rc != BF_OK) return rc;
-    if (done == 0) {
-      rc = alpha_bwd_layer(c, ws, c->affine_layers[R], C, nullptr, nullptr, nullptr, nullptr, nullptr, ws.Ahat[R - 1], 0, nullptr,
-                           nullptr, nullptr, side, M, S, nullptr, stream);
-      if (rc != BF_OK) return rc;
-      done = 1;
-    }
-    for (int r = R - done; r >= 0; --r) {
+    for (int r = R - 1; r >= 0; --r) {
       const float *dpos, *dneg, *epos = nullptr, *eneg = nullptr;
       if (side == BF_SIDE_LOWER) { dpos = ws.sl[r]; dneg = ws.au[r]; eneg = ws.bu[r]; }
       else { dpos = ws.au[r]; dneg = ws.sl[r]; epos = ws.bu[r]; }
@@ -171,21 +154,6 @@ static int alpha_adjoint(const bf_chain* c, const AlphaWs& ws, const float* cons
     const int layer = c->affine_layers[r];
     const bf_layer_desc& L = c->layers[layer];
     const float* hprev = (r == 0) ? ws.A0 : ws.H[(r - 1) & 1];
-    if (R - r <= FUSED_LAYERS) {  // Linear layers up to the last one that share one launch
-      FusedAdjointArgs a{};
-      int n = 0;
-      for (int q = r; q < R && c->layers[c->affine_layers[q]].op == BF_OP_LINEAR && adjoint_on_ffma(c, c->affine_layers[q], M); ++q, ++n) {
-        const bf_layer_desc& Q = c->layers[c->affine_layers[q]];
-        a.L[n] = FusedAdjointLayer{Q.W, Q.bias, ws.Ahat[q], ws.sl[q], ws.au[q], nullptr, ws.bu[q], pre_l[q], pre_u[q], ws.grad[q],
-                                   with_beta ? ws.gsum[q] : nullptr, Q.n_in, Q.n_out, 0};
-      }
-      if (n == R - r) {
-        a.layers = n; a.M = M; a.S = S; a.A0 = hprev; a.gw = with_beta ? gw : nullptr;
-        if (r == 0 && h0_fused) { a.mid = in.mid; a.rad = in.rad; }
-        const int rc = launch_crown_fused_adjoint(a, stream);
-        if (rc != BF_E_UNSUPPORTED) return rc;
-      }
-    }
     int rc;
     if (L.op == BF_OP_LINEAR) {
       float* hout = (r < R - 1) ? ws.H[r & 1] : nullptr;

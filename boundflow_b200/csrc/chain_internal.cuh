@@ -61,18 +61,6 @@ bool tc_may_run(const bf_chain* c, int M);
 int dispatch_bwd(const bf_chain* c, int layer, const float* A, const float* dpos, const float* dneg, const float* epos,
                  const float* eneg, const float* add, float* A_prev, float* delta, int accumulate, const float* mid,
                  const float* rad, float* partial, int side, int M, int S, int* ptiles, cudaStream_t stream);
-// One step of a backward sweep through Linear layers, as dispatch_bwd takes it.
-struct LinearStep {
-  int layer;
-  const float *dpos, *dneg, *epos, *eneg, *add;
-  float* out;
-};
-// The first layers of a sweep in one launch where the layer-by-layer path would take them on FFMA tiles: `done` receives their number
-// (0: none).  `partial` belongs to the last of the `count` steps; delta is overwritten.
-int dispatch_bwd_fused(const bf_chain* c, const float* C, const LinearStep* steps, int count, float* delta, const float* mid, const float* rad,
-                       float* partial, int side, int M, int S, int* ptiles, int* done, cudaStream_t stream);
-// True when layer `layer` of an adjoint sweep runs on FFMA tiles.
-bool adjoint_on_ffma(const bf_chain* c, int layer, int M);
 int dispatch_adjoint(const bf_chain* c, int layer, const float* Hprev, int first_layer, const float* mid, const float* rad,
                      const float* Ahat, const float* dpos, const float* dneg, const float* epos, const float* eneg,
                      const float* pre_l, const float* pre_u, float* hout, float* grad, float* gsum, int M, int S,

@@ -113,10 +113,6 @@ __global__ void __launch_bounds__(128) crown_bwd_thin_kernel(const float* __rest
   }
 }
 
-bool crown_bwd_is_thin(const float* W, const float* A_prev, int K, int N) {
-  return A_prev && K <= THIN_KMAX && N % 4 == 0 && ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(A_prev)) & 15u) == 0;
-}
-
 // 128 x 128 tiles leave most of the 148 SMs idle on small problems: below one CTA per SM the kernels switch to 64 x 64 tiles
 bool ffma_small_tiles(int M, int N) { return (long long)ceil_div(M, BM) * ceil_div(N, BN) < 148; }
 // ... and 32 x 64 tiles when even the 64 x 64 tiles give fewer CTAs than SMs
@@ -131,7 +127,8 @@ int launch_crown_bwd_linear(const float* A, const float* dpos, const float* dneg
                             const float* add, const float* W, const float* kbias, float* A_prev, float* delta,
                             int accumulate, const float* mid, const float* rad, float* partial, int side, int M, int S,
                             int K, int N, cudaStream_t stream) {
-  if (!dpos && !add && !partial && crown_bwd_is_thin(W, A_prev, K, N)) {
+  if (!dpos && !add && !partial && A_prev && K <= THIN_KMAX && N % 4 == 0 &&
+      ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(A_prev)) & 15u) == 0) {
     const int cols = ceil_div(N / 4, 128);
     int rows = THIN_ROWS;
     while (rows > 4 && ceil_div(M, rows) * cols < 4 * 148) rows /= 2;

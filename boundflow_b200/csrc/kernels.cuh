@@ -18,45 +18,6 @@ int launch_crown_adjoint_linear(const float* Hprev, int first_layer, const float
                                 float* hout, float* grad, float* gsum, int M, int S, int K, int N, cudaStream_t stream,
                                 const float* gw = nullptr);
 
-// true when [M,N] takes tiles of 64 (or fewer) rows and 64 columns
-bool ffma_small_tiles(int M, int N);
-// true when a layer without a ReLU in front takes crown_bwd_thin_kernel
-bool crown_bwd_is_thin(const float* W, const float* A_prev, int K, int N);
-
-// crown_fused.cu: sweeps of few rows through consecutive Linear layers in one launch (BF_E_UNSUPPORTED: layer by layer)
-constexpr int FUSED_LAYERS = 8;
-struct FusedSweepLayer {                           // A_prev[M,N] = relu_bwd(A)[M,K] * W[K,N]
-  const float *W, *kbias;                          // W as stored [n_out = K, n_in = N]
-  const float *dpos, *dneg, *epos, *eneg, *add;    // ReLU in front (dpos null: none)
-  float* out;                                      // [M,N]; may be null for the last layer only
-  int K, N;
-  int vec, veck;                                   // set by the launcher: 16-byte accesses along N / K
-};
-struct FusedSweepArgs {
-  FusedSweepLayer L[FUSED_LAYERS];                 // from the spec rows downwards
-  int layers, M, S, kmax, ptiles, side;
-  int thin_top;                                    // the first layer's row sums run as in crown_bwd_thin_kernel
-  const float* C;                                  // [M, L[0].K]
-  float* delta;                                    // [M], overwritten
-  const float *mid, *rad;                          // with `partial`: concretisation of the last layer's rows
-  float* partial;                                  // [M, ptiles]
-};
-int launch_crown_fused_bwd(FusedSweepArgs a, cudaStream_t stream);
-struct FusedAdjointLayer {                         // g = h[M,K] * W[N,K]^T + nbias ; h' = d*g + e ; gradient sums
-  const float *W, *nbias, *Ahat, *dpos, *dneg, *epos, *eneg, *pre_l, *pre_u;
-  float *grad, *gsum;
-  int K, N;
-  int veck;                                        // set by the launcher
-};
-struct FusedAdjointArgs {
-  FusedAdjointLayer L[FUSED_LAYERS];               // from the input upwards
-  int layers, M, S, kmax;
-  const float* A0;                                 // [M, L[0].K]: points, or coefficients when mid is given (points mid - sgn(A0) * rad)
-  const float *mid, *rad;
-  const float* gw;                                 // [M] or null: row weights of gsum
-};
-int launch_crown_fused_adjoint(FusedAdjointArgs a, cudaStream_t stream);
-
 // crown_tc.cu (tcgen05 3xTF32 path; weights pre-packed by tc_pack_weights)
 size_t tc_packed_bytes(int N, int K, int tile_rows = 0);
 int tc_pack_weights(const float* W, int rows, int cols, int transposed, unsigned char* out, cudaStream_t stream, int tile_rows = 0);
