@@ -1,7 +1,7 @@
 // CROWN backward sweep through Linear layers (fused with the ReLU backward
 // transformer and, on the first layer, with the concretisation) and the adjoint
 // (alpha-gradient) sweep, as FP32 FFMA tiles.
-#include "gemm_ffma.cuh"
+#include "gemm_small.cuh"
 #include <stdlib.h>
 
 #include "kernels.cuh"
@@ -17,31 +17,23 @@ struct BwdEpilogue {
   const float* rad;      // [D,N]
   float* partial;        // [M, ntiles] concretisation partial sums or nullptr
   int side;              // BF_SIDE_LOWER: a*mid - |a|*rad ; BF_SIDE_UPPER: a*mid + |a|*rad
-  int ntiles;            // column tiles; 32-row tiles: CTAs of a further column compute the row sums
+  int ntiles;            // column tiles; 32 x 64 tiles: CTAs of a further column compute the row sums
 };
 
 template <int PRO, int MH, int NH>
 __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_bwd_linear_kernel(GemmArgs g, BwdEpilogue e) {
-  __shared__ __align__(16) float smem[MH == 0 ? SMALL_SMEM_FLOATS : MAINLOOP_SMEM_FLOATS];
-  constexpr int TM = (MH == 0) ? 32 : 64 * MH, MR = (MH == 0) ? 2 : 4 * MH;
+  __shared__ __align__(16) float smem[MAINLOOP_SMEM_FLOATS];
+  constexpr int TM = 64 * MH, MR = 4 * MH;
   const int m0 = blockIdx.x * TM, n0 = blockIdx.y * (64 * NH);
   float acc[8][8];
-  if constexpr (MH == 0) {
-    if ((int)blockIdx.y == e.ntiles) {
-      prologue_row_sums(g, m0);
-      return;
-    }
-    gemm_small_mainloop<PRO, false>(g, m0, n0, acc, smem);
-  } else {
-    gemm_mainloop<PRO, false, MH, NH>(g, m0, n0, acc, smem);
-  }
+  gemm_mainloop<PRO, false, MH, NH>(g, m0, n0, acc, smem);
 
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const bool vN = g.vecN != 0;
   const float sgn = (e.side == BF_SIDE_LOWER) ? -1.f : 1.f;
 #pragma unroll
   for (int i = 0; i < MR; ++i) {
-    const int row = m0 + tile_row<MH>(ty, i);
+    const int row = m0 + tile_row(ty, i);
     const bool row_ok = row < g.M;
     float p = 0.f;
 #pragma unroll
@@ -70,6 +62,63 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_bwd_linear_kernel(GemmA
     }
   }
 }
+
+// 32 x 64 tiles of a small problem (gemm_small.cuh); CTAs of column e.ntiles form the row sums.
+__global__ void __launch_bounds__(GS_THREADS, 2) crown_bwd_small_kernel(GemmArgs g, BwdEpilogue e) {
+  extern __shared__ __align__(16) float dsmem[];
+  float* As = dsmem;
+  float* Bs = As + GS_STAGES * GS_A_WORDS;
+  float* part = Bs + GS_STAGES * GS_B_WORDS<false>;  // [row]: concretisation sums of the right half of the tile
+  const int m0 = blockIdx.x * GS_ROWS, n0 = blockIdx.y * GS_COLS, tid = threadIdx.x;
+  if ((int)blockIdx.y == e.ntiles) {
+    prologue_row_sums(g, m0);
+    return;
+  }
+  const int lane = tid & 31, warp = tid >> 5, tx = lane & 7, ty = lane >> 3;
+  const int r0 = (warp >> 1) * 16 + ty * 4, c0 = (warp & 1) * 32 + tx * 4, col = n0 + c0;
+  const bool vN = g.vecN != 0;
+  const float sgn = (e.side == BF_SIDE_LOWER) ? -1.f : 1.f;
+  float p[4] = {0.f, 0.f, 0.f, 0.f};
+  if (tid >= GS_COMPUTE) {
+    gs_fill<PRO_RELU, false>(g, m0, n0, As, Bs, tid - GS_COMPUTE);
+  } else {
+    float4 md[4], rd[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      md[i] = rd[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (e.partial && col < g.N) {
+        const size_t off = (size_t)(min(m0 + r0 + i, g.M - 1) / g.S) * g.N;
+        md[i] = load4_guard(e.mid + off, col, g.N, vN);
+        rd[i] = load4_guard(e.rad + off, col, g.N, vN);
+      }
+    }
+    float acc[4][4];
+    gs_compute<false>(g.K, As, Bs, r0, c0, acc);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 v = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      if (m0 + r0 + i < g.M && col < g.N && e.out) store4_guard(e.out + (size_t)(m0 + r0 + i) * g.N, col, g.N, vN, v);
+      if (e.partial) {  // the order of the 64-column kernels: sixteen groups of four columns, pairwise
+        p[i] += v.x * md[i].x + sgn * fabsf(v.x) * rd[i].x;
+        p[i] += v.y * md[i].y + sgn * fabsf(v.y) * rd[i].y;
+        p[i] += v.z * md[i].z + sgn * fabsf(v.z) * rd[i].z;
+        p[i] += v.w * md[i].w + sgn * fabsf(v.w) * rd[i].w;
+        p[i] += __shfl_xor_sync(0xffffffffu, p[i], 1);
+        p[i] += __shfl_xor_sync(0xffffffffu, p[i], 2);
+        p[i] += __shfl_xor_sync(0xffffffffu, p[i], 4);
+        if ((warp & 1) && tx == 0) part[r0 + i] = p[i];
+      }
+    }
+  }
+  if (!e.partial) return;  // uniform across the CTA
+  __syncthreads();
+  if (tid < GS_COMPUTE && !(warp & 1) && tx == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (m0 + r0 + i < g.M) e.partial[(size_t)(m0 + r0 + i) * e.ntiles + blockIdx.y] = p[i] + part[r0 + i];
+  }
+}
+constexpr int GS_BWD_SMEM = (GS_STAGES * (GS_A_WORDS + GS_B_WORDS<false>) + GS_ROWS) * (int)sizeof(float);
 
 // Top layer of a sweep (no ReLU in front, K = spec width <= 16): A_prev[M,N] = A[M,K] * W[K,N] and
 // delta[m] (+)= sum_k A[m,k] * kbias[k].  A store-bound pass, so no tiles: a thread keeps its four
@@ -151,9 +200,11 @@ int launch_crown_bwd_linear(const float* A, const float* dpos, const float* dneg
   g.delta = delta; g.accumulate = accumulate;
   BwdEpilogue e{A_prev, mid, rad, partial, side, crown_bwd_partial_tiles(N, M)};
   timing_begin(T_BWD, stream);
-  if (ffma_quarter_tiles(M, N)) {  // 32 x 64 tiles
-    dim3 grid(ceil_div(M, 32), e.ntiles + (delta ? 1 : 0));
-    crown_bwd_linear_kernel<PRO_RELU, 0, 1><<<grid, GEMM_THREADS, 0, stream>>>(g, e);
+  if (ffma_quarter_tiles(M, N)) {
+    static SmemOptIn opt_in;
+    if (int rc = ensure_dynamic_smem(crown_bwd_small_kernel, GS_BWD_SMEM, opt_in, "crown_bwd_small_kernel")) return rc;
+    dim3 grid(ceil_div(M, GS_ROWS), e.ntiles + (delta ? 1 : 0));
+    crown_bwd_small_kernel<<<grid, GS_THREADS, GS_BWD_SMEM, stream>>>(g, e);
   } else if (ffma_small_tiles(M, N)) {  // 64 x 64 tiles: four times as many CTAs
     dim3 grid(ceil_div(M, 64), ceil_div(N, 64));
     crown_bwd_linear_kernel<PRO_RELU, 1, 1><<<grid, GEMM_THREADS, 0, stream>>>(g, e);
@@ -195,18 +246,17 @@ static_assert(ADJ_SMEM_BYTES >= MAINLOOP_SMEM_FLOATS * (int)sizeof(float), "stag
 template <int PRO, int MH, int NH>
 __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_adjoint_linear_kernel(GemmArgs g, AdjEpilogue e) {
   extern __shared__ __align__(16) float dsmem[];
-  constexpr int TM = (MH == 0) ? 32 : 64 * MH, TN = 64 * NH, MR = (MH == 0) ? 2 : 4 * MH;
+  constexpr int TM = 64 * MH, TN = 64 * NH, MR = 4 * MH;
   const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
   float acc[8][8];
-  if constexpr (MH == 0) gemm_small_mainloop<PRO, true>(g, m0, n0, acc, dsmem);
-  else gemm_mainloop<PRO, true, MH, NH>(g, m0, n0, acc, dsmem);
+  gemm_mainloop<PRO, true, MH, NH>(g, m0, n0, acc, dsmem);
   // the main loop ends with __syncthreads(): the slabs may now be overwritten by the stage tile
 
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const bool vN = g.vecN != 0;
 #pragma unroll
   for (int i = 0; i < MR; ++i) {
-    const int rl = tile_row<MH>(ty, i);
+    const int rl = tile_row(ty, i);
     const int row = m0 + rl;
 #pragma unroll
     for (int jb = 0; jb < NH; ++jb) {
@@ -265,7 +315,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_adjoint_linear_kernel(G
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < MR; ++i) {
-      const int rl = tile_row<MH>(ty, i);
+      const int rl = tile_row(ty, i);
       const int row = m0 + rl;
 #pragma unroll
       for (int jb = 0; jb < NH; ++jb) {
@@ -291,6 +341,84 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_adjoint_linear_kernel(G
   }
 }
 
+// 32 x 64 tiles of a small problem (gemm_small.cuh).  What the epilogue needs is loaded first, without branches (rows and columns
+// clamped): as guarded loads after the multiply loop its seven arrays took 2 to 5 us of a 12 us launch.
+template <int PRO>
+__global__ void __launch_bounds__(GS_THREADS, 1) crown_adjoint_small_kernel(GemmArgs g, AdjEpilogue e) {
+  extern __shared__ __align__(16) float dsmem[];
+  float* As = dsmem;
+  float* Bs = As + GS_STAGES * GS_A_WORDS;
+  float* red = Bs + GS_STAGES * GS_B_WORDS<true>;  // [row][GS_COLS + 1]
+  const int m0 = blockIdx.x * GS_ROWS, n0 = blockIdx.y * GS_COLS, tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5, tx = lane & 7, ty = lane >> 3;
+  const int r0 = (warp >> 1) * 16 + ty * 4, c0 = (warp & 1) * 32 + tx;
+  float acc[4][4];
+  if (tid >= GS_COMPUTE) {
+    gs_fill<PRO, true>(g, m0, n0, As, Bs, tid - GS_COMPUTE);
+  } else {
+    float ah[4][4], dp[4][4], dn[4][4], ep[4][4], en[4][4], pl[4][4], pu[4][4], nb[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) nb[j] = e.nbias ? __ldg(e.nbias + min(n0 + c0 + 8 * j, g.N - 1)) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = min(m0 + r0 + i, g.M - 1);
+      const size_t at = (size_t)row * g.N, dom = (size_t)(row / g.S) * g.N;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int col = min(n0 + c0 + 8 * j, g.N - 1);
+        ah[i][j] = __ldg(e.Ahat + at + col);
+        dp[i][j] = __ldg(e.dpos + dom + col);
+        dn[i][j] = __ldg(e.dneg + dom + col);
+        ep[i][j] = e.epos ? __ldg(e.epos + dom + col) : 0.f;
+        en[i][j] = e.eneg ? __ldg(e.eneg + dom + col) : 0.f;
+        pl[i][j] = __ldg(e.pre_l + dom + col);
+        pu[i][j] = __ldg(e.pre_u + dom + col);
+      }
+    }
+    gs_compute<true>(g.K, As, Bs, r0, c0, acc);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = m0 + r0 + i;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int col = n0 + c0 + 8 * j;
+        const float gg = acc[i][j] + nb[j];
+        const bool sel = ah[i][j] >= 0.f;
+        const float h = (sel ? dp[i][j] : dn[i][j]) * gg + (sel ? ep[i][j] : en[i][j]);
+        if (e.hout && row < g.M && col < g.N) e.hout[(size_t)row * g.N + col] = h;
+        red[(r0 + i) * (GS_COLS + 1) + c0 + 8 * j] = (sel && pl[i][j] < 0.f && pu[i][j] > 0.f) ? ah[i][j] * gg : 0.f;
+        acc[i][j] = gg;
+      }
+    }
+  }
+  // sums over the rows of every domain that fall into this tile
+  const int m_end = min(m0 + GS_ROWS, g.M), d_first = m0 / g.S, d_last = (m_end - 1) / g.S;
+  const int c = tid % GS_COLS, col = n0 + c;
+  auto reduce = [&](float* to) {
+    __syncthreads();
+    for (int d = d_first + tid / GS_COLS; d <= d_last; d += GS_THREADS / GS_COLS) {
+      const int lo = max(d * g.S, m0) - m0, hi = min((d + 1) * g.S, m_end) - m0;
+      float s = 0.f;
+      for (int r = lo; r < hi; ++r) s += red[r * (GS_COLS + 1) + c];
+      if (col < g.N) atomicAdd(to + (size_t)d * g.N + col, s);
+    }
+  };
+  reduce(e.grad);
+  if (e.gsum) {  // sum over the domain's rows of g itself (beta)
+    __syncthreads();
+    if (tid < GS_COMPUTE) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float w = e.gw ? __ldg(e.gw + min(m0 + r0 + i, g.M - 1)) : 1.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) red[(r0 + i) * (GS_COLS + 1) + c0 + 8 * j] = e.gw ? acc[i][j] * w : acc[i][j];
+      }
+    }
+    reduce(e.gsum);
+  }
+}
+constexpr int GS_ADJ_SMEM = (GS_STAGES * (GS_A_WORDS + GS_B_WORDS<true>) + GS_ROWS * (GS_COLS + 1)) * (int)sizeof(float);
+
 int launch_crown_adjoint_linear(const float* Hprev, int first_layer, const float* mid, const float* rad, const float* W,
                                 const float* nbias, const float* Ahat, const float* dpos, const float* dneg,
                                 const float* epos, const float* eneg, const float* pre_l, const float* pre_u,
@@ -309,7 +437,7 @@ int launch_crown_adjoint_linear(const float* Hprev, int first_layer, const float
   AdjEpilogue e{nbias, Ahat, dpos, dneg, epos, eneg, pre_l, pre_u, hout, grad, gsum, gw};
   // 32-row tiles only while a domain's S rows still touch at most two row tiles (two atomic addends commute: deterministic sums)
   const bool small = ffma_small_tiles(M, N), quarter = ffma_quarter_tiles(M, N) && S <= 32;
-  dim3 grid(ceil_div(M, quarter ? 32 : (small ? 64 : BM)), ceil_div(N, small ? 64 : BN));
+  dim3 grid(ceil_div(M, quarter ? GS_ROWS : (small ? 64 : BM)), ceil_div(N, small ? 64 : BN));
   timing_begin(T_ADJ, stream);
 #define BF_ADJ_LAUNCH(PRO_, MH_, NH_, slot)                                                                                     \
   {                                                                                                                             \
@@ -318,12 +446,18 @@ int launch_crown_adjoint_linear(const float* Hprev, int first_layer, const float
       return rc;                                                                                                                \
     crown_adjoint_linear_kernel<PRO_, MH_, NH_><<<grid, GEMM_THREADS, ADJ_SMEM_BYTES, stream>>>(g, e);                          \
   }
+#define BF_ADJ_SMALL(PRO_, slot)                                                                                                  \
+  {                                                                                                                             \
+    if (int rc = ensure_dynamic_smem(crown_adjoint_small_kernel<PRO_>, GS_ADJ_SMEM, opt_in[slot], "crown_adjoint_small_kernel")) return rc; \
+    crown_adjoint_small_kernel<PRO_><<<grid, GS_THREADS, GS_ADJ_SMEM, stream>>>(g, e);                                            \
+  }
   if (first_layer) {
-    if (quarter) BF_ADJ_LAUNCH(PRO_H0, 0, 1, 4) else if (small) BF_ADJ_LAUNCH(PRO_H0, 1, 1, 0) else BF_ADJ_LAUNCH(PRO_H0, 2, 2, 1)
+    if (quarter) BF_ADJ_SMALL(PRO_H0, 4) else if (small) BF_ADJ_LAUNCH(PRO_H0, 1, 1, 0) else BF_ADJ_LAUNCH(PRO_H0, 2, 2, 1)
   } else {
-    if (quarter) BF_ADJ_LAUNCH(PRO_PLAIN, 0, 1, 5) else if (small) BF_ADJ_LAUNCH(PRO_PLAIN, 1, 1, 2) else BF_ADJ_LAUNCH(PRO_PLAIN, 2, 2, 3)
+    if (quarter) BF_ADJ_SMALL(PRO_PLAIN, 5) else if (small) BF_ADJ_LAUNCH(PRO_PLAIN, 1, 1, 2) else BF_ADJ_LAUNCH(PRO_PLAIN, 2, 2, 3)
   }
 #undef BF_ADJ_LAUNCH
+#undef BF_ADJ_SMALL
   timing_end(T_ADJ, stream, 4.0 * (double)M * K + 8.0 * (double)M * N, 2.0 * (double)M * K * N);
   BF_CHECK_LAUNCH("crown_adjoint_linear_kernel");
   return BF_OK;

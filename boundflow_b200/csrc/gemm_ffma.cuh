@@ -7,7 +7,7 @@
 // 64x128 or 128x64 tiles (4x4 ... 4x8 micro-tiles, same thread mapping, the unused half
 // simply absent) put four times as many CTAs on problems whose 128x128 tiles would leave
 // most SMs idle; problems that still do not give every SM a CTA take the 32x64 tiles of
-// gemm_small_mainloop (MH == 0 in the kernels).  `f` is the
+// gemm_small.cuh.  `f` is the
 // per-element prologue applied while the A slab moves global -> shared:
 //   PRO_PLAIN : identity                    (top linear layer, adjoint hidden layers)
 //   PRO_RELU  : ReLU backward transformer   (sign-select slope, intercept and bias row sums)
@@ -250,184 +250,8 @@ __device__ __forceinline__ void gemm_mainloop(const GemmArgs& g, const int m0, c
   }
 }
 
-// Main loop for 32 x 64 tiles (2 x 4 outputs per thread, rows / columns as tile_row<0> and tile_col) with 64-deep slabs: a
-// problem with less than one 64 x 64 tile per SM is bound by the latency of its slabs, so it takes a quarter of them, with six to
-// fourteen 128-bit loads of a thread in flight (1152 x 256 x 256: 20 -> 14 us).  Every sum runs over k in ascending order as
-// above.  Row sums are left to prologue_row_sums (CTAs of their own).  On alpha-CROWN loops with ten specs, against 16-deep slabs:
-// 128 inputs, five 256-wide layers, 20 steps 5.64 -> 5.06 ms; 37 nodes, four 512-wide layers, 10 steps 3.69 -> 3.29 ms.
-// Transposed operands are XOR-swizzled in groups of four rows / columns: stores conflict two-way, reads not at all.
-constexpr int SMALL_K = 64;
-constexpr int SMALL_SMEM_FLOATS = 2 * SMALL_K * (32 + 64);
-
-template <int PRO, bool B_NT>
-__device__ __forceinline__ void gemm_small_mainloop(const GemmArgs& g, const int m0, const int n0, float (&acc)[8][8], float* __restrict__ smem) {
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int lrow = ty, lk = tx * 4;                 // loader: rows lrow, lrow + 16 (columns lrow + 16 i of B_NT), k offset lk
-  const bool vK = g.vecK != 0, vN = g.vecN != 0;
-  float* As = smem;
-  float* Bs = smem + 2 * SMALL_K * 32;
-  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-  size_t off[2];
-  bool live[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int m = m0 + lrow + 16 * i;
-    live[i] = m < g.M;
-    off[i] = live[i] ? (size_t)(m / g.S) * g.K : 0;
-  }
-
-  float4 ar[2], dp[2], dn[2], ad[2], br[4];         // PRO_H0 keeps mid / rad in dp / dn
-  bool got[2];
-  auto load_slab = [&](int k0) {
-    const int k = k0 + lk;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      got[i] = live[i] && k < g.K;
-      ar[i] = dp[i] = dn[i] = ad[i] = z4;
-      if (got[i]) {
-        ar[i] = load4_guard(g.A + (size_t)(m0 + lrow + 16 * i) * g.K, k, g.K, vK);
-        if (PRO == PRO_RELU && g.dpos) {
-          dp[i] = load4_guard(g.dpos + off[i], k, g.K, vK);
-          dn[i] = load4_guard(g.dneg + off[i], k, g.K, vK);
-          if (g.add) ad[i] = load4_guard(g.add + off[i], k, g.K, vK);
-        } else if (PRO == PRO_H0) {
-          dp[i] = load4_guard(g.mid + off[i], k, g.K, vK);
-          dn[i] = load4_guard(g.rad + off[i], k, g.K, vK);
-        }
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      br[i] = z4;
-      if (B_NT) {
-        const int n = n0 + lrow + 16 * i;
-        if (n < g.N && k < g.K) br[i] = load4_guard(g.Bm + (size_t)n * g.K, k, g.K, vK);
-      } else {
-        const int kk = k0 + lrow + 16 * i;
-        if (kk < g.K && n0 + lk < g.N) br[i] = load4_guard(g.Bm + (size_t)kk * g.N, n0 + lk, g.N, vN);
-      }
-    }
-  };
-  auto scaled = [&](int i) -> float4 {
-    float4 a = ar[i];
-    if (!got[i]) return a;
-    if (PRO == PRO_RELU && g.dpos) {
-      a.x = a.x * (a.x >= 0.f ? dp[i].x : dn[i].x) + ad[i].x;
-      a.y = a.y * (a.y >= 0.f ? dp[i].y : dn[i].y) + ad[i].y;
-      a.z = a.z * (a.z >= 0.f ? dp[i].z : dn[i].z) + ad[i].z;
-      a.w = a.w * (a.w >= 0.f ? dp[i].w : dn[i].w) + ad[i].w;
-    } else if (PRO == PRO_H0) {
-      a.x = dp[i].x - sgnf(a.x) * dn[i].x;
-      a.y = dp[i].y - sgnf(a.y) * dn[i].y;
-      a.z = dp[i].z - sgnf(a.z) * dn[i].z;
-      a.w = dp[i].w - sgnf(a.w) * dn[i].w;
-    }
-    return a;
-  };
-  auto store_slab = [&](int stage) {
-    float* as = As + stage * SMALL_K * 32;
-    float* bs = Bs + stage * SMALL_K * 64;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float4 a = scaled(i);
-      float* d = as + lk * 32 + ((lrow + 16 * i) ^ ((tx & 7) << 2));
-      d[0] = a.x; d[32] = a.y; d[64] = a.z; d[96] = a.w;
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (B_NT) {
-        float* d = bs + lk * 64 + ((lrow + 16 * i) ^ (tx << 2));
-        d[0] = br[i].x; d[64] = br[i].y; d[128] = br[i].z; d[192] = br[i].w;
-      } else {
-        *reinterpret_cast<float4*>(bs + (lrow + 16 * i) * 64 + lk) = br[i];
-      }
-    }
-  };
-
-  const int nk = (g.K + SMALL_K - 1) / SMALL_K;
-  load_slab(0);
-  store_slab(0);
-  __syncthreads();
-  for (int kt = 0; kt < nk; ++kt) {
-    if (kt + 1 < nk) load_slab((kt + 1) * SMALL_K);
-    const float* as = As + (kt & 1) * SMALL_K * 32;
-    const float* bs = Bs + (kt & 1) * SMALL_K * 64;
-    const int left = g.K - kt * SMALL_K;              // the last slab ends with its last 16 columns
-    for (int q = 0; q < SMALL_K && q < left; q += 16)
-#pragma unroll
-    for (int kk = q; kk < q + 16; ++kk) {
-      const float2 a = *reinterpret_cast<const float2*>(&as[kk * 32 + ((ty * 2) ^ (((kk >> 2) & 7) << 2))]);
-      const float4 b = *reinterpret_cast<const float4*>(&bs[kk * 64 + (B_NT ? ((tx * 4) ^ (((kk >> 2) & 15) << 2)) : tx * 4)]);
-      acc[0][0] = fmaf(a.x, b.x, acc[0][0]); acc[0][1] = fmaf(a.x, b.y, acc[0][1]);
-      acc[0][2] = fmaf(a.x, b.z, acc[0][2]); acc[0][3] = fmaf(a.x, b.w, acc[0][3]);
-      acc[1][0] = fmaf(a.y, b.x, acc[1][0]); acc[1][1] = fmaf(a.y, b.y, acc[1][1]);
-      acc[1][2] = fmaf(a.y, b.z, acc[1][2]); acc[1][3] = fmaf(a.y, b.w, acc[1][3]);
-    }
-    if (kt + 1 < nk) store_slab((kt + 1) & 1);
-    __syncthreads();
-  }
-}
-
-// delta[m] (+)= sum_k a * intercept + lam * kbias of 32 rows, in gemm_mainloop's order: four threads per row, thread p the
-// columns 16 t + 4 p .. + 3 of every t, then their sums pairwise.
-__device__ __forceinline__ void prologue_row_sums(const GemmArgs& g, const int m0) {
-  const int row = m0 + ((int)threadIdx.x >> 2), lkc = ((int)threadIdx.x & 3) * 4;
-  if (threadIdx.x >= 128) return;
-  const bool vK = g.vecK != 0, live = row < g.M;
-  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  const float* pa = g.A + (size_t)(live ? row : 0) * g.K;
-  const size_t off = live ? (size_t)(row / g.S) * g.K : 0;
-  float r = 0.f;
-  constexpr int U = 4;                              // column groups in flight
-  for (int k0 = lkc; k0 < g.K && live; k0 += 16 * U) {
-    float4 a[U], kb[U], dp[U], dn[U], ep[U], en[U], ad[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k = k0 + 16 * u;
-      a[u] = kb[u] = dp[u] = dn[u] = ep[u] = en[u] = ad[u] = z4;
-      if (k < g.K) {
-        a[u] = load4_guard(pa, k, g.K, vK);
-        if (g.kbias) kb[u] = load4_guard(g.kbias, k, g.K, vK);
-        if (g.dpos) {
-          dp[u] = load4_guard(g.dpos + off, k, g.K, vK);
-          dn[u] = load4_guard(g.dneg + off, k, g.K, vK);
-          if (g.epos) ep[u] = load4_guard(g.epos + off, k, g.K, vK);
-          if (g.eneg) en[u] = load4_guard(g.eneg + off, k, g.K, vK);
-          if (g.add) ad[u] = load4_guard(g.add + off, k, g.K, vK);
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (k0 + 16 * u >= g.K) break;
-      if (g.dpos) {
-#define BF_ROW_SUM(c)                                                          \
-  {                                                                            \
-    const bool sel = a[u].c >= 0.f;                                            \
-    const float lam = a[u].c * (sel ? dp[u].c : dn[u].c) + ad[u].c;            \
-    r += a[u].c * (sel ? ep[u].c : en[u].c);                                   \
-    r = fmaf(lam, kb[u].c, r);                                                 \
-  }
-        BF_ROW_SUM(x) BF_ROW_SUM(y) BF_ROW_SUM(z) BF_ROW_SUM(w)
-#undef BF_ROW_SUM
-      } else {
-        r += a[u].x * kb[u].x + a[u].y * kb[u].y + a[u].z * kb[u].z + a[u].w * kb[u].w;
-      }
-    }
-  }
-  r += __shfl_xor_sync(0xffffffffu, r, 1);
-  r += __shfl_xor_sync(0xffffffffu, r, 2);
-  if (lkc == 0 && live) g.delta[row] = g.accumulate ? (g.delta[row] + r) : r;
-}
-
-// Row / column of micro-tile element (i, j) inside the CTA tile (MH == 0: 32-row tiles, two rows per thread).
-template <int MH = 2>
+// Row / column of micro-tile element (i, j) inside the CTA tile.
 __device__ __forceinline__ int tile_row(int ty, int i) {
-  if (MH == 0) return ty * 2 + i;
   return (i < 4) ? (ty * 4 + i) : (64 + ty * 4 + (i - 4));
 }
 __device__ __forceinline__ int tile_col(int tx, int jb) { return jb * 64 + tx * 4; }
