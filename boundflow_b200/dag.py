@@ -58,6 +58,7 @@ class DagTrace:
     input_name: str = ""
     norm_p: int = 0     # _lib.NORM_BOX, or 1 / 2 for an L1 / L2 ball (then mid = centre and rad = eps, the bounding box)
     eps: float = 0.0
+    clamped: bool = False  # a split was applied; without one no domain can be infeasible
 
 
 def _params(module: Any, device: torch.device) -> Dict[str, torch.Tensor]:
@@ -164,6 +165,7 @@ def forward_ibp_dag(module: Any, input_spec: Any, relu_split_state: Optional[Map
                 n = _numel(tr.shape[x])
                 t8, stride = _split_tensor(sp, B, n, device, x)
                 pl, pu = pl.clone(), pu.clone()
+                tr.clamped = True
                 _lib.check(lib.bf_relu_split_apply(_lib.ptr(pl), _lib.ptr(pu), _lib.ptr(t8), stride, _lib.ptr(tr.infeasible), B, n, s))
             tr.pre_l[x], tr.pre_u[x] = pl, pu
             yl, yu = torch.empty_like(pl), torch.empty_like(pu)
@@ -373,7 +375,7 @@ def crown_dag(module: Any, input_spec: Any, linear_spec_C: Optional[torch.Tensor
     lib = _lib.load()
     spec = normalize_input_spec(input_spec)
     tr = trace if trace is not None else forward_ibp_dag(module, spec, relu_split_state)
-    if int(tr.infeasible.sum()) != 0:
+    if tr.clamped and int(tr.infeasible.sum()) != 0:
         raise ValueError("infeasible relu split: lower > upper")
     device, B = tr.mid.device, tr.B
     params = _params(module, device)
@@ -555,7 +557,7 @@ def alpha_beta_crown_dag(module: Any, input_spec: Any, linear_spec_C: Optional[t
     with_beta = bool(optimize_beta and relu_split_state and objective == "lower")
     spec = normalize_input_spec(input_spec)
     tr = forward_ibp_dag(module, spec, relu_split_state)
-    if int(tr.infeasible.sum()) != 0:
+    if tr.clamped and int(tr.infeasible.sum()) != 0:
         raise ValueError("infeasible relu split: lower > upper")
     device, B = tr.mid.device, tr.B
     params = _params(module, device)
