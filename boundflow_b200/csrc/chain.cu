@@ -528,6 +528,13 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
   // identity-row sweeps on conv layers keep only the window of each row that can be non-zero (see conv.cu)
   bf::WindowGeom win{};
   bool windowed = false;
+  // windows that are still the kernels of this layer: copied only when something other than a ReLU pass on windows needs them
+  const bf_layer_desc* start = nullptr;
+  auto copy_start = [&]() {
+    const int rc = start ? bf::launch_onehot_conv_window(start->W, start->bias, const_cast<float*>(curA), ws.cacc, win, M, start->Ci, start->kh * start->kw, stream) : BF_OK;
+    start = nullptr;
+    return rc;
+  };
   bf::refresh_switches(chain);
   const bool windows_allowed = box && influence == nullptr && !chain->sw.no_windows;
   // rows that bound the neurons of a conv layer stay on the FP32 kernels in every layer below (see CONV_TC_MIN_TILES in conv.cu)
@@ -555,6 +562,8 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
                       (win.WH - 1) * L.sh + L.kh < L.Hi && (win.WW - 1) * L.sw + L.kw < L.Wi)) {
       // the window has grown to the feature map (or the next layer is not a ReLU + conv pair): back to full rows
       float* dense = ws.buf[toggle];
+      rc = copy_start();
+      if (rc != BF_OK) return rc;
       rc = bf::launch_window_to_dense(curA, dense, win, M, stream);
       if (rc != BF_OK) return rc;
       curA = dense;
@@ -577,7 +586,8 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
       } else if (windows_allowed && L.kh < L.Hi && L.kw < L.Wi) {
         win = bf::WindowGeom{M, onehot_first, S, L.Ho, L.Wo, L.Ci, L.kh, L.kw, L.Hi, L.Wi, L.sh, -L.ph, L.sw, -L.pw};
         windowed = true;
-        rc = bf::launch_onehot_conv_window(L.W, L.bias, dst, ws.cacc, win, M, L.Ci, L.kh * L.kw, stream);
+        start = &L;
+        rc = BF_OK;
       } else {
         rc = bf::launch_onehot_conv_rows(onehot_first, L.W, L.bias, dst, ws.cacc, M, S, L, stream);
       }
@@ -586,7 +596,9 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
                (win.WH - 1) * L.sh + L.kh < L.Hi && (win.WW - 1) * L.sw + L.kw < L.Wi) {
       // ReLU pass and transposed convolution in window coordinates (zero padding: the window grows by the kernel)
       float* lam = static_cast<float*>(ws.conv_scratch);
-      rc = bf::launch_relu_bwd_window(curA, dpos, dneg, epos, eneg, L.bias, lam, ws.cacc, win, M, stream);
+      rc = bf::launch_relu_bwd_window(curA, dpos, dneg, epos, eneg, L.bias, start ? start->W : nullptr, start ? start->bias : nullptr, lam, ws.cacc, win, M,
+                                      stream);
+      start = nullptr;
       if (rc != BF_OK) return rc;
       bf_layer_desc Lw = L;
       Lw.Ho = win.WH; Lw.Wo = win.WW;
@@ -618,7 +630,8 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
     pending = -1;
   }
   BF_REQUIRE(pending < 0, BF_E_UNSUPPORTED, "bf_chain_crown: a ReLU directly on the input is not supported");
-  int rc;
+  int rc = copy_start();
+  if (rc != BF_OK) return rc;
   if (windowed) rc = bf::launch_concretize_window(curA, mid, rad, ws.cacc, out, side, win, M, stream);
   else if (fused_concretize) rc = bf::launch_sum_partials(ws.cacc, ws.partial, ptiles, out, M, stream);
   else if (!box) rc = bf::launch_concretize_lp(curA, mid, have_c ? ws.cacc : nullptr, out, side, eps, norm_p, B, S, chain->n0, stream);

@@ -1074,16 +1074,20 @@ __global__ void __launch_bounds__(256) onehot_conv_window_kernel(const float* __
 // by the latency of its reads (the window value, then the slope and intercept that value selects, gathered from the
 // feature map), so the channel loop handles eight channels at a time: eight window values in flight, then eight slopes.
 // When the plane is smaller than T the threads split into T / plane channel groups (thread = group * plane + position).
+// wstart: the rows are those of the identity on a conv layer's output, whose windows are that layer's kernels: they are read in
+// place (wstart, bias wbias), no window is copied first, and delta starts here.
 template <int T>
 __global__ void __launch_bounds__(256) relu_bwd_window_kernel(const float* __restrict__ A, const float* __restrict__ dpos,
                                                               const float* __restrict__ dneg, const float* __restrict__ epos,
                                                               const float* __restrict__ eneg, const float* __restrict__ bias,
+                                                              const float* __restrict__ wstart, const float* __restrict__ wbias,
                                                               float* __restrict__ Lam, float* __restrict__ delta, WindowGeom w) {
   __shared__ float red[8];
   const int m = blockIdx.x * (256 / T) + threadIdx.x / T;
   const int t = threadIdx.x % T;
   const bool live = m < w.M;  // whole warps: T is a multiple of 32
   float acc = 0.f;
+  const int cb = wstart ? (w.first + m % w.S) / (w.HoB * w.WoB) : 0;  // output channel that the row bounds
   if (live) {
     const int j = w.first + m % w.S;
     const int rem = j % (w.HoB * w.WoB);
@@ -1091,7 +1095,7 @@ __global__ void __launch_bounds__(256) relu_bwd_window_kernel(const float* __res
     const int plane = w.WH * w.WW;
     const int HW = w.H * w.W;
     const size_t dom = (size_t)(m / w.S) * w.C * HW;
-    const float* a_row = A + (size_t)m * w.C * plane;
+    const float* a_row = wstart ? wstart + (size_t)cb * w.C * plane : A + (size_t)m * w.C * plane;
     float* lo_row = Lam + (size_t)m * w.C * plane;
     const int groups = (plane < T) ? T / plane : 1;          // channel groups when the plane is smaller than T
     const int c0 = (plane < T) ? t / plane : 0;              // this thread's first channel
@@ -1144,8 +1148,9 @@ __global__ void __launch_bounds__(256) relu_bwd_window_kernel(const float* __res
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  auto finish = [&](float sum) { delta[m] = (wstart ? (wbias ? __ldg(wbias + cb) : 0.f) : delta[m]) + sum; };
   if (T == 32) {
-    if (live && t == 0) delta[m] += acc;
+    if (live && t == 0) finish(acc);
   } else {
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
@@ -1153,7 +1158,7 @@ __global__ void __launch_bounds__(256) relu_bwd_window_kernel(const float* __res
       float sum = 0.f;
 #pragma unroll
       for (int i = 0; i < T / 32; ++i) sum += red[(threadIdx.x >> 5) + i];
-      delta[m] += sum;
+      finish(sum);
     }
   }
 }
@@ -1223,17 +1228,18 @@ int launch_onehot_conv_window(const float* W, const float* bias, float* out, flo
 }
 
 int launch_relu_bwd_window(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
-                           const float* bias, float* Lam, float* delta, const WindowGeom& w, int M, cudaStream_t stream) {
+                           const float* bias, const float* wstart, const float* wbias, float* Lam, float* delta, const WindowGeom& w, int M,
+                           cudaStream_t stream) {
   const int n_win = w.C * w.WH * w.WW;
   timing_begin(T_RELU_WINDOW, stream);
   if (n_win <= 512)
-    relu_bwd_window_kernel<32><<<ceil_div(M, 8), 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, Lam, delta, w);
+    relu_bwd_window_kernel<32><<<ceil_div(M, 8), 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, wstart, wbias, Lam, delta, w);
   else if (n_win <= 1536)
-    relu_bwd_window_kernel<64><<<ceil_div(M, 4), 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, Lam, delta, w);
+    relu_bwd_window_kernel<64><<<ceil_div(M, 4), 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, wstart, wbias, Lam, delta, w);
   else if (n_win <= 4096)
-    relu_bwd_window_kernel<128><<<ceil_div(M, 2), 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, Lam, delta, w);
+    relu_bwd_window_kernel<128><<<ceil_div(M, 2), 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, wstart, wbias, Lam, delta, w);
   else
-    relu_bwd_window_kernel<256><<<M, 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, Lam, delta, w);
+    relu_bwd_window_kernel<256><<<M, 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, wstart, wbias, Lam, delta, w);
   // window rows in and out; the slopes and intercepts are gathered per element (three values of the row's domain)
   timing_end(T_RELU_WINDOW, stream, 8.0 * (double)M * n_win + 12.0 * (double)M * n_win, 4.0 * (double)M * n_win);
   BF_CHECK_LAUNCH("relu_bwd_window_kernel");

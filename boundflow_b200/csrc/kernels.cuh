@@ -117,7 +117,8 @@ struct WindowGeom {
 int launch_onehot_conv_window(const float* W, const float* bias, float* out, float* delta, const WindowGeom& w, int M, int Ci, int kk,
                               cudaStream_t stream);
 int launch_relu_bwd_window(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
-                           const float* bias, float* Lam, float* delta, const WindowGeom& w, int M, cudaStream_t stream);
+                           const float* bias, const float* wstart, const float* wbias, float* Lam, float* delta, const WindowGeom& w, int M,
+                           cudaStream_t stream);
 // conv_window.cu: unpadded transposed convolution of small square maps (windows); BF_E_UNSUPPORTED leaves it to conv.cu
 int launch_conv_window(const float* Lam, const float* W, float* out, int M, int Ci, int Co, int WH, int WW, int kh, int kw, int sh, int sw,
                        cudaStream_t stream);
