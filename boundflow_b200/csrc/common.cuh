@@ -75,6 +75,30 @@ inline int ensure_dynamic_smem(Kernel kernel, int bytes, SmemOptIn& table, const
   return BF_OK;
 }
 
+// Launches that may start while the kernel before them in the stream still runs (programmatic dependent launch): their blocks are
+// placed and wait in grid_dependency() until everything before them is complete and visible, so a chain of short kernels pays
+// the launch itself (2 to 3 us) only once.  A kernel that is launched this way calls grid_dependency() before it touches memory.
+template <typename... Params, typename... Args>
+inline void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+// Returns 0, as a value that exists only after the wait: added to a block index it keeps the loads that depend on it behind the wait.
+__device__ __forceinline__ int grid_dependency() {
+  int zero;
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;\n\tmov.b32 %0, 0;" : "=r"(zero) : : "memory");
+  return zero;
+}
+
 inline cudaStream_t as_stream(bf_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }

@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
   const int tid = threadIdx.x, tx = tid % (TM / 4), ty = tid / (TM / 4);
   const int taps = g.kh * g.kw, K = g.Ci * taps, howo = g.Ho * g.Wo, hw = g.Hi * g.Wi;
   const long long npix = (long long)g.B * howo;
-  const long long p0 = (long long)blockIdx.x * TM;
+  const long long p0 = (long long)(blockIdx.x + grid_dependency()) * TM;
   const int c0 = blockIdx.y * TN;
   const int k0 = blockIdx.z * kper, k1 = min(K, k0 + kper);
   const int nk = (k1 > k0) ? (k1 - k0 + CBK - 1) / CBK : 0;
@@ -308,11 +308,13 @@ static int launch_conv_tile_n(const IbpConvArgs& g, int vec, cudaStream_t stream
   cfg.gridDim = dim3((unsigned)tiles, ctas_y, ks);
   cfg.blockDim = dim3(256);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = ks;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   cudaLaunchKernelEx(&cfg, conv_tile_kernel<INTERVAL, TN>, g, ceil_div(slabs, ks) * ConvTile<TN>::SLAB, vec);
   BF_CHECK_LAUNCH("conv_tile_kernel");
   return BF_OK;
@@ -364,7 +366,7 @@ __global__ void __launch_bounds__(256) relu_bwd_rows_kernel(const float* __restr
                                                             float* __restrict__ Lam, float* __restrict__ partial,
                                                             float* __restrict__ delta, int accumulate, int chunk, int S, int n,
                                                             int vec) {
-  const int m = blockIdx.x;
+  const int m = blockIdx.x + grid_dependency();
   const int k0 = blockIdx.y * chunk;
   const int k1 = min(n, k0 + chunk);
   const float* a = A + (size_t)m * n;
@@ -587,7 +589,7 @@ __global__ void __launch_bounds__(256, (TCI > 1 && TWP * RT > 8 ? 2 : 3)) conv_t
   const int buf_words = lam_words + w_words;
   constexpr int ROW_ZERO = -2147483647 - 1;
   int* row_off = reinterpret_cast<int*>(rs_smem + 2 * buf_words);  // [nrows] source offset of each tile row, ROW_ZERO: all zeros
-  const int m0 = blockIdx.x << a.mrl;
+  const int m0 = (blockIdx.x + grid_dependency()) << a.mrl;
   const int h0 = (blockIdx.y / a.tiles_x) << a.thl;
   const int w0 = (blockIdx.y % a.tiles_x) * (G::TW * sx);
   const int ci0 = blockIdx.z << cibl;
@@ -798,7 +800,7 @@ static int launch_rowseg_tci(const ConvTArgs& g, double* us, cudaStream_t stream
   }
   static SmemOptIn opt_in;
   if (int rc = ensure_dynamic_smem(conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT>, 110 * 1024, opt_in, "conv_transpose_rowseg_kernel")) return rc;
-  conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT><<<grid, 256, smem, stream>>>(a);
+  launch_dependent(conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT>, grid, 256, smem, stream, a);
   BF_CHECK_LAUNCH("conv_transpose_rowseg_kernel");
   return BF_OK;
 }
@@ -945,7 +947,7 @@ int launch_crown_bwd_conv2d(const float* A, const float* dpos, const float* dneg
     for (const void* q : ptrs) if (reinterpret_cast<uintptr_t>(q) & 15u) vec = 0;
     dim3 grid(M, nchunks);
     timing_begin(T_RELU_ROWS, stream);
-    relu_bwd_rows_kernel<<<grid, 256, 0, stream>>>(A, dpos, dneg, epos, eneg, dpos ? add : nullptr, bias, L.Ho * L.Wo, lam_out, partial, delta, accumulate,
+    launch_dependent(relu_bwd_rows_kernel, grid, 256, 0, stream, A, dpos, dneg, epos, eneg, dpos ? add : nullptr, bias, L.Ho * L.Wo, lam_out, partial, delta, accumulate,
                                                   chunk, S, L.n_out, vec);
     // rows in (+ out when a ReLU scales them) and the slope / intercept vectors of every domain
     timing_end(T_RELU_ROWS, stream, (lam_out ? 8.0 : 4.0) * (double)M * L.n_out + (dpos ? 12.0 * (double)(M / S) * L.n_out : 0.0),
@@ -1020,12 +1022,6 @@ __global__ void __launch_bounds__(256) onehot_conv_rows_kernel(const float* __re
     }
   }
   }
-}
-
-// grid-stride launch: enough blocks to fill the machine, at most one block per 256 elements
-static int onehot_grid(long long total) {
-  const long long blocks = (total + 255) / 256;
-  return (int)(blocks < 148LL * 16 ? blocks : 148LL * 16);
 }
 
 int launch_onehot_conv_rows(int first, const float* W, const float* bias, float* A_prev, float* delta, int M, int S,
@@ -1260,23 +1256,26 @@ int launch_concretize_window(const float* Awin, const float* mid, const float* r
   return BF_OK;
 }
 
-// Same for a linear layer: coefficient row j is row j of W, its bias term bias[j].
+// Same for a linear layer: coefficient row j is row j of W, its bias term bias[j].  A block copies one row: bound by its stores
+// (25,600 x 1568: 116 us with a division per element).
 __global__ void __launch_bounds__(256) onehot_linear_rows_kernel(const float* __restrict__ W, const float* __restrict__ bias,
                                                                  float* __restrict__ out, float* __restrict__ delta, int first,
-                                                                 int S, int n_in, long long total) {
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const int m = (int)(e / n_in);
-    const int k = (int)(e - (long long)m * n_in);
-    const int j = first + m % S;
-    out[e] = __ldg(W + (size_t)j * n_in + k);
-    if (k == 0 && delta) delta[m] = bias ? __ldg(bias + j) : 0.f;
+                                                                 int S, int n_in, int vec) {
+  const int m = blockIdx.x, j = first + m % S;
+  const float* src = W + (size_t)j * n_in;
+  float* dst = out + (size_t)m * n_in;
+  if (vec) {
+    for (int k = 4 * threadIdx.x; k < n_in; k += 1024) *reinterpret_cast<float4*>(dst + k) = __ldg(reinterpret_cast<const float4*>(src + k));
+  } else {
+    for (int k = threadIdx.x; k < n_in; k += 256) dst[k] = __ldg(src + k);
   }
+  if (threadIdx.x == 0 && delta) delta[m] = bias ? __ldg(bias + j) : 0.f;
 }
 
 int launch_onehot_linear_rows(int first, const float* W, const float* bias, float* A_prev, float* delta, int M, int S, int n_in,
                               cudaStream_t stream) {
-  const long long total = (long long)M * n_in;
-  onehot_linear_rows_kernel<<<onehot_grid(total), 256, 0, stream>>>(W, bias, A_prev, delta, first, S, n_in, total);
+  const int vec = n_in % 4 == 0 && ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(A_prev)) & 15u) == 0;
+  onehot_linear_rows_kernel<<<M, 256, 0, stream>>>(W, bias, A_prev, delta, first, S, n_in, vec);
   BF_CHECK_LAUNCH("onehot_linear_rows_kernel");
   return BF_OK;
 }
@@ -1387,7 +1386,7 @@ extern "C" int bf_crown_relu_bwd(const float* A, int side, const float* alpha_u,
   for (const void* q : ptrs) if (reinterpret_cast<uintptr_t>(q) & 15u) vec = 0;
   cudaStream_t stream = bf::as_stream(stream_);
   dim3 grid(M, nchunks);
-  bf::relu_bwd_rows_kernel<<<grid, 256, 0, stream>>>(A, dpos, dneg, epos, eneg, nullptr, nullptr, 1, A_prev, partial, delta, accumulate,
+  bf::launch_dependent(bf::relu_bwd_rows_kernel, grid, 256, 0, stream, A, dpos, dneg, epos, eneg, nullptr, nullptr, 1, A_prev, partial, delta, accumulate,
                                                     bf::RELU_ROWS_CHUNK, S, n, vec);
   BF_CHECK_LAUNCH("relu_bwd_rows_kernel");
   if (partial) return bf::launch_sum_partials(accumulate ? delta : nullptr, partial, nchunks, delta, M, stream);

@@ -24,7 +24,7 @@ template <int PRO, int MH, int NH>
 __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_bwd_linear_kernel(GemmArgs g, BwdEpilogue e) {
   __shared__ __align__(16) float smem[MAINLOOP_SMEM_FLOATS];
   constexpr int TM = 64 * MH, MR = 4 * MH;
-  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * (64 * NH);
+  const int m0 = (blockIdx.x + grid_dependency()) * TM, n0 = blockIdx.y * (64 * NH);
   float acc[8][8];
   gemm_mainloop<PRO, false, MH, NH>(g, m0, n0, acc, smem);
 
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(GS_THREADS, 2) crown_bwd_small_kernel(GemmArgs
   float* As = dsmem;
   float* Bs = As + GS_STAGES * GS_A_WORDS;
   float* part = Bs + GS_STAGES * GS_B_WORDS<false>;  // [row]: concretisation sums of the right half of the tile
-  const int m0 = blockIdx.x * GS_ROWS, n0 = blockIdx.y * GS_COLS, tid = threadIdx.x;
+  const int m0 = (blockIdx.x + grid_dependency()) * GS_ROWS, n0 = blockIdx.y * GS_COLS, tid = threadIdx.x;
   if ((int)blockIdx.y == e.ntiles) {
     prologue_row_sums(g, m0);
     return;
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(128) crown_bwd_thin_kernel(const float* __rest
                                                              const float* __restrict__ kbias, float* __restrict__ out,
                                                              float* __restrict__ delta, int accumulate, int M, int K, int N, int block_rows) {
   __shared__ float a_s[THIN_ROWS * THIN_KMAX];
-  const int m0 = blockIdx.x * block_rows;
+  const int m0 = (blockIdx.x + grid_dependency()) * block_rows;
   const int rows = min(block_rows, M - m0);
   for (int i = threadIdx.x; i < rows * K; i += blockDim.x) a_s[i] = A[(size_t)m0 * K + i];
   __syncthreads();
@@ -183,7 +183,7 @@ int launch_crown_bwd_linear(const float* A, const float* dpos, const float* dneg
     while (rows > 4 && ceil_div(M, rows) * cols < 4 * 148) rows /= 2;
     dim3 grid(ceil_div(M, rows), cols);
     timing_begin(T_THIN, stream);
-    crown_bwd_thin_kernel<<<grid, 128, 0, stream>>>(A, W, kbias, A_prev, delta, accumulate, M, K, N, rows);
+    launch_dependent(crown_bwd_thin_kernel, grid, 128, 0, stream, A, W, kbias, A_prev, delta, accumulate, M, K, N, rows);
     timing_end(T_THIN, stream, 4.0 * (double)M * N + 4.0 * (double)M * K + 4.0 * (double)K * N, 2.0 * (double)M * K * N);
     BF_CHECK_LAUNCH("crown_bwd_thin_kernel");
     return BF_OK;
@@ -204,13 +204,13 @@ int launch_crown_bwd_linear(const float* A, const float* dpos, const float* dneg
     static SmemOptIn opt_in;
     if (int rc = ensure_dynamic_smem(crown_bwd_small_kernel, GS_BWD_SMEM, opt_in, "crown_bwd_small_kernel")) return rc;
     dim3 grid(ceil_div(M, GS_ROWS), e.ntiles + (delta ? 1 : 0));
-    crown_bwd_small_kernel<<<grid, GS_THREADS, GS_BWD_SMEM, stream>>>(g, e);
+    launch_dependent(crown_bwd_small_kernel, grid, GS_THREADS, GS_BWD_SMEM, stream, g, e);
   } else if (ffma_small_tiles(M, N)) {  // 64 x 64 tiles: four times as many CTAs
     dim3 grid(ceil_div(M, 64), ceil_div(N, 64));
-    crown_bwd_linear_kernel<PRO_RELU, 1, 1><<<grid, GEMM_THREADS, 0, stream>>>(g, e);
+    launch_dependent(crown_bwd_linear_kernel<PRO_RELU, 1, 1>, grid, GEMM_THREADS, 0, stream, g, e);
   } else {
     dim3 grid(ceil_div(M, BM), ceil_div(N, BN));
-    crown_bwd_linear_kernel<PRO_RELU, 2, 2><<<grid, GEMM_THREADS, 0, stream>>>(g, e);
+    launch_dependent(crown_bwd_linear_kernel<PRO_RELU, 2, 2>, grid, GEMM_THREADS, 0, stream, g, e);
   }
   timing_end(T_BWD, stream, 4.0 * (double)M * K + (A_prev ? 4.0 * (double)M * N : 0.0), 2.0 * (double)M * K * N);
   BF_CHECK_LAUNCH("crown_bwd_linear_kernel");
@@ -247,7 +247,7 @@ template <int PRO, int MH, int NH>
 __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_adjoint_linear_kernel(GemmArgs g, AdjEpilogue e) {
   extern __shared__ __align__(16) float dsmem[];
   constexpr int TM = 64 * MH, TN = 64 * NH, MR = 4 * MH;
-  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
+  const int m0 = (blockIdx.x + grid_dependency()) * TM, n0 = blockIdx.y * TN;
   float acc[8][8];
   gemm_mainloop<PRO, true, MH, NH>(g, m0, n0, acc, dsmem);
   // the main loop ends with __syncthreads(): the slabs may now be overwritten by the stage tile
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) crown_adjoint_small_kernel(Gemm
   float* As = dsmem;
   float* Bs = As + GS_STAGES * GS_A_WORDS;
   float* red = Bs + GS_STAGES * GS_B_WORDS<true>;  // [row][GS_COLS + 1]
-  const int m0 = blockIdx.x * GS_ROWS, n0 = blockIdx.y * GS_COLS, tid = threadIdx.x;
+  const int m0 = (blockIdx.x + grid_dependency()) * GS_ROWS, n0 = blockIdx.y * GS_COLS, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5, tx = lane & 7, ty = lane >> 3;
   const int r0 = (warp >> 1) * 16 + ty * 4, c0 = (warp & 1) * 32 + tx;
   float acc[4][4];
@@ -444,12 +444,12 @@ int launch_crown_adjoint_linear(const float* Hprev, int first_layer, const float
     if (int rc = ensure_dynamic_smem(crown_adjoint_linear_kernel<PRO_, MH_, NH_>, ADJ_SMEM_BYTES, opt_in[slot],                 \
                                      "crown_adjoint_linear_kernel"))                                                            \
       return rc;                                                                                                                \
-    crown_adjoint_linear_kernel<PRO_, MH_, NH_><<<grid, GEMM_THREADS, ADJ_SMEM_BYTES, stream>>>(g, e);                          \
+    launch_dependent(crown_adjoint_linear_kernel<PRO_, MH_, NH_>, grid, GEMM_THREADS, ADJ_SMEM_BYTES, stream, g, e);            \
   }
 #define BF_ADJ_SMALL(PRO_, slot)                                                                                                  \
   {                                                                                                                             \
     if (int rc = ensure_dynamic_smem(crown_adjoint_small_kernel<PRO_>, GS_ADJ_SMEM, opt_in[slot], "crown_adjoint_small_kernel")) return rc; \
-    crown_adjoint_small_kernel<PRO_><<<grid, GS_THREADS, GS_ADJ_SMEM, stream>>>(g, e);                                            \
+    launch_dependent(crown_adjoint_small_kernel<PRO_>, grid, GS_THREADS, GS_ADJ_SMEM, stream, g, e);                              \
   }
   if (first_layer) {
     if (quarter) BF_ADJ_SMALL(PRO_H0, 4) else if (small) BF_ADJ_LAUNCH(PRO_H0, 1, 1, 0) else BF_ADJ_LAUNCH(PRO_H0, 2, 2, 1)

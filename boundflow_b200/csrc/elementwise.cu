@@ -55,7 +55,7 @@ int launch_relu_relax(const float* l, const float* u, const float* alpha, int al
 __global__ void __launch_bounds__(256) concretize_kernel(const float* __restrict__ A, const float* __restrict__ mid,
                                                          const float* __restrict__ rad, const float* __restrict__ bias_in,
                                                          float* __restrict__ out, float sgn, int M, int S, int n0, int vec) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int warp = ((blockIdx.x + grid_dependency()) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int m = warp; m < M; m += nwarps) {
@@ -89,7 +89,7 @@ int launch_concretize(const float* A, const float* mid, const float* rad, const 
   int blocks = ceil_div(M, 8);
   if (blocks > 148 * 8) blocks = 148 * 8;
   timing_begin(T_CONCRETIZE, stream);
-  concretize_kernel<<<blocks, 256, 0, stream>>>(A, mid, rad, bias_in, out, side == BF_SIDE_LOWER ? -1.f : 1.f, M, S, n0, vec);
+  launch_dependent(concretize_kernel, blocks, 256, 0, stream, A, mid, rad, bias_in, out, side == BF_SIDE_LOWER ? -1.f : 1.f, M, S, n0, vec);
   // every coefficient row once, the box of every domain once, one result per row
   timing_end(T_CONCRETIZE, stream, 4.0 * (double)M * n0 + 8.0 * (double)B * n0 + 4.0 * M, 4.0 * (double)M * n0);
   BF_CHECK_LAUNCH("concretize_kernel");
@@ -99,7 +99,7 @@ int launch_concretize(const float* A, const float* mid, const float* rad, const 
 // ---- finalisation of the fused first-layer concretisation ---------------------
 __global__ void sum_partials_kernel(const float* __restrict__ c, const float* __restrict__ partial, int ntiles,
                                     float* __restrict__ out, int M) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  const int m = (blockIdx.x + grid_dependency()) * blockDim.x + threadIdx.x;
   if (m >= M) return;
   float s = 0.f;
   for (int t = 0; t < ntiles; ++t) s += partial[(size_t)m * ntiles + t];
@@ -107,7 +107,7 @@ __global__ void sum_partials_kernel(const float* __restrict__ c, const float* __
 }
 
 int launch_sum_partials(const float* c, const float* partial, int ntiles, float* out, int M, cudaStream_t stream) {
-  sum_partials_kernel<<<ceil_div(M, 256), 256, 0, stream>>>(c, partial, ntiles, out, M);
+  launch_dependent(sum_partials_kernel, ceil_div(M, 256), 256, 0, stream, c, partial, ntiles, out, M);
   BF_CHECK_LAUNCH("sum_partials_kernel");
   return BF_OK;
 }
@@ -116,7 +116,7 @@ int launch_sum_partials(const float* c, const float* partial, int ntiles, float*
 __global__ void select_best_kernel(const float* __restrict__ cur, float* __restrict__ best_lower,
                                    float* __restrict__ best_metric, int* __restrict__ improve, int first, int spec_reduce,
                                    float soft_tau, float* __restrict__ row_weight, int B, int S) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  const int b = (blockIdx.x + grid_dependency()) * blockDim.x + threadIdx.x;
   if (b >= B) return;
   const float* row = cur + (size_t)b * S;
   float metric;
@@ -153,7 +153,7 @@ __global__ void select_best_kernel(const float* __restrict__ cur, float* __restr
 
 int launch_select_best(const float* cur, float* best_lower, float* best_metric, int* improve, int first,
                        int spec_reduce, float soft_tau, float* row_weight, int B, int S, cudaStream_t stream) {
-  select_best_kernel<<<ceil_div(B, 128), 128, 0, stream>>>(cur, best_lower, best_metric, improve, first, spec_reduce, soft_tau,
+  launch_dependent(select_best_kernel, ceil_div(B, 128), 128, 0, stream, cur, best_lower, best_metric, improve, first, spec_reduce, soft_tau,
                                                            row_weight, B, S);
   BF_CHECK_LAUNCH("select_best_kernel");
   return BF_OK;
@@ -267,7 +267,7 @@ __device__ __forceinline__ void adam_one(float& a, float& mi, float& vi, float g
 // is bound by its launches: five 256-wide layers took five launches of 5.2 us (alpha) per step.
 __global__ void __launch_bounds__(128) optimiser_step_kernel(StepArgs p, const int* __restrict__ improve, AdamScalars sc, int do_update) {
   const StepSegment& g = p.seg[blockIdx.z];
-  const int b = blockIdx.x;
+  const int b = blockIdx.x + grid_dependency();
   const int j = (blockIdx.y * blockDim.x + threadIdx.x) * (g.vec ? 4 : 1);
   if (j >= g.n) return;
   const size_t i = (size_t)b * g.n + j;
@@ -340,7 +340,7 @@ int launch_optimiser_step(const StepSegment* seg, int count, const int* improve,
     }
     BF_REQUIRE(chunks <= 65535, BF_E_UNSUPPORTED, "optimiser step: layer too wide");
     timing_begin(T_ADAM, stream);
-    optimiser_step_kernel<<<dim3(B, chunks, here), 128, 0, stream>>>(p, improve, sc, do_update);
+    launch_dependent(optimiser_step_kernel, dim3(B, chunks, here), 128, 0, stream, p, improve, sc, do_update);
     // the optimiser's own traffic: read parameter, m, v, grad and write parameter, m, v (28 B per element); the kernel also
     // reads the pre-activation bounds, clears the gradient and writes the next lower slope and the best-alpha snapshot
     // (up to 48 B per element in all), which replaces separate relaxation / snapshot passes
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(256) relu_adjoint_rows_kernel(float* __restric
                                                                 const float* __restrict__ eneg, const float* __restrict__ pre_l,
                                                                 const float* __restrict__ pre_u, float* __restrict__ grad,
                                                                 float* __restrict__ gsum, const float* __restrict__ gw, int S, int n) {
-  const int b = blockIdx.x;
+  const int b = blockIdx.x + grid_dependency();
   const int j = blockIdx.y * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const size_t o = (size_t)b * n + j;
@@ -536,7 +536,7 @@ int launch_relu_adjoint_rows(float* G, const float* Ahat, const float* dpos, con
                              const float* pre_l, const float* pre_u, float* grad, float* gsum, int B, int S, int n,
                              cudaStream_t stream, const float* gw) {
   dim3 grid(B, ceil_div(n, 256));
-  relu_adjoint_rows_kernel<<<grid, 256, 0, stream>>>(G, Ahat, dpos, dneg, eneg, pre_l, pre_u, grad, gsum, gw, S, n);
+  launch_dependent(relu_adjoint_rows_kernel, grid, 256, 0, stream, G, Ahat, dpos, dneg, eneg, pre_l, pre_u, grad, gsum, gw, S, n);
   BF_CHECK_LAUNCH("relu_adjoint_rows_kernel");
   return BF_OK;
 }
@@ -544,7 +544,7 @@ int launch_relu_adjoint_rows(float* G, const float* Ahat, const float* dpos, con
 // Start vector of the gradient sweep for a box: h0 = mid - sgn(A0) * rad, written over A0.
 __global__ void h0_box_kernel(float* __restrict__ A0, const float* __restrict__ mid, const float* __restrict__ rad, long long total,
                               int S, int n0) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+  for (long long i = (blockIdx.x + grid_dependency()) * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long m = i / n0;
     const size_t o = (size_t)(m / S) * n0 + (size_t)(i - m * n0);
     const float a = A0[i];
@@ -555,7 +555,7 @@ __global__ void h0_box_kernel(float* __restrict__ A0, const float* __restrict__ 
 
 int launch_h0_box(float* A0, const float* mid, const float* rad, int B, int S, int n0, cudaStream_t stream) {
   const long long total = (long long)B * S * n0;
-  h0_box_kernel<<<ew_grid(total, 256), 256, 0, stream>>>(A0, mid, rad, total, S, n0);
+  launch_dependent(h0_box_kernel, ew_grid(total, 256), 256, 0, stream, A0, mid, rad, total, S, n0);
   BF_CHECK_LAUNCH("h0_box_kernel");
   return BF_OK;
 }
