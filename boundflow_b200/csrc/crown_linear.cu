@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(GS_THREADS, 2) crown_bwd_small_kernel(GemmArgs
       if (m0 + r0 + i < g.M) e.partial[(size_t)(m0 + r0 + i) * e.ntiles + blockIdx.y] = p[i] + part[r0 + i];
   }
 }
+constexpr int GS_ONE_PER_SM = 116 * 1024;  // more than half of an SM's shared memory
 constexpr int GS_BWD_SMEM = (GS_STAGES * (GS_A_WORDS + GS_B_WORDS<false>) + GS_ROWS) * (int)sizeof(float);
 
 // Top layer of a sweep (no ReLU in front, K = spec width <= 16): A_prev[M,N] = A[M,K] * W[K,N] and
@@ -202,9 +203,12 @@ int launch_crown_bwd_linear(const float* A, const float* dpos, const float* dneg
   timing_begin(T_BWD, stream);
   if (ffma_quarter_tiles(M, N)) {
     static SmemOptIn opt_in;
-    if (int rc = ensure_dynamic_smem(crown_bwd_small_kernel, GS_BWD_SMEM, opt_in, "crown_bwd_small_kernel")) return rc;
+    if (int rc = ensure_dynamic_smem(crown_bwd_small_kernel, GS_ONE_PER_SM, opt_in, "crown_bwd_small_kernel")) return rc;
     dim3 grid(ceil_div(M, GS_ROWS), e.ntiles + (delta ? 1 : 0));
-    launch_dependent(crown_bwd_small_kernel, grid, GS_THREADS, GS_BWD_SMEM, stream, g, e);
+    // No more CTAs than SMs: one per SM.  They are placed while the kernel before still has its SMs and would go in pairs to those
+    // that are free (37 nodes, four 512-wide layers, 10 steps: 2.61 ms in pairs, 2.44 with one per SM).
+    const int smem = grid.x * grid.y <= 148 ? GS_ONE_PER_SM : GS_BWD_SMEM;
+    launch_dependent(crown_bwd_small_kernel, grid, GS_THREADS, smem, stream, g, e);
   } else if (ffma_small_tiles(M, N)) {  // 64 x 64 tiles: four times as many CTAs
     dim3 grid(ceil_div(M, 64), ceil_div(N, 64));
     launch_dependent(crown_bwd_linear_kernel<PRO_RELU, 1, 1>, grid, GEMM_THREADS, 0, stream, g, e);
