@@ -1049,6 +1049,35 @@ int launch_onehot_conv_rows(int first, const float* W, const float* bias, float*
 // what falls outside the feature map is cleared by the next ReLU pass or ignored by the concretisation.
 // ---------------------------------------------------------------------------
 
+// Division by a run-time constant: a handful of instructions instead of some twenty.  Rows of 100 to 300 elements are a warp each, and
+// the nine divisions of a warp (row, pixel, position) took longer than the elements.  Exact for 0 <= n < 2^31 (the quotient from the
+// rounded-down reciprocal is at most one too small).
+struct FastDiv {
+  unsigned d, magic;
+};
+static FastDiv fast_div(int d) { return FastDiv{(unsigned)d, 0xffffffffu / (unsigned)d}; }
+__device__ __forceinline__ int fast_quot(int n, FastDiv f, int* rem) {
+  unsigned q = __umulhi((unsigned)n, f.magic), r = (unsigned)n - q * f.d;
+  if (r >= f.d) { ++q; r -= f.d; }
+  *rem = (int)r;
+  return (int)q;
+}
+// divisors of the kernels on windows: spec rows per domain, pixels and row length of the bounded value, window plane and row length
+struct WindowDiv {
+  FastDiv S, pixels, wo, plane, ww;
+};
+static WindowDiv window_div(const WindowGeom& w) {
+  return WindowDiv{fast_div(w.S), fast_div(w.HoB * w.WoB), fast_div(w.WoB), fast_div(w.WH * w.WW), fast_div(w.WW)};
+}
+// the domain of row m, the output channel that it bounds and its window's origin
+__device__ __forceinline__ void window_row(const WindowGeom& w, const WindowDiv& dv, int m, int* domain, int* channel, int* top, int* left) {
+  int s, pixel, wo;
+  *domain = fast_quot(m, dv.S, &s);
+  *channel = fast_quot(w.first + s, dv.pixels, &pixel);
+  *top = fast_quot(pixel, dv.wo, &wo) * w.sy + w.ty;
+  *left = wo * w.sx + w.tx;
+}
+
 // first backward step: the window is the kernel itself (one warp per row)
 __global__ void __launch_bounds__(256) onehot_conv_window_kernel(const float* __restrict__ W, const float* __restrict__ bias,
                                                                  float* __restrict__ out, float* __restrict__ delta, WindowGeom w,
@@ -1077,31 +1106,29 @@ __global__ void __launch_bounds__(256) relu_bwd_window_kernel(const float* __res
                                                               const float* __restrict__ dneg, const float* __restrict__ epos,
                                                               const float* __restrict__ eneg, const float* __restrict__ bias,
                                                               const float* __restrict__ wstart, const float* __restrict__ wbias,
-                                                              float* __restrict__ Lam, float* __restrict__ delta, WindowGeom w) {
+                                                              float* __restrict__ Lam, float* __restrict__ delta, WindowGeom w, WindowDiv dv) {
   __shared__ float red[8];
   const int m = blockIdx.x * (256 / T) + threadIdx.x / T;
   const int t = threadIdx.x % T;
   const bool live = m < w.M;  // whole warps: T is a multiple of 32
   float acc = 0.f;
-  const int cb = wstart ? (w.first + m % w.S) / (w.HoB * w.WoB) : 0;  // output channel that the row bounds
+  int domain, cb, top, left;   // cb: output channel that the row bounds
+  window_row(w, dv, live ? m : 0, &domain, &cb, &top, &left);
   if (live) {
-    const int j = w.first + m % w.S;
-    const int rem = j % (w.HoB * w.WoB);
-    const int top = (rem / w.WoB) * w.sy + w.ty, left = (rem % w.WoB) * w.sx + w.tx;
     const int plane = w.WH * w.WW;
     const int HW = w.H * w.W;
-    const size_t dom = (size_t)(m / w.S) * w.C * HW;
+    const size_t dom = (size_t)domain * w.C * HW;
     const float* a_row = wstart ? wstart + (size_t)cb * w.C * plane : A + (size_t)m * w.C * plane;
     float* lo_row = Lam + (size_t)m * w.C * plane;
-    const int groups = (plane < T) ? T / plane : 1;          // channel groups when the plane is smaller than T
-    const int c0 = (plane < T) ? t / plane : 0;              // this thread's first channel
-    const int p0 = (plane < T) ? t - c0 * plane : t;         // and its first position
+    int p0 = t, rest;                                        // this thread's first position
+    const int c0 = (plane < T) ? fast_quot(t, dv.plane, &p0) : 0;        // and its first channel
+    const int groups = (plane < T) ? fast_quot(T, dv.plane, &rest) : 1;  // channel groups when the plane is smaller than T
     const int pstep = (plane < T) ? plane : T;               // plane < T: a single position per thread
     if (c0 < groups) {
       const size_t astep = (size_t)groups * plane, kstep = (size_t)groups * HW;
       for (int pos = p0; pos < plane; pos += pstep) {
-        const int y = pos / w.WW, x = pos - y * w.WW;
-        const int Y = top + y, X = left + x;
+        int x;
+        const int Y = top + fast_quot(pos, dv.ww, &x), X = left + x;
         const bool inside = Y >= 0 && Y < w.H && X >= 0 && X < w.W;
         const float* a = a_row + (size_t)c0 * plane + pos;
         float* lo = lo_row + (size_t)c0 * plane + pos;
@@ -1176,15 +1203,14 @@ __global__ void __launch_bounds__(256) window_to_dense_kernel(const float* __res
 // box concretisation of windows on the network input: out[m] = sum A*mid -/+ |A|*rad over the window inside the image + delta
 __global__ void __launch_bounds__(256) concretize_window_kernel(const float* __restrict__ Awin, const float* __restrict__ mid,
                                                                 const float* __restrict__ rad, const float* __restrict__ delta,
-                                                                float* __restrict__ out, float sgn, WindowGeom w) {
+                                                                float* __restrict__ out, float sgn, WindowGeom w, WindowDiv dv) {
   const int m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (m >= w.M) return;
-  const int j = w.first + m % w.S;
-  const int rem = j % (w.HoB * w.WoB);
-  const int top = (rem / w.WoB) * w.sy + w.ty, left = (rem % w.WoB) * w.sx + w.tx;
+  int domain, channel, top, left;
+  window_row(w, dv, m, &domain, &channel, &top, &left);
   const int n_win = w.C * w.WH * w.WW;
-  const size_t dom = (size_t)(m / w.S) * w.C * w.H * w.W;
+  const size_t dom = (size_t)domain * w.C * w.H * w.W;
   float acc = 0.f;
   // four elements of a lane per iteration: their index arithmetic first, then all loads, then the sums in element order
   // (the loop is bound by the latency of its gathered reads, like the ReLU pass on windows)
@@ -1195,8 +1221,9 @@ __global__ void __launch_bounds__(256) concretize_window_kernel(const float* __r
       const int e = e0 + 32 * q;
       v[q] = cm[q] = cr[q] = 0.f;
       if (e < n_win) {
-        const int c = e / (w.WH * w.WW), r2 = e - c * (w.WH * w.WW);
-        const int Y = top + r2 / w.WW, X = left + r2 % w.WW;
+        int r2, x;
+        const int c = fast_quot(e, dv.plane, &r2);
+        const int Y = top + fast_quot(r2, dv.ww, &x), X = left + x;
         if (Y >= 0 && Y < w.H && X >= 0 && X < w.W) {
           const size_t k = dom + ((size_t)c * w.H + Y) * w.W + X;
           v[q] = Awin[(size_t)m * n_win + e];
@@ -1229,13 +1256,13 @@ int launch_relu_bwd_window(const float* A, const float* dpos, const float* dneg,
   const int n_win = w.C * w.WH * w.WW;
   timing_begin(T_RELU_WINDOW, stream);
   if (n_win <= 512)
-    relu_bwd_window_kernel<32><<<ceil_div(M, 8), 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, wstart, wbias, Lam, delta, w);
+    relu_bwd_window_kernel<32><<<ceil_div(M, 8), 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, wstart, wbias, Lam, delta, w, window_div(w));
   else if (n_win <= 1536)
-    relu_bwd_window_kernel<64><<<ceil_div(M, 4), 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, wstart, wbias, Lam, delta, w);
+    relu_bwd_window_kernel<64><<<ceil_div(M, 4), 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, wstart, wbias, Lam, delta, w, window_div(w));
   else if (n_win <= 4096)
-    relu_bwd_window_kernel<128><<<ceil_div(M, 2), 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, wstart, wbias, Lam, delta, w);
+    relu_bwd_window_kernel<128><<<ceil_div(M, 2), 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, wstart, wbias, Lam, delta, w, window_div(w));
   else
-    relu_bwd_window_kernel<256><<<M, 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, wstart, wbias, Lam, delta, w);
+    relu_bwd_window_kernel<256><<<M, 256, 0, stream>>>(A, dpos, dneg, epos, eneg, bias, wstart, wbias, Lam, delta, w, window_div(w));
   // window rows in and out; the slopes and intercepts are gathered per element (three values of the row's domain)
   timing_end(T_RELU_WINDOW, stream, 8.0 * (double)M * n_win + 12.0 * (double)M * n_win, 4.0 * (double)M * n_win);
   BF_CHECK_LAUNCH("relu_bwd_window_kernel");
@@ -1251,7 +1278,7 @@ int launch_window_to_dense(const float* Awin, float* dense, const WindowGeom& w,
 int launch_concretize_window(const float* Awin, const float* mid, const float* rad, const float* delta, float* out, int side,
                              const WindowGeom& w, int M, cudaStream_t stream) {
   concretize_window_kernel<<<ceil_div((long long)M * 32, 256), 256, 0, stream>>>(Awin, mid, rad, delta, out,
-                                                                               side == BF_SIDE_LOWER ? -1.f : 1.f, w);
+                                                                               side == BF_SIDE_LOWER ? -1.f : 1.f, w, window_div(w));
   BF_CHECK_LAUNCH("concretize_window_kernel");
   return BF_OK;
 }
