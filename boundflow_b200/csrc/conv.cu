@@ -966,8 +966,8 @@ int launch_crown_bwd_conv2d(const float* A, const float* dpos, const float* dneg
   const double conv_flops = 2.0 * (double)M * L.n_out * L.Ci * L.kh * L.kw;
   timing_begin(T_CONV_T, stream);
   int rc = BF_E_UNSUPPORTED;
-  if (!gather_only && L.ph == 0 && L.pw == 0 && L.Hi == (L.Ho - 1) * L.sh + L.kh && L.Wi == (L.Wo - 1) * L.sw + L.kw)
-    rc = launch_conv_window(lam, W, A_prev, M, L.Ci, L.Co, L.Ho, L.Wo, L.kh, L.kw, L.sh, L.sw, stream);
+  if (!gather_only && L.Hi == (L.Ho - 1) * L.sh + L.kh - 2 * L.ph && L.Wi == (L.Wo - 1) * L.sw + L.kw - 2 * L.pw)
+    rc = launch_conv_window(lam, W, A_prev, M, L.Ci, L.Co, L.Ho, L.Wo, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw, stream);
   if (rc == BF_E_UNSUPPORTED && !gather_only) rc = launch_convT_rowseg(g, nullptr, stream);
   if (rc == BF_E_UNSUPPORTED) {
     if (L.Ci <= 4) rc = launch_convT<4>(g, stream);

@@ -1,4 +1,4 @@
-// Transposed convolution of narrow windows of coefficient rows (the identity-row sweeps on conv layers): no padding, square
+// Transposed convolution of narrow windows of coefficient rows (the identity-row sweeps on conv layers) and of small maps: square
 // windows, kernels and strides, lanes = coefficient rows.
 #include <math.h>
 
@@ -36,9 +36,9 @@ struct ConvWindowArgs {
 
 constexpr int CONV_WINDOW_SUMS = 72;
 
-template <int KS, int ST, int WW>
+template <int KS, int ST, int PD, int WW>
 struct ConvWindow {
-  static constexpr int OW = (WW - 1) * ST + KS;
+  static constexpr int OW = (WW - 1) * ST + KS - 2 * PD;
   static constexpr int TH0 = (CONV_WINDOW_SUMS / OW) / ST * ST;                  // whole image rows that fit
   static constexpr bool FULL = OW * OW <= CONV_WINDOW_SUMS;
   static constexpr int NB0 = FULL ? 1 : (OW + TH0 - 1) / TH0;
@@ -50,12 +50,12 @@ struct ConvWindow {
 };
 
 // One output channel (number U of CU) of a band: acc += window * weights.  lam: the channels' windows, in 16-byte words.
-template <int KS, int ST, int WW, int TCI, int BAND, int U>
-__device__ __forceinline__ void window_band(const float4* lam, const float* w, float (&acc)[TCI][ConvWindow<KS, ST, WW>::TH][ConvWindow<KS, ST, WW>::OW]) {
-  using G = ConvWindow<KS, ST, WW>;
+template <int KS, int ST, int PD, int WW, int TCI, int BAND, int U>
+__device__ __forceinline__ void window_band(const float4* lam, const float* w, float (&acc)[TCI][ConvWindow<KS, ST, PD, WW>::TH][ConvWindow<KS, ST, PD, WW>::OW]) {
+  using G = ConvWindow<KS, ST, PD, WW>;
   constexpr int H0 = BAND * G::TH;
-  constexpr int HI = (H0 + G::TH - 1) / ST < WW - 1 ? (H0 + G::TH - 1) / ST : WW - 1;
-  constexpr int LO = H0 > KS - 1 ? (H0 - KS + ST) / ST : 0;   // window rows LO to HI reach the band
+  constexpr int HI = (H0 + G::TH - 1 + PD) / ST < WW - 1 ? (H0 + G::TH - 1 + PD) / ST : WW - 1;
+  constexpr int LO = H0 + PD > KS - 1 ? (H0 + PD - KS + ST) / ST : 0;   // window rows LO to HI reach the band
   float l[G::CU * WW * WW + 4];
 #pragma unroll
   for (int iy = HI; iy >= LO; --iy) {
@@ -68,21 +68,24 @@ __device__ __forceinline__ void window_band(const float4* lam, const float* w, f
     }
 #pragma unroll
     for (int r = 0; r < KS; ++r) {
-      const int oy = iy * ST + r - H0;
+      const int oy = iy * ST + r - PD - H0;
       if (oy < 0 || oy >= G::TH) continue;
 #pragma unroll
       for (int s = 0; s < KS; ++s)
 #pragma unroll
-        for (int x = 0; x < WW; ++x)
+        for (int x = 0; x < WW; ++x) {
+          const int ox = x * ST + s - PD;
+          if (ox < 0 || ox >= G::OW) continue;
 #pragma unroll
-          for (int c = 0; c < TCI; ++c) acc[c][oy][x * ST + s] = fmaf(l[first + x], w[(r * KS + s) * TCI + c], acc[c][oy][x * ST + s]);
+          for (int c = 0; c < TCI; ++c) acc[c][oy][ox] = fmaf(l[first + x], w[(r * KS + s) * TCI + c], acc[c][oy][ox]);
+        }
     }
   }
 }
 
-template <int KS, int ST, int WW, int TCI, int BAND, int U>
+template <int KS, int ST, int PD, int WW, int TCI, int BAND, int U>
 __device__ __forceinline__ void window_channels(const float4* lam, const float4* wp, int w_step,
-                                                float (&acc)[TCI][ConvWindow<KS, ST, WW>::TH][ConvWindow<KS, ST, WW>::OW]) {
+                                                float (&acc)[TCI][ConvWindow<KS, ST, PD, WW>::TH][ConvWindow<KS, ST, PD, WW>::OW]) {
   constexpr int NWP = (KS * KS * TCI + 3) / 4 * 4;
   float w[NWP];
 #pragma unroll
@@ -90,27 +93,27 @@ __device__ __forceinline__ void window_channels(const float4* lam, const float4*
     const float4 t = wp[k];
     w[4 * k] = t.x; w[4 * k + 1] = t.y; w[4 * k + 2] = t.z; w[4 * k + 3] = t.w;
   }
-  window_band<KS, ST, WW, TCI, BAND, U>(lam, w, acc);
-  if constexpr (U + 1 < ConvWindow<KS, ST, WW>::CU) window_channels<KS, ST, WW, TCI, BAND, U + 1>(lam, wp + w_step, w_step, acc);
+  window_band<KS, ST, PD, WW, TCI, BAND, U>(lam, w, acc);
+  if constexpr (U + 1 < ConvWindow<KS, ST, PD, WW>::CU) window_channels<KS, ST, PD, WW, TCI, BAND, U + 1>(lam, wp + w_step, w_step, acc);
 }
 
 // ncc channels of a chunk for the warp's band
-template <int KS, int ST, int WW, int TCI, int BAND>
+template <int KS, int ST, int PD, int WW, int TCI, int BAND>
 __device__ __forceinline__ void window_chunk(int band, const float4* lam, const float4* wp, int w_step, int ncc,
-                                             float (&acc)[TCI][ConvWindow<KS, ST, WW>::TH][ConvWindow<KS, ST, WW>::OW]) {
-  using G = ConvWindow<KS, ST, WW>;
+                                             float (&acc)[TCI][ConvWindow<KS, ST, PD, WW>::TH][ConvWindow<KS, ST, PD, WW>::OW]) {
+  using G = ConvWindow<KS, ST, PD, WW>;
   if (band == BAND) {
 #pragma unroll 1
     for (int co = 0; co < ncc; co += G::CU, lam += G::CU * WW * WW / 4, wp += G::CU * w_step)
-      window_channels<KS, ST, WW, TCI, BAND, 0>(lam, wp, w_step, acc);
+      window_channels<KS, ST, PD, WW, TCI, BAND, 0>(lam, wp, w_step, acc);
   } else if constexpr (BAND + 1 < G::NB) {
-    window_chunk<KS, ST, WW, TCI, BAND + 1>(band, lam, wp, w_step, ncc, acc);
+    window_chunk<KS, ST, PD, WW, TCI, BAND + 1>(band, lam, wp, w_step, ncc, acc);
   }
 }
 
-template <int KS, int ST, int WW, int TCI>
-__global__ void __launch_bounds__(32 * ConvWindow<KS, ST, WW>::WARPS, ConvWindow<KS, ST, WW>::BLOCKS) conv_window_kernel(ConvWindowArgs a) {
-  using G = ConvWindow<KS, ST, WW>;
+template <int KS, int ST, int PD, int WW, int TCI>
+__global__ void __launch_bounds__(32 * ConvWindow<KS, ST, PD, WW>::WARPS, ConvWindow<KS, ST, PD, WW>::BLOCKS) conv_window_kernel(ConvWindowArgs a) {
+  using G = ConvWindow<KS, ST, PD, WW>;
   constexpr int OW = G::OW, TH = G::TH, NB = G::NB, PLANE = WW * WW;
   constexpr int NW = KS * KS * TCI, NWP = (NW + 3) / 4 * 4;
   constexpr int N = TCI * TH * OW;
@@ -156,7 +159,7 @@ __global__ void __launch_bounds__(32 * ConvWindow<KS, ST, WW>::WARPS, ConvWindow
     int next_tile = tile, next_ch = ch + 1;
     if (next_ch == nch) { next_ch = 0; next_tile += gridDim.x; }
     if (next_tile < tiles) stage(buf ^ 1, next_tile * rows, next_ch * a.cc);
-    window_chunk<KS, ST, WW, TCI, 0>(band, lamS + buf * buf4 + (rg * 32 + lane) * pitch4,
+    window_chunk<KS, ST, PD, WW, TCI, 0>(band, lamS + buf * buf4 + (rg * 32 + lane) * pitch4,
                                      reinterpret_cast<const float4*>(wS) + (ch * a.cc * a.cgb + cgl) * (NWP / 4), a.cgb * (NWP / 4),
                                      min(a.cc, a.Co - ch * a.cc), acc);
     if (next_ch == 0) {
@@ -186,9 +189,9 @@ __global__ void __launch_bounds__(32 * ConvWindow<KS, ST, WW>::WARPS, ConvWindow
   }
 }
 
-template <int KS, int ST, int WW, int TCI>
+template <int KS, int ST, int PD, int WW, int TCI>
 static int launch_window(ConvWindowArgs a, cudaStream_t stream) {
-  using G = ConvWindow<KS, ST, WW>;
+  using G = ConvWindow<KS, ST, PD, WW>;
   constexpr int NWP = (KS * KS * TCI + 3) / 4 * 4, LIMIT = (G::BLOCKS == 1 ? 224 : 112) * 1024, EPI = 32 * 33 * 4, PLANE = WW * WW;
   const int ncg = ceil_div(a.Ci, TCI);
   // channel groups per block: few of them idle, few blocks that read the same rows, and no idle warps where a block has an SM
@@ -221,37 +224,42 @@ static int launch_window(ConvWindowArgs a, cudaStream_t stream) {
   if (gx > tiles) gx = tiles;
   if (gx < 1) gx = 1;
   static SmemOptIn opt_in;
-  if (int rc = ensure_dynamic_smem(conv_window_kernel<KS, ST, WW, TCI>, LIMIT, opt_in, "conv_window_kernel")) return rc;
-  conv_window_kernel<KS, ST, WW, TCI><<<dim3(gx, gy), threads, smem, stream>>>(a);
+  if (int rc = ensure_dynamic_smem(conv_window_kernel<KS, ST, PD, WW, TCI>, LIMIT, opt_in, "conv_window_kernel")) return rc;
+  conv_window_kernel<KS, ST, PD, WW, TCI><<<dim3(gx, gy), threads, smem, stream>>>(a);
   BF_CHECK_LAUNCH("conv_window_kernel");
   return BF_OK;
 }
 
-template <int KS, int ST, int WW, int MAXW>
+template <int KS, int ST, int PD, int WW, int MAXW>
 static int launch_window_side(const ConvWindowArgs& a, int ww, cudaStream_t stream) {
   if constexpr (WW > MAXW) {
     return BF_E_UNSUPPORTED;
   } else {
-    if (ww != WW) return launch_window_side<KS, ST, WW + 1, MAXW>(a, ww, stream);
-    if constexpr (WW % 2 == 0 || WW <= 7) {
-      constexpr int TCI = ConvWindow<KS, ST, WW>::TCI;
-      if (a.Co % ConvWindow<KS, ST, WW>::CU != 0) return BF_E_UNSUPPORTED;
+    if (ww != WW) return launch_window_side<KS, ST, PD, WW + 1, MAXW>(a, ww, stream);
+    if constexpr (WW % 2 == 0 || (PD == 0 && WW <= 7)) {
+      constexpr int TCI = ConvWindow<KS, ST, PD, WW>::TCI;
+      if (a.Co % ConvWindow<KS, ST, PD, WW>::CU != 0) return BF_E_UNSUPPORTED;
       // single channels where groups would be mostly padding (three channels in groups of four or two)
-      if (TCI > 1 && 5 * (ceil_div(a.Ci, TCI) * TCI) > 6 * a.Ci) return launch_window<KS, ST, WW, 1>(a, stream);
-      return launch_window<KS, ST, WW, TCI>(a, stream);
+      if (TCI > 1 && 5 * (ceil_div(a.Ci, TCI) * TCI) > 6 * a.Ci) return launch_window<KS, ST, PD, WW, 1>(a, stream);
+      return launch_window<KS, ST, PD, WW, TCI>(a, stream);
     }
     return BF_E_UNSUPPORTED;
   }
 }
 
-// Transposed convolution without padding of M rows of WH x WW windows; BF_E_UNSUPPORTED for geometries without an instance.
+// Transposed convolution of M rows of WH x WW maps: windows (no padding), and full maps of 6 to 10 pixels under a 4x4 / 2 kernel with padding
+// 1 and one or two channels below (25,600 rows, 8 -> 1 channels, 10 x 10: 163 -> 77 us; 2048 rows: 21 -> 15; below 0.83 to 1.02 of the
+// row-segment kernel's speed).  Larger maps stay there: their ten and more bands are as many copies of the loop in the
+// instruction cache (16 -> 1 channels, 14 x 14: 333 us there, 419 here).
+// BF_E_UNSUPPORTED for geometries without an instance.
 int launch_conv_window(const float* Lam, const float* W, float* out, int M, int Ci, int Co, int WH, int WW, int kh, int kw, int sh, int sw,
-                       cudaStream_t stream) {
-  if (WH != WW || kh != kw || sh != sw || (reinterpret_cast<uintptr_t>(Lam) & 15u) != 0) return BF_E_UNSUPPORTED;
+                       int ph, int pw, cudaStream_t stream) {
+  if (WH != WW || kh != kw || sh != sw || ph != pw || (reinterpret_cast<uintptr_t>(Lam) & 15u) != 0) return BF_E_UNSUPPORTED;
   const ConvWindowArgs a{Lam, W, out, M, Co, Ci, 0, 0, 0, 0};
-  if (kh == 3 && sh == 1) return launch_window_side<3, 1, 2, 14>(a, WW, stream);
-  if (kh == 4 && sh == 2) return launch_window_side<4, 2, 2, 7>(a, WW, stream);
-  if (kh == 3 && sh == 2) return launch_window_side<3, 2, 2, 7>(a, WW, stream);
+  if (kh == 3 && sh == 1 && ph == 0) return launch_window_side<3, 1, 0, 2, 14>(a, WW, stream);
+  if (kh == 4 && sh == 2 && ph == 0) return launch_window_side<4, 2, 0, 2, 7>(a, WW, stream);
+  if (kh == 3 && sh == 2 && ph == 0) return launch_window_side<3, 2, 0, 2, 7>(a, WW, stream);
+  if (kh == 4 && sh == 2 && ph == 1 && Ci <= 2 && M >= 2048) return launch_window_side<4, 2, 1, 6, 10>(a, WW, stream);
   return BF_E_UNSUPPORTED;
 }
 

@@ -119,9 +119,9 @@ int launch_onehot_conv_window(const float* W, const float* bias, float* out, flo
 int launch_relu_bwd_window(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
                            const float* bias, const float* wstart, const float* wbias, float* Lam, float* delta, const WindowGeom& w, int M,
                            cudaStream_t stream);
-// conv_window.cu: unpadded transposed convolution of small square maps (windows); BF_E_UNSUPPORTED leaves it to conv.cu
+// conv_window.cu: transposed convolution of small square maps (windows, single-channel images); BF_E_UNSUPPORTED leaves it to conv.cu
 int launch_conv_window(const float* Lam, const float* W, float* out, int M, int Ci, int Co, int WH, int WW, int kh, int kw, int sh, int sw,
-                       cudaStream_t stream);
+                       int ph, int pw, cudaStream_t stream);
 int launch_window_to_dense(const float* Awin, float* dense, const WindowGeom& w, int M, cudaStream_t stream);
 int launch_concretize_window(const float* Awin, const float* mid, const float* rad, const float* delta, float* out, int side,
                              const WindowGeom& w, int M, cudaStream_t stream);

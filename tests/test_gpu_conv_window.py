@@ -8,15 +8,15 @@ from boundflow_b200 import _lib
 pytestmark = pytest.mark.gpu
 
 
-def _backward(A, W, stride):
+def _backward(A, W, stride, pad=0):
     """Layer-level call without slopes: A [M, Co, w, w], W [Co, Ci, k, k]."""
     M, Co, w, _ = A.shape
     Ci, k = W.shape[1], W.shape[2]
-    ow = (w - 1) * stride + k
+    ow = (w - 1) * stride + k - 2 * pad
     out = torch.full((M, Ci, ow, ow), float("nan"), device="cuda")
     lib = _lib.load()
     _lib.check(lib.bf_crown_relu_conv2d_bwd_fp32(A.data_ptr(), _lib.SIDE_LOWER, None, None, None, None, W.data_ptr(), None, out.data_ptr(), None, 1,
-                                                 None, 0, 1, M, Ci, ow, ow, Co, w, w, k, k, stride, stride, 0, 0, None))
+                                                 None, 0, 1, M, Ci, ow, ow, Co, w, w, k, k, stride, stride, pad, pad, None))
     return out
 
 
@@ -35,6 +35,18 @@ def test_windows_against_float64(k, stride, w, rows, ci, co):
     n = co * ((k + stride - 1) // stride) ** 2
     err = (_backward(A.cuda(), W.cuda(), stride).cpu().double() - ref).abs()
     assert (err <= n * 2.0**-24 * size).all()
+
+
+@pytest.mark.parametrize("w", (6, 8, 10))
+@pytest.mark.parametrize("rows, ci, co", [(2047, 1, 3), (2048, 1, 3), (2085, 2, 16)])
+def test_padded_maps_against_float64(w, rows, ci, co):
+    g = torch.Generator().manual_seed(w + ci)
+    A = torch.randn((rows, co, w, w), generator=g)
+    W = torch.randn((co, ci, 4, 4), generator=g)
+    ref = torch.nn.functional.conv_transpose2d(A.double(), W.double(), stride=2, padding=1)
+    size = torch.nn.functional.conv_transpose2d(A.double().abs(), W.double().abs(), stride=2, padding=1)
+    err = (_backward(A.cuda(), W.cuda(), 2, 1).cpu().double() - ref).abs()
+    assert (err <= 4 * co * 2.0**-24 * size).all()  # four products per channel
 
 
 @pytest.mark.parametrize("k, stride, w", [(3, 1, 3), (4, 2, 4), (3, 1, 14)])
