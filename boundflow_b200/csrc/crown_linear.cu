@@ -346,7 +346,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_adjoint_linear_kernel(G
 }
 
 // 32 x 64 tiles of a small problem (gemm_small.cuh).  What the epilogue needs is loaded first, without branches (rows and columns
-// clamped): as guarded loads after the multiply loop its seven arrays took 2 to 5 us of a 12 us launch.
+// clamped): behind a guard per element its seven arrays take 10 to 13 thousand clocks, every guard's loads after those before it.
+// 1152 x 256 x 256: 12.0 -> 9.6 us with the copying warps; 333 x 512 x 512: 21.2 -> 15.1.
 template <int PRO>
 __global__ void __launch_bounds__(GS_THREADS, 1) crown_adjoint_small_kernel(GemmArgs g, AdjEpilogue e) {
   extern __shared__ __align__(16) float dsmem[];
