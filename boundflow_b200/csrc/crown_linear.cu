@@ -99,10 +99,12 @@ __global__ void __launch_bounds__(GS_THREADS, 2) crown_bwd_small_kernel(GemmArgs
       const float4 v = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
       if (m0 + r0 + i < g.M && col < g.N && e.out) store4_guard(e.out + (size_t)(m0 + r0 + i) * g.N, col, g.N, vN, v);
       if (e.partial) {  // the order of the 64-column kernels: sixteen groups of four columns, pairwise
-        p[i] += v.x * md[i].x + sgn * fabsf(v.x) * rd[i].x;
-        p[i] += v.y * md[i].y + sgn * fabsf(v.y) * rd[i].y;
-        p[i] += v.z * md[i].z + sgn * fabsf(v.z) * rd[i].z;
-        p[i] += v.w * md[i].w + sgn * fabsf(v.w) * rd[i].w;
+        if (col < g.N) {  // columns past the end: an infinite coefficient times their zero weights is NaN
+          p[i] += v.x * md[i].x + sgn * fabsf(v.x) * rd[i].x;
+          p[i] += v.y * md[i].y + sgn * fabsf(v.y) * rd[i].y;
+          p[i] += v.z * md[i].z + sgn * fabsf(v.z) * rd[i].z;
+          p[i] += v.w * md[i].w + sgn * fabsf(v.w) * rd[i].w;
+        }
         p[i] += __shfl_xor_sync(0xffffffffu, p[i], 1);
         p[i] += __shfl_xor_sync(0xffffffffu, p[i], 2);
         p[i] += __shfl_xor_sync(0xffffffffu, p[i], 4);

@@ -64,3 +64,33 @@ def test_alpha_steps_of_ragged_layers(dev, B, widths, with_beta):
         for got, want in ((alpha.alpha_by_relu_input, out[2]),) + (((beta.beta_by_relu_input, out[3]),) if with_beta else ()):
             same = (got[n].reshape(B, -1).cpu() - want[r].reshape(B, -1)).abs() <= 1e-3
             assert same.float().mean() >= 0.95, (r, n)
+
+
+@pytest.mark.parametrize("N", (4, 60, 64, 68, 784))
+def test_infinite_coefficients_keep_their_sign(dev, N):
+    """One Linear layer with positive weights and a negative bias on a box below zero: a row with an infinite coefficient is
+    bounded by minus infinity, whatever its width."""
+    import ctypes
+
+    from boundflow_b200 import _lib
+
+    lib = _lib.load()
+    B, S, K = 3, 2, 20
+    g = torch.Generator().manual_seed(N)
+    W, b = (torch.rand((K, N), generator=g) + 0.5).to(dev), (-torch.rand((K,), generator=g) - 0.5).to(dev)
+    mid, rad = torch.full((B, N), -1.0, device=dev), torch.full((B, N), 0.25, device=dev)
+    C = torch.rand((B, S, K), generator=g).to(dev)
+    C[:, 1, 7] = float("inf")
+    desc = (_lib.LayerDesc * 1)()
+    desc[0].op, desc[0].W, desc[0].bias, desc[0].n_in, desc[0].n_out = _lib.OP_LINEAR, W.data_ptr(), b.data_ptr(), N, K
+    chain = ctypes.c_void_p()
+    _lib.check(lib.bf_chain_create(desc, 1, ctypes.byref(chain)))
+    try:
+        nbytes = int(lib.bf_chain_crown_workspace_bytes(chain, B, S, 1))
+        ws, out = torch.empty(nbytes, dtype=torch.uint8, device=dev), torch.empty((B, S), device=dev)
+        _lib.check(lib.bf_chain_crown(chain, 1, _lib.SIDE_LOWER, C.data_ptr(), None, None, None, None, mid.data_ptr(), rad.data_ptr(), _lib.NORM_BOX, 0.0,
+                                      out.data_ptr(), ws.data_ptr(), nbytes, B, S, None))
+    finally:
+        lib.bf_chain_destroy(chain)
+    assert torch.isfinite(out[:, 0]).all()
+    assert (out[:, 1] == -float("inf")).all(), out[:, 1]
