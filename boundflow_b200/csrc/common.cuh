@@ -77,7 +77,10 @@ inline int ensure_dynamic_smem(Kernel kernel, int bytes, SmemOptIn& table, const
 
 // Launches that may start while the kernel before them in the stream still runs (programmatic dependent launch): their blocks are
 // placed and wait in grid_dependency() until everything before them is complete and visible, so a chain of short kernels pays
-// the launch itself (2 to 3 us) only once.  A kernel that is launched this way calls grid_dependency() before it touches memory.
+// the launch itself (2 to 3 us) only once.  A kernel that is launched this way begins with grid_dependency() and reads global memory
+// with plain loads (or cp.async) through pointers that are not __restrict__: read-only loads (__ldg, or what a const __restrict__
+// parameter becomes) are taken for constant over the kernel's life and may be moved above the wait, and what the kernel before has
+// written (coefficients, but also a weight that the caller's kernel has just updated or transposed) would be read stale.
 template <typename... Params, typename... Args>
 inline void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -92,11 +95,8 @@ inline void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, s
   cfg.numAttrs = 1;
   (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
-// Returns 0, as a value that exists only after the wait: added to a block index it keeps the loads that depend on it behind the wait.
-__device__ __forceinline__ int grid_dependency() {
-  int zero;
-  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;\n\tmov.b32 %0, 0;" : "=r"(zero) : : "memory");
-  return zero;
+__device__ __forceinline__ void grid_dependency() {
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" : : : "memory");
 }
 
 inline cudaStream_t as_stream(bf_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
@@ -121,8 +121,7 @@ __device__ __forceinline__ float4 load4_guard(const float* __restrict__ row, int
   return v;
 }
 
-// Same for data written earlier in the same stream by another kernel but which
-// must not go through the read-only path (plain loads).
+// Same with plain loads, which the kernels of dependent launches take (see launch_dependent).
 __device__ __forceinline__ float4 load4_plain(const float* row, int idx, int n, bool vec_ok) {
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
   if (vec_ok && idx + 3 < n) {

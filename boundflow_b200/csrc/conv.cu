@@ -71,6 +71,7 @@ __device__ __forceinline__ float2 taps_inside(const IbpConvArgs& g, long long pi
 
 template <bool INTERVAL, int TN>
 __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper, int vec) {
+  grid_dependency();
   constexpr int TM = ConvTile<TN>::TM, CBK = ConvTile<TN>::SLAB, ACCS = INTERVAL ? 2 : 1;
   constexpr int NA = TM * CBK / 256, KSTEP = 256 / TM, WLD = TN + 4, NW = (TN * CBK + 255) / 256;
   constexpr int STAGE = ACCS * CBK * TM + CBK * WLD, PART = ACCS * TM * TN;
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
   const int tid = threadIdx.x, tx = tid % (TM / 4), ty = tid / (TM / 4);
   const int taps = g.kh * g.kw, K = g.Ci * taps, howo = g.Ho * g.Wo, hw = g.Hi * g.Wi;
   const long long npix = (long long)g.B * howo;
-  const long long p0 = (long long)(blockIdx.x + grid_dependency()) * TM;
+  const long long p0 = (long long)blockIdx.x * TM;
   const int c0 = blockIdx.y * TN;
   const int k0 = blockIdx.z * kper, k1 = min(K, k0 + kper);
   const int nk = (k1 > k0) ? (k1 - k0 + CBK - 1) / CBK : 0;
@@ -114,13 +115,13 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
       const int4 t = tab[kt & 1][lk + j * KSTEP];
       const int hi = h0 + t.y, wi = w0 + t.z;
       const bool ok = live && (unsigned)hi < (unsigned)g.Hi && (unsigned)wi < (unsigned)g.Wi;
-      ra[j] = ok ? __ldg(base_a + (pix_off + t.x)) : 0.f;
-      if (INTERVAL) rb[j] = ok ? __ldg(base_b + (pix_off + t.x)) : 0.f;
+      ra[j] = ok ? base_a[pix_off + t.x] : 0.f;
+      if (INTERVAL) rb[j] = ok ? base_b[pix_off + t.x] : 0.f;
     }
 #pragma unroll
     for (int j = 0; j < NW; ++j) {
       const int e = tid + j * 256, co = c0 + e / CBK, k = k0 + kt * CBK + e % CBK;
-      rw[j] = (e < TN * CBK && co < g.Co && k < k1) ? __ldg(g.W + (size_t)co * K + k) : 0.f;
+      rw[j] = (e < TN * CBK && co < g.Co && k < k1) ? g.W[(size_t)co * K + k] : 0.f;
     }
   };
   auto store_slab = [&](int stage) {
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
   for (int i = 0; i < 4; ++i) {
     const int co = c0 + ty * 4 + i;
     if (co >= g.Co || (ranks > 1 && i % ranks != (int)blockIdx.z)) continue;
-    const float bias = g.bias ? __ldg(g.bias + co) : 0.f;
+    const float bias = g.bias ? g.bias[co] : 0.f;
     float lo[4], up[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -359,14 +360,11 @@ int launch_conv_forward_rows(const float* in, const float* W, const float* bias,
 // ---------------------------------------------------------------------------
 constexpr int RELU_ROWS_CHUNK = 4096;
 
-__global__ void __launch_bounds__(256) relu_bwd_rows_kernel(const float* __restrict__ A, const float* __restrict__ dpos,
-                                                            const float* __restrict__ dneg, const float* __restrict__ epos,
-                                                            const float* __restrict__ eneg, const float* __restrict__ add,
-                                                            const float* __restrict__ bias, int chan_size,
-                                                            float* __restrict__ Lam, float* __restrict__ partial,
-                                                            float* __restrict__ delta, int accumulate, int chunk, int S, int n,
-                                                            int vec) {
-  const int m = blockIdx.x + grid_dependency();
+__global__ void __launch_bounds__(256) relu_bwd_rows_kernel(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
+                                                            const float* add, const float* bias, int chan_size, float* Lam, float* partial,
+                                                            float* delta, int accumulate, int chunk, int S, int n, int vec) {
+  grid_dependency();
+  const int m = blockIdx.x;
   const int k0 = blockIdx.y * chunk;
   const int k1 = min(n, k0 + chunk);
   const float* a = A + (size_t)m * n;
@@ -398,7 +396,7 @@ __global__ void __launch_bounds__(256) relu_bwd_rows_kernel(const float* __restr
         int ch = k / chan_size, rem = k - ch * chan_size;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          acc = fmaf(lam[c], __ldg(bias + ch), acc);
+          acc = fmaf(lam[c], bias[ch], acc);
           if (++rem == chan_size) { rem = 0; ++ch; }
         }
       }
@@ -415,7 +413,7 @@ __global__ void __launch_bounds__(256) relu_bwd_rows_kernel(const float* __restr
         acc = fmaf(v, e, acc);
         if (add) lam += add[off + k];
       }
-      if (bias) acc = fmaf(lam, __ldg(bias + k / chan_size), acc);
+      if (bias) acc = fmaf(lam, bias[k / chan_size], acc);
       if (Lam) Lam[(size_t)m * n + k] = lam;
     }
   }
@@ -572,6 +570,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // multiply-adds.  Same order of sums.
 template <int KS, int ST, int PD, int TCI, bool VEC, int TWP, int RT>
 __global__ void __launch_bounds__(256, (TCI > 1 && TWP * RT > 8 ? 2 : 3)) conv_transpose_rowseg_kernel(RowSegArgs a) {
+  grid_dependency();
   using G = RowSeg<KS, ST, PD, VEC, TWP>;
   extern __shared__ __align__(16) float rs_smem[];
   const ConvTArgs& g = a.c;
@@ -589,7 +588,7 @@ __global__ void __launch_bounds__(256, (TCI > 1 && TWP * RT > 8 ? 2 : 3)) conv_t
   const int buf_words = lam_words + w_words;
   constexpr int ROW_ZERO = -2147483647 - 1;
   int* row_off = reinterpret_cast<int*>(rs_smem + 2 * buf_words);  // [nrows] source offset of each tile row, ROW_ZERO: all zeros
-  const int m0 = (blockIdx.x + grid_dependency()) << a.mrl;
+  const int m0 = blockIdx.x << a.mrl;
   const int h0 = (blockIdx.y / a.tiles_x) << a.thl;
   const int w0 = (blockIdx.y % a.tiles_x) * (G::TW * sx);
   const int ci0 = blockIdx.z << cibl;

@@ -22,9 +22,10 @@ struct BwdEpilogue {
 
 template <int PRO, int MH, int NH>
 __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_bwd_linear_kernel(GemmArgs g, BwdEpilogue e) {
+  grid_dependency();
   __shared__ __align__(16) float smem[MAINLOOP_SMEM_FLOATS];
   constexpr int TM = 64 * MH, MR = 4 * MH;
-  const int m0 = (blockIdx.x + grid_dependency()) * TM, n0 = blockIdx.y * (64 * NH);
+  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * (64 * NH);
   float acc[8][8];
   gemm_mainloop<PRO, false, MH, NH>(g, m0, n0, acc, smem);
 
@@ -44,8 +45,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_bwd_linear_kernel(GemmA
         if (e.out) store4_guard(e.out + (size_t)row * g.N, col, g.N, vN, v);
         if (e.partial) {
           const size_t off = (size_t)(row / g.S) * g.N;
-          const float4 md = load4_guard(e.mid + off, col, g.N, vN);
-          const float4 rd = load4_guard(e.rad + off, col, g.N, vN);
+          const float4 md = load4_plain(e.mid + off, col, g.N, vN);
+          const float4 rd = load4_plain(e.rad + off, col, g.N, vN);
           p += v.x * md.x + sgn * fabsf(v.x) * rd.x;
           p += v.y * md.y + sgn * fabsf(v.y) * rd.y;
           p += v.z * md.z + sgn * fabsf(v.z) * rd.z;
@@ -65,11 +66,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_bwd_linear_kernel(GemmA
 
 // 32 x 64 tiles of a small problem (gemm_small.cuh); CTAs of column e.ntiles form the row sums.
 __global__ void __launch_bounds__(GS_THREADS, 2) crown_bwd_small_kernel(GemmArgs g, BwdEpilogue e) {
+  grid_dependency();
   extern __shared__ __align__(16) float dsmem[];
   float* As = dsmem;
   float* Bs = As + GS_STAGES * GS_A_WORDS;
   float* part = Bs + GS_STAGES * GS_B_WORDS<false>;  // [row]: concretisation sums of the right half of the tile
-  const int m0 = (blockIdx.x + grid_dependency()) * GS_ROWS, n0 = blockIdx.y * GS_COLS, tid = threadIdx.x;
+  const int m0 = blockIdx.x * GS_ROWS, n0 = blockIdx.y * GS_COLS, tid = threadIdx.x;
   if ((int)blockIdx.y == e.ntiles) {
     prologue_row_sums(g, m0);
     return;
@@ -88,8 +90,8 @@ __global__ void __launch_bounds__(GS_THREADS, 2) crown_bwd_small_kernel(GemmArgs
       md[i] = rd[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (e.partial && col < g.N) {
         const size_t off = (size_t)(min(m0 + r0 + i, g.M - 1) / g.S) * g.N;
-        md[i] = load4_guard(e.mid + off, col, g.N, vN);
-        rd[i] = load4_guard(e.rad + off, col, g.N, vN);
+        md[i] = load4_plain(e.mid + off, col, g.N, vN);
+        rd[i] = load4_plain(e.rad + off, col, g.N, vN);
       }
     }
     float acc[4][4];
@@ -128,20 +130,20 @@ constexpr int GS_BWD_SMEM = (GS_STAGES * (GS_A_WORDS + GS_B_WORDS<false>) + GS_R
 // columns of W in registers and walks the block's rows, whose K values sit in shared memory.
 constexpr int THIN_KMAX = 16;
 constexpr int THIN_ROWS = 64;   // rows of a block, at most: a small problem takes fewer (its blocks' rows are a serial chain)
-__global__ void __launch_bounds__(128) crown_bwd_thin_kernel(const float* __restrict__ A, const float* __restrict__ W,
-                                                             const float* __restrict__ kbias, float* __restrict__ out,
-                                                             float* __restrict__ delta, int accumulate, int M, int K, int N, int block_rows) {
+__global__ void __launch_bounds__(128) crown_bwd_thin_kernel(const float* A, const float* W, const float* kbias, float* out, float* delta,
+                                                             int accumulate, int M, int K, int N, int block_rows) {
+  grid_dependency();
   __shared__ float a_s[THIN_ROWS * THIN_KMAX];
-  const int m0 = (blockIdx.x + grid_dependency()) * block_rows;
+  const int m0 = blockIdx.x * block_rows;
   const int rows = min(block_rows, M - m0);
+  const int cg = blockIdx.y * blockDim.x + threadIdx.x;  // group of four columns
+  float4 w[THIN_KMAX];                                   // in flight together with the rows
+#pragma unroll
+  for (int k = 0; k < THIN_KMAX; ++k)
+    w[k] = (k < K && cg * 4 < N) ? *reinterpret_cast<const float4*>(W + (size_t)k * N + cg * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
   for (int i = threadIdx.x; i < rows * K; i += blockDim.x) a_s[i] = A[(size_t)m0 * K + i];
   __syncthreads();
-  const int cg = blockIdx.y * blockDim.x + threadIdx.x;  // group of four columns
   if (cg * 4 < N) {
-    float4 w[THIN_KMAX];
-#pragma unroll
-    for (int k = 0; k < THIN_KMAX; ++k)
-      w[k] = (k < K) ? *reinterpret_cast<const float4*>(W + (size_t)k * N + cg * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
     for (int r = 0; r < rows; ++r) {
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(128) crown_bwd_thin_kernel(const float* __rest
     for (int r = threadIdx.x; r < rows; r += blockDim.x) {
       float sum = 0.f;
       if (kbias)
-        for (int k = 0; k < K; ++k) sum = fmaf(a_s[r * K + k], __ldg(kbias + k), sum);
+        for (int k = 0; k < K; ++k) sum = fmaf(a_s[r * K + k], kbias[k], sum);
       delta[m0 + r] = accumulate ? delta[m0 + r] + sum : sum;
     }
   }
@@ -251,9 +253,10 @@ static_assert(ADJ_SMEM_BYTES >= MAINLOOP_SMEM_FLOATS * (int)sizeof(float), "stag
 
 template <int PRO, int MH, int NH>
 __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_adjoint_linear_kernel(GemmArgs g, AdjEpilogue e) {
+  grid_dependency();
   extern __shared__ __align__(16) float dsmem[];
   constexpr int TM = 64 * MH, TN = 64 * NH, MR = 4 * MH;
-  const int m0 = (blockIdx.x + grid_dependency()) * TM, n0 = blockIdx.y * TN;
+  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
   float acc[8][8];
   gemm_mainloop<PRO, true, MH, NH>(g, m0, n0, acc, dsmem);
   // the main loop ends with __syncthreads(): the slabs may now be overwritten by the stage tile
@@ -272,15 +275,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_adjoint_linear_kernel(G
       if (row < g.M && col < g.N) {
         const size_t off = (size_t)(row / g.S) * g.N;
         float4 nb = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (e.nbias) nb = load4_guard(e.nbias, col, g.N, vN);
-        const float4 ah = load4_guard(e.Ahat + (size_t)row * g.N, col, g.N, vN);
-        const float4 dp = load4_guard(e.dpos + off, col, g.N, vN);
-        const float4 dn = load4_guard(e.dneg + off, col, g.N, vN);
+        if (e.nbias) nb = load4_plain(e.nbias, col, g.N, vN);
+        const float4 ah = load4_plain(e.Ahat + (size_t)row * g.N, col, g.N, vN);
+        const float4 dp = load4_plain(e.dpos + off, col, g.N, vN);
+        const float4 dn = load4_plain(e.dneg + off, col, g.N, vN);
         float4 ep = make_float4(0.f, 0.f, 0.f, 0.f), en = ep;
-        if (e.epos) ep = load4_guard(e.epos + off, col, g.N, vN);
-        if (e.eneg) en = load4_guard(e.eneg + off, col, g.N, vN);
-        const float4 pl = load4_guard(e.pre_l + off, col, g.N, vN);
-        const float4 pu = load4_guard(e.pre_u + off, col, g.N, vN);
+        if (e.epos) ep = load4_plain(e.epos + off, col, g.N, vN);
+        if (e.eneg) en = load4_plain(e.eneg + off, col, g.N, vN);
+        const float4 pl = load4_plain(e.pre_l + off, col, g.N, vN);
+        const float4 pu = load4_plain(e.pre_u + off, col, g.N, vN);
         float4 h;
 #define BF_ADJ(c, idx)                                               \
   {                                                                  \
@@ -330,8 +333,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_adjoint_linear_kernel(G
         for (int q = 0; q < 4; ++q) {
           const int cc = n0 + cl + q;
           float gg = 0.f;
-          if (row < g.M && cc < g.N) gg = acc[i][jb * 4 + q] + (e.nbias ? __ldg(e.nbias + cc) : 0.f);
-          if (e.gw != nullptr && row < g.M) gg *= __ldg(e.gw + row);
+          if (row < g.M && cc < g.N) gg = acc[i][jb * 4 + q] + (e.nbias ? e.nbias[cc] : 0.f);
+          if (e.gw != nullptr && row < g.M) gg *= e.gw[row];
           dsmem[rl * STAGE_LD + cl + q] = gg;
         }
       }
@@ -352,11 +355,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_adjoint_linear_kernel(G
 // 1152 x 256 x 256: 12.0 -> 9.6 us with the copying warps; 333 x 512 x 512: 21.2 -> 15.1.
 template <int PRO>
 __global__ void __launch_bounds__(GS_THREADS, 1) crown_adjoint_small_kernel(GemmArgs g, AdjEpilogue e) {
+  grid_dependency();
   extern __shared__ __align__(16) float dsmem[];
   float* As = dsmem;
   float* Bs = As + GS_STAGES * GS_A_WORDS;
   float* red = Bs + GS_STAGES * GS_B_WORDS<true>;  // [row][GS_COLS + 1]
-  const int m0 = (blockIdx.x + grid_dependency()) * GS_ROWS, n0 = blockIdx.y * GS_COLS, tid = threadIdx.x;
+  const int m0 = blockIdx.x * GS_ROWS, n0 = blockIdx.y * GS_COLS, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5, tx = lane & 7, ty = lane >> 3;
   const int r0 = (warp >> 1) * 16 + ty * 4, c0 = (warp & 1) * 32 + tx;
   float acc[4][4];
@@ -365,7 +369,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) crown_adjoint_small_kernel(Gemm
   } else {
     float ah[4][4], dp[4][4], dn[4][4], ep[4][4], en[4][4], pl[4][4], pu[4][4], nb[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) nb[j] = e.nbias ? __ldg(e.nbias + min(n0 + c0 + 8 * j, g.N - 1)) : 0.f;
+    for (int j = 0; j < 4; ++j) nb[j] = e.nbias ? e.nbias[min(n0 + c0 + 8 * j, g.N - 1)] : 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int row = min(m0 + r0 + i, g.M - 1);
@@ -373,13 +377,13 @@ __global__ void __launch_bounds__(GS_THREADS, 1) crown_adjoint_small_kernel(Gemm
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int col = min(n0 + c0 + 8 * j, g.N - 1);
-        ah[i][j] = __ldg(e.Ahat + at + col);
-        dp[i][j] = __ldg(e.dpos + dom + col);
-        dn[i][j] = __ldg(e.dneg + dom + col);
-        ep[i][j] = e.epos ? __ldg(e.epos + dom + col) : 0.f;
-        en[i][j] = e.eneg ? __ldg(e.eneg + dom + col) : 0.f;
-        pl[i][j] = __ldg(e.pre_l + dom + col);
-        pu[i][j] = __ldg(e.pre_u + dom + col);
+        ah[i][j] = e.Ahat[at + col];
+        dp[i][j] = e.dpos[dom + col];
+        dn[i][j] = e.dneg[dom + col];
+        ep[i][j] = e.epos ? e.epos[dom + col] : 0.f;
+        en[i][j] = e.eneg ? e.eneg[dom + col] : 0.f;
+        pl[i][j] = e.pre_l[dom + col];
+        pu[i][j] = e.pre_u[dom + col];
       }
     }
     gs_compute<true>(g.K, As, Bs, r0, c0, acc);
@@ -416,7 +420,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) crown_adjoint_small_kernel(Gemm
     if (tid < GS_COMPUTE) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float w = e.gw ? __ldg(e.gw + min(m0 + r0 + i, g.M - 1)) : 1.f;
+        const float w = e.gw ? e.gw[min(m0 + r0 + i, g.M - 1)] : 1.f;
 #pragma unroll
         for (int j = 0; j < 4; ++j) red[(r0 + i) * (GS_COLS + 1) + c0 + 8 * j] = e.gw ? acc[i][j] * w : acc[i][j];
       }

@@ -127,20 +127,20 @@ __device__ __forceinline__ void gemm_mainloop(const GemmArgs& g, const int m0, c
       const bool ok = m < g.M && k < g.K;
       float4 a = z4, kb = z4, dp = z4, dn = z4, ep = z4, en = z4, ad = z4;
       if (ok) {
-        a = load4_guard(g.A + (size_t)m * g.K, k, g.K, vK);
+        a = load4_plain(g.A + (size_t)m * g.K, k, g.K, vK);
         const size_t off = (size_t)dom[i] * g.K;
         if (PRO == PRO_RELU) {
-          if (g.kbias) kb = load4_guard(g.kbias, k, g.K, vK);
+          if (g.kbias) kb = load4_plain(g.kbias, k, g.K, vK);
           if (g.dpos) {
-            dp = load4_guard(g.dpos + off, k, g.K, vK);
-            dn = load4_guard(g.dneg + off, k, g.K, vK);
-            if (g.epos) ep = load4_guard(g.epos + off, k, g.K, vK);
-            if (g.eneg) en = load4_guard(g.eneg + off, k, g.K, vK);
-            if (g.add) ad = load4_guard(g.add + off, k, g.K, vK);
+            dp = load4_plain(g.dpos + off, k, g.K, vK);
+            dn = load4_plain(g.dneg + off, k, g.K, vK);
+            if (g.epos) ep = load4_plain(g.epos + off, k, g.K, vK);
+            if (g.eneg) en = load4_plain(g.eneg + off, k, g.K, vK);
+            if (g.add) ad = load4_plain(g.add + off, k, g.K, vK);
           }
         } else if (PRO == PRO_H0) {
-          dp = load4_guard(g.mid + off, k, g.K, vK);
-          dn = load4_guard(g.rad + off, k, g.K, vK);
+          dp = load4_plain(g.mid + off, k, g.K, vK);
+          dn = load4_plain(g.rad + off, k, g.K, vK);
         }
       }
       if (DEFER) {
@@ -154,7 +154,7 @@ __device__ __forceinline__ void gemm_mainloop(const GemmArgs& g, const int m0, c
       for (int i = 0; i < NH; ++i) {
         const int n = n0 + lrow + i * 64;
         float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (n < g.N && k < g.K) b = load4_guard(g.Bm + (size_t)n * g.K, k, g.K, vK);
+        if (n < g.N && k < g.K) b = load4_plain(g.Bm + (size_t)n * g.K, k, g.K, vK);
         breg[i] = b;
       }
     } else {
@@ -163,7 +163,7 @@ __device__ __forceinline__ void gemm_mainloop(const GemmArgs& g, const int m0, c
         const int kk = kt * BK + bkr + i * 8;
         const int n = n0 + bnc;
         float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (kk < g.K && n < g.N && bnc < 64 * NH) b = load4_guard(g.Bm + (size_t)kk * g.N, n, g.N, vN);
+        if (kk < g.K && n < g.N && bnc < 64 * NH) b = load4_plain(g.Bm + (size_t)kk * g.N, n, g.N, vN);
         breg[i] = b;
       }
     }

@@ -83,14 +83,14 @@ __device__ __forceinline__ void gs_fill(const GemmArgs& g, const int m0, const i
       r.got[h] = live[h] && k < g.K;
       r.a[h] = r.p[h] = r.n[h] = r.d[h] = z4;
       if (r.got[h]) {
-        r.a[h] = load4_guard(pa[h], k, g.K, vK);
+        r.a[h] = load4_plain(pa[h], k, g.K, vK);
         if (PRO == PRO_RELU && g.dpos) {
-          r.p[h] = load4_guard(g.dpos + off[h], k, g.K, vK);
-          r.n[h] = load4_guard(g.dneg + off[h], k, g.K, vK);
-          if (g.add) r.d[h] = load4_guard(g.add + off[h], k, g.K, vK);
+          r.p[h] = load4_plain(g.dpos + off[h], k, g.K, vK);
+          r.n[h] = load4_plain(g.dneg + off[h], k, g.K, vK);
+          if (g.add) r.d[h] = load4_plain(g.add + off[h], k, g.K, vK);
         } else if (PRO == PRO_H0) {
-          r.p[h] = load4_guard(g.mid + off[h], k, g.K, vK);
-          r.n[h] = load4_guard(g.rad + off[h], k, g.K, vK);
+          r.p[h] = load4_plain(g.mid + off[h], k, g.K, vK);
+          r.n[h] = load4_plain(g.rad + off[h], k, g.K, vK);
         }
       }
     }
@@ -201,14 +201,14 @@ __device__ __forceinline__ void prologue_row_sums(const GemmArgs& g, const int m
       const int k = k0 + 16 * u;
       a[u] = kb[u] = dp[u] = dn[u] = ep[u] = en[u] = ad[u] = z4;
       if (k < g.K) {
-        a[u] = load4_guard(pa, k, g.K, vK);
-        if (g.kbias) kb[u] = load4_guard(g.kbias, k, g.K, vK);
+        a[u] = load4_plain(pa, k, g.K, vK);
+        if (g.kbias) kb[u] = load4_plain(g.kbias, k, g.K, vK);
         if (g.dpos) {
-          dp[u] = load4_guard(g.dpos + off, k, g.K, vK);
-          dn[u] = load4_guard(g.dneg + off, k, g.K, vK);
-          if (g.epos) ep[u] = load4_guard(g.epos + off, k, g.K, vK);
-          if (g.eneg) en[u] = load4_guard(g.eneg + off, k, g.K, vK);
-          if (g.add) ad[u] = load4_guard(g.add + off, k, g.K, vK);
+          dp[u] = load4_plain(g.dpos + off, k, g.K, vK);
+          dn[u] = load4_plain(g.dneg + off, k, g.K, vK);
+          if (g.epos) ep[u] = load4_plain(g.epos + off, k, g.K, vK);
+          if (g.eneg) en[u] = load4_plain(g.eneg + off, k, g.K, vK);
+          if (g.add) ad[u] = load4_plain(g.add + off, k, g.K, vK);
         }
       }
     }

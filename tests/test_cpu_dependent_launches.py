@@ -1,0 +1,49 @@
+"""Kernels that may start before the one in front of them has finished (launch_dependent): each waits before anything else, and neither it
+nor a device function that it calls reads global memory through the read-only path, whose loads may be moved above the wait."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "boundflow_b200", "csrc")
+READ_ONLY = re.compile(r"__ldg\b|\bld\.global\.nc\b|\bconst\b[^,;(){}]*__restrict__")
+
+
+def _functions():
+    """({kernel: (parameters, body)}, {device function: text}, all sources without comments)"""
+    kernels, device, sources = {}, {}, ""
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, name)) as fh:
+                text = re.sub(r"//[^\n]*|/\*.*?\*/", "", fh.read(), flags=re.S)
+            sources += text
+            for m in re.finditer(r"(__global__|__device__)\b[^;{}()]*?(?:__launch_bounds__\([^{;]*?\)\s*)?(\w+)\s*\(([^;{}]*)\)\s*\{", text):
+                depth, end = 1, m.end()
+                while depth:
+                    depth += {"{": 1, "}": -1}.get(text[end], 0)
+                    end += 1
+                if m.group(1) == "__global__":
+                    assert m.group(2) not in kernels, m.group(2)
+                    kernels[m.group(2)] = (m.group(3), text[m.end():end])
+                else:
+                    device[m.group(2)] = device.get(m.group(2), "") + m.group(3) + text[m.end():end]
+    return kernels, device, sources
+
+
+def test_dependent_kernels_wait_first_and_read_with_plain_loads():
+    kernels, device, sources = _functions()
+    launched = set(re.findall(r"launch_dependent\(\s*(?:bf::)?(\w+_kernel)", sources))
+    # the clusters of conv_tile_kernel are launched with the attribute among others
+    launched |= set(re.findall(r"cudaLaunchKernelEx\(&cfg, (\w+_kernel)", sources)) & {"conv_tile_kernel"}
+    assert len(launched) >= 14 and launched <= set(kernels), launched - set(kernels)
+    waiting = {k for k, (_, body) in kernels.items() if "grid_dependency()" in body}
+    assert waiting == launched, waiting ^ launched
+    for k in sorted(launched):
+        params, body = kernels[k]
+        assert re.match(r"\s*grid_dependency\(\);", body), f"{k}: the wait is not the first statement"
+        assert "__restrict__" not in params, f"{k}: a __restrict__ parameter's loads may pass the wait"
+        seen, todo = set(), [body]
+        while todo:
+            text = todo.pop()
+            assert not READ_ONLY.search(text), f"{k}: {READ_ONLY.search(text).group(0)}"
+            for f in set(re.findall(r"\b(\w+)\s*(?:<[^;(){}]*>)?\s*\(", text)) & set(device) - seen:
+                seen.add(f)
+                todo.append(device[f])
