@@ -350,11 +350,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_adjoint_linear_kernel(G
   }
 }
 
-// 32 x 64 tiles of a small problem (gemm_small.cuh).  What the epilogue needs is loaded first, without branches (rows and columns
-// clamped): behind a guard per element its seven arrays take 10 to 13 thousand clocks, every guard's loads after those before it.
+// 32 x 64 tiles of a small problem (gemm_small.cuh).  What the epilogue needs is loaded without branches (rows and columns clamped):
+// behind a guard per element its seven arrays take 10 to 13 thousand clocks, every guard's loads after those before it.  AHEAD: of
+// all four rows of a thread before the first slab, 209 registers, for launches of at most one CTA per SM.  Otherwise two rows
+// at a time after the last slab, so that two CTAs share an SM (10 steps on four 512-wide layers, 128 inputs, 288 CTAs: 3.82 ms with one CTA
+// per SM, 3.51 with two, 4.33 on 64 x 64 tiles; 500 inputs, 128-wide, 282 CTAs: 1.85, 1.70, 1.90).
 // 1152 x 256 x 256: 12.0 -> 9.6 us with the copying warps; 333 x 512 x 512: 21.2 -> 15.1.
-template <int PRO>
-__global__ void __launch_bounds__(GS_THREADS, 1) crown_adjoint_small_kernel(GemmArgs g, AdjEpilogue e) {
+template <int PRO, bool AHEAD>
+__global__ void __launch_bounds__(GS_THREADS, AHEAD ? 1 : 2) crown_adjoint_small_kernel(GemmArgs g, AdjEpilogue e) {
   grid_dependency();
   extern __shared__ __align__(16) float dsmem[];
   float* As = dsmem;
@@ -367,38 +370,46 @@ __global__ void __launch_bounds__(GS_THREADS, 1) crown_adjoint_small_kernel(Gemm
   if (tid >= GS_COMPUTE) {
     gs_fill<PRO, true>(g, m0, n0, As, Bs, tid - GS_COMPUTE);
   } else {
-    float ah[4][4], dp[4][4], dn[4][4], ep[4][4], en[4][4], pl[4][4], pu[4][4], nb[4];
+    constexpr int R = AHEAD ? 4 : 2;
+    float ah[R][4], dp[R][4], dn[R][4], ep[R][4], en[R][4], pl[R][4], pu[R][4], nb[4];
+    auto load = [&](int first) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) nb[j] = e.nbias ? e.nbias[min(n0 + c0 + 8 * j, g.N - 1)] : 0.f;
+      for (int j = 0; j < 4; ++j) nb[j] = e.nbias ? e.nbias[min(n0 + c0 + 8 * j, g.N - 1)] : 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int row = min(m0 + r0 + i, g.M - 1);
-      const size_t at = (size_t)row * g.N, dom = (size_t)(row / g.S) * g.N;
+      for (int i = 0; i < R; ++i) {
+        const int row = min(m0 + r0 + first + i, g.M - 1);
+        const size_t at = (size_t)row * g.N, dom = (size_t)(row / g.S) * g.N;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int col = min(n0 + c0 + 8 * j, g.N - 1);
-        ah[i][j] = e.Ahat[at + col];
-        dp[i][j] = e.dpos[dom + col];
-        dn[i][j] = e.dneg[dom + col];
-        ep[i][j] = e.epos ? e.epos[dom + col] : 0.f;
-        en[i][j] = e.eneg ? e.eneg[dom + col] : 0.f;
-        pl[i][j] = e.pre_l[dom + col];
-        pu[i][j] = e.pre_u[dom + col];
+        for (int j = 0; j < 4; ++j) {
+          const int col = min(n0 + c0 + 8 * j, g.N - 1);
+          ah[i][j] = e.Ahat[at + col];
+          dp[i][j] = e.dpos[dom + col];
+          dn[i][j] = e.dneg[dom + col];
+          ep[i][j] = e.epos ? e.epos[dom + col] : 0.f;
+          en[i][j] = e.eneg ? e.eneg[dom + col] : 0.f;
+          pl[i][j] = e.pre_l[dom + col];
+          pu[i][j] = e.pre_u[dom + col];
+        }
       }
-    }
+    };
+    if (AHEAD) load(0);
     gs_compute<true>(g.K, As, Bs, r0, c0, acc);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int row = m0 + r0 + i;
+    for (int first = 0; first < 4; first += R) {
+      if (!AHEAD) load(first);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int col = n0 + c0 + 8 * j;
-        const float gg = acc[i][j] + nb[j];
-        const bool sel = ah[i][j] >= 0.f;
-        const float h = (sel ? dp[i][j] : dn[i][j]) * gg + (sel ? ep[i][j] : en[i][j]);
-        if (e.hout && row < g.M && col < g.N) e.hout[(size_t)row * g.N + col] = h;
-        red[(r0 + i) * (GS_COLS + 1) + c0 + 8 * j] = (sel && pl[i][j] < 0.f && pu[i][j] > 0.f) ? ah[i][j] * gg : 0.f;
-        acc[i][j] = gg;
+      for (int i = 0; i < R; ++i) {
+        const int row = m0 + r0 + first + i;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int col = n0 + c0 + 8 * j;
+          const float gg = acc[first + i][j] + nb[j];
+          const bool sel = ah[i][j] >= 0.f;
+          const float h = (sel ? dp[i][j] : dn[i][j]) * gg + (sel ? ep[i][j] : en[i][j]);
+          if (e.hout && row < g.M && col < g.N) e.hout[(size_t)row * g.N + col] = h;
+          red[(r0 + first + i) * (GS_COLS + 1) + c0 + 8 * j] = (sel && pl[i][j] < 0.f && pu[i][j] > 0.f) ? ah[i][j] * gg : 0.f;
+          acc[first + i][j] = gg;
+        }
       }
     }
   }
@@ -435,7 +446,7 @@ int launch_crown_adjoint_linear(const float* Hprev, int first_layer, const float
                                 const float* epos, const float* eneg, const float* pre_l, const float* pre_u,
                                 float* hout, float* grad, float* gsum, int M, int S, int K, int N, cudaStream_t stream,
                                 const float* gw) {
-  static SmemOptIn opt_in[6];
+  static SmemOptIn opt_in[8];
   GemmArgs g{};
   g.A = Hprev; g.Bm = W; g.M = M; g.N = N; g.K = K; g.S = S;
   const void* kptrs[] = {Hprev, W, mid, rad};
@@ -449,6 +460,7 @@ int launch_crown_adjoint_linear(const float* Hprev, int first_layer, const float
   // 32-row tiles only while a domain's S rows still touch at most two row tiles (two atomic addends commute: deterministic sums)
   const bool small = ffma_small_tiles(M, N), quarter = ffma_quarter_tiles(M, N) && S <= 32;
   dim3 grid(ceil_div(M, quarter ? GS_ROWS : (small ? 64 : BM)), ceil_div(N, small ? 64 : BN));
+  const bool one_each = grid.x * grid.y <= 148;
   timing_begin(T_ADJ, stream);
 #define BF_ADJ_LAUNCH(PRO_, MH_, NH_, slot)                                                                                     \
   {                                                                                                                             \
@@ -457,15 +469,15 @@ int launch_crown_adjoint_linear(const float* Hprev, int first_layer, const float
       return rc;                                                                                                                \
     launch_dependent(crown_adjoint_linear_kernel<PRO_, MH_, NH_>, grid, GEMM_THREADS, ADJ_SMEM_BYTES, stream, g, e);            \
   }
-#define BF_ADJ_SMALL(PRO_, slot)                                                                                                  \
+#define BF_ADJ_SMALL(PRO_, AHEAD_, slot)                                                                                          \
   {                                                                                                                             \
-    if (int rc = ensure_dynamic_smem(crown_adjoint_small_kernel<PRO_>, GS_ADJ_SMEM, opt_in[slot], "crown_adjoint_small_kernel")) return rc; \
-    launch_dependent(crown_adjoint_small_kernel<PRO_>, grid, GS_THREADS, GS_ADJ_SMEM, stream, g, e);                              \
+    if (int rc = ensure_dynamic_smem(crown_adjoint_small_kernel<PRO_, AHEAD_>, GS_ADJ_SMEM, opt_in[slot], "crown_adjoint_small_kernel")) return rc; \
+    launch_dependent(crown_adjoint_small_kernel<PRO_, AHEAD_>, grid, GS_THREADS, GS_ADJ_SMEM, stream, g, e);                      \
   }
   if (first_layer) {
-    if (quarter) BF_ADJ_SMALL(PRO_H0, 4) else if (small) BF_ADJ_LAUNCH(PRO_H0, 1, 1, 0) else BF_ADJ_LAUNCH(PRO_H0, 2, 2, 1)
+    if (quarter && one_each) BF_ADJ_SMALL(PRO_H0, true, 4) else if (quarter) BF_ADJ_SMALL(PRO_H0, false, 6) else if (small) BF_ADJ_LAUNCH(PRO_H0, 1, 1, 0) else BF_ADJ_LAUNCH(PRO_H0, 2, 2, 1)
   } else {
-    if (quarter) BF_ADJ_SMALL(PRO_PLAIN, 5) else if (small) BF_ADJ_LAUNCH(PRO_PLAIN, 1, 1, 2) else BF_ADJ_LAUNCH(PRO_PLAIN, 2, 2, 3)
+    if (quarter && one_each) BF_ADJ_SMALL(PRO_PLAIN, true, 5) else if (quarter) BF_ADJ_SMALL(PRO_PLAIN, false, 7) else if (small) BF_ADJ_LAUNCH(PRO_PLAIN, 1, 1, 2) else BF_ADJ_LAUNCH(PRO_PLAIN, 2, 2, 3)
   }
 #undef BF_ADJ_LAUNCH
 #undef BF_ADJ_SMALL

@@ -66,6 +66,60 @@ def test_alpha_steps_of_ragged_layers(dev, B, widths, with_beta):
             assert same.float().mean() >= 0.95, (r, n)
 
 
+# the last three: more tiles than SMs (two adjoint CTAs per SM), the others fewer
+@pytest.mark.parametrize("B, S, n0, widths", [(7, 9, 33, (33, 70, 65)), (2, 9, 784, (64, 32)), (40, 9, 50, (31, 129)), (70, 1, 65, (65,)), (3, 32, 40, (100, 100)),
+                                              (72, 9, 784, (512, 512)), (300, 9, 64, (128, 100)), (147, 9, 61, (197, 130))])
+def test_alpha_gradient_is_exact_on_small_integers(dev, B, S, n0, widths):
+    """Integer weights and inputs, slopes in quarters: every sum is exact in FP32 in any order, so the gradient of every neuron of every
+    domain, and the bounds, have to be those of float64."""
+    from boundflow_b200 import workloads as W
+    from boundflow_b200.crown import alpha_grad_from_trace, ibp_trace
+    from boundflow_b200.ir import InputSpec
+
+    g = torch.Generator().manual_seed(B + n0)
+    pick = lambda values, *shape: torch.tensor(values)[torch.randint(0, len(values), shape, generator=g)]
+    wl = W.make_workload("c1", batch=1, net=W.NetSpec((n0,), [("fc", w) for w in widths] + [("fc", 10)]))
+    params, dims = wl.module.bindings["params"], (n0,) + tuple(widths) + (10,)
+    for k in range(1, len(dims)):
+        keep = torch.rand((dims[k], dims[k - 1]), generator=g) < min(1.0, 24.0 / dims[k - 1])
+        params[f"W{k}"], params[f"b{k}"] = pick((-1.0, 1.0), dims[k], dims[k - 1]) * keep, pick((-2.0, -1.0, 1.0, 2.0), dims[k])
+    mid, rad = pick((-2.0, -1.0, 0.0, 1.0, 3.0), B, n0), pick((0.0, 1.0, 2.0), B, n0)
+    C = pick((-1.0, 0.0, 1.0), B, S, 10)
+    pre_l = [pick((-1.0, -1.0, -1.0, -2.0, 0.5), B, n) for n in widths]          # slope 1/2, inactive, active
+    pre_u = [torch.where(l == -2.0, -1.0, 1.0) for l in pre_l]
+    alpha = [pick((0.0, 0.25, 0.5, 1.0), B, n) for n in widths]
+    trace = ibp_trace(wl.module, InputSpec.box(value_name="input", lower=(mid - rad).to(dev), upper=(mid + rad).to(dev)))
+    trace.pre_l, trace.pre_u = [t.to(dev) for t in pre_l], [t.to(dev) for t in pre_u]
+    grads, lower = alpha_grad_from_trace(trace, C.to(dev), [a.to(dev) for a in alpha], spec_reduce="sum")
+
+    def contract(x, M, quarters):  # x M in float64; its terms' magnitudes stay below 2^24 of the grid of the values
+        assert (x.abs() @ M.abs()).max() * 4.0**quarters < 2.0**23
+        return x @ M
+
+    Ws, bs = [params[f"W{k}"].double() for k in range(1, len(dims))], [params[f"b{k}"].double() for k in range(1, len(dims))]
+    open_ = [(l < 0) & (u > 0) for l, u in zip(pre_l, pre_u)]
+    up = [torch.where(o, 0.5, (l > 0).double())[:, None].double() for o, l in zip(open_, pre_l)]
+    low = [torch.where(o, a.double(), (l > 0).double())[:, None] for o, l, a in zip(open_, pre_l, alpha)]
+    icpt = [o.double()[:, None] * 0.5 for o in open_]
+    A, R, bound, Ahat = C.double(), len(widths), 0.0, [None] * len(widths)
+    for r in reversed(range(R)):
+        bound = bound + A @ bs[r + 1]
+        Ahat[r] = contract(A, Ws[r + 1], R - 1 - r)
+        bound = bound + (torch.where(Ahat[r] < 0, Ahat[r], 0.0) * icpt[r]).sum(-1)
+        A = Ahat[r] * torch.where(Ahat[r] >= 0, low[r], up[r])
+    bound = bound + A @ bs[0]
+    A = contract(A, Ws[0], R)
+    want = bound + (A * mid.double()[:, None]).sum(-1) - (A.abs() * rad.double()[:, None]).sum(-1)
+    assert torch.equal(lower.cpu().double(), want)
+    h = mid.double()[:, None] - A.sign() * rad.double()[:, None]
+    for r in range(R):
+        v = contract(h, Ws[r].t(), r) + bs[r]
+        terms = torch.where((Ahat[r] >= 0) & open_[r][:, None], Ahat[r] * v, 0.0)
+        assert terms.abs().sum(1).max() * 4.0**R < 2.0**23
+        assert torch.equal(grads[r].cpu().double(), -terms.sum(1)), r
+        h = torch.where(Ahat[r] >= 0, low[r] * v, up[r] * v + icpt[r])
+
+
 @pytest.mark.parametrize("N", (4, 60, 64, 68, 784))
 def test_infinite_coefficients_keep_their_sign(dev, N):
     """One Linear layer with positive weights and a negative bias on a box below zero: a row with an infinite coefficient is
