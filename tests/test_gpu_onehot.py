@@ -71,3 +71,34 @@ def test_intermediate_recipe_on_mlp_matches_oracle(dev):
     for r, nm in enumerate(wl.relu_names):
         assert_close(pre[nm].lower, ref_tr.pre[r][0], f"pre {nm} lower")
         assert_close(pre[nm].upper, ref_tr.pre[r][1], f"pre {nm} upper")
+
+
+@pytest.mark.parametrize("n_in", (1, 2, 3, 4, 5, 12, 31, 33, 100, 128, 255, 1020, 1024, 1030))
+@pytest.mark.parametrize("B, first, S", [(1, 0, 1), (3, 2, 11), (29, 5, 35)])
+def test_identity_rows_of_one_linear_layer(dev, n_in, B, first, S):
+    """Rows shorter and longer than the threads that copy them, counts that do not fill a block, and the neighbours of the rows untouched."""
+    import ctypes
+
+    from boundflow_b200 import _lib
+
+    lib = _lib.load()
+    g = torch.Generator().manual_seed(n_in + S)
+    W, b = torch.randn((40, n_in), generator=g), torch.randn((40,), generator=g)
+    mid, rad = torch.randn((B, n_in), generator=g), torch.rand((B, n_in), generator=g)
+    d = {k: t.to(dev) for k, t in dict(W=W, b=b, mid=mid, rad=rad).items()}
+    desc = (_lib.LayerDesc * 1)()
+    desc[0].op, desc[0].W, desc[0].bias, desc[0].n_in, desc[0].n_out = _lib.OP_LINEAR, d["W"].data_ptr(), d["b"].data_ptr(), n_in, 40
+    chain = ctypes.c_void_p()
+    _lib.check(lib.bf_chain_create(desc, 1, ctypes.byref(chain)))
+    try:
+        nbytes = int(lib.bf_chain_crown_workspace_bytes(chain, B, S, 1))
+        ws, out = torch.full((nbytes + 4096,), 0x55, dtype=torch.uint8, device=dev), torch.empty((B, S), device=dev)
+        _lib.check(lib.bf_chain_crown_onehot(chain, 1, _lib.SIDE_UPPER, first, None, None, None, None, d["mid"].data_ptr(), d["rad"].data_ptr(), _lib.NORM_BOX, 0.0,
+                                             out.data_ptr(), ws.data_ptr(), nbytes, B, S, None))
+    finally:
+        lib.bf_chain_destroy(chain)
+    rows, size = W[first:first + S].double(), mid.double().abs() + rad.double()
+    want = mid.double() @ rows.t() + rad.double() @ rows.abs().t() + b[first:first + S].double()
+    # 2 n_in products and the bias in any order
+    assert ((out.cpu().double() - want).abs() <= (2 * n_in + 2) * 2.0**-24 * (size @ rows.abs().t() + b[first:first + S].double().abs())).all()
+    assert (ws[nbytes:] == 0x55).all()
