@@ -210,9 +210,14 @@ int launch_crown_bwd_linear(const float* A, const float* dpos, const float* dneg
     if (int rc = ensure_dynamic_smem(crown_bwd_small_kernel, GS_ONE_PER_SM, opt_in, "crown_bwd_small_kernel")) return rc;
     dim3 grid(ceil_div(M, GS_ROWS), e.ntiles + (delta ? 1 : 0));
     // No more CTAs than SMs: one per SM.  They are placed while the kernel before still has its SMs and would go in pairs to those
-    // that are free (37 nodes, four 512-wide layers, 10 steps: 2.61 ms in pairs, 2.44 with one per SM).
+    // that are free (10 steps in pairs and one per SM: 37 inputs, four 512-wide layers 2.35 and 2.16 ms; 64, three 384-wide 1.67 and 1.57; 16,
+    // two 1024-wide 1.90 and 1.71; 64, five 256-wide 1.85 and 1.80; 33 other sizes within 2 %).
     const int smem = grid.x * grid.y <= 148 ? GS_ONE_PER_SM : GS_BWD_SMEM;
-    launch_dependent(crown_bwd_small_kernel, grid, GS_THREADS, smem, stream, g, e);
+    // More CTAs than SMs only with those of the row sums: a plain launch, whose tiles all find an SM of their own, where the sums are long
+    // (576 x 512 x 512 24.2 us early, 19.4 plain; 10 steps on 512-wide layers, 64 inputs, 2.46 and 2.32 ms, on 256-wide ones, 120 inputs, 2.22
+    // and 2.18; below 256 terms the early start is worth more: 128 wide, 220 inputs, 1.36 and 1.38).
+    if (grid.x * grid.y > 148 && grid.x * e.ntiles <= 148 && K >= 256) crown_bwd_small_kernel<<<grid, GS_THREADS, smem, stream>>>(g, e);
+    else launch_dependent(crown_bwd_small_kernel, grid, GS_THREADS, smem, stream, g, e);
   } else if (ffma_small_tiles(M, N)) {  // 64 x 64 tiles: four times as many CTAs
     dim3 grid(ceil_div(M, 64), ceil_div(N, 64));
     launch_dependent(crown_bwd_linear_kernel<PRO_RELU, 1, 1>, grid, GEMM_THREADS, 0, stream, g, e);

@@ -66,9 +66,9 @@ def test_alpha_steps_of_ragged_layers(dev, B, widths, with_beta):
             assert same.float().mean() >= 0.95, (r, n)
 
 
-# the last three: more tiles than SMs (two adjoint CTAs per SM), the others fewer
+# the last three: more tiles than SMs (two adjoint CTAs per SM), the others fewer; the one before them: more only with the CTAs of the row sums
 @pytest.mark.parametrize("B, S, n0, widths", [(7, 9, 33, (33, 70, 65)), (2, 9, 784, (64, 32)), (40, 9, 50, (31, 129)), (70, 1, 65, (65,)), (3, 32, 40, (100, 100)),
-                                              (72, 9, 784, (512, 512)), (300, 9, 64, (128, 100)), (147, 9, 61, (197, 130))])
+                                              (64, 9, 70, (512, 512)), (72, 9, 784, (512, 512)), (300, 9, 64, (128, 100)), (147, 9, 61, (197, 130))])
 def test_alpha_gradient_is_exact_on_small_integers(dev, B, S, n0, widths):
     """Integer weights and inputs, slopes in quarters: every sum is exact in FP32 in any order, so the gradient of every neuron of every
     domain, and the bounds, have to be those of float64."""
