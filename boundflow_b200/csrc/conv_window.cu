@@ -239,8 +239,12 @@ static int launch_window_side(const ConvWindowArgs& a, int ww, cudaStream_t stre
     if constexpr (WW % 2 == 0 || (PD == 0 && WW <= 7)) {
       constexpr int TCI = ConvWindow<KS, ST, PD, WW>::TCI;
       if (a.Co % ConvWindow<KS, ST, PD, WW>::CU != 0) return BF_E_UNSUPPORTED;
-      // single channels where groups would be mostly padding (three channels in groups of four or two)
-      if (TCI > 1 && 5 * (ceil_div(a.Ci, TCI) * TCI) > 6 * a.Ci) return launch_window<KS, ST, PD, WW, 1>(a, stream);
+      // single channels where groups would be mostly padding (three channels in groups of four or two), and while the warps of single
+      // channels are no more than the chip holds at once: TCI times the warps, each with 1 / TCI of the multiply-adds in series.
+      // 3x3 / 1, 4 -> 6 pixels, groups and single channels (row segments): 64 -> 32 channels, 512 rows 44.5 and 25.4 us (42.3), 2048 rows 45.1
+      // and 39.3, 4096 rows (twice the line) 71.5 and 69.8; 16 -> 16, 512 rows 14.0 and 9.0 (13.3), 8192 rows (twice the line) 22.5 and 23.3.
+      if (TCI > 1 && (5 * (ceil_div(a.Ci, TCI) * TCI) > 6 * a.Ci || (long long)ceil_div(a.M, 32) * a.Ci <= 16 * 148))
+        return launch_window<KS, ST, PD, WW, 1>(a, stream);
       return launch_window<KS, ST, PD, WW, TCI>(a, stream);
     }
     return BF_E_UNSUPPORTED;

@@ -49,6 +49,46 @@ def test_padded_maps_against_float64(w, rows, ci, co):
     assert (err <= 4 * co * 2.0**-24 * size).all()  # four products per channel
 
 
+def _serial(A, W, stride, pad=0):
+    """Each sum over output channels, kernel rows, kernel columns ascending, one rounding a term: on inputs in steps of 2^-12 every
+    product and sum is exact in float64 before it is rounded to float32 (products in steps of 2^-24, sums below 2^20)."""
+    M, Co, w, _ = A.shape
+    Ci, k = W.shape[1], W.shape[2]
+    ow = (w - 1) * stride + k - 2 * pad
+    out = torch.zeros((M, Ci, ow, ow), device="cuda")
+    for co in range(Co):
+        for r in range(k):
+            for c in range(k):
+                ys = [y for y in range(w) if 0 <= y * stride + r - pad < ow]
+                xs = [x for x in range(w) if 0 <= x * stride + c - pad < ow]
+                part = out[:, :, ys[0] * stride + r - pad:ys[-1] * stride + r - pad + 1:stride, xs[0] * stride + c - pad:xs[-1] * stride + c - pad + 1:stride]
+                x = A[:, co, ys[0]:ys[-1] + 1, xs[0]:xs[-1] + 1].double()[:, None]
+                part.copy_((x * W[co, :, r, c].double()[None, :, None, None] + part.double()).float())
+    return out
+
+
+def _grid(shape, g):
+    return (torch.randn(shape, generator=g, device="cuda") * 4096).round() / 4096
+
+
+# few rows (single channels), rows of several tiles per block with a ragged last one (groups of channels, odd counts of chunks), channel
+# counts that no 16-byte window word fits
+@pytest.mark.parametrize("k, stride, w", GEOMETRIES)
+@pytest.mark.parametrize("rows, ci, co", [(40, 12, 8), (33, 3, 5), (40, 9, 31), (700, 32, 8), (20011, 4, 12), (5003, 24, 20)])
+def test_windows_keep_the_order_of_sums(k, stride, w, rows, ci, co):
+    g = torch.Generator("cuda").manual_seed(1000 * w + 10 * k + ci)
+    A, W = _grid((rows, co, w, w), g), _grid((co, ci, k, k), g)
+    assert torch.equal(_backward(A, W, stride), _serial(A, W, stride))
+
+
+@pytest.mark.parametrize("w", (6, 8, 10))
+@pytest.mark.parametrize("rows, ci, co", [(2048, 1, 5), (3001, 2, 7), (20011, 1, 12), (25601, 2, 6)])
+def test_padded_maps_keep_the_order_of_sums(w, rows, ci, co):
+    g = torch.Generator("cuda").manual_seed(w + rows)
+    A, W = _grid((rows, co, w, w), g), _grid((co, ci, 4, 4), g)
+    assert torch.equal(_backward(A, W, 2, 1), _serial(A, W, 2, 1))
+
+
 @pytest.mark.parametrize("k, stride, w", [(3, 1, 3), (4, 2, 4), (3, 1, 14)])
 def test_infinite_weight_reaches_only_its_taps(k, stride, w):
     A = torch.ones((40, 4, w, w), device="cuda")
