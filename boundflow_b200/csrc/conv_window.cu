@@ -206,7 +206,9 @@ static int launch_window(ConvWindowArgs a, cudaStream_t stream) {
     const long long left = LIMIT - (long long)a.Co * c * NWP * 4 - c * G::NB * r * EPI;
     const long long room = left / (2 * 32 * r * 16) - 1;                  // 16-byte words of a row's chunk
     if (room < G::CU * PLANE / 4 || used <= best + 1e-9) continue;
-    long long cc = room * 4 / PLANE, want = (G::BLOCKS == 1 ? 40 : 24) * 1024 / (32 * r * 4 * PLANE);
+    // Chunks of up to 40 KB: 24 KB were one output channel of 10-pixel windows (3x3 / 1, 64 -> 32 channels, 64 rows: 85 us, 71 with 40 KB, row
+    // segments 82).  Time of all shapes against 24 KB: 8 KB 1.10, 16 KB 1.02, 32 KB 0.96, 40 KB 0.95, 56 KB 0.96.
+    long long cc = room * 4 / PLANE, want = 40 * 1024 / (32 * r * 4 * PLANE);
     if (want < G::CU) want = G::CU;
     if (cc > want) cc = want;
     if (cc > 16) cc = 16;
