@@ -202,7 +202,19 @@ static int launch_window(ConvWindowArgs a, cudaStream_t stream) {
     const int y = ceil_div(ncg, c);
     int r = G::WARPS / (c * G::NB);
     const double used = (double)ncg / (y * c) / (1.0 + 0.1 * y) * (G::BLOCKS == 1 ? sqrt((double)(c * G::NB * r) / G::WARPS) : 1.0);
-    while (r > 1 && (long long)ceil_div(a.M, 32 * r) * y < 148) --r;      // few rows: more blocks with longer chunks
+    if (G::BLOCKS == 1) {
+      // Row groups for the least rounds of blocks times a block's time, as its warps and a start that four more would take: 188 blocks of four
+      // warps are two rounds on 148 SMs, 94 of eight one (4x4 / 2, padding 1, 8 -> 16 pixels, 16 -> 2 channels: 3000 rows 19.1 -> 15.4 us, 8192
+      // rows 39.1 -> 28.6; row segments 17.8 and 38.1).
+      const int gx = y < 148 ? 148 / y : 1;
+      long long least = -1;
+      for (int t = r; t >= 1; --t) {
+        const long long time = (long long)ceil_div(ceil_div(a.M, 32 * t), gx) * (c * G::NB * t + 4);
+        if (least < 0 || time < least) { least = time; r = t; }
+      }
+    } else {
+      while (r > 1 && (long long)ceil_div(a.M, 32 * r) * y < 148) --r;    // few rows: more blocks with longer chunks
+    }
     const long long left = LIMIT - (long long)a.Co * c * NWP * 4 - c * G::NB * r * EPI;
     const long long room = left / (2 * 32 * r * 16) - 1;                  // 16-byte words of a row's chunk
     if (room < G::CU * PLANE / 4 || used <= best + 1e-9) continue;
