@@ -750,9 +750,15 @@ static int ilog2_ceil(int v) {
   return l;
 }
 
-// us: only the time that the launch is expected to take, without its start (nothing is launched)
+// A launch's expected time without its start, its blocks, and the share of the sums it forms that are results (not padding)
+struct RowSegCost {
+  double us;
+  long long blocks;
+  double used;
+};
+// cost: only that (nothing is launched)
 template <int KS, int ST, int PD, int TCI, bool VEC, int TWP, int RT = 1>
-static int launch_rowseg_tci(const ConvTArgs& g, double* us, cudaStream_t stream) {
+static int launch_rowseg_tci(const ConvTArgs& g, RowSegCost* cost, cudaStream_t stream) {
   using G = RowSeg<KS, ST, PD, VEC, TWP>;
   RowSegArgs a{};
   a.c = g;
@@ -787,14 +793,16 @@ static int launch_rowseg_tci(const ConvTArgs& g, double* us, cudaStream_t stream
   const size_t smem = 2 * (lam_words + w_words) * sizeof(float) + (size_t)(1 << a.mrl) * cc * G::tile_h(1 << a.thl) * sizeof(int);
   dim3 grid(ceil_div(g.M, 1 << a.mrl), a.tiles_x * a.tiles_y, ceil_div(g.Ci, cib));
   if (grid.y > 65535 || grid.z > 65535) return BF_E_UNSUPPORTED;
-  if (us) {
+  if (cost) {
     // multiply-adds of a block at a rate per kernel shape, and its chunks; blocks share an SM up to its shared memory
     const double blocks = (double)grid.x * grid.y * grid.z / 148.0;
     double room = (TCI > 1 && TWP * RT > 8) ? 2 : 3;
     if (room > 227 * 1024 / (double)(smem + 1024)) room = (double)(int)(227 * 1024 / (smem + 1024));
     const double waves = blocks > room ? blocks / room : 1.0, side = blocks > room ? room : (blocks > 1.0 ? blocks : 1.0);
     const double rate = KS == 5 ? 1.17e-3 : (KS == 4 ? 2.4e-3 : (ST == 1 ? 1.67e-3 : 3.3e-3));
-    *us = waves * (side * rate * g.Co * KS * KS * TCI * TWP * RT / (ST * ST) + 0.4 * g.Co / cc) * (TWP == 8 ? 1.35 : 1.0);
+    cost->us = waves * (side * rate * g.Co * KS * KS * TCI * TWP * RT / (ST * ST) + 0.4 * g.Co / cc) * (TWP == 8 ? 1.35 : 1.0);
+    cost->blocks = (long long)grid.x * grid.y * grid.z;
+    cost->used = (double)g.Ci * g.Hi * g.Wi / ((double)grid.z * cib * ((long long)a.tiles_y << a.thl) * ((long long)a.tiles_x << a.sxl) * G::TW);
     return BF_OK;
   }
   static SmemOptIn opt_in;
@@ -805,9 +813,9 @@ static int launch_rowseg_tci(const ConvTArgs& g, double* us, cudaStream_t stream
 }
 
 template <int KS, int ST, int PD>
-static int launch_rowseg(const ConvTArgs& g, double* us, cudaStream_t stream) {
+static int launch_rowseg(const ConvTArgs& g, RowSegCost* cost, cudaStream_t stream) {
   const bool vec = (g.Wo % 4 == 0) && ((reinterpret_cast<uintptr_t>(g.Lam) & 15u) == 0);
-  if (g.Ci <= 2) return vec ? launch_rowseg_tci<KS, ST, PD, 1, true, 16>(g, us, stream) : launch_rowseg_tci<KS, ST, PD, 1, false, 16>(g, us, stream);
+  if (g.Ci <= 2) return vec ? launch_rowseg_tci<KS, ST, PD, 1, true, 16>(g, cost, stream) : launch_rowseg_tci<KS, ST, PD, 1, false, 16>(g, cost, stream);
   // 8-pixel segments when they waste fewer lanes than 16-pixel ones (narrow windows of the windowed sweeps)
   const bool narrow = ((g.Wi + 7) / 8) * 8 < ((g.Wi + 15) / 16) * 16;
   if constexpr (KS == 4) {
@@ -815,23 +823,23 @@ static int launch_rowseg(const ConvTArgs& g, double* us, cudaStream_t stream) {
     // kernels on five to eight rows from 24 -> 32 channels on (1.03 to 1.18 of the speed), elsewhere mostly slower (4x4 / 2 on 17 to
     // 24 rows 0.90 to 0.98, 3x3 / 1 0.66 to 1.02, 5x5 / 1 0.8 to 1.05), and with few channels its tile can outgrow shared memory.
     if (narrow && g.Ci >= 24 && g.Co >= 32 && g.Hi >= 5 && g.Hi <= 8)
-      return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 8, 2>(g, us, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 8, 2>(g, us, stream);
+      return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 8, 2>(g, cost, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 8, 2>(g, cost, stream);
   }
-  if (narrow) return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 8>(g, us, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 8>(g, us, stream);
-  return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 16>(g, us, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 16>(g, us, stream);
+  if (narrow) return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 8>(g, cost, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 8>(g, cost, stream);
+  return vec ? launch_rowseg_tci<KS, ST, PD, 4, true, 16>(g, cost, stream) : launch_rowseg_tci<KS, ST, PD, 4, false, 16>(g, cost, stream);
 }
 
 // Row-segment kernel for the geometries it is instantiated for; BF_E_UNSUPPORTED otherwise.
-static int launch_convT_rowseg(const ConvTArgs& g, double* us, cudaStream_t stream) {
+static int launch_convT_rowseg(const ConvTArgs& g, RowSegCost* cost, cudaStream_t stream) {
   if (g.kh != g.kw || g.sh != g.sw || g.ph != g.pw) return BF_E_UNSUPPORTED;
-  if (g.kh == 3 && g.sh == 1 && g.ph == 1) return launch_rowseg<3, 1, 1>(g, us, stream);
-  if (g.kh == 4 && g.sh == 2 && g.ph == 1) return launch_rowseg<4, 2, 1>(g, us, stream);
-  if (g.kh == 3 && g.sh == 2 && g.ph == 1) return launch_rowseg<3, 2, 1>(g, us, stream);
+  if (g.kh == 3 && g.sh == 1 && g.ph == 1) return launch_rowseg<3, 1, 1>(g, cost, stream);
+  if (g.kh == 4 && g.sh == 2 && g.ph == 1) return launch_rowseg<4, 2, 1>(g, cost, stream);
+  if (g.kh == 3 && g.sh == 2 && g.ph == 1) return launch_rowseg<3, 2, 1>(g, cost, stream);
   // zero padding: the windowed sweeps below run every transposed convolution in window coordinates
-  if (g.kh == 3 && g.sh == 1 && g.ph == 0) return launch_rowseg<3, 1, 0>(g, us, stream);
-  if (g.kh == 4 && g.sh == 2 && g.ph == 0) return launch_rowseg<4, 2, 0>(g, us, stream);
-  if (g.kh == 3 && g.sh == 2 && g.ph == 0) return launch_rowseg<3, 2, 0>(g, us, stream);
-  if (g.kh == 5 && g.sh == 1 && g.ph == 2) return launch_rowseg<5, 1, 2>(g, us, stream);
+  if (g.kh == 3 && g.sh == 1 && g.ph == 0) return launch_rowseg<3, 1, 0>(g, cost, stream);
+  if (g.kh == 4 && g.sh == 2 && g.ph == 0) return launch_rowseg<4, 2, 0>(g, cost, stream);
+  if (g.kh == 3 && g.sh == 2 && g.ph == 0) return launch_rowseg<3, 2, 0>(g, cost, stream);
+  if (g.kh == 5 && g.sh == 1 && g.ph == 2) return launch_rowseg<5, 1, 2>(g, cost, stream);
   return BF_E_UNSUPPORTED;
 }
 
@@ -885,7 +893,8 @@ static ConvTcProblem conv_tc_geometry(int M, int S, const bf_layer_desc& L) {
 }
 static bool conv_tc_rule(const ConvTcProblem& c, int* slots) {
   int tiles = 0;
-  double tc = 0.0, fp32 = 0.0;
+  double tc = 0.0;
+  RowSegCost fp32{};
   const int taps = ceil_div(c.kh, c.sh) * ceil_div(c.kw, c.sw);
   if (c.Ci < CONV_TC_MIN_CI || taps > CONV_TC_MAX_TAPS || !conv_tc_supports(c, slots, &tiles, &tc) || tiles < CONV_TC_MIN_TILES) return false;
   ConvTArgs g{nullptr, nullptr, nullptr, c.M, c.Ci, c.Hi, c.Wi, c.Co, c.WH, c.WW, c.kh, c.kw, c.sh, c.sw, c.ph, c.pw, 0};
@@ -893,7 +902,7 @@ static bool conv_tc_rule(const ConvTcProblem& c, int* slots) {
     const int npix = c.Hi * c.Wi, idle = npix < 32 ? 32 : npix;  // the gather kernel's threads of a small map
     return (long long)c.kh * c.kw * c.Ci * (c.Co < 32 ? c.Co : 32) * idle / npix >= (c.sh * c.sw > 1 ? 384 : 1024);
   }
-  return tc < fp32 + 13.0 + 2.5e-6 * c.M * c.Co * c.WH * c.WW;  // and the ReLU pass
+  return tc < fp32.us + 13.0 + 2.5e-6 * c.M * c.Co * c.WH * c.WW;  // and the ReLU pass
 }
 bool conv_rows_on_tensor_cores(int M, const bf_layer_desc& L) {
   int slots = 0;
@@ -923,6 +932,23 @@ static int launch_conv_tc_bwd(const float* A, const float* dpos, const float* dn
              2.0 * (double)M * L.n_out * L.Ci * L.kh * L.kw);
   if (rc == BF_OK && sums) rc = launch_sum_partials(accumulate ? delta : nullptr, c.partial, slots, delta, M, stream);
   return rc;
+}
+
+// Windows that the row-segment kernel keeps: results of 14 and 16 pixels (windows of 12 and 14 under 3x3 / 1, of 7 under 4x4 / 2) fill
+// its segments, and its blocks cut a row finer, so it is the faster one where few of its lanes idle (from the channels
+// rounded up to a block's) or its blocks fit the SMs at once.  Window kernel against it, time ratios over 8 to 64 output, 1 to 64 input
+// channels, 32 to 8192 rows, where this rule takes the one or the other:
+//   3x3 / 1, 12 -> 14: 0.43 to 0.88 | 1.02 to 1.25 (16 channels, few rows, also 0.98)    14 -> 16: 0.38 to 1.00 | 1.02 to 1.43 (16 channels 0.94 to 1.25)
+//   4x4 / 2,  7 -> 16: 0.73 to 0.95 | 1.05 to 1.57 (1 and 8 channels, few rows, 0.92 to 0.99)
+static bool rowseg_keeps(const ConvTArgs& g) {
+  const bool s1 = g.kh == 3 && g.sh == 1 && g.Wi >= 14, s2 = g.kh == 4 && g.sh == 2 && g.Wi == 16;
+  if (g.Hi != g.Wi || g.kh != g.kw || g.sh != g.sw || g.ph != 0 || g.pw != 0 || (!s1 && !s2)) return false;
+  RowSegCost cost{};
+  if (launch_convT_rowseg(g, &cost, nullptr) != BF_OK) return false;
+  const bool full = cost.used >= 0.8, one_wave = cost.blocks <= 148;
+  if (s2) return full || (one_wave && g.Ci > 8);
+  if (g.Ci > 8) return full || one_wave;
+  return g.Wi == 14 && g.Ci <= 2 && one_wave;
 }
 
 int launch_crown_bwd_conv2d(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
@@ -965,7 +991,7 @@ int launch_crown_bwd_conv2d(const float* A, const float* dpos, const float* dneg
   const double conv_flops = 2.0 * (double)M * L.n_out * L.Ci * L.kh * L.kw;
   timing_begin(T_CONV_T, stream);
   int rc = BF_E_UNSUPPORTED;
-  if (!gather_only && L.Hi == (L.Ho - 1) * L.sh + L.kh - 2 * L.ph && L.Wi == (L.Wo - 1) * L.sw + L.kw - 2 * L.pw)
+  if (!gather_only && L.Hi == (L.Ho - 1) * L.sh + L.kh - 2 * L.ph && L.Wi == (L.Wo - 1) * L.sw + L.kw - 2 * L.pw && !rowseg_keeps(g))
     rc = launch_conv_window(lam, W, A_prev, M, L.Ci, L.Co, L.Ho, L.Wo, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw, stream);
   if (rc == BF_E_UNSUPPORTED && !gather_only) rc = launch_convT_rowseg(g, nullptr, stream);
   if (rc == BF_E_UNSUPPORTED) {

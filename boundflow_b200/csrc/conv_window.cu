@@ -22,7 +22,7 @@ namespace bf {
 // the chip reaches), by the chunks' copies and the results' stores with one to three channels.  65,536 rows, against the
 // row-segment kernels: 32 -> 32 channels, 3 x 3 -> 8 x 8 of 4x4 / 2: 1293 -> 472 us; 64 -> 32, 4 x 4 -> 6 x 6 of 3x3: 3674 -> 841;
 // 32 -> 32, 6 x 6 -> 14 x 14 of 4x4 / 2: 5490 -> 2515; 32 -> 3, 8 x 8 -> 10 x 10 of 3x3: 1124 -> 218; 32 -> 1, 4 x 4 -> 10 x 10 of
-// 4x4 / 2: 223 -> 60.  64 rows: 0.9 (7 x 7, 4x4 / 2) to 3.8 of the speed, so no line in the rows.
+// 4x4 / 2: 223 -> 60.  Few rows: no slower (32 rows of 220 shapes: 0.1 to 1.0 of the time), except where rowseg_keeps (conv.cu) says so.
 struct ConvWindowArgs {
   const float* Lam;  // [M, Co, WW, WW]
   const float* W;    // [Co, Ci, KS, KS]
@@ -266,9 +266,13 @@ static int launch_window_side(const ConvWindowArgs& a, int ww, cudaStream_t stre
 }
 
 // Transposed convolution of M rows of WH x WW maps: windows (no padding), and full maps of 6 to 10 pixels under a 4x4 / 2 kernel with padding
-// 1 and one or two channels below (25,600 rows, 8 -> 1 channels, 10 x 10: 163 -> 77 us; 2048 rows: 21 -> 15; below 0.83 to 1.02 of the
-// row-segment kernel's speed).  Larger maps stay there: their ten and more bands are as many copies of the loop in the
-// instruction cache (16 -> 1 channels, 14 x 14: 333 us there, 419 here).
+// 1 and one or two channels below, from 2048 rows on (row segments -> here, us):
+//   pixels, channels   2048 rows      8192 rows     25,600 rows
+//    6, 16 -> 1 | 2    15 -> 11 | 15 -> 9     38 -> 12 | 45 -> 13     93 -> 35 | 130 -> 34
+//    8, 16 -> 1 | 2    12 -> 11 | 13 -> 11    31 -> 16 | 38 -> 29     74 -> 45 | 112 -> 81
+//   10, 16 -> 1 | 2    32 -> 19 | 36 -> 25    97 -> 50 | 132 -> 92    294 -> 124 | 401 -> 243
+// Fewer rows are 0.83 to 1.02 of the row-segment kernel's speed, and larger maps stay there: their ten and more bands are as many copies
+// of the loop in the instruction cache (16 -> 1 channels, 14 x 14: 333 us there, 419 here).
 // BF_E_UNSUPPORTED for geometries without an instance.
 int launch_conv_window(const float* Lam, const float* W, float* out, int M, int Ci, int Co, int WH, int WW, int kh, int kw, int sh, int sw,
                        int ph, int pw, cudaStream_t stream) {
