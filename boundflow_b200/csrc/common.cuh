@@ -76,8 +76,8 @@ inline int ensure_dynamic_smem(Kernel kernel, int bytes, SmemOptIn& table, const
 }
 
 // Launches that may start while the kernel before them in the stream still runs (programmatic dependent launch): their blocks are
-// placed and wait in grid_dependency() until everything before them is complete and visible, so a chain of short kernels pays
-// the launch itself (2 to 3 us) only once.  A kernel that is launched this way begins with grid_dependency() and reads global memory
+// placed and wait in grid_wait() until everything before them is complete and visible, so a chain of short kernels pays
+// the launch itself (2 to 3 us) only once.  A kernel that is launched this way begins with grid_wait() and reads global memory
 // with plain loads (or cp.async) through pointers that are not __restrict__: read-only loads (__ldg, or what a const __restrict__
 // parameter becomes) are taken for constant over the kernel's life and may be moved above the wait, and what the kernel before has
 // written (coefficients, but also a weight that the caller's kernel has just updated or transposed) would be read stale.
@@ -95,9 +95,11 @@ inline void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, s
   cfg.numAttrs = 1;
   (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
-__device__ __forceinline__ void grid_dependency() {
-  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" : : : "memory");
-}
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" : : : "memory"); }
+// When every block has come here or ended, the blocks of the next dependent launch are placed.  Where SMs are still unevenly busy they go in
+// bunches to those that are free, as many as fit, and a launch of fewer blocks than the chip holds then leaves SMs idle: so behind the
+// work of a block, not before it, and kernels of long blocks that rarely fill the chip evenly (conv.cu) are plain launches.
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" : : : "memory"); }
 
 inline cudaStream_t as_stream(bf_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 

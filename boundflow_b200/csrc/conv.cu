@@ -71,7 +71,7 @@ __device__ __forceinline__ float2 taps_inside(const IbpConvArgs& g, long long pi
 
 template <bool INTERVAL, int TN>
 __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper, int vec) {
-  grid_dependency();
+  grid_wait();
   constexpr int TM = ConvTile<TN>::TM, CBK = ConvTile<TN>::SLAB, ACCS = INTERVAL ? 2 : 1;
   constexpr int NA = TM * CBK / 256, KSTEP = 256 / TM, WLD = TN + 4, NW = (TN * CBK + 255) / 256;
   constexpr int STAGE = ACCS * CBK * TM + CBK * WLD, PART = ACCS * TM * TN;
@@ -190,6 +190,8 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
     if (kt + 1 < nk) store_slab(stage ^ 1);
     __syncthreads();
   }
+
+  grid_release();
 
   const int ranks = gridDim.z;
   if (ranks > 1) {  // four: rank z finishes channel z of every thread
@@ -315,7 +317,10 @@ static int launch_conv_tile_n(const IbpConvArgs& g, int vec, cudaStream_t stream
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  // Fewer blocks than the chip holds, or clusters, are not placed early, unless they are short: bunched on the SMs that are free first, 400
+  // of them took 88 us for 71 (200 x 32 x 32 x 32 -> 32, 4x4 / 2), 128 in clusters of four 37 for 30 (16 x 128 x 8 x 8 -> 128, 3x3, intervals);
+  // 110 of 16 taps (144 x 1 x 28 x 28 -> 16) 4.0 for 4.6.
+  cfg.numAttrs = ks == 1 && (K <= 64 || tiles * ctas_y >= 4 * 148) ? 2 : 1;
   cudaLaunchKernelEx(&cfg, conv_tile_kernel<INTERVAL, TN>, g, ceil_div(slabs, ks) * ConvTile<TN>::SLAB, vec);
   BF_CHECK_LAUNCH("conv_tile_kernel");
   return BF_OK;
@@ -363,7 +368,7 @@ constexpr int RELU_ROWS_CHUNK = 4096;
 __global__ void __launch_bounds__(256) relu_bwd_rows_kernel(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
                                                             const float* add, const float* bias, int chan_size, float* Lam, float* partial,
                                                             float* delta, int accumulate, int chunk, int S, int n, int vec) {
-  grid_dependency();
+  grid_wait();
   const int m = blockIdx.x;
   const int k0 = blockIdx.y * chunk;
   const int k1 = min(n, k0 + chunk);
@@ -417,6 +422,7 @@ __global__ void __launch_bounds__(256) relu_bwd_rows_kernel(const float* A, cons
       if (Lam) Lam[(size_t)m * n + k] = lam;
     }
   }
+  grid_release();
   if (!partial && !delta) return;
   __shared__ float red[8];
 #pragma unroll
@@ -566,11 +572,12 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// Plain launches: placed early, behind the short ReLU pass, the blocks of a sweep of a few hundred rows bunched on half of the SMs (256 rows,
+// 64 -> 32 channels, 3x3 on 8 x 8, with the pass: 113 us, 48 plain; 856 sizes: 0.97 of the time, 78 of them under 0.95).
 // RT = 2 (8-pixel segments): a thread owns two image rows that meet the same kernel rows, and each weight read feeds twice the
 // multiply-adds.  Same order of sums.
 template <int KS, int ST, int PD, int TCI, bool VEC, int TWP, int RT>
 __global__ void __launch_bounds__(256, (TCI > 1 && TWP * RT > 8 ? 2 : 3)) conv_transpose_rowseg_kernel(RowSegArgs a) {
-  grid_dependency();
   using G = RowSeg<KS, ST, PD, VEC, TWP>;
   extern __shared__ __align__(16) float rs_smem[];
   const ConvTArgs& g = a.c;
@@ -807,7 +814,7 @@ static int launch_rowseg_tci(const ConvTArgs& g, RowSegCost* cost, cudaStream_t 
   }
   static SmemOptIn opt_in;
   if (int rc = ensure_dynamic_smem(conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT>, 110 * 1024, opt_in, "conv_transpose_rowseg_kernel")) return rc;
-  launch_dependent(conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT>, grid, 256, smem, stream, a);
+  conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT><<<grid, 256, smem, stream>>>(a);
   BF_CHECK_LAUNCH("conv_transpose_rowseg_kernel");
   return BF_OK;
 }

@@ -22,12 +22,13 @@ struct BwdEpilogue {
 
 template <int PRO, int MH, int NH>
 __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_bwd_linear_kernel(GemmArgs g, BwdEpilogue e) {
-  grid_dependency();
+  grid_wait();
   __shared__ __align__(16) float smem[MAINLOOP_SMEM_FLOATS];
   constexpr int TM = 64 * MH, MR = 4 * MH;
   const int m0 = blockIdx.x * TM, n0 = blockIdx.y * (64 * NH);
   float acc[8][8];
   gemm_mainloop<PRO, false, MH, NH>(g, m0, n0, acc, smem);
+  grid_release();
 
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const bool vN = g.vecN != 0;
@@ -66,7 +67,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_bwd_linear_kernel(GemmA
 
 // 32 x 64 tiles of a small problem (gemm_small.cuh); CTAs of column e.ntiles form the row sums.
 __global__ void __launch_bounds__(GS_THREADS, 2) crown_bwd_small_kernel(GemmArgs g, BwdEpilogue e) {
-  grid_dependency();
+  grid_wait();
   extern __shared__ __align__(16) float dsmem[];
   float* As = dsmem;
   float* Bs = As + GS_STAGES * GS_A_WORDS;
@@ -83,6 +84,7 @@ __global__ void __launch_bounds__(GS_THREADS, 2) crown_bwd_small_kernel(GemmArgs
   float p[4] = {0.f, 0.f, 0.f, 0.f};
   if (tid >= GS_COMPUTE) {
     gs_fill<PRO_RELU, false>(g, m0, n0, As, Bs, tid - GS_COMPUTE);
+    grid_release();
   } else {
     float4 md[4], rd[4];
 #pragma unroll
@@ -96,6 +98,7 @@ __global__ void __launch_bounds__(GS_THREADS, 2) crown_bwd_small_kernel(GemmArgs
     }
     float acc[4][4];
     gs_compute<false>(g.K, As, Bs, r0, c0, acc);
+    grid_release();
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float4 v = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
@@ -132,7 +135,7 @@ constexpr int THIN_KMAX = 16;
 constexpr int THIN_ROWS = 64;   // rows of a block, at most: a small problem takes fewer (its blocks' rows are a serial chain)
 __global__ void __launch_bounds__(128) crown_bwd_thin_kernel(const float* A, const float* W, const float* kbias, float* out, float* delta,
                                                              int accumulate, int M, int K, int N, int block_rows) {
-  grid_dependency();
+  grid_wait();
   __shared__ float a_s[THIN_ROWS * THIN_KMAX];
   const int m0 = blockIdx.x * block_rows;
   const int rows = min(block_rows, M - m0);
@@ -144,19 +147,24 @@ __global__ void __launch_bounds__(128) crown_bwd_thin_kernel(const float* A, con
   for (int i = threadIdx.x; i < rows * K; i += blockDim.x) a_s[i] = A[(size_t)m0 * K + i];
   __syncthreads();
   if (cg * 4 < N) {
-    for (int r = 0; r < rows; ++r) {
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r = 0; r < rows; r += 2) {  // two rows a turn: a store holds back the next row's reads
+      const float* a0 = a_s + r * K;
+      const float* a1 = a0 + (r + 1 < rows ? K : 0);
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
 #pragma unroll
       for (int k = 0; k < THIN_KMAX; ++k) {
         if (k < K) {
-          const float a = a_s[r * K + k];
-          acc.x = fmaf(a, w[k].x, acc.x); acc.y = fmaf(a, w[k].y, acc.y);
-          acc.z = fmaf(a, w[k].z, acc.z); acc.w = fmaf(a, w[k].w, acc.w);
+          const float p = a0[k], q = a1[k];
+          x.x = fmaf(p, w[k].x, x.x); x.y = fmaf(p, w[k].y, x.y); x.z = fmaf(p, w[k].z, x.z); x.w = fmaf(p, w[k].w, x.w);
+          y.x = fmaf(q, w[k].x, y.x); y.y = fmaf(q, w[k].y, y.y); y.z = fmaf(q, w[k].z, y.z); y.w = fmaf(q, w[k].w, y.w);
         }
       }
-      *reinterpret_cast<float4*>(out + (size_t)(m0 + r) * N + cg * 4) = acc;
+      float* to = out + (size_t)(m0 + r) * N + cg * 4;
+      *reinterpret_cast<float4*>(to) = x;
+      if (r + 1 < rows) *reinterpret_cast<float4*>(to + N) = y;
     }
   }
+  grid_release();
   if (delta && blockIdx.y == 0) {
     for (int r = threadIdx.x; r < rows; r += blockDim.x) {
       float sum = 0.f;
@@ -210,12 +218,11 @@ int launch_crown_bwd_linear(const float* A, const float* dpos, const float* dneg
     if (int rc = ensure_dynamic_smem(crown_bwd_small_kernel, GS_ONE_PER_SM, opt_in, "crown_bwd_small_kernel")) return rc;
     dim3 grid(ceil_div(M, GS_ROWS), e.ntiles + (delta ? 1 : 0));
     // No more CTAs than SMs: one per SM.  They are placed while the kernel before still has its SMs and would go in pairs to those
-    // that are free (10 steps in pairs and one per SM: 37 inputs, four 512-wide layers 2.35 and 2.16 ms; 64, three 384-wide 1.67 and 1.57; 16,
-    // two 1024-wide 1.90 and 1.71; 64, five 256-wide 1.85 and 1.80; 33 other sizes within 2 %).
+    // that are free (alpha loops of 99 to 145 CTAs in pairs: 1.02 to 1.07 of the time over nine sizes from 128 to 1000 wide; fewer CTAs: the same).
     const int smem = grid.x * grid.y <= 148 ? GS_ONE_PER_SM : GS_BWD_SMEM;
     // More CTAs than SMs only with those of the row sums: a plain launch, whose tiles all find an SM of their own, where the sums are long
-    // (576 x 512 x 512 24.2 us early, 19.4 plain; 10 steps on 512-wide layers, 64 inputs, 2.46 and 2.32 ms, on 256-wide ones, 120 inputs, 2.22
-    // and 2.18; below 256 terms the early start is worth more: 128 wide, 220 inputs, 1.36 and 1.38).
+    // (576 x 512 x 512 21.4 us early, 19.6 plain, 1152 x 256 x 256 12.8 and 11.3; alpha loops of 256 to 1000 wide layers early: 0.98 to 1.06 of
+    // the time, 1.02 on average; of 64 to 128 wide layers plain: 1.00 to 1.07).
     if (grid.x * grid.y > 148 && grid.x * e.ntiles <= 148 && K >= 256) crown_bwd_small_kernel<<<grid, GS_THREADS, smem, stream>>>(g, e);
     else launch_dependent(crown_bwd_small_kernel, grid, GS_THREADS, smem, stream, g, e);
   } else if (ffma_small_tiles(M, N)) {  // 64 x 64 tiles: four times as many CTAs
@@ -258,12 +265,13 @@ static_assert(ADJ_SMEM_BYTES >= MAINLOOP_SMEM_FLOATS * (int)sizeof(float), "stag
 
 template <int PRO, int MH, int NH>
 __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_adjoint_linear_kernel(GemmArgs g, AdjEpilogue e) {
-  grid_dependency();
+  grid_wait();
   extern __shared__ __align__(16) float dsmem[];
   constexpr int TM = 64 * MH, TN = 64 * NH, MR = 4 * MH;
   const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
   float acc[8][8];
   gemm_mainloop<PRO, true, MH, NH>(g, m0, n0, acc, dsmem);
+  grid_release();
   // the main loop ends with __syncthreads(): the slabs may now be overwritten by the stage tile
 
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -363,7 +371,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) crown_adjoint_linear_kernel(G
 // 1152 x 256 x 256: 12.0 -> 9.6 us with the copying warps; 333 x 512 x 512: 21.2 -> 15.1.
 template <int PRO, bool AHEAD>
 __global__ void __launch_bounds__(GS_THREADS, AHEAD ? 1 : 2) crown_adjoint_small_kernel(GemmArgs g, AdjEpilogue e) {
-  grid_dependency();
+  grid_wait();
   extern __shared__ __align__(16) float dsmem[];
   float* As = dsmem;
   float* Bs = As + GS_STAGES * GS_A_WORDS;
@@ -374,6 +382,7 @@ __global__ void __launch_bounds__(GS_THREADS, AHEAD ? 1 : 2) crown_adjoint_small
   float acc[4][4];
   if (tid >= GS_COMPUTE) {
     gs_fill<PRO, true>(g, m0, n0, As, Bs, tid - GS_COMPUTE);
+    grid_release();
   } else {
     constexpr int R = AHEAD ? 4 : 2;
     float ah[R][4], dp[R][4], dn[R][4], ep[R][4], en[R][4], pl[R][4], pu[R][4], nb[4];
@@ -399,6 +408,7 @@ __global__ void __launch_bounds__(GS_THREADS, AHEAD ? 1 : 2) crown_adjoint_small
     };
     if (AHEAD) load(0);
     gs_compute<true>(g.K, As, Bs, r0, c0, acc);
+    grid_release();
 #pragma unroll
     for (int first = 0; first < 4; first += R) {
       if (!AHEAD) load(first);

@@ -54,7 +54,8 @@ int launch_relu_relax(const float* l, const float* u, const float* alpha, int al
 // ---- concretisation: one warp per coefficient row -----------------------------
 __global__ void __launch_bounds__(256) concretize_kernel(const float* A, const float* mid, const float* rad, const float* bias_in, float* out,
                                                          float sgn, int M, int S, int n0, int vec) {
-  grid_dependency();
+  grid_wait();
+  grid_release();  // the blocks fill every SM (and the loop has no register to spare for a later place)
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -98,7 +99,7 @@ int launch_concretize(const float* A, const float* mid, const float* rad, const 
 
 // ---- finalisation of the fused first-layer concretisation ---------------------
 __global__ void sum_partials_kernel(const float* c, const float* partial, int ntiles, float* out, int M) {
-  grid_dependency();
+  grid_wait();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= M) return;
   float s = 0.f;
@@ -115,7 +116,7 @@ int launch_sum_partials(const float* c, const float* partial, int ntiles, float*
 // ---- per-domain objective and strict best-of ----------------------------------
 __global__ void select_best_kernel(const float* cur, float* best_lower, float* best_metric, int* improve, int first, int spec_reduce,
                                    float soft_tau, float* row_weight, int B, int S) {
-  grid_dependency();
+  grid_wait();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
   const float* row = cur + (size_t)b * S;
@@ -266,7 +267,7 @@ __device__ __forceinline__ void adam_one(float& a, float& mi, float& vi, float g
 // parameter tensor per blockIdx.z; a chunk is 512 columns where 16-byte accesses are legal, else 128.  A step of a small loop
 // is bound by its launches: five 256-wide layers took five launches of 5.2 us (alpha) per step.
 __global__ void __launch_bounds__(128) optimiser_step_kernel(StepArgs p, const int* improve, AdamScalars sc, int do_update) {
-  grid_dependency();
+  grid_wait();
   const StepSegment& g = p.seg[blockIdx.z];
   const int b = blockIdx.x;
   const int j = (blockIdx.y * blockDim.x + threadIdx.x) * (g.vec ? 4 : 1);
@@ -512,7 +513,7 @@ int launch_colmax_abs(const float* A, float* out, int B, int S, int n, cudaStrea
 __global__ void __launch_bounds__(256) relu_adjoint_rows_kernel(float* G, const float* Ahat, const float* dpos, const float* dneg, const float* eneg,
                                                                 const float* pre_l, const float* pre_u, float* grad, float* gsum,
                                                                 const float* gw, int S, int n) {
-  grid_dependency();
+  grid_wait();
   const int b = blockIdx.x;
   const int j = blockIdx.y * blockDim.x + threadIdx.x;
   if (j >= n) return;
@@ -540,6 +541,7 @@ __global__ void __launch_bounds__(256) relu_adjoint_rows_kernel(float* G, const 
       G[((size_t)b * S + s0 + u) * n + j] = sel ? dp * g[u] : fmaf(dn, g[u], en);
     }
   }
+  grid_release();
   grad[o] += acc;
   if (gsum) gsum[o] += gs;
 }
@@ -555,7 +557,7 @@ int launch_relu_adjoint_rows(float* G, const float* Ahat, const float* dpos, con
 
 // Start vector of the gradient sweep for a box: h0 = mid - sgn(A0) * rad, written over A0.
 __global__ void h0_box_kernel(float* A0, const float* mid, const float* rad, long long total, int S, int n0) {
-  grid_dependency();
+  grid_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long m = i / n0;
     const size_t o = (size_t)(m / S) * n0 + (size_t)(i - m * n0);

@@ -33,12 +33,12 @@ def test_dependent_kernels_wait_first_and_read_with_plain_loads():
     launched = set(re.findall(r"launch_dependent\(\s*(?:bf::)?(\w+_kernel)", sources))
     # the clusters of conv_tile_kernel are launched with the attribute among others
     launched |= set(re.findall(r"cudaLaunchKernelEx\(&cfg, (\w+_kernel)", sources)) & {"conv_tile_kernel"}
-    assert len(launched) >= 14 and launched <= set(kernels), launched - set(kernels)
-    waiting = {k for k, (_, body) in kernels.items() if "grid_dependency()" in body}
+    assert len(launched) >= 13 and launched <= set(kernels), launched - set(kernels)
+    waiting = {k for k, (_, body) in kernels.items() if "grid_wait()" in body}
     assert waiting == launched, waiting ^ launched
     for k in sorted(launched):
         params, body = kernels[k]
-        assert re.match(r"\s*grid_dependency\(\);", body), f"{k}: the wait is not the first statement"
+        assert re.match(r"\s*grid_wait\(\);", body), f"{k}: the wait is not the first statement"
         assert "__restrict__" not in params, f"{k}: a __restrict__ parameter's loads may pass the wait"
         seen, todo = set(), [body]
         while todo:
