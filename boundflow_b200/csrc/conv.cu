@@ -855,6 +855,9 @@ static int launch_convT_rowseg(const ConvTArgs& g, RowSegCost* cost, cudaStream_
 // 5x5 kernels, 8 to 256 channels, 7 to 32 pixels) it takes 2211, 33 of them at less than 0.9 of the FP32 speed (worst 0.72), and leaves
 // 44 that would gain 1.3 and more.  (All layers of 148 tiles, 8 channels and up to 9 taps: 266 below 0.9, worst 0.39, namely 8 to 16
 // input channels at stride 1, 8 output channels, and weights of so many blocks that the rows are staged four and eight times.)
+// The FP32 time is that of the row-segment kernel, also for unpadded square maps, which conv_window.cu takes: of 378 such layers that
+// this rule sends here (3x3 / 1, 4x4 / 2, 3x3 / 2 on 3 to 14 pixels, 8 to 128 channels, 256 to 16,384 rows) the time is 0.76 of the FP32 kernels' on
+// average, but 97 are slower than them, 39 by more than 1.25 (worst 1.72, 8 and 16 channels).  They stay: their sums are nearer to float64.
 // Kernels without a row-segment form take it unless a staged element feeds few multiply-adds: 1x1 / 1 from 32 -> 32 channels on (0.9 to
 // 1.4 of the gather kernel's speed; 16 -> 32: 0.7 to 1.1), 2x2 / 1 from 8 -> 32 or 16 -> 16 (0.8 to 1.6), strided ones from 12 -> 32 at
 // 1x1 (0.8 to 1.8) and 12 -> 8 at 2x2 (0.8 to 2.0).
@@ -945,7 +948,8 @@ static int launch_conv_tc_bwd(const float* A, const float* dpos, const float* dn
 // its segments, and its blocks cut a row finer, so it is the faster one where few of its lanes idle (from the channels
 // rounded up to a block's) or its blocks fit the SMs at once.  Window kernel against it, time ratios over 8 to 64 output, 1 to 64 input
 // channels, 32 to 8192 rows, where this rule takes the one or the other:
-//   3x3 / 1, 12 -> 14: 0.43 to 0.88 | 1.02 to 1.25 (16 channels, few rows, also 0.98)    14 -> 16: 0.38 to 1.00 | 1.02 to 1.43 (16 channels 0.94 to 1.25)
+//   3x3 / 1, 12 -> 14: 0.43 to 0.88 | 1.02 to 1.25 (16 channels, few rows, also 0.98)
+//            14 -> 16: 0.38 to 1.00 | 1.02 to 1.43 (16 channels 0.94 to 1.25)
 //   4x4 / 2,  7 -> 16: 0.73 to 0.95 | 1.05 to 1.57 (1 and 8 channels, few rows, 0.92 to 0.99)
 static bool rowseg_keeps(const ConvTArgs& g) {
   const bool s1 = g.kh == 3 && g.sh == 1 && g.Wi >= 14, s2 = g.kh == 4 && g.sh == 2 && g.Wi == 16;

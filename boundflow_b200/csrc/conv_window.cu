@@ -18,11 +18,12 @@ namespace bf {
 // Blocks stay: a block keeps the weights of its channel groups and walks tiles of 32 * R rows, whose windows come in chunks of
 // cc output channels with 16-byte cp.async (4-byte copies took eight clocks of the SM for 128 bytes and bound the kernel), one
 // chunk ahead.  Results leave through a 32 x 33 tile per warp, 128 bytes of a row at a time.
-// Bound by FFMA issue next to the shared-memory reads where a block's channels are many (20 to 23 of 31 T multiply-adds/s that
-// the chip reaches), by the chunks' copies and the results' stores with one to three channels.  65,536 rows, against the
-// row-segment kernels: 32 -> 32 channels, 3 x 3 -> 8 x 8 of 4x4 / 2: 1293 -> 472 us; 64 -> 32, 4 x 4 -> 6 x 6 of 3x3: 3674 -> 841;
-// 32 -> 32, 6 x 6 -> 14 x 14 of 4x4 / 2: 5490 -> 2515; 32 -> 3, 8 x 8 -> 10 x 10 of 3x3: 1124 -> 218; 32 -> 1, 4 x 4 -> 10 x 10 of
-// 4x4 / 2: 223 -> 60.  Few rows: no slower (32 rows of 220 shapes: 0.1 to 1.0 of the time), except where rowseg_keeps (conv.cu) says so.
+// Bound by instruction issue (slots 62 to 79 % busy with 12 to 16 warps an SM, FFMA pipe 46 to 67 %, shared memory 29 to 43 %): 15 to 23 of the
+// 31 T multiply-adds/s that the chip reaches where a block's channels are many; with one to three channels the chunks' copies and the
+// results' stores count too (DRAM 35 %).  65,536 rows, against the row-segment kernels: 32 -> 32 channels, 3 x 3 -> 8 x 8 of 4x4 / 2:
+// 1291 -> 471 us; 64 -> 32, 4 x 4 -> 6 x 6 of 3x3: 3672 -> 838; 32 -> 32, 6 x 6 -> 14 x 14 of 4x4 / 2: 5486 -> 2514; 32 -> 3, 8 x 8 -> 10 x 10 of
+// 3x3: 1124 -> 201; 32 -> 1, 4 x 4 -> 10 x 10 of 4x4 / 2: 221 -> 53.  Few rows: no slower (32 rows of 220 shapes: 0.1 to 1.0 of the time),
+// except where rowseg_keeps (conv.cu) says so.
 struct ConvWindowArgs {
   const float* Lam;  // [M, Co, WW, WW]
   const float* W;    // [Co, Ci, KS, KS]
@@ -194,7 +195,9 @@ static int launch_window(ConvWindowArgs a, cudaStream_t stream) {
   using G = ConvWindow<KS, ST, PD, WW>;
   constexpr int NWP = (KS * KS * TCI + 3) / 4 * 4, LIMIT = (G::BLOCKS == 1 ? 224 : 112) * 1024, EPI = 32 * 33 * 4, PLANE = WW * WW;
   const int ncg = ceil_div(a.Ci, TCI);
-  // channel groups per block: few of them idle, few blocks that read the same rows, and no idle warps where a block has an SM
+  // Channel groups per block: few of them idle, few blocks that read the same rows (a tenth for each), and no idle warps where a block has an
+  // SM.  Over 198 shapes (11 windows, 6 pairs of channels, 512 to 16,384 rows) the best other count is 5 % faster on average, more than 6 % on 46 of
+  // them, 38 of these at 512 rows, where fewer groups in more blocks would take down to 0.68 of the time.
   double best = 0.0;
   int gy = 0;
   for (int c = G::WARPS / G::NB; c >= 1; --c) {
