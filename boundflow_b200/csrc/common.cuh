@@ -98,8 +98,11 @@ inline void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, s
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" : : : "memory"); }
 // When every block has come here or ended, the blocks of the next dependent launch are placed.  Where SMs are still unevenly busy they go in
 // bunches to those that are free, as many as fit, and a launch of fewer blocks than the chip holds then leaves SMs idle: so behind the
-// work of a block, not before it, and kernels of long blocks that rarely fill the chip evenly (conv.cu) are plain launches.
+// work of a block, not before it, and kernels of long blocks that do not fill the chip evenly (conv.cu) are plain launches.
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" : : : "memory"); }
+
+// A dependent launch of no more blocks than SMs asks for ONE_PER_SM bytes of shared memory instead: they cannot bunch then.
+constexpr int ONE_PER_SM = 116 * 1024;  // more than half of an SM's shared memory
 
 inline cudaStream_t as_stream(bf_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 

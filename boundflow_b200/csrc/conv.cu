@@ -317,10 +317,16 @@ static int launch_conv_tile_n(const IbpConvArgs& g, int vec, cudaStream_t stream
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  // Fewer blocks than the chip holds, or clusters, are not placed early, unless they are short: bunched on the SMs that are free first, 400
-  // of them took 88 us for 71 (200 x 32 x 32 x 32 -> 32, 4x4 / 2), 128 in clusters of four 37 for 30 (16 x 128 x 8 x 8 -> 128, 3x3, intervals);
-  // 110 of 16 taps (144 x 1 x 28 x 28 -> 16) 4.0 for 4.6.
-  cfg.numAttrs = ks == 1 && (K <= 64 || tiles * ctas_y >= 4 * 148) ? 2 : 1;
+  // Fewer blocks than the chip holds, or clusters, are not placed early, unless they are short or one to an SM: bunched on the SMs that are
+  // free first, 400 of them took 88 us for 71 (200 x 32 x 32 x 32 -> 32, 4x4 / 2), 128 in clusters of four 37 for 30 (16 x 128 x 8 x 8 -> 128, 3x3,
+  // intervals); 110 of 16 taps (144 x 1 x 28 x 28 -> 16) 4.0 for 4.6.  One to an SM: 10 steps of alpha on a CNN of 48 inputs 2.03 -> 2.00 ms.
+  const bool one_each = ks == 1 && tiles * ctas_y <= 148;
+  cfg.numAttrs = one_each || (ks == 1 && (K <= 64 || tiles * ctas_y >= 4 * 148)) ? 2 : 1;
+  if (one_each) {
+    static SmemOptIn opt_in;
+    if (int rc = ensure_dynamic_smem(conv_tile_kernel<INTERVAL, TN>, ONE_PER_SM, opt_in, "conv_tile_kernel")) return rc;
+    cfg.dynamicSmemBytes = ONE_PER_SM;
+  }
   cudaLaunchKernelEx(&cfg, conv_tile_kernel<INTERVAL, TN>, g, ceil_div(slabs, ks) * ConvTile<TN>::SLAB, vec);
   BF_CHECK_LAUNCH("conv_tile_kernel");
   return BF_OK;
@@ -572,12 +578,13 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Plain launches: placed early, behind the short ReLU pass, the blocks of a sweep of a few hundred rows bunched on half of the SMs (256 rows,
-// 64 -> 32 channels, 3x3 on 8 x 8, with the pass: 113 us, 48 plain; 856 sizes: 0.97 of the time, 78 of them under 0.95).
+// A plain launch unless its blocks are one to an SM: placed early, behind the short ReLU pass, the blocks of a sweep of a few hundred rows bunched on
+// half of the SMs (256 rows, 64 -> 32 channels, 3x3 on 8 x 8, with the pass: 113 us, 48 plain; 856 sizes: 0.97 of the time, 78 of them under 0.95).
 // RT = 2 (8-pixel segments): a thread owns two image rows that meet the same kernel rows, and each weight read feeds twice the
 // multiply-adds.  Same order of sums.
 template <int KS, int ST, int PD, int TCI, bool VEC, int TWP, int RT>
 __global__ void __launch_bounds__(256, (TCI > 1 && TWP * RT > 8 ? 2 : 3)) conv_transpose_rowseg_kernel(RowSegArgs a) {
+  grid_wait();
   using G = RowSeg<KS, ST, PD, VEC, TWP>;
   extern __shared__ __align__(16) float rs_smem[];
   const ConvTArgs& g = a.c;
@@ -728,6 +735,7 @@ __global__ void __launch_bounds__(256, (TCI > 1 && TWP * RT > 8 ? 2 : 3)) conv_t
     }
     __syncthreads();
   }
+  grid_release();
   if (!row_ok) return;
   const int wleft = g.Wi - (w0 + colseg * G::TW);
 #pragma unroll
@@ -813,8 +821,11 @@ static int launch_rowseg_tci(const ConvTArgs& g, RowSegCost* cost, cudaStream_t 
     return BF_OK;
   }
   static SmemOptIn opt_in;
-  if (int rc = ensure_dynamic_smem(conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT>, 110 * 1024, opt_in, "conv_transpose_rowseg_kernel")) return rc;
-  conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT><<<grid, 256, smem, stream>>>(a);
+  if (int rc = ensure_dynamic_smem(conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT>, ONE_PER_SM, opt_in, "conv_transpose_rowseg_kernel")) return rc;
+  if ((long long)grid.x * grid.y * grid.z <= 148)
+    launch_dependent(conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT>, grid, 256, ONE_PER_SM, stream, a);
+  else
+    conv_transpose_rowseg_kernel<KS, ST, PD, TCI, VEC, TWP, RT><<<grid, 256, smem, stream>>>(a);
   BF_CHECK_LAUNCH("conv_transpose_rowseg_kernel");
   return BF_OK;
 }

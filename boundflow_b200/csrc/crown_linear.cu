@@ -125,7 +125,6 @@ __global__ void __launch_bounds__(GS_THREADS, 2) crown_bwd_small_kernel(GemmArgs
       if (m0 + r0 + i < g.M) e.partial[(size_t)(m0 + r0 + i) * e.ntiles + blockIdx.y] = p[i] + part[r0 + i];
   }
 }
-constexpr int GS_ONE_PER_SM = 116 * 1024;  // more than half of an SM's shared memory
 constexpr int GS_BWD_SMEM = (GS_STAGES * (GS_A_WORDS + GS_B_WORDS<false>) + GS_ROWS) * (int)sizeof(float);
 
 // Top layer of a sweep (no ReLU in front, K = spec width <= 16): A_prev[M,N] = A[M,K] * W[K,N] and
@@ -215,11 +214,11 @@ int launch_crown_bwd_linear(const float* A, const float* dpos, const float* dneg
   timing_begin(T_BWD, stream);
   if (ffma_quarter_tiles(M, N)) {
     static SmemOptIn opt_in;
-    if (int rc = ensure_dynamic_smem(crown_bwd_small_kernel, GS_ONE_PER_SM, opt_in, "crown_bwd_small_kernel")) return rc;
+    if (int rc = ensure_dynamic_smem(crown_bwd_small_kernel, ONE_PER_SM, opt_in, "crown_bwd_small_kernel")) return rc;
     dim3 grid(ceil_div(M, GS_ROWS), e.ntiles + (delta ? 1 : 0));
     // No more CTAs than SMs: one per SM.  They are placed while the kernel before still has its SMs and would go in pairs to those
     // that are free (alpha loops of 99 to 145 CTAs in pairs: 1.02 to 1.07 of the time over nine sizes from 128 to 1000 wide; fewer CTAs: the same).
-    const int smem = grid.x * grid.y <= 148 ? GS_ONE_PER_SM : GS_BWD_SMEM;
+    const int smem = grid.x * grid.y <= 148 ? ONE_PER_SM : GS_BWD_SMEM;
     // More CTAs than SMs only with those of the row sums: a plain launch, whose tiles all find an SM of their own, where the sums are long
     // (576 x 512 x 512 21.4 us early, 19.6 plain, 1152 x 256 x 256 12.8 and 11.3; alpha loops of 256 to 1000 wide layers early: 0.98 to 1.06 of
     // the time, 1.02 on average; of 64 to 128 wide layers plain: 1.00 to 1.07).
