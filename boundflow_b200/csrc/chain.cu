@@ -237,11 +237,18 @@ void refresh_switches(const bf_chain* c) {
   c->sw.tc_auto = !(rows && atoi(rows) > 0);
 }
 
+// few rows: crown_small_tc.cu
+static bool small_rows(const bf_chain* c, int M, int N, int K, int S, bool adjoint) {
+  return !c->pk_small_bwd.empty() && !c->sw.force_ffma && c->sw.tc_auto && small_tc_supports(M, N, K, S, adjoint);
+}
+
 bool tc_may_run(const bf_chain* c, int M) {
   if (c->status == nullptr || c->sw.force_ffma) return false;
   if (!c->pk_bwd.empty() && M >= c->sw.tc_min_rows) return true;
-  for (const bf_layer_desc& L : c->layers)
+  for (const bf_layer_desc& L : c->layers) {
     if (L.op == BF_OP_CONV2D && conv_rows_on_tensor_cores(M, L)) return true;
+    if (L.op == BF_OP_LINEAR && (small_rows(c, M, L.n_in, L.n_out, 1, false) || small_rows(c, M, L.n_out, L.n_in, 1, true))) return true;
+  }
   return false;
 }
 
@@ -270,6 +277,11 @@ int dispatch_bwd(const bf_chain* c, int layer, const float* A, const float* dpos
                         cudaStream_t stream) {
   const bf_layer_desc& L = c->layers[layer];
   const int K = L.n_out, N = L.n_in;
+  if ((A_prev || partial) && small_rows(c, M, N, K, S, false)) {
+    if (ptiles) *ptiles = small_tc_tiles(M, N, K);
+    return launch_crown_bwd_small_tc(A, dpos, dneg, epos, eneg, add, c->pk_small_bwd[layer], L.W, L.bias, A_prev, delta, accumulate, mid, rad,
+                                     partial, side, M, S, K, N, c->status, stream);
+  }
   const unsigned char* pk = tc_weights(c, layer, false, M, K, N);
   if (pk && c->sw.persistent_bwd && crown_tc_persistent_supports(epos, eneg, add)) {
     if (ptiles) *ptiles = crown_tc_persist_partial_tiles(M, N, K);
@@ -292,6 +304,9 @@ int dispatch_adjoint(const bf_chain* c, int layer, const float* Hprev, int first
                             int M, int S, cudaStream_t stream, const float* gw) {
   const bf_layer_desc& L = c->layers[layer];
   const int K = L.n_in, N = L.n_out;
+  if (small_rows(c, M, N, K, S, true))
+    return launch_crown_adjoint_small_tc(Hprev, first_layer, mid, rad, c->pk_small_adj[layer], L.W, L.bias, Ahat, dpos, dneg, epos, eneg, pre_l,
+                                         pre_u, hout, grad, gsum, M, S, K, N, c->status, stream, gw);
   const unsigned char* pk = tc_weights(c, layer, true, M, K, N);
   // gw (row weights of the beta sums, min / softmin with beta parameters) is implemented by the row-major and FFMA kernels
   if (pk && gw == nullptr && adjoint_feature_major(c, M, N))
@@ -312,7 +327,8 @@ extern "C" size_t bf_chain_tc_bytes(const bf_chain* chain) {
   for (const bf_layer_desc& L : chain->layers)
     if (L.op == BF_OP_LINEAR)
       total += bf::align_up(bf::tc_packed_bytes(L.n_in, L.n_out)) + bf::align_up(bf::tc_packed_bytes(L.n_out, L.n_in)) +
-               bf::align_up(bf::tc_packed_bytes(L.n_out, L.n_in, bf::tc_adjoint_tile_rows()));
+               bf::align_up(bf::tc_packed_bytes(L.n_out, L.n_in, bf::tc_adjoint_tile_rows())) +
+               bf::align_up(bf::small_tc_packed_bytes(L.n_in, L.n_out)) + bf::align_up(bf::small_tc_packed_bytes(L.n_out, L.n_in));
   return total;
 }
 
@@ -331,6 +347,9 @@ extern "C" int bf_chain_tc_prepare(bf_chain* chain, void* buffer, size_t bytes, 
   chain->pk_bwd.assign(chain->layers.size(), nullptr);
   chain->pk_adj.assign(chain->layers.size(), nullptr);
   chain->pk_adj_fm.assign(chain->layers.size(), nullptr);
+  std::vector<bf::SmallPack> small;
+  chain->pk_small_bwd.assign(chain->layers.size(), nullptr);
+  chain->pk_small_adj.assign(chain->layers.size(), nullptr);
   for (size_t i = 0; i < chain->layers.size(); ++i) {
     const bf_layer_desc& L = chain->layers[i];
     if (L.op != BF_OP_LINEAR) continue;
@@ -349,11 +368,19 @@ extern "C" int bf_chain_tc_prepare(bf_chain* chain, void* buffer, size_t bytes, 
     off += bf::align_up(bf::tc_packed_bytes(L.n_out, L.n_in, bf::tc_adjoint_tile_rows()));
     rc = bf::tc_pack_weights(L.W, L.n_out, L.n_in, 0, pf, stream, bf::tc_adjoint_tile_rows());
     if (rc != BF_OK) return rc;
+    unsigned char* sb = base + off;
+    off += bf::align_up(bf::small_tc_packed_bytes(L.n_in, L.n_out));
+    unsigned char* sa = base + off;
+    off += bf::align_up(bf::small_tc_packed_bytes(L.n_out, L.n_in));
+    small.push_back({L.W, L.n_out, L.n_in, 1, sb});
+    small.push_back({L.W, L.n_out, L.n_in, 0, sa});
+    chain->pk_small_bwd[i] = sb;
+    chain->pk_small_adj[i] = sa;
     chain->pk_adj_fm[i] = pf;
     chain->pk_bwd[i] = pb;
     chain->pk_adj[i] = pa;
   }
-  return BF_OK;
+  return bf::small_tc_pack(small.data(), (int)small.size(), stream);
 }
 
 extern "C" int bf_chain_tc_status(const bf_chain* chain, int* status_out) {

@@ -16,6 +16,7 @@ struct bf_chain {
   // tensor-core path: per layer, packed hi/lo weight images for the backward (W^T as B) and
   // adjoint (W as B) orientation inside a caller-owned buffer, plus a device status word
   std::vector<const unsigned char*> pk_bwd, pk_adj, pk_adj_fm;  // pk_adj_fm: 128-row images for the feature-major adjoint kernel
+  std::vector<const unsigned char*> pk_small_bwd, pk_small_adj;  // bfloat16 parts for sweeps of few rows (crown_small_tc.cu)
   int* status = nullptr;
   // A/B switches (environment variables BF_B200_*), refreshed at the start of every whole-chain call and read by
   // the per-layer dispatch of that call

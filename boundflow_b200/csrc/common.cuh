@@ -95,6 +95,27 @@ inline void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, s
   cfg.numAttrs = 1;
   (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
+// The same for kernels that fetch weight images while they wait.  What they read in front of weights_wait() has to be older than the launch before
+// them: images packed before the sweep, in a kernel that is not the first of it.  The blocks of a dependent launch are placed when
+// those of the launch before have passed their own wait or ended (grid_release comes behind it), so all older launches are complete and visible then.
+template <typename... Params, typename... Args>
+inline void launch_behind_weights(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+__device__ __forceinline__ void weights_wait() { asm volatile("griddepcontrol.wait;" : : : "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" : : : "memory"); }
 // When every block has come here or ended, the blocks of the next dependent launch are placed.  Where SMs are still unevenly busy they go in
 // bunches to those that are free, as many as fit, and a launch of fewer blocks than the chip holds then leaves SMs idle: so behind the

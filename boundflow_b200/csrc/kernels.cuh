@@ -33,6 +33,24 @@ int launch_crown_adjoint_linear_tc(const float* Hprev, int first_layer, const fl
 int crown_tc_partial_tiles(int N, int K);
 void tc_tile_shape(int N, int K, int* BN, int* ntiles, int* nkb);
 
+// crown_small_tc.cu (few coefficient rows on the tensor cores; weights packed by small_tc_pack)
+bool small_tc_supports(int M, int N, int K, int S, bool adjoint);
+int small_tc_tiles(int M, int N, int K);  // feature tiles (= partial sums per row)
+size_t small_tc_packed_bytes(int N, int K);
+struct SmallPack {
+  const float* W;  // [rows, cols]; features are its rows, or its columns (transposed)
+  int rows, cols, transposed;
+  unsigned char* out;
+};
+int small_tc_pack(const SmallPack* packs, int count, cudaStream_t stream);
+int launch_crown_bwd_small_tc(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg, const float* add,
+                              const unsigned char* Wpk, const float* W, const float* kbias, float* A_prev, float* delta, int accumulate, const float* mid,
+                              const float* rad, float* partial, int side, int M, int S, int K, int N, int* status, cudaStream_t stream);
+int launch_crown_adjoint_small_tc(const float* Hprev, int first_layer, const float* mid, const float* rad, const unsigned char* Wpk, const float* W,
+                                  const float* nbias, const float* Ahat, const float* dpos, const float* dneg, const float* epos, const float* eneg,
+                                  const float* pre_l, const float* pre_u, float* hout, float* grad, float* gsum, int M, int S, int K, int N, int* status,
+                                  cudaStream_t stream, const float* gw);
+
 // crown_tc_persist.cu (persistent, warp-specialised backward contraction; same packed weights as crown_tc.cu)
 int launch_crown_bwd_linear_tc_persistent(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
                                           const float* add, const unsigned char* Wpk, const float* kbias, float* A_prev,
