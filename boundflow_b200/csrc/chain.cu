@@ -506,7 +506,7 @@ static size_t crown_ws_layout(const bf_chain* c, int B, int S, int upto, void* b
   float* b0 = cv.take<float>(M * maxw);
   float* b1 = cv.take<float>(M * maxw);
   float* cacc = cv.take<float>(M);
-  float* partial = cv.take<float>(M * (size_t)std::max(std::max(crown_bwd_partial_tiles(c->n0), crown_tc_partial_tiles(c->n0, 32)), crown_tc_persist_max_partial_tiles(c->n0)));
+  float* partial = cv.take<float>(M * (size_t)max_partial_tiles(c->n0));
   char* cs = cv.take<char>(conv_scratch);
   if (ws) {
     ws->buf[0] = b0; ws->buf[1] = b1; ws->cacc = cacc; ws->partial = partial; ws->conv_scratch = cs; ws->bytes = cv.off;

@@ -1,5 +1,6 @@
 // Shared between the chain drivers (chain.cu, chain_alpha.cu).
 #pragma once
+#include <algorithm>
 #include <vector>
 
 #include "kernels.cuh"
@@ -50,6 +51,11 @@ struct Carver {
   }
 };
 
+// Concretisation partial sums per row, at most, of whichever backward kernel takes a first layer of n0 inputs
+inline int max_partial_tiles(int n0) {
+  return std::max(std::max(std::max(crown_bwd_partial_tiles(n0), crown_tc_partial_tiles(n0, 32)), crown_tc_persist_max_partial_tiles(n0)),
+                  small_tc_max_tiles(n0));
+}
 
 // Re-reads the BF_B200_* environment switches into chain->sw (called once per whole-chain entry point).
 void refresh_switches(const bf_chain* c);

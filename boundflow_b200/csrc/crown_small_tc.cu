@@ -701,6 +701,7 @@ static int small_tc_cluster(int M, int N, int K) {
 
 bool small_tc_supports(int M, int N, int K, int S, bool adjoint) { return small_tc_cluster(M, N, K) > 0 && (!adjoint || S <= stc::NR); }
 int small_tc_tiles(int M, int N, int K) { return ceil_div(N, stc::TF) * small_tc_cluster(M, N, K); }
+int small_tc_max_tiles(int N) { return ceil_div(N, stc::TF) * 4; }
 size_t small_tc_packed_bytes(int N, int K) { return (size_t)ceil_div(N, stc::TF) * ceil_div(K, stc::KS) * stc::W_STAGE; }
 
 int small_tc_pack(const SmallPack* packs, int count, cudaStream_t stream) {

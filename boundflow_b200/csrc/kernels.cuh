@@ -35,7 +35,8 @@ void tc_tile_shape(int N, int K, int* BN, int* ntiles, int* nkb);
 
 // crown_small_tc.cu (few coefficient rows on the tensor cores; weights packed by small_tc_pack)
 bool small_tc_supports(int M, int N, int K, int S, bool adjoint);
-int small_tc_tiles(int M, int N, int K);  // feature tiles (= partial sums per row)
+int small_tc_tiles(int M, int N, int K);  // parts of the features (= partial sums per row)
+int small_tc_max_tiles(int N);            // the largest count any M and K give (workspace sizing)
 size_t small_tc_packed_bytes(int N, int K);
 struct SmallPack {
   const float* W;  // [rows, cols]; features are its rows, or its columns (transposed)

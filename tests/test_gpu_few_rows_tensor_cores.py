@@ -132,3 +132,21 @@ def test_infinities_pass_as_on_the_fp32_units(dev, N):
     # two sums of K + N positive terms, each rounding at most n * 2^-24 of the result
     assert ((out[:, [0, 2, 3]].cpu().double() - want).abs() <= (K + N + 8) * 2.0**-24 * want.abs()).all()
     assert (out[:, 1] == -float("inf")).all(), out[:, 1]
+
+
+# (rows of a domain, inputs, terms): one CTA a tile and clusters of two and four, first layers of 1 to 13 tiles
+@pytest.mark.parametrize("B, S, n0, K", [(6, 9, 784, 512), (6, 9, 784, 1100), (40, 9, 784, 256), (1, 1, 65, 1100), (3, 2, 1600, 200), (160, 9, 129, 100)])
+def test_sweeps_stay_inside_their_workspace(dev, B, S, n0, K):
+    """What lies behind the bytes that the library asks for stays as it was (partial sums per row: one per part of the features)."""
+    g = torch.Generator().manual_seed(n0 + K)
+    chain = _Chain([torch.randn((K, n0), generator=g)], [torch.randn((K,), generator=g)], dev)
+    lib, _lib = chain.lib, chain._lib
+    C, mid, rad = (torch.rand(s, generator=g).to(dev) for s in ((B, S, K), (B, n0), (B, n0)))
+    n, guard = int(lib.bf_chain_crown_workspace_bytes(chain.h, B, S, 1)), 1 << 20
+    ws, out = torch.full((n + guard,), 0xA5, dtype=torch.uint8, device=dev), torch.empty((B, S), device=dev)
+    launches = _lib.tc_launch_count()
+    _lib.check(lib.bf_chain_crown(chain.h, 1, _lib.SIDE_LOWER, C.data_ptr(), None, None, None, None, mid.data_ptr(), rad.data_ptr(), _lib.NORM_BOX, 0.0,
+                                  out.data_ptr(), ws.data_ptr(), n, B, S, None))
+    assert _lib.tc_launch_count() == launches + 1
+    assert (ws[n:] == 0xA5).all() and torch.isfinite(out).all()
+    chain.close()
