@@ -95,11 +95,10 @@ inline void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, s
   cfg.numAttrs = 1;
   (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
-// The same for kernels that fetch weight images while they wait.  What they read in front of weights_wait() has to be older than the launch before
-// them: images packed before the sweep, in a kernel that is not the first of it.  The blocks of a dependent launch are placed when
-// those of the launch before have passed their own wait or ended (grid_release comes behind it), so all older launches are complete and visible then.
+// The same for kernels that set up barriers and tensor memory before they wait (1 to 2 thousand clocks), and in clusters: nothing in front of
+// grid_wait_after_setup() reads or writes global memory.
 template <typename... Params, typename... Args>
-inline void launch_behind_weights(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t stream, Args&&... args) {
+inline void launch_after_setup(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -115,7 +114,7 @@ inline void launch_behind_weights(void (*kernel)(Params...), dim3 grid, dim3 blo
   cfg.numAttrs = cluster > 1 ? 2 : 1;
   (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
-__device__ __forceinline__ void weights_wait() { asm volatile("griddepcontrol.wait;" : : : "memory"); }
+__device__ __forceinline__ void grid_wait_after_setup() { asm volatile("griddepcontrol.wait;" : : : "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" : : : "memory"); }
 // When every block has come here or ended, the blocks of the next dependent launch are placed.  Where SMs are still unevenly busy they go in
 // bunches to those that are free, as many as fit, and a launch of fewer blocks than the chip holds then leaves SMs idle: so behind the

@@ -49,21 +49,19 @@ def test_dependent_kernels_wait_first_and_read_with_plain_loads():
                 todo.append(device[f])
 
 
-def test_kernels_that_fetch_weights_while_they_wait_read_nothing_else():
-    """launch_behind_weights: in front of weights_wait() a kernel may set up barriers and tensor memory and copy weight images (g.Wpk), which no
-    launch of a sweep writes; it takes them early only where another launch of its sweep lies between it and the packing."""
+def test_kernels_that_wait_after_their_setup_touch_no_global_memory_before():
+    """launch_after_setup: in front of grid_wait_after_setup() a kernel sets up barriers, tensor memory and indices only."""
     kernels, device, sources = _functions()
-    launched = set(re.findall(r"launch_behind_weights\(\s*(?:\w+::)*(\w+_kernel)", sources))
-    waiting = {k for k, (_, body) in kernels.items() if "weights_wait()" in body}
+    launched = set(re.findall(r"launch_after_setup\(\s*(?:\w+::)*(\w+_kernel)", sources))
+    waiting = {k for k, (_, body) in kernels.items() if "grid_wait_after_setup()" in body}
     assert launched and launched == waiting, launched ^ waiting
     for k in sorted(launched):
         params, body = kernels[k]
-        front, behind = body.split("weights_wait();")
+        front, behind = body.split("grid_wait_after_setup();")
         assert "__restrict__" not in params and "grid_release()" not in front and "grid_release()" in behind
-        assert not re.search(r"\bload\w*\(|\bld_?\w*\(|\*\s*reinterpret_cast|ld\.global|atomic", front), k
-        # the only global memory it names by subscript or copies from
-        assert set(re.findall(r"bulk_copy_g2s\([^;]*?,\s*(\w+)", front)) == {"wsrc"} and re.search(r"\bwsrc = g\.Wpk\b", front), k
-        assert re.search(r"if \([^;]*g\.early\)\s*for", front), k
+        # no loads, stores, copies or atomics; the only subscripts are those of barriers in shared memory
+        assert not re.search(r"\bload\w*\(|\bld_\w*\(|\bbulk_copy|\*\s*reinterpret_cast|\.global\b|atomic|\bg\.\w+\[", front), k
+        assert set(re.findall(r"(\w+(?:\.\w+)?)\[[^\]]*\]\s*[;,)=+]", front)) <= {"ctl.full", "ctl.summed", "ctl.drained", "row_part", "con_part", "st_smem"}, k
         seen, todo = set(), [body]
         while todo:
             text = todo.pop()
@@ -71,4 +69,3 @@ def test_kernels_that_fetch_weights_while_they_wait_read_nothing_else():
             for f in set(re.findall(r"\b(\w+)\s*(?:<[^;(){}]*>)?\s*\(", text)) & set(device) - seen:
                 seen.add(f)
                 todo.append(device[f])
-    assert re.findall(r"g\.early = ([^;]*);", sources) == ["dpos != nullptr", "1"]
