@@ -85,6 +85,17 @@ struct InputSetArg {
   bool box() const { return norm_p == BF_NORM_BOX; }
 };
 
+// Relaxations of every ReLU at `alpha` (one row for all domains if shared)
+static int relax_all(const bf_chain* c, const AlphaWs& ws, const float* const* pre_l, const float* const* pre_u, const float* const* alpha, bool shared,
+                     int B, cudaStream_t stream) {
+  std::vector<RelaxSegment> seg;
+  for (size_t r = 0; r < c->relu_layers.size(); ++r) {
+    const int n = c->layers[c->relu_layers[r]].n_in;
+    seg.push_back({pre_l[r], pre_u[r], alpha[r], ws.au[r], ws.bu[r], ws.sl[r], shared ? 0 : n, n});
+  }
+  return launch_relu_relax(seg.data(), (int)seg.size(), B, stream);
+}
+
 // One lower- or upper-side sweep with the relaxations in ws; `use_add` adds the split term of
 // every ReLU to the lower coefficients (beta-CROWN).
 // Backward step of affine layer `layer` (Linear: tensor-core / FFMA GEMM with optional fused box concretisation;
@@ -259,10 +270,9 @@ static int alpha_loop(const char* who, const bf_chain* chain, const float* C, co
     bf::set_error("%s: cudaMemsetAsync failed", who);
     return BF_E_CUDA;
   }
+  if ((rc = bf::relax_all(chain, ws, pre_l, pre_u, alpha, false, B, stream)) != BF_OK) return rc;
   for (int r = 0; r < R; ++r) {
     const int n = chain->layers[chain->relu_layers[r]].n_in;
-    rc = bf::launch_relu_relax(pre_l[r], pre_u[r], alpha[r], n, ws.au[r], ws.bu[r], ws.sl[r], B, n, stream);
-    if (rc != BF_OK) return rc;
     if (with_beta) {  // split term of the start beta (no update, no snapshot: improve flags are not set yet)
       bf::AdamScalars none{};
       rc = bf::launch_beta_step(beta[r], ws.mb[r], ws.vb[r], ws.gsum[r], splits[r], split_strides ? split_strides[r] : n, nullptr,
@@ -304,11 +314,7 @@ static int alpha_loop(const char* who, const bf_chain* chain, const float* C, co
   }
   if (best_upper) {
     // the upper bound of each domain's best iteration = the upper sweep at its best alpha (beta acts on the lower side only)
-    for (int r = 0; r < R; ++r) {
-      const int n = chain->layers[chain->relu_layers[r]].n_in;
-      rc = bf::launch_relu_relax(pre_l[r], pre_u[r], best_alpha[r], n, ws.au[r], ws.bu[r], ws.sl[r], B, n, stream);
-      if (rc != BF_OK) return rc;
-    }
+    if ((rc = bf::relax_all(chain, ws, pre_l, pre_u, best_alpha, false, B, stream)) != BF_OK) return rc;
     rc = bf::alpha_sweep(chain, ws, C, BF_SIDE_UPPER, false, false, in, best_upper, B, S, stream);
     if (rc != BF_OK) return rc;
   }
@@ -374,11 +380,7 @@ extern "C" int bf_chain_alpha_grad(const bf_chain* chain, const float* C, const 
     bf::set_error("bf_chain_alpha_grad: cudaMemsetAsync failed");
     return BF_E_CUDA;
   }
-  for (int r = 0; r < R; ++r) {
-    const int n = chain->layers[chain->relu_layers[r]].n_in;
-    rc = bf::launch_relu_relax(pre_l[r], pre_u[r], alpha[r], n, ws.au[r], ws.bu[r], ws.sl[r], B, n, stream);
-    if (rc != BF_OK) return rc;
-  }
+  if ((rc = bf::relax_all(chain, ws, pre_l, pre_u, alpha, false, B, stream)) != BF_OK) return rc;
   rc = bf::alpha_sweep(chain, ws, C, BF_SIDE_LOWER, true, false, in, lower, B, S, stream);
   if (rc != BF_OK) return rc;
   rc = bf::alpha_adjoint(chain, ws, pre_l, pre_u, false, in, B, S, stream);
@@ -486,16 +488,9 @@ static int shared_loop(const char* who, const bf_chain* chain, const float* C, c
   int rc;
   auto width = [&](int r) { return chain->layers[chain->relu_layers[r]].n_in; };
   auto stride = [&](int r) { return split_strides ? split_strides[r] : width(r); };
-  auto relax_all = [&](float* const* a) -> int {
-    for (int r = 0; r < R; ++r) {
-      int e = bf::launch_relu_relax(pre_l[r], pre_u[r], a[r], /*alpha_stride=*/0, ws.au[r], ws.bu[r], ws.sl[r], B, width(r), stream);
-      if (e != BF_OK) return e;
-    }
-    return BF_OK;
-  };
   for (int t = 0; t <= steps; ++t) {
     const bool last = (t == steps);
-    if ((rc = relax_all(alpha)) != BF_OK) return rc;
+    if ((rc = bf::relax_all(chain, ws, pre_l, pre_u, alpha, true, B, stream)) != BF_OK) return rc;
     if (with_beta)
       for (int r = 0; r < R; ++r)
         if (splits[r] && (rc = bf::launch_shared_beta_add(beta[r], splits[r], stride(r), ws.addv[r], B, width(r), stream)) != BF_OK)
@@ -540,7 +535,7 @@ static int shared_loop(const char* who, const bf_chain* chain, const float* C, c
     }
   }
   if (best_upper) {  // beta acts on the lower side only
-    if ((rc = relax_all(best_alpha)) != BF_OK) return rc;
+    if ((rc = bf::relax_all(chain, ws, pre_l, pre_u, best_alpha, true, B, stream)) != BF_OK) return rc;
     rc = bf::alpha_sweep(chain, ws, C, BF_SIDE_UPPER, false, false, in, best_upper, B, S, stream);
     if (rc != BF_OK) return rc;
   }

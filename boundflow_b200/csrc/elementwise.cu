@@ -2,6 +2,9 @@
 // per-domain best tracking, the fused Adam/projection/slope kernel and verdicts.
 #include <float.h>
 
+#include <algorithm>
+#include <vector>
+
 #include "kernels.cuh"
 
 namespace bf {
@@ -19,21 +22,25 @@ __device__ __forceinline__ void relax_one(float l, float u, float& au, float& bu
   }
 }
 
-__global__ void relu_relax_kernel(const float* __restrict__ l, const float* __restrict__ u, const float* __restrict__ alpha,
-                                  int alpha_stride, float* __restrict__ alpha_u, float* __restrict__ beta_u,
-                                  float* __restrict__ alpha_l, int n, long long total) {
+// The ReLUs of a sweep in one launch, blocks (x, ReLU): a query of small layers spent 2 us of the GPU and 4 of the host on each.
+struct RelaxArgs {
+  RelaxSegment seg[RELAX_SEGMENTS];
+};
+__global__ void __launch_bounds__(256) relu_relax_kernel(const __grid_constant__ RelaxArgs args, int B) {
+  const RelaxSegment& g = args.seg[blockIdx.y];
+  const long long total = (long long)B * g.n;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const float lo = l[i], up = u[i];
+    const float lo = __ldg(g.l + i), up = __ldg(g.u + i);
     float au, bu, al;
     relax_one(lo, up, au, bu, al);
-    if (alpha != nullptr && lo < 0.f && up > 0.f) {
+    if (g.alpha != nullptr && lo < 0.f && up > 0.f) {
       // alpha_stride is n (per-domain rows, same flat index) or 0 (one shared row)
-      const float a = (alpha_stride != 0) ? alpha[i] : alpha[i % n];
+      const float a = __ldg(g.alpha + ((g.alpha_stride != 0) ? i : i % g.n));
       al = fminf(fmaxf(a, 0.f), 1.f);
     }
-    alpha_u[i] = au;
-    beta_u[i] = bu;
-    alpha_l[i] = al;
+    g.alpha_u[i] = au;
+    g.beta_u[i] = bu;
+    g.alpha_l[i] = al;
   }
 }
 
@@ -43,12 +50,24 @@ static int ew_grid(long long total, int threads) {
   return (int)(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
+int launch_relu_relax(const RelaxSegment* seg, int count, int B, cudaStream_t stream) {
+  for (int first = 0; first < count; first += RELAX_SEGMENTS) {
+    RelaxArgs args;
+    const int c = std::min(count - first, RELAX_SEGMENTS);
+    long long widest = 0;
+    for (int i = 0; i < c; ++i) {
+      args.seg[i] = seg[first + i];
+      widest = std::max(widest, (long long)B * args.seg[i].n);
+    }
+    relu_relax_kernel<<<dim3(ew_grid(widest, 256), c), 256, 0, stream>>>(args, B);
+    BF_CHECK_LAUNCH("relu_relax_kernel");
+  }
+  return BF_OK;
+}
 int launch_relu_relax(const float* l, const float* u, const float* alpha, int alpha_stride, float* alpha_u,
                       float* beta_u, float* alpha_l, int B, int n, cudaStream_t stream) {
-  const long long total = (long long)B * n;
-  relu_relax_kernel<<<ew_grid(total, 256), 256, 0, stream>>>(l, u, alpha, alpha_stride, alpha_u, beta_u, alpha_l, n, total);
-  BF_CHECK_LAUNCH("relu_relax_kernel");
-  return BF_OK;
+  const RelaxSegment seg{l, u, alpha, alpha_u, beta_u, alpha_l, alpha_stride, n};
+  return launch_relu_relax(&seg, 1, B, stream);
 }
 
 // ---- concretisation: one warp per coefficient row -----------------------------
@@ -740,38 +759,44 @@ int launch_beta_step(float* beta, float* m, float* v, float* gsum, const int8_t*
   return launch_optimiser_step(&g, 1, improve, sc, do_update, B, stream);
 }
 
-__global__ void fill_kernel(float* __restrict__ dst, float value, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = value;
-}
-
-// Widest unstable gap of one ReLU per domain: one warp per domain, first index wins ties; the caller
-// combines ReLUs in chain order with a strict comparison (earlier ReLUs win ties).
-__global__ void __launch_bounds__(256) branch_score_kernel(const float* __restrict__ l, const float* __restrict__ u, int n, int B,
-                                                           int relu_index, float* __restrict__ best_gap,
+// Widest unstable gap per domain over the ReLUs in chain order: one warp per domain; the first index of a tie and the earlier ReLU win.  `first`
+// is 0 where earlier launches have left the best of the ReLUs before these.
+constexpr int SCORE_SEGMENTS = 16;
+struct ScoreArgs {
+  const float *l[SCORE_SEGMENTS], *u[SCORE_SEGMENTS];
+  int n[SCORE_SEGMENTS];
+  int count, relu0;
+};
+__global__ void __launch_bounds__(256) branch_score_kernel(const __grid_constant__ ScoreArgs a, int B, int first, float* __restrict__ best_gap,
                                                            int* __restrict__ best_relu, int* __restrict__ best_idx) {
   const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (b >= B) return;
-  float gap = -INFINITY;
-  int idx = 0x7fffffff;
-  for (int j = lane; j < n; j += 32) {
-    const float lo = l[(size_t)b * n + j], up = u[(size_t)b * n + j];
-    if (lo < 0.f && up > 0.f) {
-      const float g = fmaxf(up - lo, 0.f);
-      if (g > gap) { gap = g; idx = j; }  // j increases: the first index of a tie is kept
+  float best = first ? -INFINITY : best_gap[b];
+  int relu = -1, at = -1;
+  for (int r = 0; r < a.count; ++r) {
+    const float *l = a.l[r] + (size_t)b * a.n[r], *u = a.u[r] + (size_t)b * a.n[r];
+    float gap = -INFINITY;
+    int idx = 0x7fffffff;
+    for (int j = lane; j < a.n[r]; j += 32) {
+      const float lo = __ldg(l + j), up = __ldg(u + j);
+      if (lo < 0.f && up > 0.f) {
+        const float g = fmaxf(up - lo, 0.f);
+        if (g > gap) { gap = g; idx = j; }  // j increases: the first index of a tie is kept
+      }
     }
-  }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float og = __shfl_xor_sync(0xffffffffu, gap, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-    if (og > gap || (og == gap && oi < idx)) { gap = og; idx = oi; }
+    for (int o = 16; o > 0; o >>= 1) {
+      const float og = __shfl_xor_sync(0xffffffffu, gap, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+      if (og > gap || (og == gap && oi < idx)) { gap = og; idx = oi; }
+    }
+    if (gap > best) { best = gap; relu = a.relu0 + r; at = idx; }
   }
-  if (lane == 0 && gap > best_gap[b]) {
-    best_gap[b] = gap;
-    best_relu[b] = relu_index;
-    best_idx[b] = idx;
+  if (lane == 0 && (first || relu >= 0)) {
+    best_gap[b] = best;
+    best_relu[b] = relu;
+    best_idx[b] = at;
   }
 }
 
@@ -781,21 +806,19 @@ extern "C" int bf_branch_scores(const float* const* pre_l, const float* const* p
                                 float* best_gap, int* best_relu, int* best_idx, int B, bf_stream_t stream_) {
   BF_REQUIRE(pre_l && pre_u && widths && best_gap && best_relu && best_idx, BF_E_INVALID, "bf_branch_scores: null argument");
   BF_REQUIRE(B > 0 && n_relu >= 0, BF_E_INVALID, "bf_branch_scores: bad sizes");
-  cudaStream_t stream = bf::as_stream(stream_);
-  // best_relu / best_idx start at -1 ("no unstable neuron"), best_gap at -inf
-  if (cudaMemsetAsync(best_relu, 0xff, sizeof(int) * (size_t)B, stream) != cudaSuccess ||
-      cudaMemsetAsync(best_idx, 0xff, sizeof(int) * (size_t)B, stream) != cudaSuccess) {
-    bf::set_error("bf_branch_scores: cudaMemsetAsync failed");
-    return BF_E_CUDA;
-  }
-  bf::fill_kernel<<<bf::ceil_div(B, 256), 256, 0, stream>>>(best_gap, -INFINITY, B);
-  BF_CHECK_LAUNCH("fill_kernel");
-  for (int r = 0; r < n_relu; ++r) {
-    BF_REQUIRE(pre_l[r] && pre_u[r] && widths[r] > 0, BF_E_INVALID, "bf_branch_scores: bad ReLU %d", r);
-    bf::branch_score_kernel<<<bf::ceil_div((long long)B * 32, 256), 256, 0, stream>>>(pre_l[r], pre_u[r], widths[r], B, r, best_gap,
-                                                                                  best_relu, best_idx);
+  for (int r = 0; r < n_relu; ++r) BF_REQUIRE(pre_l[r] && pre_u[r] && widths[r] > 0, BF_E_INVALID, "bf_branch_scores: bad ReLU %d", r);
+  int r0 = 0;
+  do {  // one launch also where there is no ReLU: "no unstable neuron" everywhere
+    bf::ScoreArgs a{};
+    a.relu0 = r0;
+    for (; r0 < n_relu && a.count < bf::SCORE_SEGMENTS; ++r0, ++a.count) {
+      a.l[a.count] = pre_l[r0];
+      a.u[a.count] = pre_u[r0];
+      a.n[a.count] = widths[r0];
+    }
+    bf::branch_score_kernel<<<bf::ceil_div((long long)B * 32, 256), 256, 0, bf::as_stream(stream_)>>>(a, B, a.relu0 == 0 ? 1 : 0, best_gap, best_relu, best_idx);
     BF_CHECK_LAUNCH("branch_score_kernel");
-  }
+  } while (r0 < n_relu);
   return BF_OK;
 }
 

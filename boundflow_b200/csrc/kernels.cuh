@@ -79,6 +79,13 @@ int launch_concretize_lp(const float* A, const float* center, const float* bias_
                          int S, int n0, cudaStream_t stream);
 
 // elementwise.cu
+struct RelaxSegment {  // one ReLU: bounds [B,n], alpha [B,n] (stride n), [n] (stride 0) or null -> slopes and intercept [B,n]
+  const float *l, *u, *alpha;
+  float *alpha_u, *beta_u, *alpha_l;
+  int alpha_stride, n;
+};
+constexpr int RELAX_SEGMENTS = 16;  // per launch
+int launch_relu_relax(const RelaxSegment* seg, int count, int B, cudaStream_t stream);
 int launch_relu_relax(const float* l, const float* u, const float* alpha, int alpha_stride, float* alpha_u,
                       float* beta_u, float* alpha_l, int B, int n, cudaStream_t stream);
 int launch_concretize(const float* A, const float* mid, const float* rad, const float* bias_in, float* out, int side,

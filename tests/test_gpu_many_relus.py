@@ -41,3 +41,29 @@ def test_more_tensors_than_one_launch(dev, with_beta):
             same = (got - want).abs() <= 1e-3
             assert same.float().mean() >= 0.9, (r, n)
             assert ((want - start).abs() > 0.05).any() == ((got - start).abs() > 0.05).any()
+
+
+@pytest.mark.parametrize("R,B", [(0, 3), (1, 1), (16, 9), (19, 300)])
+def test_branch_scores_of_many_relus(dev, R, B):
+    """Widest unstable gap: the first neuron of a tie and the earlier ReLU win, also over the edge of a launch (16 ReLUs); -inf and -1 without one."""
+    from boundflow_b200 import _lib
+
+    lib, g = _lib.load(), torch.Generator().manual_seed(R)
+    widths = [1 + (7 * r) % 45 for r in range(R)]
+    # bounds on a grid of quarters: many equal gaps; the last domain has no unstable neuron
+    pre = [(-torch.randint(0, 5, (B, n), generator=g) / 4, torch.randint(0, 5, (B, n), generator=g) / 4) for n in widths]
+    for l, _ in pre:
+        l[-1] = 0
+    want = (torch.full((B,), -float("inf")), torch.full((B,), -1), torch.full((B,), -1))
+    for r, (l, u) in enumerate(pre):
+        gap = torch.where((l < 0) & (u > 0), u - l, torch.tensor(-float("inf")))
+        best = gap.max(1).values
+        better = best > want[0]
+        for w, v in zip(want, (best, torch.full((B,), r), (gap == best[:, None]).int().argmax(1))):
+            w[better] = v[better].to(w.dtype)
+    l, u = [x[0].to(dev) for x in pre], [x[1].to(dev) for x in pre]
+    gap, relu, idx = torch.empty(B, device=dev), torch.empty(B, dtype=torch.int32, device=dev), torch.empty(B, dtype=torch.int32, device=dev)
+    arr = lambda ts: _lib.ptr_array(ts) if ts else _lib.ptr_array([gap])
+    _lib.check(lib.bf_branch_scores(arr(l), arr(u), _lib.int_array(widths or [1]), R, _lib.ptr(gap), _lib.ptr(relu), _lib.ptr(idx), B, None))
+    for got, w in zip((gap, relu, idx), want):
+        assert torch.equal(got.cpu(), w.to(got.dtype))
