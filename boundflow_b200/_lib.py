@@ -112,6 +112,11 @@ SIGNATURES = {
     "bf_shared_adam_step": (_i, [_p, _p, _p, _p, _p, _i, _p, _p, _p, _i, _f, _f, _i, _i, _i, _i, _p]),
     "bf_shared_beta_add": (_i, [_p, _p, _i, _p, _i, _i, _p]),
     "bf_chain_alpha_crown_shared_objective": (_i, [_p] * 8 + [_i, _f, _p, _p, _p, _i, _f, _i, _i, _f, _f, _f, _p, _sz, _i, _i, _p]),
+    "bf_relu_relax_many": (_i, [_p] * 8 + [_i, _i, _p]),
+    "bf_chain_query_workspace_bytes": (_sz, [_p, _i, _i, _i]),
+    "bf_chain_ibp_query": (_i, [_p, _p, _p, _f, _p, _p, _p, _sz, _i, _p]),
+    "bf_chain_crown_query": (_i, [_p, _p, _p, _f, _p, _p, _p, _p, _sz, _i, _i, _p]),
+    "bf_chain_crown_intermediate": (_i, [_p, _p, _p, _f] + [_p] * 6 + [_i, _p, _sz, _i, _i, _p]),
     "bf_branch_scores": (_i, [_p, _p, _p, _i, _p, _p, _p, _i, _p]),
     "bf_chain_alpha_grad": (_i, [_p, _p, _p, _p, _p, _p, _p, _i, _f, _p, _p, _i, _p, _sz, _i, _i, _p]),
     "bf_chain_alpha_shared_workspace_bytes": (_sz, [_p, _i, _i, _i]),

@@ -87,7 +87,8 @@ def _f32(t: torch.Tensor, device: torch.device) -> torch.Tensor:
 
 
 def _stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """Handle of the current stream (`torch.cuda.current_stream(device).cuda_stream` without the Stream object)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
 
 
 class _Workspace:
@@ -147,6 +148,24 @@ def _prepare_input(module: Any, input_spec: Any, batch: Optional[int] = None):
         mid = mid.expand(B, -1).contiguous()
         rad = rad.expand(B, -1).contiguous()
     return spec, chain, device, B, mid, rad, center.device
+
+
+def _plain_set(spec: Any):
+    """(lower, upper, 0.0) of a box or (centre, None, eps) of an L-inf ball whose tensors the library can read where they are (CUDA, fp32,
+    contiguous), else None: the input sets of the calls that bound a whole query in the library."""
+    pert = spec.perturbation
+    if hasattr(pert, "lower") and hasattr(pert, "upper"):
+        a, b, eps = pert.lower, pert.upper, 0.0
+    elif hasattr(pert, "eps") and (pert.norm() if hasattr(pert, "norm") else pert._normalize_p()) == "inf":
+        a, b, eps = spec.center, None, float(pert.eps)
+    else:
+        return None
+    for t in (a, b):
+        if t is not None and not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()):
+            return None
+    if b is not None and (b.shape != a.shape or b.device != a.device or a.shape != spec.center.shape or spec.center.device != a.device):
+        return None
+    return a, b, eps
 
 
 def _split_tensor(raw: Any, B: int, n: int, device: torch.device, name: str):
@@ -375,28 +394,33 @@ def _alpha_rows(raw: Any, B: int, n: int, device: torch.device, name: str) -> Tu
 
 def _relaxations(trace: ForwardTrace, relu_alpha: Optional[Mapping[str, torch.Tensor]], n_relu: int):
     chain, B, device = trace.chain, trace.B, trace.mid.device
-    au, bu, al = [], [], []
-    keep = []
-    for r in range(n_relu):
-        n = chain.relu_widths[r]
-        name = chain.relu_input_names[r]
-        a_u = torch.empty(B, n, dtype=torch.float32, device=device)
-        b_u = torch.empty_like(a_u)
-        a_l = torch.empty_like(a_u)
-        alpha, stride = (None, 0)
-        if relu_alpha is not None and name in relu_alpha:
-            alpha, stride = _alpha_rows(relu_alpha[name], B, n, device, name)
-            keep.append(alpha)
-        _lib.check(
-            chain.lib.bf_relu_relax(
-                _lib.ptr(trace.pre_l[r]), _lib.ptr(trace.pre_u[r]), _lib.ptr(alpha), stride,
-                _lib.ptr(a_u), _lib.ptr(b_u), _lib.ptr(a_l), B, n, _stream_ptr(device),
-            )
-        )
-        au.append(a_u)
-        bu.append(b_u)
-        al.append(a_l)
-    return au, bu, al, keep
+    widths = chain.relu_widths[:n_relu]
+    alpha: List[Optional[torch.Tensor]] = [None] * n_relu
+    strides = [0] * n_relu
+    if relu_alpha is not None:
+        for r, (n, name) in enumerate(zip(widths, chain.relu_input_names)):
+            if name in relu_alpha:
+                alpha[r], strides[r] = _alpha_rows(relu_alpha[name], B, n, device, name)
+    au, bu, al = relax_all(chain.lib, trace.pre_l[:n_relu], trace.pre_u[:n_relu], alpha, strides, widths, B, device)
+    return au, bu, al, alpha
+
+
+def relax_all(lib, pre_l, pre_u, alpha, strides, widths, B: int, device: torch.device):
+    """Slopes and intercepts (upper slope, upper intercept, lower slope) of several ReLUs in one launch, [B, n_r] each."""
+    pitch = [(B * n + 63) // 64 * 64 for n in widths]  # every table starts on a 256-byte boundary
+    slab = torch.empty(3 * sum(pitch), dtype=torch.float32, device=device)
+    tables, at = [], 0
+    for _ in range(3):
+        row = []
+        for n, p in zip(widths, pitch):
+            row.append(slab.as_strided((B, n), (n, 1), at))
+            at += p
+        tables.append(row)
+    au, bu, al = tables
+    R = len(widths)
+    _lib.check(lib.bf_relu_relax_many(_lib.ptr_array(pre_l), _lib.ptr_array(pre_u), _lib.ptr_array(alpha), _lib.int_array(strides), _lib.ptr_array(au),
+                                      _lib.ptr_array(bu), _lib.ptr_array(al), _lib.int_array(widths), R, B, _stream_ptr(device)))
+    return au, bu, al
 
 
 def crown_from_trace(
@@ -509,12 +533,45 @@ def run_crown_ibp_mlp(
         return run_crown_ibp_dag(module, input_spec, linear_spec_C=linear_spec_C, output_value=output_value, relu_alpha=relu_alpha,
                                  relu_pre_add_coeff_l=relu_pre_add_coeff_l, relu_pre_add_coeff_u=relu_pre_add_coeff_u,
                                  relu_split_state=relu_split_state)
+    spec = normalize_input_spec(input_spec)
+    if not (relu_split_state or relu_alpha or relu_pre_add_coeff_l or relu_pre_add_coeff_u):
+        plain = _plain_set(spec)
+        if plain is not None:
+            center = spec.center
+            chain = compile_chain(module, center.shape[1:], center.device)
+            if output_value is None or output_value == chain.output_name:
+                return _crown_query(chain, plain, linear_spec_C, center.device, int(center.shape[0]))
     trace = ibp_trace(module, input_spec, relu_split_state=relu_split_state)
     _raise_if_infeasible(trace, "relu split")
     lo, up = crown_from_trace(trace, linear_spec_C, output_value=output_value, relu_alpha=relu_alpha, relu_pre_add_coeff_l=relu_pre_add_coeff_l,
                               relu_pre_add_coeff_u=relu_pre_add_coeff_u)
-    dev = normalize_input_spec(input_spec).center.device
+    dev = spec.center.device
     return IntervalState(lower=lo.to(dev), upper=up.to(dev))
+
+
+def _crown_query(chain: CudaChain, plain, linear_spec_C: Optional[torch.Tensor], device: torch.device, B: int) -> IntervalState:
+    """Both CROWN bounds of the chain's output in one call of the library: what lies between stays in one workspace."""
+    C = _expand_spec(linear_spec_C, B, chain.output_width, device)
+    S = int(C.shape[1])
+    lower, upper = torch.empty(B, S, dtype=torch.float32, device=device), torch.empty(B, S, dtype=torch.float32, device=device)
+    nbytes = chain.lib.bf_chain_query_workspace_bytes(chain.handle, B, S, 0)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    a, b, eps = plain
+    _lib.check(chain.lib.bf_chain_crown_query(chain.handle, a.data_ptr(), _lib.ptr(b), eps, C.data_ptr(), lower.data_ptr(), upper.data_ptr(), ws.data_ptr(),
+                                              nbytes, B, S, _stream_ptr(device)))
+    return IntervalState(lower=lower, upper=upper)
+
+
+def ibp_query(chain: CudaChain, plain, device: torch.device, B: int) -> IntervalState:
+    """Interval bounds of the chain's output in one call of the library."""
+    shape = (B,) + tuple(chain.output_shape)
+    lower, upper = torch.empty(shape, dtype=torch.float32, device=device), torch.empty(shape, dtype=torch.float32, device=device)
+    nbytes = chain.lib.bf_chain_query_workspace_bytes(chain.handle, B, 0, 0)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    a, b, eps = plain
+    _lib.check(chain.lib.bf_chain_ibp_query(chain.handle, a.data_ptr(), _lib.ptr(b), eps, lower.data_ptr(), upper.data_ptr(), ws.data_ptr(), nbytes, B,
+                                            _stream_ptr(device)))
+    return IntervalState(lower=lower, upper=upper)
 
 
 def run_crown_ibp_mlp_from_forward_trace(
@@ -1215,6 +1272,10 @@ def run_crown_intermediate_mlp(
     current bounds, and re-propagate IBP under those constraints; then bound the
     spec rows.  Restates runtime/native_intermediate_refinement.py:923-988 on
     the device.  Returns (final bounds, refined pre-activation bounds)."""
+    spec = normalize_input_spec(input_spec)
+    plain = _plain_set(spec)
+    if plain is not None and int(chunk_rows) > 0:
+        return _crown_intermediate_query(module, spec, plain, linear_spec_C, int(chunk_rows))
     trace = ibp_trace(module, input_spec)
     chain, B, device = trace.chain, trace.B, trace.mid.device
     names = chain.relu_input_names
@@ -1244,6 +1305,32 @@ def run_crown_intermediate_mlp(
     dev = normalize_input_spec(input_spec).center.device
     pre = {nm: IntervalState(lower=trace.pre_l[k].reshape((B,) + tuple(chain.relu_shapes[k])).to(dev), upper=trace.pre_u[k].reshape((B,) + tuple(chain.relu_shapes[k])).to(dev)) for k, nm in enumerate(names)}
     return IntervalState(lower=lo.to(dev), upper=up.to(dev)), pre
+
+
+def _crown_intermediate_query(module: Any, spec: Any, plain, linear_spec_C: Optional[torch.Tensor], chunk_rows: int):
+    """`run_crown_intermediate_mlp` in one call of the library."""
+    center = spec.center
+    device, B = center.device, int(center.shape[0])
+    chain = compile_chain(module, center.shape[1:], device)
+    C = _expand_spec(linear_spec_C, B, chain.output_width, device)
+    S, R = int(C.shape[1]), len(chain.relu_widths)
+    lower, upper = torch.empty(B, S, dtype=torch.float32, device=device), torch.empty(B, S, dtype=torch.float32, device=device)
+    pre = {name: IntervalState(lower=torch.empty((B,) + tuple(s), dtype=torch.float32, device=device), upper=torch.empty((B,) + tuple(s), dtype=torch.float32, device=device))
+           for name, s in zip(chain.relu_input_names, chain.relu_shapes)}
+    infeasible = torch.empty(max(R, 1), B, dtype=torch.int32, device=device)
+    chunk_rows = min(chunk_rows, max(chain.relu_widths[1:], default=1))  # the workspace holds a chunk
+    nbytes = chain.lib.bf_chain_query_workspace_bytes(chain.handle, B, S, chunk_rows)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    a, b, eps = plain
+    states = [pre[n] for n in chain.relu_input_names]
+    _lib.check(chain.lib.bf_chain_crown_intermediate(
+        chain.handle, a.data_ptr(), _lib.ptr(b), eps, C.data_ptr(), lower.data_ptr(), upper.data_ptr(), _lib.ptr_array([t.lower for t in states]),
+        _lib.ptr_array([t.upper for t in states]), infeasible.data_ptr(), chunk_rows, ws.data_ptr(), nbytes, B, S, _stream_ptr(device)))
+    if R > 1 and bool(infeasible.any().item()):
+        step = infeasible[int(torch.nonzero(infeasible.any(dim=1))[0])]  # the first step that found a contradiction
+        bad = torch.nonzero(step).flatten().tolist()
+        raise ValueError(f"infeasible ReLU pre-activation intersection: lower>upper after applying split/constraint (domains {bad[:8]}{'...' if len(bad) > 8 else ''})")
+    return IntervalState(lower=lower, upper=upper), pre
 
 
 @dataclass

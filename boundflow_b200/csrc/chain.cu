@@ -397,13 +397,12 @@ extern "C" int bf_chain_tc_status(const bf_chain* chain, int* status_out) {
 // ---------------------------------------------------------------------------
 // IBP trace
 // ---------------------------------------------------------------------------
-extern "C" int bf_chain_ibp(const bf_chain* chain, const float* in_a, const float* in_b, int in_mode,
+// out_l / out_u null: only the pre-activation bounds are wanted, the last affine layer is left out
+static int ibp_sweep(const bf_chain* chain, const float* in_a, const float* in_b, int in_mode,
                             const int8_t* const* splits, const int* split_strides, const float* const* cons_l,
                             const float* const* cons_u, float* const* pre_l, float* const* pre_u, float* out_l,
                             float* out_u, int* infeasible, float* scratch, size_t scratch_bytes, int B,
                             bf_stream_t stream_) {
-  BF_REQUIRE(chain && in_a && in_b && out_l && out_u, BF_E_INVALID, "bf_chain_ibp: null argument");
-  BF_REQUIRE(B > 0, BF_E_INVALID, "bf_chain_ibp: B must be positive");
   cudaStream_t stream = bf::as_stream(stream_);
   const int nl = (int)chain->layers.size();
   const size_t need = 4 * bf::align_up((size_t)B * chain->max_width * sizeof(float));
@@ -427,6 +426,7 @@ extern "C" int bf_chain_ibp(const bf_chain* chain, const float* in_a, const floa
       relu_pending = 1;
       continue;
     }
+    if (i == last_affine && !out_l) break;
     // affine layer: where does its output go?
     int j = i + 1;
     while (j < nl && chain->layers[j].op == BF_OP_FLATTEN) ++j;
@@ -476,6 +476,17 @@ extern "C" int bf_chain_ibp(const bf_chain* chain, const float* in_a, const floa
     relu_pending = 0;
   }
   return BF_OK;
+}
+
+extern "C" int bf_chain_ibp(const bf_chain* chain, const float* in_a, const float* in_b, int in_mode,
+                            const int8_t* const* splits, const int* split_strides, const float* const* cons_l,
+                            const float* const* cons_u, float* const* pre_l, float* const* pre_u, float* out_l,
+                            float* out_u, int* infeasible, float* scratch, size_t scratch_bytes, int B,
+                            bf_stream_t stream) {
+  BF_REQUIRE(chain && in_a && in_b && out_l && out_u, BF_E_INVALID, "bf_chain_ibp: null argument");
+  BF_REQUIRE(B > 0, BF_E_INVALID, "bf_chain_ibp: B must be positive");
+  return ibp_sweep(chain, in_a, in_b, in_mode, splits, split_strides, cons_l, cons_u, pre_l, pre_u, out_l, out_u, infeasible, scratch,
+                   scratch_bytes, B, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -695,3 +706,163 @@ extern "C" int bf_chain_crown_onehot(const bf_chain* chain, int upto_layer, int 
                      workspace, workspace_bytes, B, S, stream);
 }
 
+
+// ---------------------------------------------------------------------------
+// Whole queries in one call: input set, IBP, relaxations and sweeps in one caller-owned workspace
+// ---------------------------------------------------------------------------
+namespace bf {
+
+struct QueryWs {
+  float *mid, *rad, *scratch;
+  size_t scratch_bytes;
+  std::vector<float*> pre_l, pre_u, au, bu, al;
+  float *chunk_l, *chunk_u;                         // bounds of a chunk of neurons
+  std::vector<float*> alt_l, alt_u, new_l, new_u;   // intermediate queries: the other set of bounds, the sweeps' bounds
+  char* sweep;
+  size_t sweep_bytes, bytes;
+};
+
+// S: spec rows (0: IBP only); chunk > 0: neuron bounds too, at most `chunk` rows of a value per sweep
+static size_t query_layout(const bf_chain* c, int B, int S, int chunk, void* base, QueryWs* out) {
+  Carver cv(base);
+  QueryWs w{};
+  w.mid = cv.take<float>((size_t)B * c->n0);
+  w.rad = cv.take<float>((size_t)B * c->n0);
+  w.scratch_bytes = 4 * align_up((size_t)B * c->max_width * sizeof(float));
+  w.scratch = cv.take<float>(w.scratch_bytes / sizeof(float));
+  const int nl = (int)c->layers.size();
+  w.sweep_bytes = S > 0 ? crown_ws_layout(c, B, S, nl, nullptr, nullptr) : 0;
+  for (size_t r = 0; r < c->relu_layers.size(); ++r) {
+    const int n = c->layers[c->relu_layers[r]].n_in;
+    w.pre_l.push_back(cv.take<float>((size_t)B * n));
+    w.pre_u.push_back(cv.take<float>((size_t)B * n));
+    if (S > 0) {
+      w.au.push_back(cv.take<float>((size_t)B * n));
+      w.bu.push_back(cv.take<float>((size_t)B * n));
+      w.al.push_back(cv.take<float>((size_t)B * n));
+    }
+    if (chunk > 0) {
+      w.alt_l.push_back(cv.take<float>((size_t)B * n));
+      w.alt_u.push_back(cv.take<float>((size_t)B * n));
+      w.new_l.push_back(cv.take<float>((size_t)B * n));
+      w.new_u.push_back(cv.take<float>((size_t)B * n));
+      w.sweep_bytes = std::max(w.sweep_bytes, crown_ws_layout(c, B, std::min(chunk, n), c->relu_layers[r], nullptr, nullptr));
+    }
+  }
+  if (chunk > 0) {
+    w.chunk_l = cv.take<float>((size_t)B * chunk);
+    w.chunk_u = cv.take<float>((size_t)B * chunk);
+  }
+  w.sweep = cv.take<char>(w.sweep_bytes);
+  w.bytes = cv.off;
+  if (out) *out = w;
+  return cv.off;
+}
+
+// mid, rad of the input set: a box [a, b], or (b null) an L-inf ball of radius eps around a, whose centre is read in place
+static int query_input(const float* a, const float* b, float eps, QueryWs& w, size_t n, cudaStream_t stream) {
+  if (!b) w.mid = const_cast<float*>(a);
+  return launch_input_set(a, b, eps, w.mid, w.rad, (long long)n, stream);
+}
+
+static int query_relax(const bf_chain* c, const QueryWs& w, float* const* pre_l, float* const* pre_u, int n_relu, int B, cudaStream_t stream) {
+  std::vector<RelaxSegment> seg;
+  for (int r = 0; r < n_relu; ++r) {
+    const int n = c->layers[c->relu_layers[r]].n_in;
+    seg.push_back({pre_l[r], pre_u[r], nullptr, w.au[r], w.bu[r], w.al[r], 0, n});
+  }
+  return launch_relu_relax(seg.data(), n_relu, B, stream);
+}
+
+}  // namespace bf
+
+extern "C" size_t bf_chain_query_workspace_bytes(const bf_chain* chain, int B, int S, int chunk_rows) {
+  if (!chain || B <= 0 || S < 0 || chunk_rows < 0) return 0;
+  return bf::query_layout(chain, B, S, chunk_rows, nullptr, nullptr);
+}
+
+extern "C" int bf_chain_ibp_query(const bf_chain* chain, const float* in_a, const float* in_b, float eps, float* out_l, float* out_u,
+                                  void* workspace, size_t workspace_bytes, int B, bf_stream_t stream) {
+  BF_REQUIRE(chain && in_a && out_l && out_u && workspace, BF_E_INVALID, "bf_chain_ibp_query: null argument");
+  BF_REQUIRE(B > 0, BF_E_INVALID, "bf_chain_ibp_query: B must be positive");
+  bf::QueryWs w;
+  const size_t need = bf::query_layout(chain, B, 0, 0, workspace, &w);
+  BF_REQUIRE(workspace_bytes >= need, BF_E_WORKSPACE, "bf_chain_ibp_query: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
+  int rc = bf::query_input(in_a, in_b, eps, w, (size_t)B * chain->n0, bf::as_stream(stream));
+  if (rc != BF_OK) return rc;
+  return ibp_sweep(chain, w.mid, w.rad, BF_IN_MID_RAD, nullptr, nullptr, nullptr, nullptr, w.pre_l.data(), w.pre_u.data(), out_l, out_u, nullptr,
+                   w.scratch, w.scratch_bytes, B, stream);
+}
+
+extern "C" int bf_chain_crown_query(const bf_chain* chain, const float* in_a, const float* in_b, float eps, const float* C, float* out_l,
+                                    float* out_u, void* workspace, size_t workspace_bytes, int B, int S, bf_stream_t stream) {
+  BF_REQUIRE(chain && in_a && C && out_l && out_u && workspace, BF_E_INVALID, "bf_chain_crown_query: null argument");
+  BF_REQUIRE(B > 0 && S > 0 && (long long)B * S < 2147483647LL, BF_E_INVALID, "bf_chain_crown_query: bad B/S");
+  bf::QueryWs w;
+  const size_t need = bf::query_layout(chain, B, S, 0, workspace, &w);
+  BF_REQUIRE(workspace_bytes >= need, BF_E_WORKSPACE, "bf_chain_crown_query: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
+  int rc = bf::query_input(in_a, in_b, eps, w, (size_t)B * chain->n0, bf::as_stream(stream));
+  if (rc == BF_OK)
+    rc = ibp_sweep(chain, w.mid, w.rad, BF_IN_MID_RAD, nullptr, nullptr, nullptr, nullptr, w.pre_l.data(), w.pre_u.data(), nullptr, nullptr,
+                   nullptr, w.scratch, w.scratch_bytes, B, stream);
+  if (rc == BF_OK) rc = bf::query_relax(chain, w, w.pre_l.data(), w.pre_u.data(), (int)chain->relu_layers.size(), B, bf::as_stream(stream));
+  for (int side = 0; side < 2 && rc == BF_OK; ++side)
+    rc = crown_sweep(chain, 0, side, C, -1, w.au.data(), w.bu.data(), w.al.data(), nullptr, w.mid, w.rad, BF_NORM_BOX, 0.f,
+                     side == BF_SIDE_LOWER ? out_l : out_u, w.sweep, w.sweep_bytes, B, S, stream);
+  return rc;
+}
+
+extern "C" int bf_chain_crown_intermediate(const bf_chain* chain, const float* in_a, const float* in_b, float eps, const float* C, float* out_l,
+                                           float* out_u, float* const* pre_l, float* const* pre_u, int* infeasible, int chunk_rows, void* workspace,
+                                           size_t workspace_bytes, int B, int S, bf_stream_t stream_) {
+  BF_REQUIRE(chain && in_a && C && out_l && out_u && pre_l && pre_u && infeasible && workspace, BF_E_INVALID, "bf_chain_crown_intermediate: null argument");
+  BF_REQUIRE(B > 0 && S > 0 && chunk_rows > 0 && (long long)B * S < 2147483647LL && (long long)B * chunk_rows < 2147483647LL, BF_E_INVALID,
+             "bf_chain_crown_intermediate: bad sizes");
+  bf::QueryWs w;
+  const size_t need = bf::query_layout(chain, B, S, chunk_rows, workspace, &w);
+  BF_REQUIRE(workspace_bytes >= need, BF_E_WORKSPACE, "bf_chain_crown_intermediate: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
+  cudaStream_t stream = bf::as_stream(stream_);
+  const int R = (int)chain->relu_layers.size();
+  if (cudaMemsetAsync(infeasible, 0, sizeof(int) * (size_t)B * std::max(R, 1), stream) != cudaSuccess) {
+    bf::set_error("bf_chain_crown_intermediate: cudaMemsetAsync failed");
+    return BF_E_CUDA;
+  }
+  // every interval pass reads the bounds of the one before as constraints: two sets by turns, the last pass into the caller's
+  std::vector<float*> set_l[2], set_u[2];
+  set_l[0].assign(pre_l, pre_l + R); set_u[0].assign(pre_u, pre_u + R);
+  set_l[1] = w.alt_l; set_u[1] = w.alt_u;
+  int cur = R > 0 ? (R - 1) & 1 : 0;
+  int rc = bf::query_input(in_a, in_b, eps, w, (size_t)B * chain->n0, stream);
+  if (rc != BF_OK) return rc;
+  rc = ibp_sweep(chain, w.mid, w.rad, BF_IN_MID_RAD, nullptr, nullptr, nullptr, nullptr, set_l[cur].data(), set_u[cur].data(), nullptr, nullptr,
+                 nullptr, w.scratch, w.scratch_bytes, B, stream_);
+  if (rc != BF_OK) return rc;
+  for (int r = 1; r < R; ++r) {  // the first ReLU's CROWN bounds are its interval bounds
+    const int n = chain->layers[chain->relu_layers[r]].n_in, upto = chain->relu_layers[r];
+    if ((rc = bf::query_relax(chain, w, set_l[cur].data(), set_u[cur].data(), r, B, stream)) != BF_OK) return rc;
+    for (int s = 0; s < n; s += chunk_rows) {
+      const int cnt = std::min(chunk_rows, n - s);
+      for (int side = 0; side < 2; ++side) {
+        float* all = side == BF_SIDE_LOWER ? w.new_l[r] : w.new_u[r];
+        float* to = cnt == n ? all : (side == BF_SIDE_LOWER ? w.chunk_l : w.chunk_u);
+        rc = crown_sweep(chain, upto, side, nullptr, s, w.au.data(), w.bu.data(), w.al.data(), nullptr, w.mid, w.rad, BF_NORM_BOX, 0.f, to, w.sweep,
+                         w.sweep_bytes, B, cnt, stream_);
+        if (rc != BF_OK) return rc;
+      }
+      if (cnt < n && (rc = bf::launch_place_columns(w.chunk_l, w.chunk_u, w.new_l[r], w.new_u[r], B, cnt, n, s, stream)) != BF_OK) return rc;
+    }
+    // interval pass constrained by the new bounds of this ReLU and the current ones of the others
+    std::vector<const float*> cons_l(set_l[cur].begin(), set_l[cur].end()), cons_u(set_u[cur].begin(), set_u[cur].end());
+    cons_l[r] = w.new_l[r];
+    cons_u[r] = w.new_u[r];
+    cur ^= 1;
+    rc = ibp_sweep(chain, w.mid, w.rad, BF_IN_MID_RAD, nullptr, nullptr, cons_l.data(), cons_u.data(), set_l[cur].data(), set_u[cur].data(), nullptr,
+                   nullptr, infeasible + (size_t)r * B, w.scratch, w.scratch_bytes, B, stream_);
+    if (rc != BF_OK) return rc;
+  }
+  if ((rc = bf::query_relax(chain, w, set_l[cur].data(), set_u[cur].data(), R, B, stream)) != BF_OK) return rc;
+  for (int side = 0; side < 2 && rc == BF_OK; ++side)
+    rc = crown_sweep(chain, 0, side, C, -1, w.au.data(), w.bu.data(), w.al.data(), nullptr, w.mid, w.rad, BF_NORM_BOX, 0.f,
+                     side == BF_SIDE_LOWER ? out_l : out_u, w.sweep, w.sweep_bytes, B, S, stream_);
+  return rc;
+}

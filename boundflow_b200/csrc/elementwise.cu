@@ -70,6 +70,39 @@ int launch_relu_relax(const float* l, const float* u, const float* alpha, int al
   return launch_relu_relax(&seg, 1, B, stream);
 }
 
+__global__ void __launch_bounds__(256) input_set_kernel(const float* __restrict__ a, const float* __restrict__ b, float eps, float* __restrict__ mid,
+                                                        float* __restrict__ rad, long long n) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    if (b) {
+      const float lo = a[i], up = b[i];
+      mid[i] = (lo + up) / 2.f;
+      rad[i] = (up - lo) / 2.f;
+    } else {
+      rad[i] = eps;
+    }
+  }
+}
+int launch_input_set(const float* a, const float* b, float eps, float* mid, float* rad, long long n, cudaStream_t stream) {
+  input_set_kernel<<<ew_grid(n, 256), 256, 0, stream>>>(a, b, eps, mid, rad, n);
+  BF_CHECK_LAUNCH("input_set_kernel");
+  return BF_OK;
+}
+
+__global__ void __launch_bounds__(256) place_columns_kernel(const float* __restrict__ l, const float* __restrict__ u, float* __restrict__ to_l,
+                                                            float* __restrict__ to_u, int cnt, int n, int at, long long total) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const long long b = i / cnt, o = b * n + at + (i - b * cnt);
+    to_l[o] = l[i];
+    to_u[o] = u[i];
+  }
+}
+int launch_place_columns(const float* l, const float* u, float* to_l, float* to_u, int B, int cnt, int n, int at, cudaStream_t stream) {
+  const long long total = (long long)B * cnt;
+  place_columns_kernel<<<ew_grid(total, 256), 256, 0, stream>>>(l, u, to_l, to_u, cnt, n, at, total);
+  BF_CHECK_LAUNCH("place_columns_kernel");
+  return BF_OK;
+}
+
 // ---- concretisation: one warp per coefficient row -----------------------------
 __global__ void __launch_bounds__(256) concretize_kernel(const float* A, const float* mid, const float* rad, const float* bias_in, float* out,
                                                          float sgn, int M, int S, int n0, int vec) {
@@ -707,6 +740,22 @@ extern "C" int bf_accumulate(float* dst, const float* src, long long n, bf_strea
   bf::accumulate_kernel<<<bf::ew_grid(n, 256), 256, 0, bf::as_stream(stream)>>>(dst, src, n);
   BF_CHECK_LAUNCH("accumulate_kernel");
   return BF_OK;
+}
+
+extern "C" int bf_relu_relax_many(const float* const* l, const float* const* u, const float* const* alpha, const int* alpha_strides,
+                                  float* const* alpha_u, float* const* beta_u, float* const* alpha_l, const int* widths, int n_relu, int B,
+                                  bf_stream_t stream) {
+  BF_REQUIRE(l && u && alpha_u && beta_u && alpha_l && widths, BF_E_INVALID, "bf_relu_relax_many: null argument");
+  BF_REQUIRE(B > 0 && n_relu >= 0, BF_E_INVALID, "bf_relu_relax_many: bad sizes");
+  std::vector<bf::RelaxSegment> seg;
+  for (int r = 0; r < n_relu; ++r) {
+    const float* a = alpha ? alpha[r] : nullptr;
+    const int stride = a && alpha_strides ? alpha_strides[r] : 0;
+    BF_REQUIRE(l[r] && u[r] && alpha_u[r] && beta_u[r] && alpha_l[r] && widths[r] > 0 && (stride == 0 || stride == widths[r]), BF_E_INVALID,
+               "bf_relu_relax_many: bad ReLU %d", r);
+    seg.push_back({l[r], u[r], a, alpha_u[r], beta_u[r], alpha_l[r], stride, widths[r]});
+  }
+  return bf::launch_relu_relax(seg.data(), n_relu, B, bf::as_stream(stream));
 }
 
 extern "C" int bf_relu_relax(const float* l, const float* u, const float* alpha, int alpha_stride, float* alpha_u,

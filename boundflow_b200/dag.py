@@ -22,7 +22,7 @@ from typing import Any, Dict, List, Mapping, Optional, Tuple
 import torch
 
 from . import _lib
-from .crown import _alpha_rows, _cuda_device, _f32, _split_tensor, _stream_ptr
+from .crown import _alpha_rows, _cuda_device, _f32, _split_tensor, _stream_ptr, relax_all
 from .ir import IntervalState, input_mid_rad, lp_ball_of, normalize_input_spec
 from .network import dense_conv_weight
 
@@ -59,6 +59,7 @@ class DagTrace:
     norm_p: int = 0     # _lib.NORM_BOX, or 1 / 2 for an L1 / L2 ball (then mid = centre and rad = eps, the bounding box)
     eps: float = 0.0
     clamped: bool = False  # a split was applied; without one no domain can be infeasible
+    params: Dict[str, torch.Tensor] = field(default_factory=dict)  # the device parameters this pass has used
 
 
 def _params(module: Any, device: torch.device) -> Dict[str, torch.Tensor]:
@@ -95,6 +96,7 @@ def forward_ibp_dag(module: Any, input_spec: Any, relu_split_state: Optional[Map
     params = _params(module, device)
     B = int(spec.center.shape[0])
     tr = DagTrace(B=B, input_name=spec.value_name)
+    tr.params = params
     tr.infeasible = torch.zeros(B, dtype=torch.int32, device=device)
     if ball is not None:
         # L1 / L2 ball (LpBallPerturbation, perturbation.py:73-222): a Linear op on the input value uses the dual row norms,
@@ -237,18 +239,18 @@ def _relax(lib, tr: DagTrace, relu_alpha: Optional[Mapping[str, torch.Tensor]], 
     """Slopes / intercepts of every ReLU from its (split) pre-activation bounds; alpha overrides the lower slope of
     unstable neurons (crown_ibp.py:1176-1208)."""
     device, B = tr.mid.device, tr.B
-    relax = {}
-    for x in tr.relu_inputs:
-        if x in relax:
-            continue
-        n = _numel(tr.shape[x])
-        au, bu, al = (torch.empty(B, n, device=device) for _ in range(3))
-        a, stride = (None, 0)
-        if relu_alpha is not None and x in relu_alpha and relu_alpha[x] is not None:
-            a, stride = _alpha_rows(relu_alpha[x], B, n, device, x)
-        _lib.check(lib.bf_relu_relax(_lib.ptr(tr.pre_l[x]), _lib.ptr(tr.pre_u[x]), _lib.ptr(a), stride, _lib.ptr(au), _lib.ptr(bu), _lib.ptr(al), B, n, s))
-        relax[x] = (au, bu, al)
-    return relax
+    names = list(dict.fromkeys(tr.relu_inputs))
+    widths = [_numel(tr.shape[x]) for x in names]
+    alpha: List[Optional[torch.Tensor]] = [None] * len(names)
+    strides = [0] * len(names)
+    if relu_alpha is not None:
+        for r, (x, n) in enumerate(zip(names, widths)):
+            if x in relu_alpha and relu_alpha[x] is not None:
+                alpha[r], strides[r] = _alpha_rows(relu_alpha[x], B, n, device, x)
+    if not names:
+        return {}
+    au, bu, al = relax_all(lib, [tr.pre_l[x] for x in names], [tr.pre_u[x] for x in names], alpha, strides, widths, B, device)
+    return dict(zip(names, zip(au, bu, al)))
 
 
 def _sweep(lib, module: Any, tr: DagTrace, params: Dict[str, torch.Tensor], relax, C: torch.Tensor, side: int, output_value: str, *,
@@ -265,6 +267,13 @@ def _sweep(lib, module: Any, tr: DagTrace, params: Dict[str, torch.Tensor], rela
     neurons = len(tr.shape[output_value]) == 3 and (output_value not in task.output_values or S == _numel(tr.shape[output_value]))
     conv_bwd = lib.bf_crown_relu_conv2d_bwd_fp32 if neurons else lib.bf_crown_relu_conv2d_bwd
     adj: Dict[str, _State] = {output_value: _State(C.clone(), torch.zeros(B, S, device=device))}
+    scratch = torch.empty(16, dtype=torch.uint8, device=device)  # of one step at a time, on this stream
+
+    def need(nb: int) -> torch.Tensor:
+        nonlocal scratch
+        if scratch.numel() < nb:
+            scratch = torch.empty(nb, dtype=torch.uint8, device=device)
+        return scratch
 
     def push(name: str, A: torch.Tensor, d: torch.Tensor) -> None:
         cur = adj.get(name)
@@ -297,21 +306,18 @@ def _sweep(lib, module: Any, tr: DagTrace, params: Dict[str, torch.Tensor], rela
             kh, kw = int(W.shape[2]), int(W.shape[3])
             sth, pdh = _pair(op.attrs.get("stride", 1)), _pair(op.attrs.get("padding", 0))
             Ap = torch.empty(B, S, Ci * Hi * Wi, device=device)
-            nb = int(lib.bf_crown_relu_conv2d_bwd_scratch_bytes(B, S, Co, Ho, Wo))
-            scratch = torch.empty(max(nb, 16), dtype=torch.uint8, device=device)
+            buf = need(int(lib.bf_crown_relu_conv2d_bwd_scratch_bytes(B, S, Co, Ho, Wo)))
             _lib.check(conv_bwd(_lib.ptr(st.A), side, None, None, None, None, _lib.ptr(W), _lib.ptr(b), _lib.ptr(Ap), _lib.ptr(st.d), 1,
-                                _lib.ptr(scratch), scratch.numel(), B, S, Ci, Hi, Wi, Co, Ho, Wo, kh, kw, sth[0], sth[1], pdh[0], pdh[1], s))
+                                _lib.ptr(buf), buf.numel(), B, S, Ci, Hi, Wi, Co, Ho, Wo, kh, kw, sth[0], sth[1], pdh[0], pdh[1], s))
             push(op.inputs[0], Ap, st.d)
         elif t == "relu":
             x = op.inputs[0]
             n = _numel(tr.shape[x])
             au, bu, al = relax[x]
-            zb = torch.zeros(B, n, device=device)
-            nb = int(lib.bf_crown_relu_bwd_scratch_bytes(B, S, n))
-            scratch = torch.empty(max(nb, 16), dtype=torch.uint8, device=device)
+            buf = need(int(lib.bf_crown_relu_bwd_scratch_bytes(B, S, n)))
             Ap = torch.empty_like(st.A)
-            _lib.check(lib.bf_crown_relu_bwd(_lib.ptr(st.A), side, _lib.ptr(au), _lib.ptr(al), _lib.ptr(bu), _lib.ptr(zb), _lib.ptr(Ap),
-                                             _lib.ptr(st.d), 1, _lib.ptr(scratch), scratch.numel(), B, S, n, s))
+            _lib.check(lib.bf_crown_relu_bwd(_lib.ptr(st.A), side, _lib.ptr(au), _lib.ptr(al), _lib.ptr(bu), None, _lib.ptr(Ap),
+                                             _lib.ptr(st.d), 1, _lib.ptr(buf), buf.numel(), B, S, n, s))
             if ahat is not None:
                 ahat[x] = st.A  # left untouched by the call above
             if add_l is not None and add_l.get(x) is not None:
@@ -378,7 +384,7 @@ def crown_dag(module: Any, input_spec: Any, linear_spec_C: Optional[torch.Tensor
     if tr.clamped and int(tr.infeasible.sum()) != 0:
         raise ValueError("infeasible relu split: lower > upper")
     device, B = tr.mid.device, tr.B
-    params = _params(module, device)
+    params = tr.params if trace is None else _params(module, device)  # a caller's trace may be older than the module's parameters
     output_value = _output_value(module, tr, output_value)
     C = _spec_rows(linear_spec_C, B, _numel(tr.shape[output_value]), device)
     s = _stream_ptr(device)

@@ -18,9 +18,9 @@ from typing import Any, Dict, Optional
 import torch
 
 from . import _lib
-from .crown import _cuda_device, _f32, _stream_ptr, ibp_trace, needs_graph_path
+from .crown import _cuda_device, _f32, _plain_set, _stream_ptr, ibp_query, ibp_trace, needs_graph_path
 from .ir import IntervalState, input_mid_rad, lp_ball_of, normalize_input_spec
-from .network import _pair, dense_conv_weight
+from .network import _pair, compile_chain, dense_conv_weight
 
 
 def _is_interval_kind(kind: Any) -> bool:
@@ -168,6 +168,11 @@ class CudaTaskExecutor:
             from .dag import run_ibp_dag
 
             return run_ibp_dag(module, spec, output_value=output_value)
+        plain = _plain_set(spec)
+        if plain is not None:
+            chain = compile_chain(module, spec.center.shape[1:], spec.center.device)
+            if output_value == chain.output_name:
+                return ibp_query(chain, plain, spec.center.device, int(spec.center.shape[0]))
         trace = ibp_trace(module, spec)
         chain = trace.chain
         dev = spec.center.device

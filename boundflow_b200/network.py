@@ -159,6 +159,7 @@ class CudaChain:
             shape = out_shape
         self.layers = layers
         self.output_shape = shape
+        self.output_width = _numel(shape)
         self.relu_layer_ids = [i for i, l in enumerate(layers) if l.op == "relu"]
         self.relu_input_names = [layers[i].in_name for i in self.relu_layer_ids]
         self.relu_shapes = [layers[i].in_shape for i in self.relu_layer_ids]

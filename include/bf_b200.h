@@ -126,6 +126,12 @@ int bf_relu_relax(const float* l, const float* u, const float* alpha, int alpha_
                   float* alpha_u, float* beta_u, float* alpha_l,
                   int B, int n, bf_stream_t stream);
 
+/* The same for n_relu ReLUs in one launch: HOST arrays of device pointers, widths and strides (alpha NULL or with NULL entries:
+ * the default slopes). */
+int bf_relu_relax_many(const float* const* l, const float* const* u, const float* const* alpha, const int* alpha_strides,
+                       float* const* alpha_u, float* const* beta_u, float* const* alpha_l, const int* widths, int n_relu,
+                       int B, bf_stream_t stream);
+
 /* Start value of the per-domain lower slopes: 1 where l >= 0 or (l < 0 < u and u > -l), else 0.
  *   replaces _initial_alpha_state, boundflow/runtime/native_alpha_beta_optimizer_schedule.py:635-656.
  * l,u,alpha [B,n]. */
@@ -410,6 +416,23 @@ int bf_chain_crown_influence(const bf_chain* chain, int upto_layer, int side,
                              const float* mid, const float* rad, int norm_p, float eps, float* out,
                              float* const* influence,
                              void* workspace, size_t workspace_bytes, int B, int S, bf_stream_t stream);
+
+/* Whole queries in one call, for an input set that is a box [in_a, in_b] or, with in_b NULL, the L-inf ball of radius eps around in_a
+ * ([B,n0] each), without splits, constraints or given slopes.  The workspace (bf_chain_query_workspace_bytes: S = 0 for the IBP
+ * query, chunk_rows = 0 except for the intermediate query) holds everything in between.
+ *   bf_chain_ibp_query:     interval bounds of the chain's output (run_ibp, runtime/task_executor.py)          out [B,n_out]
+ *   bf_chain_crown_query:   IBP, relaxations and both sweeps (run_crown_ibp_mlp crown_ibp.py:2054)            out [B,S]
+ *   bf_chain_crown_intermediate: CROWN whose ReLU-input bounds are CROWN bounds, identity rows in chunks of chunk_rows per domain
+ *     (boundflow/runtime/native_intermediate_refinement.py:923-988); pre_l / pre_u: HOST arrays of [B,n_r] outputs; infeasible [R,B] int32:
+ *     row r is raised where the bounds of ReLU r's step contradict the interval pass. */
+size_t bf_chain_query_workspace_bytes(const bf_chain* chain, int B, int S, int chunk_rows);
+int bf_chain_ibp_query(const bf_chain* chain, const float* in_a, const float* in_b, float eps, float* out_l, float* out_u,
+                       void* workspace, size_t workspace_bytes, int B, bf_stream_t stream);
+int bf_chain_crown_query(const bf_chain* chain, const float* in_a, const float* in_b, float eps, const float* C, float* out_l,
+                         float* out_u, void* workspace, size_t workspace_bytes, int B, int S, bf_stream_t stream);
+int bf_chain_crown_intermediate(const bf_chain* chain, const float* in_a, const float* in_b, float eps, const float* C, float* out_l,
+                                float* out_u, float* const* pre_l, float* const* pre_u, int* infeasible, int chunk_rows,
+                                void* workspace, size_t workspace_bytes, int B, int S, bf_stream_t stream);
 
 /* bf_chain_crown for spec rows that are rows first_row .. first_row+S-1 of the identity, the same
  * for every domain: the sweeps that bound an intermediate value neuron by neuron

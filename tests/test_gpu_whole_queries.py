@@ -1,0 +1,106 @@
+"""Queries that the library answers in one call against the same queries step by step (an input set whose tensors it cannot read in place): same bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    assert torch.cuda.is_available(), "GPU tests need a CUDA device"
+    from boundflow_b200.csrc import build
+
+    build.build()
+    return torch.device("cuda", 0)
+
+
+def _wide(t):
+    """t with a gap behind every element: not contiguous."""
+    out = torch.empty(tuple(t.shape) + (2,), device=t.device)[..., 0]
+    out.copy_(t)
+    return out
+
+
+NETS = [((784,), [("fc", 10)]), ((784,), [("fc", 33), ("fc", 10)]), ((784,), [("fc", 100), ("fc", 257), ("fc", 65), ("fc", 10)]),
+        ((784,), [("fc", 9 + r) for r in range(18)] + [("fc", 10)]), ((1, 28, 28), [("conv", 8, 4, 2, 1), ("conv", 5, 4, 2, 1), ("fc", 37), ("fc", 10)])]
+
+
+@pytest.mark.parametrize("ball", ["box", "linf"])
+@pytest.mark.parametrize("net", range(len(NETS)))
+@pytest.mark.parametrize("B", [1, 17])
+def test_one_call_and_many_agree(dev, net, ball, B):
+    from boundflow_b200 import crown
+    from boundflow_b200 import workloads as W
+    from boundflow_b200.executor import CudaTaskExecutor
+    from boundflow_b200.ir import InputSpec, normalize_input_spec
+
+    wl = W.make_workload("c1" if len(NETS[net][0]) == 1 else "c2", batch=B, eps=1e-3, net=W.NetSpec(*NETS[net]))
+    lo, up, C = wl.lo.to(dev), wl.up.to(dev), wl.C.to(dev)
+    make = (lambda f: InputSpec.box(value_name="input", lower=f(lo), upper=f(up))) if ball == "box" else (
+        lambda f: InputSpec.linf(value_name="input", center=f(lo), eps=1e-3))
+    one, many = make(lambda t: t.contiguous()), make(_wide)
+    assert crown._plain_set(normalize_input_spec(one)) is not None and crown._plain_set(normalize_input_spec(many)) is None
+    for f in (lambda s: CudaTaskExecutor().run_ibp(wl.module, s), lambda s: crown.run_crown_ibp_mlp(wl.module, s, linear_spec_C=C),
+              lambda s: crown.run_crown_ibp_mlp(wl.module, s)):
+        a, b = f(one), f(many)
+        assert torch.equal(a.lower, b.lower) and torch.equal(a.upper, b.upper) and a.lower.shape == b.lower.shape
+    for chunk in (7, 1024, 10**12):
+        (a, pa), (b, pb) = (crown.run_crown_intermediate_mlp(wl.module, s, linear_spec_C=C, chunk_rows=chunk) for s in (one, many))
+        assert torch.equal(a.lower, b.lower) and torch.equal(a.upper, b.upper) and list(pa) == list(pb)
+        for n in pa:
+            assert torch.equal(pa[n].lower, pb[n].lower) and torch.equal(pa[n].upper, pb[n].upper) and pa[n].lower.shape == pb[n].lower.shape
+
+
+def test_contradictions_are_reported(dev):
+    """lower > upper in one input set: both routes raise, and name the same domains."""
+    from boundflow_b200 import crown
+    from boundflow_b200 import workloads as W
+    from boundflow_b200.ir import InputSpec
+
+    wl = W.make_workload("c1", batch=5, eps=1e-3, net=W.NetSpec(*NETS[2]))
+    lo, up = wl.lo.to(dev).clone(), wl.up.to(dev).clone()
+    lo[3], up[3] = up[3].clone() + 1, lo[3].clone()
+    said = []
+    for f in (lambda t: t.contiguous(), _wide):
+        with pytest.raises(ValueError) as e:
+            crown.run_crown_intermediate_mlp(wl.module, InputSpec.box(value_name="input", lower=f(lo), upper=f(up)), linear_spec_C=wl.C.to(dev))
+        said.append(str(e.value))
+    assert said[0] == said[1] and "[3]" in said[0]
+
+
+def test_other_norms_stay_refused(dev):
+    """Only "inf" balls are read as boxes of radius eps."""
+    from boundflow_b200 import crown
+    from boundflow_b200.ir import InputSpec, normalize_input_spec
+
+    spec = normalize_input_spec(InputSpec.linf(value_name="input", center=torch.zeros(2, 4, device=dev), eps=0.1))
+
+    class Odd:
+        eps = 0.1
+
+        def norm(self):
+            return "3"
+
+    class Spec:
+        center, perturbation = spec.center, Odd()
+
+    assert crown._plain_set(spec) is not None and crown._plain_set(Spec()) is None
+
+
+@pytest.mark.parametrize("R,B", [(1, 1), (16, 5), (19, 33)])
+def test_relaxations_in_one_launch_or_many(dev, R, B):
+    """bf_relu_relax_many against bf_relu_relax: default slopes, slopes per domain and shared ones, past the edge of a launch (16 ReLUs)."""
+    from boundflow_b200 import _lib
+    from boundflow_b200.crown import relax_all
+
+    lib, g = _lib.load(), torch.Generator("cuda").manual_seed(R)
+    widths = [1 + (13 * r) % 70 for r in range(R)]
+    l = [torch.randn(B, n, generator=g, device=dev) - 0.5 for n in widths]
+    u = [x + torch.rand(x.shape, generator=g, device=dev) * 2 for x in l]
+    alpha = [None if r % 3 == 0 else torch.rand(B if r % 3 == 1 else 1, n, generator=g, device=dev) for r, n in enumerate(widths)]
+    strides = [n if r % 3 == 1 else 0 for r, n in enumerate(widths)]
+    many = relax_all(lib, l, u, alpha, strides, widths, B, dev)
+    for r, n in enumerate(widths):
+        one = [torch.empty(B, n, device=dev) for _ in range(3)]
+        _lib.check(lib.bf_relu_relax(l[r].data_ptr(), u[r].data_ptr(), _lib.ptr(alpha[r]), strides[r], *[t.data_ptr() for t in one], B, n, None))
+        assert all(torch.equal(a[r], b) for a, b in zip(many, one))
