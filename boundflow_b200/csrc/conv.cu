@@ -34,13 +34,29 @@ struct IbpConvArgs {
 // Bound by FFMA issue and the slab's shared-memory reads (three 128-bit reads for 32 FMAs; issue slots 66 %, shared memory 51 %, FMA
 // pipe 44 % busy): 200 images, 32 -> 32 channels, 4x4 / 2
 // kernel on 32 x 32: 138 us = 24 TFLOP/s (one thread per output, weights and pixels read through L1 for every tap, before: 1.1 ms);
-// plain rows, 432 x 16 x 14 x 14 -> 32, 4x4 / 2: 32 us (164).
-constexpr int CONV_SERIAL_K = 1024, CONV_PARTS = 4;
+// plain rows, 432 x 16 x 14 x 14 -> 32, 4x4 / 2: 27 us (164).
+// Plain rows of few tiles are cut too (conv_row_parts): one tile an SM is bound by the latency of its slabs (copy, barrier, 16 taps: 1.4 us).  They are
+// points of a gradient, not bounds: the order of their sums follows the tile count.  (One order for every batch, the parts of a tile added one by one
+// by one, two or four CTAs: 1.02 to 1.07 of the time where the tiles are many.)
+// TC channels a thread: eight for plain rows of more than 32 channels and more than two tiles an SM (three 128-bit reads per 32 FMAs instead of four; 128 threads): 1152 x 64 x 8 x 8 ->
+// 64, 3x3: 195 -> 179 us, 4608 rows 755 -> 672.  Not for intervals (128 registers: 30 -> 36 us and 92 -> 142 us at 16 images, 0.92 of the time at best) nor
+// for few tiles (9 x 128 x 8 x 8 -> 128, 3x3: 26 -> 33; 72 x 16 x 14 x 14 -> 48, 3x3, 221 tiles: 19 -> 21) or channels (32: 11 -> 13 us at 36 rows, 148 -> 134 at 4608).
+constexpr int CONV_SERIAL_K = 1024, CONV_PARTS = 4, CONV_ROWS_CUT_4 = 128, CONV_ROWS_CUT_2 = 256;
 
 template <int TN>
 struct ConvTile {
   static constexpr int TM = 4096 / TN, SLAB = (TN == 16) ? 8 : 16;
 };
+
+// Parts that a sum of K taps of plain rows is cut into, a CTA each: four while the CTAs are two an SM at most, else two.  16 -> 32 channels, 14 x 14, 4x4 / 2
+// (256 taps), one / two / four parts: 36 rows 22 / 17 / 11 us, 144 rows (56 tiles) 22 / 17 / 14, 288 rows (111) 22 / 21 / 21, 432 rows (166) 31 / 27 / 29,
+// 576 rows (221) 32 / 27 / 33, 1152 rows (441) 44 / 49 / 54; 32 -> 32, 16 x 16, 4x4 / 2 (512 taps): 38 / 25 / 19 at 36 tiles, 39 / 33 / 38 at 144, 56 / 53 / 62
+// at 288.  128 taps: 12 / 9 in four parts, 12.3 -> 13.1 in two (144 tiles); 135 taps 13 / 12 in four (55 tiles), 13.2 -> 14.7 in two (110).
+static int conv_row_parts(long long tiles, int K) {
+  if (K > CONV_SERIAL_K) return CONV_PARTS;
+  if (tiles * 4 <= 2 * 148) return K >= CONV_ROWS_CUT_4 ? 4 : 1;
+  return tiles <= 2 * 148 && K >= CONV_ROWS_CUT_2 ? 2 : 1;
+}
 
 // Sums of one output (pixel of all images, channel) over the taps inside the image: centre, radius
 template <bool INTERVAL>
@@ -69,11 +85,11 @@ __device__ __forceinline__ float2 taps_inside(const IbpConvArgs& g, long long pi
   return t;
 }
 
-template <bool INTERVAL, int TN>
-__global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper, int vec) {
+template <bool INTERVAL, int TN, int TC>
+__global__ void __launch_bounds__(1024 / TC) conv_tile_kernel(IbpConvArgs g, int kper, int vec) {
   grid_wait();
   constexpr int TM = ConvTile<TN>::TM, CBK = ConvTile<TN>::SLAB, ACCS = INTERVAL ? 2 : 1;
-  constexpr int NA = TM * CBK / 256, KSTEP = 256 / TM, WLD = TN + 4, NW = (TN * CBK + 255) / 256;
+  constexpr int T = 1024 / TC, NA = TM * CBK / T, KSTEP = T / TM, WLD = TN + 4, NW = (TN * CBK + T - 1) / T;
   constexpr int STAGE = ACCS * CBK * TM + CBK * WLD, PART = ACCS * TM * TN;
   __shared__ __align__(16) float smem[2 * STAGE > PART ? 2 * STAGE : PART];
   __shared__ int4 tab[2][CBK];
@@ -120,7 +136,7 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
     }
 #pragma unroll
     for (int j = 0; j < NW; ++j) {
-      const int e = tid + j * 256, co = c0 + e / CBK, k = k0 + kt * CBK + e % CBK;
+      const int e = tid + j * T, co = c0 + e / CBK, k = k0 + kt * CBK + e % CBK;
       rw[j] = (e < TN * CBK && co < g.Co && k < k1) ? g.W[(size_t)co * K + k] : 0.f;
     }
   };
@@ -145,14 +161,14 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
     }
 #pragma unroll
     for (int j = 0; j < NW; ++j) {
-      const int e = tid + j * 256;
+      const int e = tid + j * T;
       if (e < TN * CBK) ws[(e % CBK) * WLD + e / CBK] = rw[j];
     }
   };
 
-  float accC[4][4], accR[INTERVAL ? 4 : 1][4];  // [channel][pixel]
+  float accC[TC][4], accR[INTERVAL ? TC : 1][4];  // [channel][pixel]
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < TC; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       accC[i][j] = 0.f;
@@ -175,12 +191,17 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
 #pragma unroll
     for (int kk = 0; kk < CBK; ++kk) {
       const float4 c4 = *reinterpret_cast<const float4*>(as + kk * TM + tx * 4);
-      const float4 w4 = *reinterpret_cast<const float4*>(ws + kk * WLD + ty * 4);
+      float w[TC];
+#pragma unroll
+      for (int q = 0; q < TC; q += 4) {
+        const float4 w4 = *reinterpret_cast<const float4*>(ws + kk * WLD + ty * TC + q);
+        w[q] = w4.x; w[q + 1] = w4.y; w[q + 2] = w4.z; w[q + 3] = w4.w;
+      }
       float4 r4 = c4;
       if (INTERVAL) r4 = *reinterpret_cast<const float4*>(as + CBK * TM + kk * TM + tx * 4);
-      const float c[4] = {c4.x, c4.y, c4.z, c4.w}, r[4] = {r4.x, r4.y, r4.z, r4.w}, w[4] = {w4.x, w4.y, w4.z, w4.w};
+      const float c[4] = {c4.x, c4.y, c4.z, c4.w}, r[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < TC; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           accC[i][j] = fmaf(c[j], w[i], accC[i][j]);
@@ -194,16 +215,16 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
   grid_release();
 
   const int ranks = gridDim.z;
-  if (ranks > 1) {  // four: rank z finishes channel z of every thread
-    const int at = ty * 4 * TM + tx * 4;  // part[acc][channel][pixel]
+  if (ranks > 1) {
+    const int at = ty * TC * TM + tx * 4;  // part[acc][channel][pixel]
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < TC; ++i) {
       *reinterpret_cast<float4*>(smem + at + i * TM) = make_float4(accC[i][0], accC[i][1], accC[i][2], accC[i][3]);
       if (INTERVAL) *reinterpret_cast<float4*>(smem + TM * TN + at + i * TM) = make_float4(accR[i][0], accR[i][1], accR[i][2], accR[i][3]);
     }
     cluster.sync();
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < TC; ++i) {
       if (i % ranks != (int)blockIdx.z) continue;  // rank z finishes channels z, z + ranks, ... of every thread
       float4 c = make_float4(0.f, 0.f, 0.f, 0.f), r = c;
       for (int q = 0; q < ranks; ++q) {
@@ -227,24 +248,24 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
   // formed again from the taps inside.
   bool finite = true;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < TC; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       finite &= fabsf(accC[i][j]) <= FLT_MAX;
       if (INTERVAL) finite &= fabsf(accR[i][j]) <= FLT_MAX;
     }
   if (!finite) {
-    for (int e = 0; e < 16; ++e) {
+    for (int e = 0; e < 4 * TC; ++e) {
       const int i = e >> 2, j = e & 3;
-      if (pt + j >= npix || c0 + ty * 4 + i >= g.Co) continue;
-      const float2 t = taps_inside<INTERVAL>(g, pt + j, c0 + ty * 4 + i);
-      smem[e * 256 + tid] = t.x;  // the slabs are read no more; a thread has words of its own
-      if (INTERVAL) smem[4096 + e * 256 + tid] = t.y;
+      if (pt + j >= npix || c0 + ty * TC + i >= g.Co) continue;
+      const float2 t = taps_inside<INTERVAL>(g, pt + j, c0 + ty * TC + i);
+      smem[e * T + tid] = t.x;  // the slabs are read no more; a thread has words of its own
+      if (INTERVAL) smem[4096 + e * T + tid] = t.y;
     }
 #pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      accC[e >> 2][e & 3] = smem[e * 256 + tid];
-      if (INTERVAL) accR[e >> 2][e & 3] = smem[4096 + e * 256 + tid];
+    for (int e = 0; e < 4 * TC; ++e) {
+      accC[e >> 2][e & 3] = smem[e * T + tid];
+      if (INTERVAL) accR[e >> 2][e & 3] = smem[4096 + e * T + tid];
     }
   }
   int b4[4], q4[4];
@@ -254,8 +275,8 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
     q4[j] = (int)((pt + j) - (long long)b4[j] * howo);
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int co = c0 + ty * 4 + i;
+  for (int i = 0; i < TC; ++i) {
+    const int co = c0 + ty * TC + i;
     if (co >= g.Co || (ranks > 1 && i % ranks != (int)blockIdx.z)) continue;
     const float bias = g.bias ? g.bias[co] : 0.f;
     float lo[4], up[4];
@@ -300,16 +321,16 @@ __global__ void __launch_bounds__(256) conv_tile_kernel(IbpConvArgs g, int kper,
   }
 }
 
-template <bool INTERVAL, int TN>
+template <bool INTERVAL, int TN, int TC>
 static int launch_conv_tile_n(const IbpConvArgs& g, int vec, cudaStream_t stream) {
   const long long npix = (long long)g.B * g.Ho * g.Wo;
   const long long tiles = (npix + ConvTile<TN>::TM - 1) / ConvTile<TN>::TM;
   const int K = g.Ci * g.kh * g.kw, slabs = ceil_div(K, ConvTile<TN>::SLAB), ctas_y = ceil_div(g.Co, TN);
   BF_REQUIRE(ctas_y <= 65535 && tiles <= 2147483647LL, BF_E_UNSUPPORTED, "conv2d: too many output channels or pixels");
-  const int ks = K > CONV_SERIAL_K ? CONV_PARTS : 1;
+  const int ks = !INTERVAL ? conv_row_parts(tiles * ctas_y, K) : K > CONV_SERIAL_K ? CONV_PARTS : 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)tiles, ctas_y, ks);
-  cfg.blockDim = dim3(256);
+  cfg.blockDim = dim3(1024 / TC);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -324,10 +345,10 @@ static int launch_conv_tile_n(const IbpConvArgs& g, int vec, cudaStream_t stream
   cfg.numAttrs = one_each || (ks == 1 && (K <= 64 || tiles * ctas_y >= 4 * 148)) ? 2 : 1;
   if (one_each) {
     static SmemOptIn opt_in;
-    if (int rc = ensure_dynamic_smem(conv_tile_kernel<INTERVAL, TN>, ONE_PER_SM, opt_in, "conv_tile_kernel")) return rc;
+    if (int rc = ensure_dynamic_smem(conv_tile_kernel<INTERVAL, TN, TC>, ONE_PER_SM, opt_in, "conv_tile_kernel")) return rc;
     cfg.dynamicSmemBytes = ONE_PER_SM;
   }
-  cudaLaunchKernelEx(&cfg, conv_tile_kernel<INTERVAL, TN>, g, ceil_div(slabs, ks) * ConvTile<TN>::SLAB, vec);
+  cudaLaunchKernelEx(&cfg, conv_tile_kernel<INTERVAL, TN, TC>, g, ceil_div(slabs, ks) * ConvTile<TN>::SLAB, vec);
   BF_CHECK_LAUNCH("conv_tile_kernel");
   return BF_OK;
 }
@@ -336,9 +357,11 @@ static int launch_conv_tile_n(const IbpConvArgs& g, int vec, cudaStream_t stream
 template <bool INTERVAL>
 static int launch_conv_tile(const IbpConvArgs& g, cudaStream_t stream) {
   int vec = (g.Ho * g.Wo) % 4 == 0 && ((reinterpret_cast<uintptr_t>(g.out_l) | reinterpret_cast<uintptr_t>(g.out_u)) & 15u) == 0;
-  if (g.Co <= 16) return launch_conv_tile_n<INTERVAL, 16>(g, vec, stream);
-  if (g.Co <= 32) return launch_conv_tile_n<INTERVAL, 32>(g, vec, stream);
-  return launch_conv_tile_n<INTERVAL, 64>(g, vec, stream);
+  if (g.Co <= 16) return launch_conv_tile_n<INTERVAL, 16, 4>(g, vec, stream);
+  if (g.Co <= 32) return launch_conv_tile_n<INTERVAL, 32, 4>(g, vec, stream);
+  const long long tiles = ((long long)g.B * g.Ho * g.Wo + 63) / 64 * ceil_div(g.Co, 64);
+  if (INTERVAL || tiles <= 2 * 148) return launch_conv_tile_n<INTERVAL, 64, 4>(g, vec, stream);
+  return launch_conv_tile_n<false, 64, 8>(g, vec, stream);
 }
 
 int launch_ibp_conv2d(const float* in_a, const float* in_b, int in_mode, int relu_in, const float* W, const float* bias,

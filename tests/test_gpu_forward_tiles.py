@@ -195,3 +195,32 @@ def test_forward_conv_bits_do_not_depend_on_the_batch(dev, Ci, H, W, Co, k, s, p
     bias = b.double()[:, None, None]
     for got, ref in zip(whole, (conv(x, w) - conv(r, w.abs()), conv(x, w) + conv(r, w.abs()), conv(x, w))):
         assert ((got[:7].double() - (ref + bias)).abs() <= tol).all()
+
+
+# (rows, Ci, map, Co, kernel, stride, padding): plain rows whose sums are cut in four, two and not at all, on both sides of each line (74 and 76, 296 and 298
+# tiles; 126 and 128, 252 and 261 taps), parts of unequal length, a part without taps, one row, and eight channels a thread with channels past the end
+@pytest.mark.parametrize("M,Ci,H,Co,k,s,p", [(1, 16, 14, 32, 4, 2, 1), (37, 32, 16, 20, 3, 1, 1), (38, 32, 16, 20, 3, 1, 1), (148, 32, 16, 20, 3, 1, 1), (149, 32, 16, 20, 3, 1, 1),
+                                             (5, 14, 8, 17, 3, 1, 1), (5, 8, 8, 17, 4, 2, 1), (40, 28, 16, 20, 3, 1, 1), (40, 29, 16, 20, 3, 1, 1), (149, 16, 8, 64, 4, 1, 0), (7, 33, 7, 33, 3, 1, 1), (3, 40, 9, 70, 5, 2, 2), (74, 16, 8, 64, 3, 1, 1),
+                                             (75, 32, 8, 64, 3, 1, 1), (300, 16, 8, 64, 3, 1, 1), (2, 130, 6, 65, 3, 1, 1), (9, 2, 10, 16, 8, 1, 0)])
+def test_plain_rows_cut_in_parts(dev, M, Ci, H, Co, k, s, p):
+    from boundflow_b200 import _lib
+
+    lib, g = _lib.load(), torch.Generator("cuda").manual_seed(M + Ci + Co)
+    x, w, b = torch.randn(M, Ci, H, H, generator=g, device=dev), torch.randn(Co, Ci, k, k, generator=g, device=dev), torch.randn(Co, generator=g, device=dev)
+    Ho = (H + 2 * p - k) // s + 1
+    conv = lambda t, u, v: torch.nn.functional.conv2d(t.double(), u.double(), v.double(), stride=s, padding=p)
+
+    def run():
+        y = torch.full((M, Co, Ho, Ho), float("nan"), device=dev)
+        _lib.check(lib.bf_rows_conv2d_fwd(x.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), M, Ci, H, H, Co, Ho, Ho, k, k, s, s, p, p, None))
+        return y
+
+    # a sum of K products in any order is off by at most (K + 4) u times the sum of their magnitudes, u = 2^-24
+    bound = (Ci * k * k + 4) * 2.0**-24 * conv(x.abs(), w.abs(), b.abs())
+    assert ((run().double() - conv(x, w, b)).abs() <= bound).all()
+    # an infinite weight counts where its tap lies inside the image, also in the middle parts of a sum
+    w[Co - 1, Ci // 2, 0, 0] = float("inf")
+    want, got = conv(x, torch.where(w.isinf(), 0, w), b), run()
+    inside = torch.nn.functional.conv2d(x[:, Ci // 2 : Ci // 2 + 1].sign().double(), torch.nn.functional.pad(torch.ones(1, 1, 1, 1, device=dev, dtype=torch.float64), (0, k - 1, 0, k - 1)), stride=s, padding=p)
+    assert torch.equal(got[:, Co - 1].isposinf(), inside[:, 0] > 0) and torch.equal(got[:, Co - 1].isneginf(), inside[:, 0] < 0)
+    assert not got.isnan().any() and ((got.double() - want).abs() <= bound)[:, : Co - 1].all()
