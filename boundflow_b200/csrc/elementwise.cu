@@ -808,44 +808,54 @@ int launch_beta_step(float* beta, float* m, float* v, float* gsum, const int8_t*
   return launch_optimiser_step(&g, 1, improve, sc, do_update, B, stream);
 }
 
-// Widest unstable gap per domain over the ReLUs in chain order: one warp per domain; the first index of a tie and the earlier ReLU win.  `first`
-// is 0 where earlier launches have left the best of the ReLUs before these.
+// Widest unstable gap per domain over the ReLUs in chain order; the first index of a tie and the earlier ReLU win.  `first` is 0 where earlier launches
+// have left the best of the ReLUs before these.  T threads a domain: bound by the latency of its reads, a warp took 33 us for 48 domains of 4804 neurons
+// (98 reads in a row), a block takes 8; 1000 domains of 4 x 512 18.5 and 8.3, 2000 of 4804 60 and 21, but 8192 of 4 x 512 45 and 56, 16384 of 200 10 and 31.
+constexpr int SCORE_BLOCK_DOMAINS = 2000;  // up to here a block each
 constexpr int SCORE_SEGMENTS = 16;
 struct ScoreArgs {
   const float *l[SCORE_SEGMENTS], *u[SCORE_SEGMENTS];
   int n[SCORE_SEGMENTS];
   int count, relu0;
 };
+template <int T>
 __global__ void __launch_bounds__(256) branch_score_kernel(const __grid_constant__ ScoreArgs a, int B, int first, float* __restrict__ best_gap,
                                                            int* __restrict__ best_relu, int* __restrict__ best_idx) {
-  const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (b >= B) return;
+  const int b = blockIdx.x * (256 / T) + threadIdx.x / T, t = threadIdx.x % T, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (b >= B) return;  // whole warps
+  __shared__ float gaps[8];
+  __shared__ int at[8];
   float best = first ? -INFINITY : best_gap[b];
-  int relu = -1, at = -1;
+  int relu = -1, best_at = -1;
   for (int r = 0; r < a.count; ++r) {
     const float *l = a.l[r] + (size_t)b * a.n[r], *u = a.u[r] + (size_t)b * a.n[r];
     float gap = -INFINITY;
     int idx = 0x7fffffff;
-    for (int j = lane; j < a.n[r]; j += 32) {
+#pragma unroll 4
+    for (int j = t; j < a.n[r]; j += T) {
       const float lo = __ldg(l + j), up = __ldg(u + j);
       if (lo < 0.f && up > 0.f) {
         const float g = fmaxf(up - lo, 0.f);
         if (g > gap) { gap = g; idx = j; }  // j increases: the first index of a tie is kept
       }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float og = __shfl_xor_sync(0xffffffffu, gap, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+    auto take = [&](float og, int oi) {
       if (og > gap || (og == gap && oi < idx)) { gap = og; idx = oi; }
+    };
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) take(__shfl_xor_sync(0xffffffffu, gap, o), __shfl_xor_sync(0xffffffffu, idx, o));
+    if (T == 256) {
+      if (lane == 0) { gaps[warp] = gap; at[warp] = idx; }
+      __syncthreads();
+      for (int w = 0; w < 8; ++w) take(gaps[w], at[w]);
+      __syncthreads();
     }
-    if (gap > best) { best = gap; relu = a.relu0 + r; at = idx; }
+    if (gap > best) { best = gap; relu = a.relu0 + r; best_at = idx; }
   }
-  if (lane == 0 && (first || relu >= 0)) {
+  if (t == 0 && (first || relu >= 0)) {
     best_gap[b] = best;
     best_relu[b] = relu;
-    best_idx[b] = at;
+    best_idx[b] = best_at;
   }
 }
 
@@ -865,7 +875,11 @@ extern "C" int bf_branch_scores(const float* const* pre_l, const float* const* p
       a.u[a.count] = pre_u[r0];
       a.n[a.count] = widths[r0];
     }
-    bf::branch_score_kernel<<<bf::ceil_div((long long)B * 32, 256), 256, 0, bf::as_stream(stream_)>>>(a, B, a.relu0 == 0 ? 1 : 0, best_gap, best_relu, best_idx);
+    const int first = a.relu0 == 0 ? 1 : 0;
+    if (B <= bf::SCORE_BLOCK_DOMAINS)
+      bf::branch_score_kernel<256><<<B, 256, 0, bf::as_stream(stream_)>>>(a, B, first, best_gap, best_relu, best_idx);
+    else
+      bf::branch_score_kernel<32><<<bf::ceil_div(B, 8), 256, 0, bf::as_stream(stream_)>>>(a, B, first, best_gap, best_relu, best_idx);
     BF_CHECK_LAUNCH("branch_score_kernel");
   } while (r0 < n_relu);
   return BF_OK;

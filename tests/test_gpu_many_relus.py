@@ -43,13 +43,13 @@ def test_more_tensors_than_one_launch(dev, with_beta):
             assert ((want - start).abs() > 0.05).any() == ((got - start).abs() > 0.05).any()
 
 
-@pytest.mark.parametrize("R,B", [(0, 3), (1, 1), (16, 9), (19, 300)])
+@pytest.mark.parametrize("R,B", [(0, 3), (1, 1), (16, 9), (19, 300), (19, 2000), (18, 2001), (2, 2009)])
 def test_branch_scores_of_many_relus(dev, R, B):
     """Widest unstable gap: the first neuron of a tie and the earlier ReLU win, also over the edge of a launch (16 ReLUs); -inf and -1 without one."""
     from boundflow_b200 import _lib
 
     lib, g = _lib.load(), torch.Generator().manual_seed(R)
-    widths = [1 + (7 * r) % 45 for r in range(R)]
+    widths = [1 + (37 * r) % 301 for r in range(R)]
     # bounds on a grid of quarters: many equal gaps; the last domain has no unstable neuron
     pre = [(-torch.randint(0, 5, (B, n), generator=g) / 4, torch.randint(0, 5, (B, n), generator=g) / 4) for n in widths]
     for l, _ in pre:
