@@ -16,9 +16,9 @@
 // 2e-7 and 2 to 5e-7, TF32 kernels 2e-6), and fewer signs of small coefficients on the wrong side.
 // Layouts are K-major; weights without swizzle (8-row x 16-byte core matrices), [16 terms][part][8-term chunk][128 features][16 bytes], rows
 // [part][32 rows][64 bytes] with the 64-byte swizzle: four lanes read 128 bytes of a row and a warp's stores meet different banks.
-// From the end of one launch to the end of the next, FP32 kernels -> here: 1152 x 256 x 256 backward 12.5 -> 7.1 us, adjoint 9.3 -> 6.6; 1152 rows, 256 -> 784
-// 28.4 -> 14; 784 -> 256 adjoint 28 -> 13; 333 x 512 x 512 20 -> 9.7 and 15 -> 7.7; 432 rows, 1568 -> 100 adjoint 39 -> 10.
-// Of the 6.6 us (13 thousand clocks) 1.5 are the loads of the rows, 4 the MMAs (480 to 700 a stage: shared memory is busy with their operands), 2.5 the epilogue.
+// From the end of one launch to the end of the next, FP32 kernels -> here: 1152 x 256 x 256 backward 12.5 -> 6.8 us, adjoint 9.3 -> 6.5; 1152 rows, 256 -> 784
+// 28.4 -> 17.3; 784 -> 256 adjoint 28 -> 12.5; 333 x 512 x 512 20 -> 9.9 and 15 -> 7.8; 432 rows, 1568 -> 100 adjoint 39 -> 9.9.
+// Of some 6.6 us (13 thousand clocks) 1.5 are the loads of the rows, 4 the MMAs (480 to 700 a stage: shared memory is busy with their operands), 2.5 the epilogue.
 // Every wait is bounded; on expiry the status word is raised, whose reader replaces the call's results by NaN.
 #include <float.h>
 
@@ -678,17 +678,18 @@ __global__ void __launch_bounds__(256) pack_small_weights_kernel(const __grid_co
 }  // namespace stc
 
 // CTAs that share the terms of a tile; 0: the problem is not small.
-// Gradient evaluations (one sweep down, one up) of 784-input networks, other kernels -> here, us: up to two tiles per SM three 256-wide layers, 300 inputs
-// 241 -> 174, 500 inputs 247 -> 187, three 128-wide ones, 1000 inputs 201 -> 173; three per SM 256-wide, 600 inputs 235 -> 242, but sums above 256 terms
-// amortise a tile's start: 512-wide, 300 inputs 370 -> 306, 800-wide, 200 inputs 307 -> 260; four per SM 256-wide, 900 inputs 252 -> 303.
-// Sums of up to 64 terms are short on the FP32 units, too: three 64-wide layers, 3 inputs 62 there and 66 here, 30 inputs 70 and 72; 100-wide, 500 inputs
-// 125 and 114.
-// Clusters while all CTAs find an SM: four 512-wide layers, 37 inputs 156 us with one CTA a tile, 127 with two.  Four CTAs share sums above 1024 terms
-// (432 rows, 1568 -> 100: 39 us on FP32 units, 27, 16 and 10 here); a shorter sum gains little more (500-wide, 9 inputs 120, 91 and 77 us), and with two
-// the loops of the 784-input network that the tests follow step by step choose their best steps as in FP32 where two steps' objectives are equal up to rounding.
+// Gradient evaluations (one sweep down, one up) of 784-input networks, other kernels -> here, us: up to two tiles an SM three 256-wide layers, 300 inputs
+// 234 -> 161, 500 inputs 242 -> 171, three 128-wide ones, 1000 inputs 195 -> 150; three an SM 256-wide, 530 inputs 218 -> 208, 785 inputs 236 -> 230, five such
+// layers 345 -> 308 and 357 -> 339, 512-wide, 300 inputs 363 -> 291, 800-wide, 200 inputs 456 -> 358, but 128-wide, 1200 inputs 203 -> 210 and 100-wide 204 -> 208;
+// four an SM 256-wide, 900 inputs 250 -> 271.
+// Sums of up to 64 terms are short on the FP32 units, too: three 33-, 48- and 64-wide layers, 1 to 128 inputs 50 to 69 there and 52 to 72 here.
+// Clusters while all CTAs find an SM: four 512-wide layers, 37 inputs 145 us with one CTA a tile, 115 with two, 784-100-100-10, 64 inputs 60 and 52.  Four CTAs
+// share sums above 1024 terms (1568-1568-100-10, 48 inputs: 190 with one CTA a tile, 174); a shorter sum gains little more (500-wide, 9 inputs: 120, 91 and 77 us
+// with one, two and four), and with two the loops of the 784-input network that the tests follow step by step choose their best steps as in FP32 where two
+// steps' objectives are equal up to rounding.
 static int small_tc_cluster(int M, int N, int K) {
   const long long tiles = (long long)ceil_div(N, stc::TF) * ceil_div(M, stc::NR);
-  if (K <= 64 || tiles > (K > 256 ? 3 : 2) * 148) return 0;
+  if (K <= 64 || tiles > (K >= 256 ? 3 : 2) * 148) return 0;
   int cs = K > 1024 ? 4 : (K > 96 ? 2 : 1);
   while (tiles * cs > 148 && cs > 1) cs /= 2;
   return cs;

@@ -60,7 +60,7 @@ class _Chain:
 # per domain 1, 7 (more than two domains in a block), 8, 32; one tile and 129 features; more tiles than SMs, one CTA each; the largest counts of the rule
 @pytest.mark.parametrize("D, S, dims", [(1, 1, (65, 65, 3)), (34, 1, (70, 96, 66, 5)), (5, 7, (97, 129, 128, 8)), (9, 8, (128, 255, 100, 9)), (3, 32, (300, 127, 33)),
                                         (2, 9, (1000, 777, 10)), (11, 9, (1570, 100, 10)), (48, 9, (784, 256, 256, 10)), (37, 9, (512, 512, 512, 10)),
-                                        (263, 9, (256, 256, 256, 10)), (160, 9, (784, 512, 10)), (1, 9, (4100, 130, 10))])
+                                        (263, 9, (256, 256, 256, 10)), (785, 9, (256, 256, 255, 10)), (160, 9, (784, 512, 10)), (1, 9, (4100, 130, 10))])
 def test_gradients_and_bounds_against_float64(dev, D, S, dims):
     g = torch.Generator().manual_seed(D + sum(dims))
     Ws = [torch.randn((n, k), generator=g) * (2.0 / k) ** 0.5 for k, n in zip(dims, dims[1:])]
