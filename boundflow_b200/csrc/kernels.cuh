@@ -89,7 +89,11 @@ int launch_relu_relax(const RelaxSegment* seg, int count, int B, cudaStream_t st
 int launch_relu_relax(const float* l, const float* u, const float* alpha, int alpha_stride, float* alpha_u,
                       float* beta_u, float* alpha_l, int B, int n, cudaStream_t stream);
 // mid = (a + b) / 2, rad = (b - a) / 2; b null: rad = eps (mid is a itself)
-int launch_input_set(const float* a, const float* b, float eps, float* mid, float* rad, long long n, cudaStream_t stream);
+// and, with C2, C2[b] = (C[b], -C[b]) for B blocks of `per` values
+int launch_input_set(const float* a, const float* b, float eps, float* mid, float* rad, long long n, const float* C, float* C2, long long per, int B,
+                     cudaStream_t stream);
+// lower, -upper [B,S] from both [B,2S]
+int launch_split_sides(const float* both, float* lower, float* upper, int B, int S, cudaStream_t stream);
 // columns at .. at + cnt - 1 of [B,n] matrices from [B,cnt] ones
 int launch_place_columns(const float* l, const float* u, float* to_l, float* to_u, int B, int cnt, int n, int at, cudaStream_t stream);
 int launch_concretize(const float* A, const float* mid, const float* rad, const float* bias_in, float* out, int side,

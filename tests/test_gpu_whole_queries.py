@@ -27,7 +27,7 @@ NETS = [((784,), [("fc", 10)]), ((784,), [("fc", 33), ("fc", 10)]), ((784,), [("
 
 @pytest.mark.parametrize("ball", ["box", "linf"])
 @pytest.mark.parametrize("net", range(len(NETS)))
-@pytest.mark.parametrize("B", [1, 17])
+@pytest.mark.parametrize("B", [1, 17, 150])  # both sides join in one sweep for some, not for others
 def test_one_call_and_many_agree(dev, net, ball, B):
     from boundflow_b200 import crown
     from boundflow_b200 import workloads as W
