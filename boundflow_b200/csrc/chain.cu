@@ -724,9 +724,9 @@ struct QueryWs {
 };
 
 // Both sides in one sweep: the upper bound of a row is minus the lower bound of its negation, bit for bit (every kernel of a sweep is symmetric in the sign
-// of a row), so S rows and their negations go down together: half the launches, and fuller waves.  784-100-100-10, 64 inputs: 67 -> 57 us; 784-512x4-10, 500 inputs 557 -> 378, 3000
-// inputs (three waves of CTAs for four) 1366 -> 1224.  Not where twice the rows would take a layer to another kernel or split of its sums (other bits, or fewer of them right), nor where the rows' workspace grows
-// beyond JOIN_BYTES: sweeps that large fill their waves.
+// of a row), so S rows and their negations go down together: half the launches, and fuller waves.  784-100-100-10, 64 inputs: 67 -> 57 us;
+// 784-512x4-10, 500 inputs 557 -> 378, 3000 inputs (three waves of CTAs for four) 1366 -> 1224.  Not where twice the rows would take a layer to another
+// kernel or split of its sums (other bits, or fewer of them right), nor where the rows' workspace grows beyond JOIN_BYTES: sweeps that large fill their waves.
 constexpr size_t JOIN_BYTES = (size_t)1 << 30;
 static bool join_sides(const bf_chain* c, int B, int S) {
   if ((long long)B * S * 2 >= 2147483647LL || crown_ws_layout(c, B, 2 * S, (int)c->layers.size(), nullptr, nullptr) > JOIN_BYTES) return false;
@@ -737,7 +737,10 @@ static bool join_sides(const bf_chain* c, int B, int S) {
     const bool small = small_rows(c, M, L.n_in, L.n_out, S, false);
     if (small != small_rows(c, 2 * M, L.n_in, L.n_out, 2 * S, false)) return false;
     if (small && small_tc_tiles(M, L.n_in, L.n_out) != small_tc_tiles(2 * M, L.n_in, L.n_out)) return false;
-    if (!small && (tc_weights(c, 0, false, M, L.n_out, L.n_in) != nullptr) != (tc_weights(c, 0, false, 2 * M, L.n_out, L.n_in) != nullptr)) return false;
+    if (small) continue;
+    const bool tc = tc_weights(c, 0, false, M, L.n_out, L.n_in) != nullptr;
+    if (tc != (tc_weights(c, 0, false, 2 * M, L.n_out, L.n_in) != nullptr)) return false;
+    if (!tc && crown_bwd_partial_tiles(L.n_in, M) != crown_bwd_partial_tiles(L.n_in, 2 * M)) return false;  // another tile width: other partial sums
   }
   return true;
 }
