@@ -104,3 +104,29 @@ def test_relaxations_in_one_launch_or_many(dev, R, B):
         one = [torch.empty(B, n, device=dev) for _ in range(3)]
         _lib.check(lib.bf_relu_relax(l[r].data_ptr(), u[r].data_ptr(), _lib.ptr(alpha[r]), strides[r], *[t.data_ptr() for t in one], B, n, None))
         assert all(torch.equal(a[r], b) for a, b in zip(many, one))
+
+
+@pytest.mark.parametrize("B", [1, 3, 40])
+def test_graph_sides_in_one_sweep_or_two(dev, B):
+    """The graph walker's joined sweep against one sweep a side (zero terms behind a ReLU keep the sides apart).  Twice the rows may take a convolution
+    to the tensor cores: the roundings of sums of up to 1152 products, about sqrt(1152) 2^-24 = 2e-6 of the bounds, 1e-5 leaves a factor of five."""
+    from boundflow_b200 import dag
+    from boundflow_b200.ir import BFTaskModule, BoundTask, InputSpec, TaskKind, TaskOp
+
+    g = torch.Generator().manual_seed(B)
+    P = {"w1": torch.randn(8, 3, 3, 3, generator=g) * 0.2, "b1": torch.randn(8, generator=g) * 0.1, "w2": torch.randn(8, 8, 3, 3, generator=g) * 0.1,
+         "w3": torch.randn(10, 8 * 12 * 12, generator=g) * 0.03, "b3": torch.randn(10, generator=g) * 0.1}
+    conv = {"stride": 1, "padding": 1, "dilation": 1, "groups": 1}
+    ops = [TaskOp("conv2d", "c1", ["x", "w1", "b1"], ["y1"], conv), TaskOp("relu", "r1", ["y1"], ["z1"]), TaskOp("conv2d", "c2", ["z1", "w2"], ["y2"], conv),
+           TaskOp("add", "a", ["y2", "z1"], ["y3"]), TaskOp("relu", "r2", ["y3"], ["z3"]), TaskOp("flatten", "f", ["z3"], ["z4"], {"start_dim": 1, "end_dim": -1}),
+           TaskOp("linear", "l", ["z4", "w3", "b3"], ["out"])]
+    module = BFTaskModule([BoundTask("t", TaskKind.INTERVAL_IBP, ops, ["x"], ["out"])], "t", bindings={"params": {k: v.to(dev) for k, v in P.items()}})
+    x = torch.rand(B, 3, 12, 12, generator=g).to(dev)
+    spec = InputSpec.box(value_name="x", lower=x - 0.02, upper=x + 0.02)
+    C = torch.randn(B, 9, 10, generator=g).to(dev)
+    lo, up, tr = dag.crown_dag(module, spec, C)
+    assert dag._sides_join(module, tr, tr.params, 9, "out")
+    zero = {"y1": torch.zeros(B, 8 * 12 * 12, device=dev)}
+    lo2, up2, _ = dag.crown_dag(module, spec, C, relu_pre_add_coeff_l=zero, relu_pre_add_coeff_u=zero)
+    scale = torch.maximum(lo2.abs(), up2.abs()).max()
+    assert (lo - lo2).abs().max() <= 1e-5 * scale and (up - up2).abs().max() <= 1e-5 * scale and lo.shape == up.shape == (B, 9)
