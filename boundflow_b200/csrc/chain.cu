@@ -238,17 +238,51 @@ void refresh_switches(const bf_chain* c) {
 }
 
 // few rows: crown_small_tc.cu
+static bool small_rows_allowed(const bf_chain* c) { return c->status && !c->sw.force_ffma && c->sw.tc_auto; }
 static bool small_rows(const bf_chain* c, int M, int N, int K, int S, bool adjoint) {
-  return !c->pk_small_bwd.empty() && !c->sw.force_ffma && c->sw.tc_auto && small_tc_supports(M, N, K, S, adjoint);
+  return small_rows_allowed(c) && small_tc_supports(M, N, K, S, adjoint);
 }
 
-bool tc_may_run(const bf_chain* c, int M) {
+void small_images_layout(const bf_chain* c, int M, int S, int upto, bool adjoint, Carver& cv, SmallImages* images) {
+  if (images) *images = SmallImages{};
+  for (int i = 0; i < upto; ++i) {
+    const bf_layer_desc& L = c->layers[i];
+    if (L.op != BF_OP_LINEAR) continue;
+    auto place = [&](int N, int K, bool adj) {
+      if (!small_tc_supports(M, N, K, S, adj)) return;
+      unsigned char* p = cv.take<unsigned char>(small_tc_packed_bytes(N, K) + 15);
+      if (!images) return;
+      std::vector<unsigned char*>& to = adj ? images->adj : images->bwd;
+      to.resize(c->layers.size(), nullptr);
+      to[i] = p + ((0 - reinterpret_cast<uintptr_t>(p)) & 15u);  // the bulk copies' alignment, whatever the workspace's is
+    };
+    place(L.n_in, L.n_out, false);
+    if (adjoint) place(L.n_out, L.n_in, true);
+  }
+}
+
+std::vector<SmallPack> small_images_packs(const bf_chain* c, SmallImages* images) {
+  if (!small_rows_allowed(c)) *images = SmallImages{};
+  std::vector<SmallPack> packs;
+  for (size_t i = 0; i < c->layers.size(); ++i) {
+    const bf_layer_desc& L = c->layers[i];
+    if (images->backward(i)) packs.push_back({L.W, L.n_out, L.n_in, 1, images->bwd[i]});
+    if (images->adjoint(i)) packs.push_back({L.W, L.n_out, L.n_in, 0, images->adj[i]});
+  }
+  images->packed = true;
+  return packs;
+}
+int small_images_pack(const bf_chain* c, SmallImages* images, cudaStream_t stream) {
+  const std::vector<SmallPack> packs = small_images_packs(c, images);
+  return small_tc_pack(packs.data(), (int)packs.size(), stream);
+}
+
+bool tc_may_run(const bf_chain* c, int M, const SmallImages& images) {
   if (c->status == nullptr || c->sw.force_ffma) return false;
   if (!c->pk_bwd.empty() && M >= c->sw.tc_min_rows) return true;
-  for (const bf_layer_desc& L : c->layers) {
+  if (!images.bwd.empty() || !images.adj.empty()) return true;
+  for (const bf_layer_desc& L : c->layers)
     if (L.op == BF_OP_CONV2D && conv_rows_on_tensor_cores(M, L)) return true;
-    if (L.op == BF_OP_LINEAR && (small_rows(c, M, L.n_in, L.n_out, 1, false) || small_rows(c, M, L.n_out, L.n_in, 1, true))) return true;
-  }
   return false;
 }
 
@@ -271,15 +305,16 @@ static const unsigned char* tc_weights(const bf_chain* c, int layer, bool adjoin
 
 // Backward contraction of linear layer `layer`; *ptiles receives the number of column tiles
 // (the second dimension of the concretisation partial-sum buffer).
-int dispatch_bwd(const bf_chain* c, int layer, const float* A, const float* dpos, const float* dneg,
+int dispatch_bwd(const bf_chain* c, const SmallImages& images, int layer, const float* A, const float* dpos, const float* dneg,
                         const float* epos, const float* eneg, const float* add, float* A_prev, float* delta, int accumulate,
                         const float* mid, const float* rad, float* partial, int side, int M, int S, int* ptiles,
                         cudaStream_t stream) {
   const bf_layer_desc& L = c->layers[layer];
   const int K = L.n_out, N = L.n_in;
-  if ((A_prev || partial) && small_rows(c, M, N, K, S, false)) {
+  const unsigned char* small = images.backward(layer);
+  if ((A_prev || partial) && small) {
     if (ptiles) *ptiles = small_tc_tiles(M, N, K);
-    return launch_crown_bwd_small_tc(A, dpos, dneg, epos, eneg, add, c->pk_small_bwd[layer], L.W, L.bias, A_prev, delta, accumulate, mid, rad,
+    return launch_crown_bwd_small_tc(A, dpos, dneg, epos, eneg, add, small, L.W, L.bias, A_prev, delta, accumulate, mid, rad,
                                      partial, side, M, S, K, N, c->status, stream);
   }
   const unsigned char* pk = tc_weights(c, layer, false, M, K, N);
@@ -298,14 +333,14 @@ int dispatch_bwd(const bf_chain* c, int layer, const float* A, const float* dpos
                                  M, S, K, N, stream);
 }
 
-int dispatch_adjoint(const bf_chain* c, int layer, const float* Hprev, int first_layer, const float* mid,
+int dispatch_adjoint(const bf_chain* c, const SmallImages& images, int layer, const float* Hprev, int first_layer, const float* mid,
                             const float* rad, const float* Ahat, const float* dpos, const float* dneg, const float* epos,
                             const float* eneg, const float* pre_l, const float* pre_u, float* hout, float* grad, float* gsum,
                             int M, int S, cudaStream_t stream, const float* gw) {
   const bf_layer_desc& L = c->layers[layer];
   const int K = L.n_in, N = L.n_out;
-  if (small_rows(c, M, N, K, S, true))
-    return launch_crown_adjoint_small_tc(Hprev, first_layer, mid, rad, c->pk_small_adj[layer], L.W, L.bias, Ahat, dpos, dneg, epos, eneg, pre_l,
+  if (const unsigned char* small = images.adjoint(layer))
+    return launch_crown_adjoint_small_tc(Hprev, first_layer, mid, rad, small, L.W, L.bias, Ahat, dpos, dneg, epos, eneg, pre_l,
                                          pre_u, hout, grad, gsum, M, S, K, N, c->status, stream, gw);
   const unsigned char* pk = tc_weights(c, layer, true, M, K, N);
   // gw (row weights of the beta sums, min / softmin with beta parameters) is implemented by the row-major and FFMA kernels
@@ -327,8 +362,7 @@ extern "C" size_t bf_chain_tc_bytes(const bf_chain* chain) {
   for (const bf_layer_desc& L : chain->layers)
     if (L.op == BF_OP_LINEAR)
       total += bf::align_up(bf::tc_packed_bytes(L.n_in, L.n_out)) + bf::align_up(bf::tc_packed_bytes(L.n_out, L.n_in)) +
-               bf::align_up(bf::tc_packed_bytes(L.n_out, L.n_in, bf::tc_adjoint_tile_rows())) +
-               bf::align_up(bf::small_tc_packed_bytes(L.n_in, L.n_out)) + bf::align_up(bf::small_tc_packed_bytes(L.n_out, L.n_in));
+               bf::align_up(bf::tc_packed_bytes(L.n_out, L.n_in, bf::tc_adjoint_tile_rows()));
   return total;
 }
 
@@ -347,9 +381,6 @@ extern "C" int bf_chain_tc_prepare(bf_chain* chain, void* buffer, size_t bytes, 
   chain->pk_bwd.assign(chain->layers.size(), nullptr);
   chain->pk_adj.assign(chain->layers.size(), nullptr);
   chain->pk_adj_fm.assign(chain->layers.size(), nullptr);
-  std::vector<bf::SmallPack> small;
-  chain->pk_small_bwd.assign(chain->layers.size(), nullptr);
-  chain->pk_small_adj.assign(chain->layers.size(), nullptr);
   for (size_t i = 0; i < chain->layers.size(); ++i) {
     const bf_layer_desc& L = chain->layers[i];
     if (L.op != BF_OP_LINEAR) continue;
@@ -368,19 +399,11 @@ extern "C" int bf_chain_tc_prepare(bf_chain* chain, void* buffer, size_t bytes, 
     off += bf::align_up(bf::tc_packed_bytes(L.n_out, L.n_in, bf::tc_adjoint_tile_rows()));
     rc = bf::tc_pack_weights(L.W, L.n_out, L.n_in, 0, pf, stream, bf::tc_adjoint_tile_rows());
     if (rc != BF_OK) return rc;
-    unsigned char* sb = base + off;
-    off += bf::align_up(bf::small_tc_packed_bytes(L.n_in, L.n_out));
-    unsigned char* sa = base + off;
-    off += bf::align_up(bf::small_tc_packed_bytes(L.n_out, L.n_in));
-    small.push_back({L.W, L.n_out, L.n_in, 1, sb});
-    small.push_back({L.W, L.n_out, L.n_in, 0, sa});
-    chain->pk_small_bwd[i] = sb;
-    chain->pk_small_adj[i] = sa;
     chain->pk_adj_fm[i] = pf;
     chain->pk_bwd[i] = pb;
     chain->pk_adj[i] = pa;
   }
-  return bf::small_tc_pack(small.data(), (int)small.size(), stream);
+  return BF_OK;
 }
 
 extern "C" int bf_chain_tc_status(const bf_chain* chain, int* status_out) {
@@ -499,6 +522,7 @@ struct CrownWs {
   float* cacc;
   float* partial;
   void* conv_scratch;
+  SmallImages images;
   size_t bytes;
 };
 
@@ -519,6 +543,7 @@ static size_t crown_ws_layout(const bf_chain* c, int B, int S, int upto, void* b
   float* cacc = cv.take<float>(M);
   float* partial = cv.take<float>(M * (size_t)max_partial_tiles(c->n0));
   char* cs = cv.take<char>(conv_scratch);
+  small_images_layout(c, (int)M, S, upto, false, cv, ws ? &ws->images : nullptr);
   if (ws) {
     ws->buf[0] = b0; ws->buf[1] = b1; ws->cacc = cacc; ws->partial = partial; ws->conv_scratch = cs; ws->bytes = cv.off;
   }
@@ -534,12 +559,12 @@ extern "C" size_t bf_chain_crown_workspace_bytes(const bf_chain* chain, int B, i
 }
 
 // One sweep; `C` dense [B,S,width of the bounded value], or NULL with onehot_first >= 0: the spec rows are rows
-// onehot_first .. onehot_first+S-1 of the identity for every domain.
+// onehot_first .. onehot_first+S-1 of the identity for every domain.  shared: images that sweeps of the same sizes in the same workspace have in common.
 static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const float* C, int onehot_first,
                        const float* const* alpha_u, const float* const* beta_u, const float* const* alpha_l,
                        const float* const* add, const float* mid, const float* rad, int norm_p, float eps, float* out,
                        void* workspace, size_t workspace_bytes, int B, int S, bf_stream_t stream_,
-                       float* const* influence = nullptr) {
+                       float* const* influence = nullptr, bf::SmallImages* shared = nullptr) {
   BF_REQUIRE(chain && (C || onehot_first >= 0) && mid && out && workspace, BF_E_INVALID, "bf_chain_crown: null argument");
   BF_REQUIRE(norm_p == BF_NORM_BOX || norm_p == BF_NORM_INF || norm_p == BF_NORM_L2 || norm_p == BF_NORM_L1, BF_E_INVALID,
              "bf_chain_crown: bad norm");
@@ -574,6 +599,12 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
     return rc;
   };
   bf::refresh_switches(chain);
+  if (shared && shared->packed) {
+    ws.images = *shared;
+  } else {
+    if (int rc = bf::small_images_pack(chain, &ws.images, stream)) return rc;
+    if (shared) *shared = ws.images;
+  }
   const bool windows_allowed = box && influence == nullptr && !chain->sw.no_windows;
   // rows that bound the neurons of a conv layer stay on the FP32 kernels in every layer below (see CONV_TC_MIN_TILES in conv.cu)
   int top = upto_layer - 1;
@@ -652,7 +683,7 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
     } else if (L.op == BF_OP_LINEAR) {
       const bool last = box && (i == low);  // the fused concretisation handles boxes; Lp balls concretise separately
       float* dst = last ? nullptr : ws.buf[toggle];
-      rc = bf::dispatch_bwd(chain, i, curA, dpos, dneg, epos, eneg, ad, dst, ws.cacc, have_c, last ? mid : nullptr,
+      rc = bf::dispatch_bwd(chain, ws.images, i, curA, dpos, dneg, epos, eneg, ad, dst, ws.cacc, have_c, last ? mid : nullptr,
                             last ? rad : nullptr, last ? ws.partial : nullptr, side, M, S, &ptiles, stream);
       if (last) fused_concretize = true;
       curA = dst;
@@ -674,7 +705,7 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
   else if (fused_concretize) rc = bf::launch_sum_partials(ws.cacc, ws.partial, ptiles, out, M, stream);
   else if (!box) rc = bf::launch_concretize_lp(curA, mid, have_c ? ws.cacc : nullptr, out, side, eps, norm_p, B, S, chain->n0, stream);
   else rc = bf::launch_concretize(curA, mid, rad, have_c ? ws.cacc : nullptr, out, side, B, S, chain->n0, stream);
-  if (rc == BF_OK && bf::tc_may_run(chain, M)) rc = bf::launch_poison_on_status(chain->status, out, M, nullptr, 0, stream);
+  if (rc == BF_OK && bf::tc_may_run(chain, M, ws.images)) rc = bf::launch_poison_on_status(chain->status, out, M, nullptr, 0, stream);
   return rc;
 }
 
@@ -788,9 +819,10 @@ static size_t query_layout(const bf_chain* c, int B, int S, int chunk, void* bas
 }
 
 // mid, rad of the input set: a box [a, b], or (b null) an L-inf ball of radius eps around a, whose centre is read in place
-static int query_input(const float* a, const float* b, float eps, QueryWs& w, size_t n, cudaStream_t stream, const float* C = nullptr, long long per = 0, int B = 0) {
+static int query_input(const float* a, const float* b, float eps, QueryWs& w, size_t n, cudaStream_t stream, const float* C = nullptr, long long per = 0, int B = 0,
+                       const std::vector<SmallPack>& packs = {}) {
   if (!b) w.mid = const_cast<float*>(a);
-  return launch_input_set(a, b, eps, w.mid, w.rad, (long long)n, C, C ? w.both_C : nullptr, per, B, stream);
+  return launch_query_start(a, b, eps, w.mid, w.rad, (long long)n, C, C ? w.both_C : nullptr, per, B, packs.data(), (int)packs.size(), stream);
 }
 
 static int query_relax(const bf_chain* c, const QueryWs& w, float* const* pre_l, float* const* pre_u, int n_relu, int B, cudaStream_t stream) {
@@ -829,7 +861,13 @@ extern "C" int bf_chain_crown_query(const bf_chain* chain, const float* in_a, co
   bf::QueryWs w;
   const size_t need = bf::query_layout(chain, B, S, 0, workspace, &w);
   BF_REQUIRE(workspace_bytes >= need, BF_E_WORKSPACE, "bf_chain_crown_query: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
-  int rc = bf::query_input(in_a, in_b, eps, w, (size_t)B * chain->n0, bf::as_stream(stream), w.both_C ? C : nullptr, (long long)S * chain->layers.back().n_out, B);
+  const int rows = w.both_C ? 2 * S : S;  // of a domain in a sweep
+  bf::refresh_switches(chain);
+  bf::CrownWs sweep;
+  bf::crown_ws_layout(chain, B, rows, (int)chain->layers.size(), w.sweep, &sweep);
+  const std::vector<bf::SmallPack> packs = bf::small_images_packs(chain, &sweep.images);
+  int rc = bf::query_input(in_a, in_b, eps, w, (size_t)B * chain->n0, bf::as_stream(stream), w.both_C ? C : nullptr, (long long)S * chain->layers.back().n_out, B,
+                           packs);
   if (rc == BF_OK)
     rc = ibp_sweep(chain, w.mid, w.rad, BF_IN_MID_RAD, nullptr, nullptr, nullptr, nullptr, w.pre_l.data(), w.pre_u.data(), nullptr, nullptr,
                    nullptr, w.scratch, w.scratch_bytes, B, stream);
@@ -837,12 +875,12 @@ extern "C" int bf_chain_crown_query(const bf_chain* chain, const float* in_a, co
   if (w.both_C) {
     if (rc == BF_OK)
       rc = crown_sweep(chain, 0, BF_SIDE_LOWER, w.both_C, -1, w.au.data(), w.bu.data(), w.al.data(), nullptr, w.mid, w.rad, BF_NORM_BOX, 0.f, w.both, w.sweep,
-                       w.sweep_bytes, B, 2 * S, stream);
+                       w.sweep_bytes, B, rows, stream, nullptr, &sweep.images);
     return rc == BF_OK ? bf::launch_split_sides(w.both, out_l, out_u, B, S, bf::as_stream(stream)) : rc;
   }
   for (int side = 0; side < 2 && rc == BF_OK; ++side)
     rc = crown_sweep(chain, 0, side, C, -1, w.au.data(), w.bu.data(), w.al.data(), nullptr, w.mid, w.rad, BF_NORM_BOX, 0.f,
-                     side == BF_SIDE_LOWER ? out_l : out_u, w.sweep, w.sweep_bytes, B, S, stream);
+                     side == BF_SIDE_LOWER ? out_l : out_u, w.sweep, w.sweep_bytes, B, rows, stream, nullptr, &sweep.images);
   return rc;
 }
 
@@ -876,11 +914,12 @@ extern "C" int bf_chain_crown_intermediate(const bf_chain* chain, const float* i
     if ((rc = bf::query_relax(chain, w, set_l[cur].data(), set_u[cur].data(), r, B, stream)) != BF_OK) return rc;
     for (int s = 0; s < n; s += chunk_rows) {
       const int cnt = std::min(chunk_rows, n - s);
+      bf::SmallImages images;
       for (int side = 0; side < 2; ++side) {
         float* all = side == BF_SIDE_LOWER ? w.new_l[r] : w.new_u[r];
         float* to = cnt == n ? all : (side == BF_SIDE_LOWER ? w.chunk_l : w.chunk_u);
         rc = crown_sweep(chain, upto, side, nullptr, s, w.au.data(), w.bu.data(), w.al.data(), nullptr, w.mid, w.rad, BF_NORM_BOX, 0.f, to, w.sweep,
-                         w.sweep_bytes, B, cnt, stream_);
+                         w.sweep_bytes, B, cnt, stream_, nullptr, &images);
         if (rc != BF_OK) return rc;
       }
       if (cnt < n && (rc = bf::launch_place_columns(w.chunk_l, w.chunk_u, w.new_l[r], w.new_u[r], B, cnt, n, s, stream)) != BF_OK) return rc;
@@ -895,8 +934,9 @@ extern "C" int bf_chain_crown_intermediate(const bf_chain* chain, const float* i
     if (rc != BF_OK) return rc;
   }
   if ((rc = bf::query_relax(chain, w, set_l[cur].data(), set_u[cur].data(), R, B, stream)) != BF_OK) return rc;
+  bf::SmallImages images;
   for (int side = 0; side < 2 && rc == BF_OK; ++side)
     rc = crown_sweep(chain, 0, side, C, -1, w.au.data(), w.bu.data(), w.al.data(), nullptr, w.mid, w.rad, BF_NORM_BOX, 0.f,
-                     side == BF_SIDE_LOWER ? out_l : out_u, w.sweep, w.sweep_bytes, B, S, stream_);
+                     side == BF_SIDE_LOWER ? out_l : out_u, w.sweep, w.sweep_bytes, B, S, stream_, nullptr, &images);
   return rc;
 }

@@ -24,6 +24,7 @@ struct AlphaWs {
   float* row_weight;  // [M] d objective / d lower per spec row (min / softmin objectives)
   float* metric;
   int* improve;
+  SmallImages images;
   void* conv_scratch;  // ReLU-scaled coefficients of a conv layer's backward step
   size_t state_begin, state_bytes;  // grad/m/v (+ beta state) region, zero-initialised per call
   size_t bytes;
@@ -71,6 +72,7 @@ static size_t alpha_ws_layout(const bf_chain* c, int B, int S, bool with_beta, v
   for (const bf_layer_desc& L : c->layers)
     if (L.op == BF_OP_CONV2D) conv_scratch = std::max(conv_scratch, crown_bwd_conv2d_scratch_bytes((int)M, L));
   w.conv_scratch = cv.take<char>(conv_scratch);
+  small_images_layout(c, (int)M, S, (int)c->layers.size(), true, cv, &w.images);
   w.bytes = cv.off;
   if (ws) *ws = w;
   return cv.off;
@@ -105,7 +107,7 @@ static int alpha_bwd_layer(const bf_chain* c, const AlphaWs& ws, int layer, cons
                            const float* rad, float* partial, int side, int M, int S, int* ptiles, cudaStream_t stream) {
   const bf_layer_desc& L = c->layers[layer];
   if (L.op == BF_OP_LINEAR)
-    return dispatch_bwd(c, layer, A, dpos, dneg, epos, eneg, add, dst, ws.cacc, accumulate, mid, rad, partial, side, M, S, ptiles, stream);
+    return dispatch_bwd(c, ws.images, layer, A, dpos, dneg, epos, eneg, add, dst, ws.cacc, accumulate, mid, rad, partial, side, M, S, ptiles, stream);
   return launch_crown_bwd_conv2d(A, dpos, dneg, epos, eneg, L.W, L.bias, dst, ws.cacc, accumulate, M, S, L, ws.conv_scratch, stream, add,
                                  c->status != nullptr, c->status);
 }
@@ -169,7 +171,7 @@ static int alpha_adjoint(const bf_chain* c, const AlphaWs& ws, const float* cons
     if (L.op == BF_OP_LINEAR) {
       float* hout = (r < R - 1) ? ws.H[r & 1] : nullptr;
       const bool from_box = (r == 0) && h0_fused;
-      rc = dispatch_adjoint(c, layer, hprev, from_box ? 1 : 0, from_box ? in.mid : nullptr, from_box ? in.rad : nullptr, ws.Ahat[r],
+      rc = dispatch_adjoint(c, ws.images, layer, hprev, from_box ? 1 : 0, from_box ? in.mid : nullptr, from_box ? in.rad : nullptr, ws.Ahat[r],
                             ws.sl[r], ws.au[r], nullptr, ws.bu[r], pre_l[r], pre_u[r], hout, ws.grad[r],
                             with_beta ? ws.gsum[r] : nullptr, M, S, stream, with_beta ? gw : nullptr);
     } else {
@@ -270,6 +272,7 @@ static int alpha_loop(const char* who, const bf_chain* chain, const float* C, co
     bf::set_error("%s: cudaMemsetAsync failed", who);
     return BF_E_CUDA;
   }
+  if ((rc = bf::small_images_pack(chain, &ws.images, stream)) != BF_OK) return rc;
   if ((rc = bf::relax_all(chain, ws, pre_l, pre_u, alpha, false, B, stream)) != BF_OK) return rc;
   for (int r = 0; r < R; ++r) {
     const int n = chain->layers[chain->relu_layers[r]].n_in;
@@ -318,7 +321,7 @@ static int alpha_loop(const char* who, const bf_chain* chain, const float* C, co
     rc = bf::alpha_sweep(chain, ws, C, BF_SIDE_UPPER, false, false, in, best_upper, B, S, stream);
     if (rc != BF_OK) return rc;
   }
-  if (bf::tc_may_run(chain, B * S)) {  // a tensor-core wait that expired invalidates every bound of this call
+  if (bf::tc_may_run(chain, B * S, ws.images)) {  // a tensor-core wait that expired invalidates every bound of this call
     rc = bf::launch_poison_on_status(chain->status, best_lower, (long long)B * S, best_upper, best_upper ? (long long)B * S : 0, stream);
     if (rc != BF_OK) return rc;
     rc = bf::launch_poison_on_status(chain->status, metric, B, nullptr, 0, stream);
@@ -380,6 +383,7 @@ extern "C" int bf_chain_alpha_grad(const bf_chain* chain, const float* C, const 
     bf::set_error("bf_chain_alpha_grad: cudaMemsetAsync failed");
     return BF_E_CUDA;
   }
+  if ((rc = bf::small_images_pack(chain, &ws.images, stream)) != BF_OK) return rc;
   if ((rc = bf::relax_all(chain, ws, pre_l, pre_u, alpha, false, B, stream)) != BF_OK) return rc;
   rc = bf::alpha_sweep(chain, ws, C, BF_SIDE_LOWER, true, false, in, lower, B, S, stream);
   if (rc != BF_OK) return rc;
@@ -390,7 +394,7 @@ extern "C" int bf_chain_alpha_grad(const bf_chain* chain, const float* C, const 
     const int n = chain->layers[chain->relu_layers[r]].n_in;
     rc = bf::launch_scale_copy(ws.grad[r], scale, grad[r], (long long)B * n, stream);
     if (rc != BF_OK) return rc;
-    if (bf::tc_may_run(chain, B * S)) {
+    if (bf::tc_may_run(chain, B * S, ws.images)) {
       rc = bf::launch_poison_on_status(chain->status, grad[r], (long long)B * n, r == 0 ? lower : nullptr, (long long)B * S, stream);
       if (rc != BF_OK) return rc;
     }
@@ -485,7 +489,8 @@ static int shared_loop(const char* who, const bf_chain* chain, const float* C, c
     bf::set_error("%s: cudaMemsetAsync failed", who);
     return BF_E_CUDA;
   }
-  int rc;
+  int rc = bf::small_images_pack(chain, &ws.images, stream);
+  if (rc != BF_OK) return rc;
   auto width = [&](int r) { return chain->layers[chain->relu_layers[r]].n_in; };
   auto stride = [&](int r) { return split_strides ? split_strides[r] : width(r); };
   for (int t = 0; t <= steps; ++t) {
@@ -539,7 +544,7 @@ static int shared_loop(const char* who, const bf_chain* chain, const float* C, c
     rc = bf::alpha_sweep(chain, ws, C, BF_SIDE_UPPER, false, false, in, best_upper, B, S, stream);
     if (rc != BF_OK) return rc;
   }
-  if (bf::tc_may_run(chain, B * S)) {  // a tensor-core wait that expired invalidates every bound of this call
+  if (bf::tc_may_run(chain, B * S, ws.images)) {  // a tensor-core wait that expired invalidates every bound of this call
     rc = bf::launch_poison_on_status(chain->status, best_lower, (long long)B * S, best_upper, best_upper ? (long long)B * S : 0, stream);
     if (rc != BF_OK) return rc;
     rc = bf::launch_poison_on_status(chain->status, metric, B, nullptr, 0, stream);

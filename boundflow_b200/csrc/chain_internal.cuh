@@ -17,7 +17,6 @@ struct bf_chain {
   // tensor-core path: per layer, packed hi/lo weight images for the backward (W^T as B) and
   // adjoint (W as B) orientation inside a caller-owned buffer, plus a device status word
   std::vector<const unsigned char*> pk_bwd, pk_adj, pk_adj_fm;  // pk_adj_fm: 128-row images for the feature-major adjoint kernel
-  std::vector<const unsigned char*> pk_small_bwd, pk_small_adj;  // bfloat16 parts for sweeps of few rows (crown_small_tc.cu)
   int* status = nullptr;
   // A/B switches (environment variables BF_B200_*), refreshed at the start of every whole-chain call and read by
   // the per-layer dispatch of that call
@@ -51,6 +50,20 @@ struct Carver {
   }
 };
 
+// Images of the Linear weights that crown_small_tc.cu multiplies by: they lie in the workspace of the call that reads them and are packed at its start
+// (a launch of 3 to 4 us, or part of a query's first), so a call sees the weights as they are when it runs, on whichever stream.
+struct SmallImages {
+  std::vector<unsigned char*> bwd, adj;  // per layer; null: another kernel takes the step
+  bool packed = false;
+  const unsigned char* backward(int layer) const { return bwd.empty() ? nullptr : bwd[layer]; }
+  const unsigned char* adjoint(int layer) const { return adj.empty() ? nullptr : adj[layer]; }
+};
+// Places for the layers below `upto` of a sweep of M rows, S per domain (adjoint: and of its gradient sweep)
+void small_images_layout(const bf_chain* c, int M, int S, int upto, bool adjoint, Carver& cv, SmallImages* images);
+// Fills them, or drops them all where the switches or an unprepared chain leave the rows to other kernels.  Behind refresh_switches().
+int small_images_pack(const bf_chain* c, SmallImages* images, cudaStream_t stream);
+std::vector<SmallPack> small_images_packs(const bf_chain* c, SmallImages* images);  // what there is to fill
+
 // Concretisation partial sums per row, at most, of whichever backward kernel takes a first layer of n0 inputs
 inline int max_partial_tiles(int n0) {
   return std::max(std::max(std::max(crown_bwd_partial_tiles(n0), crown_tc_partial_tiles(n0, 32)), crown_tc_persist_max_partial_tiles(n0)),
@@ -60,15 +73,15 @@ inline int max_partial_tiles(int n0) {
 // Re-reads the BF_B200_* environment switches into chain->sw (called once per whole-chain entry point).
 void refresh_switches(const bf_chain* c);
 // True when a sweep over M coefficient rows may have run tensor-core kernels (whose status word then guards the results).
-bool tc_may_run(const bf_chain* c, int M);
+bool tc_may_run(const bf_chain* c, int M, const SmallImages& images);
 
 // Backward contraction of linear layer `layer` (tensor-core path when the packed weights exist and the
-// problem is large enough, FFMA tiles otherwise); *ptiles receives the number of column tiles of the
+// problem is small or large enough, FFMA tiles otherwise); *ptiles receives the number of column tiles of the
 // concretisation partial-sum buffer.
-int dispatch_bwd(const bf_chain* c, int layer, const float* A, const float* dpos, const float* dneg, const float* epos,
+int dispatch_bwd(const bf_chain* c, const SmallImages& images, int layer, const float* A, const float* dpos, const float* dneg, const float* epos,
                  const float* eneg, const float* add, float* A_prev, float* delta, int accumulate, const float* mid,
                  const float* rad, float* partial, int side, int M, int S, int* ptiles, cudaStream_t stream);
-int dispatch_adjoint(const bf_chain* c, int layer, const float* Hprev, int first_layer, const float* mid, const float* rad,
+int dispatch_adjoint(const bf_chain* c, const SmallImages& images, int layer, const float* Hprev, int first_layer, const float* mid, const float* rad,
                      const float* Ahat, const float* dpos, const float* dneg, const float* epos, const float* eneg,
                      const float* pre_l, const float* pre_u, float* hout, float* grad, float* gsum, int M, int S,
                      cudaStream_t stream, const float* gw = nullptr);

@@ -4,7 +4,7 @@
 //
 // Such a launch is a chain of latencies: operands, contraction, epilogue, next launch.  On FP32 units the contraction alone is 40 clocks a
 // term (gemm_small.cuh: shared-memory reads).  Here a CTA owns 128 output features x 32 coefficient rows:
-//   * features are the MMA's M side: weights are packed once (pack_small_weights_kernel) as the shared-memory images that the MMA reads, per
+//   * features are the MMA's M side: weights are packed at the start of a call (pack_small_weights_kernel) as the shared-memory images that the MMA reads, per
 //     (feature tile, 16 terms), and come by bulk copies, 32 terms (24 KB) a stage of a ring of seven;
 //   * rows are its N side: sixteen warps load, scale and split them, and read the accumulators back afterwards.
 // Where there are fewer tiles than SMs a cluster of two or four CTAs shares a tile: each takes a part of the terms, leaves its sums in shared memory
@@ -648,7 +648,8 @@ __global__ void __launch_bounds__(THREADS, 1) crown_small_tc_kernel(const __grid
   if (CS > 1) cluster_wait();
 }
 
-// Images of up to PACK_JOBS weights in one launch: a block takes 256 (feature, eight terms) items of a job.
+// Images of up to PACK_JOBS weights in one launch: a block takes 256 (feature, eight terms) items of a job.  The blocks behind those form the input set and
+// the negated spec rows of a query (a launch of its own in front of it cost 784-100-100-10, 64 inputs, 3.8 us of 61).
 constexpr int PACK_JOBS = 16;
 struct PackJob {
   const float* W;
@@ -659,7 +660,38 @@ struct PackJobs {
   PackJob job[PACK_JOBS];
   int count;
 };
-__global__ void __launch_bounds__(256) pack_small_weights_kernel(const __grid_constant__ PackJobs jobs) {
+struct QueryStart {
+  const float *a, *b, *C;
+  float *mid, *rad, *C2;
+  float eps;
+  long long n, per, total;
+  int set_blocks;  // blocks for the input set; the rest of the grid is for the spec rows
+};
+__device__ __forceinline__ void query_start_block(const QueryStart& q, int block, int blocks) {
+  if (block >= q.set_blocks) {  // C2[b] = (C[b], -C[b])
+    for (long long i = (block - q.set_blocks) * 256ll + threadIdx.x; i < q.total; i += (blocks - q.set_blocks) * 256ll) {
+      const long long o = i + i / q.per * q.per;
+      const float c = q.C[i];
+      q.C2[o] = c;
+      q.C2[o + q.per] = -c;
+    }
+    return;
+  }
+  for (long long i = block * 256ll + threadIdx.x; i < q.n; i += q.set_blocks * 256ll) {
+    if (q.b) {
+      const float lo = q.a[i], up = q.b[i];
+      q.mid[i] = (lo + up) / 2.f;
+      q.rad[i] = (up - lo) / 2.f;
+    } else {
+      q.rad[i] = q.eps;
+    }
+  }
+}
+__global__ void __launch_bounds__(256) pack_small_weights_kernel(const __grid_constant__ PackJobs jobs, int pack_blocks, const __grid_constant__ QueryStart q) {
+  if ((int)blockIdx.x >= pack_blocks) {
+    query_start_block(q, (int)blockIdx.x - pack_blocks, (int)gridDim.x - pack_blocks);
+    return;
+  }
   int j = 0;
   while (j + 1 < jobs.count && (int)blockIdx.x >= jobs.job[j + 1].first_block) ++j;
   const PackJob& p = jobs.job[j];
@@ -700,22 +732,31 @@ int small_tc_tiles(int M, int N, int K) { return ceil_div(N, stc::TF) * small_tc
 int small_tc_max_tiles(int N) { return ceil_div(N, stc::TF) * 4; }
 size_t small_tc_packed_bytes(int N, int K) { return (size_t)ceil_div(N, stc::TF) * ceil_div(K, stc::KS) * stc::W_STAGE; }
 
-int small_tc_pack(const SmallPack* packs, int count, cudaStream_t stream) {
-  for (int first = 0; first < count; first += stc::PACK_JOBS) {
+static int pack_images(const SmallPack* packs, int count, const stc::QueryStart* start, int start_blocks, cudaStream_t stream) {
+  int first = 0;
+  do {
     stc::PackJobs jobs{};
     int blocks = 0;
-    for (int i = first; i < count && jobs.count < stc::PACK_JOBS; ++i) {
-      const SmallPack& p = packs[i];
+    for (; first < count && jobs.count < stc::PACK_JOBS; ++first) {
+      const SmallPack& p = packs[first];
       const int N = p.transposed ? p.cols : p.rows, K = p.transposed ? p.rows : p.cols, nst = ceil_div(K, stc::KS);
       jobs.job[jobs.count++] = {p.W, p.out, p.cols, p.transposed, N, K, nst, blocks};
       blocks += ceil_div(N, stc::TF) * nst * 4 * stc::TF / 256;
     }
-    stc::pack_small_weights_kernel<<<blocks, 256, 0, stream>>>(jobs);
+    stc::pack_small_weights_kernel<<<blocks + start_blocks, 256, 0, stream>>>(jobs, blocks, start ? *start : stc::QueryStart{});
     BF_CHECK_LAUNCH("pack_small_weights_kernel");
-  }
+    start_blocks = 0;
+  } while (first < count);
   return BF_OK;
 }
+int launch_query_start(const float* a, const float* b, float eps, float* mid, float* rad, long long n, const float* C, float* C2, long long per, int B,
+                       const SmallPack* packs, int count, cudaStream_t stream) {
+  auto blocks = [](long long items) { return (int)std::min((items + 255) / 256, 148ll * 16); };
+  const stc::QueryStart q{a, b, C, mid, rad, C2, eps, n, per, B * per, blocks(n)};
+  return pack_images(packs, count, &q, q.set_blocks + (C2 ? blocks(q.total) : 0), stream);
+}
 
+int small_tc_pack(const SmallPack* packs, int count, cudaStream_t stream) { return count ? pack_images(packs, count, nullptr, 0, stream) : BF_OK; }
 template <int MODE, int PRO, int CS>
 static int launch_small_n(stc::Args g, cudaStream_t stream) {
   g.dS.set((uint32_t)g.S);

@@ -70,35 +70,6 @@ int launch_relu_relax(const float* l, const float* u, const float* alpha, int al
   return launch_relu_relax(&seg, 1, B, stream);
 }
 
-__global__ void __launch_bounds__(256) input_set_kernel(const float* __restrict__ a, const float* __restrict__ b, float eps, float* __restrict__ mid,
-                                                        float* __restrict__ rad, long long n, const float* __restrict__ C, float* __restrict__ C2,
-                                                        long long per, long long total) {
-  if (blockIdx.y == 1) {  // C2[b] = (C[b], -C[b])
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-      const long long o = i + i / per * per;
-      const float c = C[i];
-      C2[o] = c;
-      C2[o + per] = -c;
-    }
-    return;
-  }
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    if (b) {
-      const float lo = a[i], up = b[i];
-      mid[i] = (lo + up) / 2.f;
-      rad[i] = (up - lo) / 2.f;
-    } else {
-      rad[i] = eps;
-    }
-  }
-}
-int launch_input_set(const float* a, const float* b, float eps, float* mid, float* rad, long long n, const float* C, float* C2, long long per, int B,
-                     cudaStream_t stream) {
-  input_set_kernel<<<dim3(ew_grid(std::max(n, C2 ? B * per : 0), 256), C2 ? 2 : 1), 256, 0, stream>>>(a, b, eps, mid, rad, n, C, C2, per, B * per);
-  BF_CHECK_LAUNCH("input_set_kernel");
-  return BF_OK;
-}
-
 __global__ void __launch_bounds__(256) split_sides_kernel(const float* __restrict__ both, float* __restrict__ lower, float* __restrict__ upper, int S, long long total) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long o = i + i / S * S;

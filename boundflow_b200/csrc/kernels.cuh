@@ -33,7 +33,7 @@ int launch_crown_adjoint_linear_tc(const float* Hprev, int first_layer, const fl
 int crown_tc_partial_tiles(int N, int K);
 void tc_tile_shape(int N, int K, int* BN, int* ntiles, int* nkb);
 
-// crown_small_tc.cu (few coefficient rows on the tensor cores; weights packed by small_tc_pack)
+// crown_small_tc.cu (few coefficient rows on the tensor cores; weights packed by small_tc_pack in every call)
 bool small_tc_supports(int M, int N, int K, int S, bool adjoint);
 int small_tc_tiles(int M, int N, int K);  // parts of the features (= partial sums per row)
 int small_tc_max_tiles(int N);            // the largest count any M and K give (workspace sizing)
@@ -44,6 +44,10 @@ struct SmallPack {
   unsigned char* out;
 };
 int small_tc_pack(const SmallPack* packs, int count, cudaStream_t stream);
+// What a query begins with, in one launch: mid = (a + b) / 2, rad = (b - a) / 2; b null: rad = eps (mid is a itself); with C2, C2[b] = (C[b], -C[b]) for
+// B blocks of `per` values; and the images
+int launch_query_start(const float* a, const float* b, float eps, float* mid, float* rad, long long n, const float* C, float* C2, long long per, int B,
+                       const SmallPack* packs, int count, cudaStream_t stream);
 int launch_crown_bwd_small_tc(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg, const float* add,
                               const unsigned char* Wpk, const float* W, const float* kbias, float* A_prev, float* delta, int accumulate, const float* mid,
                               const float* rad, float* partial, int side, int M, int S, int K, int N, int* status, cudaStream_t stream);
@@ -88,10 +92,6 @@ constexpr int RELAX_SEGMENTS = 16;  // per launch
 int launch_relu_relax(const RelaxSegment* seg, int count, int B, cudaStream_t stream);
 int launch_relu_relax(const float* l, const float* u, const float* alpha, int alpha_stride, float* alpha_u,
                       float* beta_u, float* alpha_l, int B, int n, cudaStream_t stream);
-// mid = (a + b) / 2, rad = (b - a) / 2; b null: rad = eps (mid is a itself)
-// and, with C2, C2[b] = (C[b], -C[b]) for B blocks of `per` values
-int launch_input_set(const float* a, const float* b, float eps, float* mid, float* rad, long long n, const float* C, float* C2, long long per, int B,
-                     cudaStream_t stream);
 // lower, -upper [B,S] from both [B,2S]
 int launch_split_sides(const float* both, float* lower, float* upper, int B, int S, cudaStream_t stream);
 // columns at .. at + cnt - 1 of [B,n] matrices from [B,cnt] ones

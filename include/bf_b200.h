@@ -361,7 +361,9 @@ int bf_chain_num_relu(const bf_chain* chain);
  * shared-memory image the MMA consumes.  bf_chain_tc_prepare does that packing into a
  * caller-owned device buffer of bf_chain_tc_bytes(chain) bytes (256-byte aligned) that must
  * outlive the chain; without it, or with the environment variable BF_B200_FORCE_FFMA=1, or
- * for tiny problems, the FP32 FFMA kernels are used (for Conv2d layers too).  Every wait inside the tensor-core
+ * for tiny problems, the FP32 FFMA kernels are used (for Conv2d layers too).  These images are the
+ * weights as they were then: prepare again after changing a weight in place.  Sweeps of few rows
+ * read images that every call packs into its own workspace.  Every wait inside the tensor-core
  * kernels is bounded; bf_chain_tc_status (synchronous) returns non-zero in *status if a
  * wait ever expired, in which case results of that call are invalid. */
 size_t bf_chain_tc_bytes(const bf_chain* chain);
