@@ -237,7 +237,7 @@ def ibp_trace(
         in_b, in_mode = row_dev, _lib.IN_CENTER_DEV
     _lib.check(
         lib.bf_chain_ibp(
-            chain.handle, _lib.ptr(mid), _lib.ptr(in_b), in_mode,
+            chain.interval_handle, _lib.ptr(mid), _lib.ptr(in_b), in_mode,
             _lib.ptr_array(splits), _lib.int_array(strides),
             _lib.ptr_array(cons_l), _lib.ptr_array(cons_u),
             _lib.ptr_array(pre_l), _lib.ptr_array(pre_u),
@@ -566,10 +566,10 @@ def ibp_query(chain: CudaChain, plain, device: torch.device, B: int) -> Interval
     """Interval bounds of the chain's output in one call of the library."""
     shape = (B,) + tuple(chain.output_shape)
     lower, upper = torch.empty(shape, dtype=torch.float32, device=device), torch.empty(shape, dtype=torch.float32, device=device)
-    nbytes = chain.lib.bf_chain_query_workspace_bytes(chain.handle, B, 0, 0)
+    nbytes = chain.lib.bf_chain_query_workspace_bytes(chain.interval_handle, B, 0, 0)
     ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
     a, b, eps = plain
-    _lib.check(chain.lib.bf_chain_ibp_query(chain.handle, a.data_ptr(), _lib.ptr(b), eps, lower.data_ptr(), upper.data_ptr(), ws.data_ptr(), nbytes, B,
+    _lib.check(chain.lib.bf_chain_ibp_query(chain.interval_handle, a.data_ptr(), _lib.ptr(b), eps, lower.data_ptr(), upper.data_ptr(), ws.data_ptr(), nbytes, B,
                                             _stream_ptr(device)))
     return IntervalState(lower=lower, upper=upper)
 

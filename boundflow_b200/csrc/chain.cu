@@ -372,15 +372,19 @@ extern "C" int bf_chain_tc_prepare(bf_chain* chain, void* buffer, size_t bytes, 
   BF_REQUIRE(bytes >= bf_chain_tc_bytes(chain), BF_E_WORKSPACE, "bf_chain_tc_prepare: %zu bytes needed", bf_chain_tc_bytes(chain));
   cudaStream_t stream = bf::as_stream(stream_);
   unsigned char* base = static_cast<unsigned char*>(buffer);
-  if (cudaMemsetAsync(base, 0, 256, stream) != cudaSuccess) {
-    bf::set_error("bf_chain_tc_prepare: cudaMemsetAsync failed");
-    return BF_E_CUDA;
+  // the same buffer again: new images in the old places, and nothing that a call in another thread reads is touched
+  const bool again = chain->status == reinterpret_cast<int*>(base);
+  if (!again) {
+    if (cudaMemsetAsync(base, 0, 256, stream) != cudaSuccess) {
+      bf::set_error("bf_chain_tc_prepare: cudaMemsetAsync failed");
+      return BF_E_CUDA;
+    }
+    chain->status = reinterpret_cast<int*>(base);
+    chain->pk_bwd.assign(chain->layers.size(), nullptr);
+    chain->pk_adj.assign(chain->layers.size(), nullptr);
+    chain->pk_adj_fm.assign(chain->layers.size(), nullptr);
   }
-  chain->status = reinterpret_cast<int*>(base);
   size_t off = 256;
-  chain->pk_bwd.assign(chain->layers.size(), nullptr);
-  chain->pk_adj.assign(chain->layers.size(), nullptr);
-  chain->pk_adj_fm.assign(chain->layers.size(), nullptr);
   for (size_t i = 0; i < chain->layers.size(); ++i) {
     const bf_layer_desc& L = chain->layers[i];
     if (L.op != BF_OP_LINEAR) continue;
@@ -399,6 +403,7 @@ extern "C" int bf_chain_tc_prepare(bf_chain* chain, void* buffer, size_t bytes, 
     off += bf::align_up(bf::tc_packed_bytes(L.n_out, L.n_in, bf::tc_adjoint_tile_rows()));
     rc = bf::tc_pack_weights(L.W, L.n_out, L.n_in, 0, pf, stream, bf::tc_adjoint_tile_rows());
     if (rc != BF_OK) return rc;
+    if (again) continue;
     chain->pk_adj_fm[i] = pf;
     chain->pk_bwd[i] = pb;
     chain->pk_adj[i] = pa;

@@ -12,6 +12,7 @@ to the kernels as the equal dense convolution (`dense_conv_weight`).
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from dataclasses import dataclass
 from typing import Any, Dict, List, Optional, Sequence, Tuple
 
@@ -93,8 +94,18 @@ def _numel(shape: Sequence[int]) -> int:
     return n
 
 
+def _version(t: torch.Tensor) -> int:
+    """In-place version counter; tensors made in inference mode have none."""
+    return 0 if t.is_inference() else int(t._version)
+
+
 class CudaChain:
-    """Validated chain with device parameters and its `bf_chain` handle."""
+    """Validated chain with device parameters and its `bf_chain` handle.
+
+    Contiguous fp32 CUDA parameters are read where they are, others from device copies.  What is derived from a parameter follows it: the packed
+    images of the large tensor-core kernels are packed again, in place, when a Linear weight's version counter has moved (`handle`), and
+    `compile_chain` compiles again when that of a copied parameter has.  Images and copies are made on the stream of the call that makes them; calls on
+    other streams wait for that work."""
 
     def __init__(self, module: Any, input_shape: Sequence[int], device: torch.device, *, input_name: Optional[str] = None):
         self.lib = _lib.load()
@@ -111,10 +122,18 @@ class CudaChain:
         self.output_name = task.output_values[0]
         self.input_shape = tuple(int(d) for d in input_shape)
 
-        def dev(t: Any) -> torch.Tensor:
-            if not torch.is_tensor(t):
-                t = torch.as_tensor(t)
-            return t.detach().to(device=self.device, dtype=torch.float32).contiguous()
+        self._copied: Dict[str, int] = {}  # parameters with a device copy: version copied
+        self._owned: List[torch.Tensor] = []  # device memory of the chain's own
+
+        def dev(name: str, attrs: Any = None) -> torch.Tensor:
+            t = params[name]
+            given = t if torch.is_tensor(t) else torch.as_tensor(t)
+            out = dense_conv_weight(given.detach().to(device=self.device, dtype=torch.float32).contiguous(), attrs)
+            if torch.is_tensor(t) and out.data_ptr() != t.data_ptr():
+                self._copied[name] = _version(t)
+            if out.data_ptr() != given.data_ptr():
+                self._owned.append(out)
+            return out
 
         layers: List[ChainLayer] = []
         shape = self.input_shape
@@ -124,15 +143,15 @@ class CudaChain:
                 raise NotImplementedError(f"op '{op.name}' does not continue the chain at value '{cur}'")
             t = op.op_type
             if t == "linear":
-                W = dev(params[op.inputs[1]])
-                b = dev(params[op.inputs[2]]) if len(op.inputs) == 3 else None
+                W = dev(op.inputs[1])
+                b = dev(op.inputs[2]) if len(op.inputs) == 3 else None
                 if W.dim() != 2 or len(shape) != 1 or W.shape[1] != shape[0]:
                     raise ValueError(f"linear '{op.name}': weight {tuple(W.shape)} does not match input shape {shape}")
                 out_shape = (int(W.shape[0]),)
                 layers.append(ChainLayer("linear", op.name, cur, op.outputs[0], shape, out_shape, W, b))
             elif t == "conv2d":
-                W = dense_conv_weight(dev(params[op.inputs[1]]), op.attrs)
-                b = dev(params[op.inputs[2]]) if len(op.inputs) == 3 else None
+                W = dev(op.inputs[1], op.attrs)
+                b = dev(op.inputs[2]) if len(op.inputs) == 3 else None
                 st, pd = _pair(op.attrs.get("stride", 1)), _pair(op.attrs.get("padding", 0))
                 if len(shape) != 3 or W.dim() != 4 or W.shape[1] != shape[0]:
                     raise ValueError(f"conv2d '{op.name}': weight {tuple(W.shape)} does not match input shape {shape}")
@@ -186,26 +205,74 @@ class CudaChain:
                 d.ph, d.pw = l.padding
         handle = C.c_void_p()
         _lib.check(self.lib.bf_chain_create(descs, len(layers), C.byref(handle)))
-        self.handle = handle
-        # tensor-core path: split + pack the static weights once (buffer owned here, freed with the chain)
-        nbytes = int(self.lib.bf_chain_tc_bytes(handle))
-        self._tc_buffer = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
-        _lib.check(self.lib.bf_chain_tc_prepare(handle, self._tc_buffer.data_ptr(), nbytes, torch.cuda.current_stream(self.device).cuda_stream))
+        self._handle = handle
+        # tensor-core path: split + pack the weights (buffer owned here, freed with the chain)
+        self._linear = [l.W for l in layers if l.op == "linear"]
+        self._lock = threading.Lock()
+        self._packed: Optional[Tuple[int, ...]] = None  # versions of the Linear weights in the images
+        self._work: Optional[Tuple[torch.cuda.Event, int]] = None  # behind the copies and images, and the stream that made them
+        self._tc_buffer = torch.empty(int(self.lib.bf_chain_tc_bytes(handle)), dtype=torch.uint8, device=self.device)
+        self._owned.append(self._tc_buffer)
+        self._pack()
+
+    def _versions(self) -> Tuple[int, ...]:
+        return tuple([_version(W) for W in self._linear])
+
+    def _raw_stream(self) -> int:
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if self.device.index is None else self.device.index)
+
+    def _pack(self) -> None:
+        versions = self._versions()
+        _lib.check(self.lib.bf_chain_tc_prepare(self._handle, self._tc_buffer.data_ptr(), self._tc_buffer.numel(), self._raw_stream()))
+        if not torch.cuda.is_current_stream_capturing():  # else packed when the graph runs: by calls inside it, not for those outside
+            ready = torch.cuda.Event()
+            ready.record(torch.cuda.current_stream(self.device))
+            self._work, self._packed = (ready, self._raw_stream()), versions
+
+    def _behind_own_work(self) -> None:
+        """The current stream continues behind the stream that has made images and copies.  (A graph is captured on an idle device.)"""
+        work = self._work
+        if work is not None and self._raw_stream() != work[1] and not torch.cuda.is_current_stream_capturing():
+            stream = torch.cuda.current_stream(self.device)
+            stream.wait_event(work[0])
+            for t in self._owned:
+                t.record_stream(stream)
+
+    @property
+    def handle(self) -> C.c_void_p:
+        """The `bf_chain` for calls that multiply coefficient rows: images of the Linear weights as they are now."""
+        if self._packed != self._versions():
+            with self._lock:
+                if self._packed != self._versions():
+                    self._behind_own_work()
+                    self._pack()
+        self._behind_own_work()
+        return self._handle
+
+    @property
+    def interval_handle(self) -> C.c_void_p:
+        """The `bf_chain` for interval passes, which read the weights themselves."""
+        self._behind_own_work()
+        return self._handle
+
+    def copies_current(self, params: Any) -> bool:
+        """Whether the parameters that the chain has copied are as they were then."""
+        return all(_version(params[name]) == v for name, v in self._copied.items())
 
     def tc_status(self) -> int:
         """Synchronous read of the tensor-core kernels' status word (non-zero: a bounded wait expired)."""
         st = C.c_int(0)
-        _lib.check(self.lib.bf_chain_tc_status(self.handle, C.byref(st)))
+        _lib.check(self.lib.bf_chain_tc_status(self._handle, C.byref(st)))
         return int(st.value)
 
     def __del__(self):
-        h = getattr(self, "handle", None)
+        h = getattr(self, "_handle", None)
         if h:
             try:
                 self.lib.bf_chain_destroy(h)
             except Exception:
                 pass
-            self.handle = None
+            self._handle = None
 
     # layer count that produces `value_name` (for intermediate-value bounds)
     def layers_upto(self, value_name: Optional[str]) -> int:
@@ -227,7 +294,8 @@ _CHAIN_CACHE: Dict[Tuple, CudaChain] = {}
 
 def compile_chain(module: Any, input_shape: Sequence[int], device: torch.device) -> CudaChain:
     """Cached by module identity, parameter storage and device (a module whose
-    parameter tensors are replaced gets a fresh chain)."""
+    parameter tensors are replaced gets a fresh chain, and so does one whose copied
+    parameters have been changed in place)."""
     raw = module.bindings.get("params", {})
     key = (
         id(module),
@@ -236,9 +304,10 @@ def compile_chain(module: Any, input_shape: Sequence[int], device: torch.device)
         tuple((k, v.data_ptr() if torch.is_tensor(v) else id(v)) for k, v in raw.items()) if isinstance(raw, dict) else (),
     )
     chain = _CHAIN_CACHE.get(key)
-    if chain is None:
+    if chain is None or not chain.copies_current(raw):
         if len(_CHAIN_CACHE) > 64:
             _CHAIN_CACHE.clear()
         chain = CudaChain(module, input_shape, device)
-        _CHAIN_CACHE[key] = chain
+        if not torch.cuda.is_current_stream_capturing():  # copies and images of a captured compilation are made when the graph runs
+            _CHAIN_CACHE[key] = chain
     return chain
