@@ -767,15 +767,16 @@ constexpr size_t JOIN_BYTES = (size_t)1 << 30;
 static bool join_sides(const bf_chain* c, int B, int S) {
   if ((long long)B * S * 2 >= 2147483647LL || crown_ws_layout(c, B, 2 * S, (int)c->layers.size(), nullptr, nullptr) > JOIN_BYTES) return false;
   const int M = B * S;
-  for (const bf_layer_desc& L : c->layers) {
+  for (int i = 0; i < (int)c->layers.size(); ++i) {
+    const bf_layer_desc& L = c->layers[i];
     if (L.op == BF_OP_CONV2D && conv_rows_on_tensor_cores(M, L) != conv_rows_on_tensor_cores(2 * M, L)) return false;
     if (L.op != BF_OP_LINEAR) continue;
     const bool small = small_rows(c, M, L.n_in, L.n_out, S, false);
     if (small != small_rows(c, 2 * M, L.n_in, L.n_out, 2 * S, false)) return false;
     if (small && small_tc_tiles(M, L.n_in, L.n_out) != small_tc_tiles(2 * M, L.n_in, L.n_out)) return false;
     if (small) continue;
-    const bool tc = tc_weights(c, 0, false, M, L.n_out, L.n_in) != nullptr;
-    if (tc != (tc_weights(c, 0, false, 2 * M, L.n_out, L.n_in) != nullptr)) return false;
+    const bool tc = tc_weights(c, i, false, M, L.n_out, L.n_in) != nullptr;
+    if (tc != (tc_weights(c, i, false, 2 * M, L.n_out, L.n_in) != nullptr)) return false;
     if (!tc && crown_bwd_partial_tiles(L.n_in, M) != crown_bwd_partial_tiles(L.n_in, 2 * M)) return false;  // another tile width: other partial sums
   }
   return true;

@@ -51,6 +51,22 @@ def test_one_call_and_many_agree(dev, net, ball, B):
             assert torch.equal(pa[n].lower, pb[n].lower) and torch.equal(pa[n].upper, pb[n].upper) and pa[n].lower.shape == pb[n].lower.shape
 
 
+# Chains that begin with a flatten or a convolution, on both sides of where a Linear layer of 48, 50 or 64 outputs leaves the FP32 tiles (one wave of
+# 64 x 64 tiles): neither sweep, the joined one only, both
+@pytest.mark.parametrize("body, batches", [([("fc", 48), ("fc", 10)], (40, 78, 79, 100, 149, 157, 170)), ([("fc", 64), ("fc", 10)], (78, 80, 150, 160)),
+                                           ([("conv", 16, 4, 2, 1), ("conv", 32, 4, 2, 1), ("fc", 50), ("fc", 10)], (39, 40, 60, 78, 90))])
+def test_sides_join_where_no_layer_changes_its_kernel(dev, body, batches):
+    from boundflow_b200 import crown
+    from boundflow_b200 import workloads as W
+    from boundflow_b200.ir import InputSpec
+
+    for B in batches:
+        wl = W.make_workload("c2", batch=B, eps=1e-3, net=W.NetSpec((1, 28, 28), body))
+        lo, up, C = wl.lo.to(dev), wl.up.to(dev), wl.C.to(dev)
+        a, b = (crown.run_crown_ibp_mlp(wl.module, InputSpec.box(value_name="input", lower=f(lo), upper=f(up)), linear_spec_C=C) for f in (torch.clone, _wide))
+        assert torch.equal(a.lower, b.lower) and torch.equal(a.upper, b.upper), B
+
+
 def test_contradictions_are_reported(dev):
     """lower > upper in one input set: both routes raise, and name the same domains."""
     from boundflow_b200 import crown
