@@ -782,8 +782,8 @@ static bool join_sides(const bf_chain* c, int B, int S) {
   return true;
 }
 
-// S: spec rows (0: IBP only); chunk > 0: neuron bounds too, at most `chunk` rows of a value per sweep
-static size_t query_layout(const bf_chain* c, int B, int S, int chunk, void* base, QueryWs* out) {
+// S: spec rows (0: IBP only); chunk > 0: neuron bounds too, at most `chunk` rows of a value per sweep; join: both sides in one sweep
+static size_t query_layout(const bf_chain* c, int B, int S, int chunk, bool join, void* base, QueryWs* out) {
   Carver cv(base);
   QueryWs w{};
   w.mid = cv.take<float>((size_t)B * c->n0);
@@ -791,7 +791,6 @@ static size_t query_layout(const bf_chain* c, int B, int S, int chunk, void* bas
   w.scratch_bytes = 4 * align_up((size_t)B * c->max_width * sizeof(float));
   w.scratch = cv.take<float>(w.scratch_bytes / sizeof(float));
   const int nl = (int)c->layers.size();
-  const bool join = S > 0 && chunk == 0 && join_sides(c, B, S);
   w.sweep_bytes = S > 0 ? crown_ws_layout(c, B, join ? 2 * S : S, nl, nullptr, nullptr) : 0;
   if (join) {
     w.both_C = cv.take<float>((size_t)B * 2 * S * c->layers.back().n_out);
@@ -844,7 +843,8 @@ static int query_relax(const bf_chain* c, const QueryWs& w, float* const* pre_l,
 
 extern "C" size_t bf_chain_query_workspace_bytes(const bf_chain* chain, int B, int S, int chunk_rows) {
   if (!chain || B <= 0 || S < 0 || chunk_rows < 0) return 0;
-  return bf::query_layout(chain, B, S, chunk_rows, nullptr, nullptr);
+  bf::refresh_switches(chain);
+  return bf::query_layout(chain, B, S, chunk_rows, S > 0 && chunk_rows == 0 && bf::join_sides(chain, B, S), nullptr, nullptr);
 }
 
 extern "C" int bf_chain_ibp_query(const bf_chain* chain, const float* in_a, const float* in_b, float eps, float* out_l, float* out_u,
@@ -852,7 +852,7 @@ extern "C" int bf_chain_ibp_query(const bf_chain* chain, const float* in_a, cons
   BF_REQUIRE(chain && in_a && out_l && out_u && workspace, BF_E_INVALID, "bf_chain_ibp_query: null argument");
   BF_REQUIRE(B > 0, BF_E_INVALID, "bf_chain_ibp_query: B must be positive");
   bf::QueryWs w;
-  const size_t need = bf::query_layout(chain, B, 0, 0, workspace, &w);
+  const size_t need = bf::query_layout(chain, B, 0, 0, false, workspace, &w);
   BF_REQUIRE(workspace_bytes >= need, BF_E_WORKSPACE, "bf_chain_ibp_query: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
   int rc = bf::query_input(in_a, in_b, eps, w, (size_t)B * chain->n0, bf::as_stream(stream));
   if (rc != BF_OK) return rc;
@@ -864,11 +864,13 @@ extern "C" int bf_chain_crown_query(const bf_chain* chain, const float* in_a, co
                                     float* out_u, void* workspace, size_t workspace_bytes, int B, int S, bf_stream_t stream) {
   BF_REQUIRE(chain && in_a && C && out_l && out_u && workspace, BF_E_INVALID, "bf_chain_crown_query: null argument");
   BF_REQUIRE(B > 0 && S > 0 && (long long)B * S < 2147483647LL, BF_E_INVALID, "bf_chain_crown_query: bad B/S");
+  bf::refresh_switches(chain);
   bf::QueryWs w;
-  const size_t need = bf::query_layout(chain, B, S, 0, workspace, &w);
+  // Other switches than when the workspace was sized may join the sides now: the sweeps one after the other need less and give the same bits.
+  size_t need = bf::query_layout(chain, B, S, 0, bf::join_sides(chain, B, S), workspace, &w);
+  if (w.both_C && workspace_bytes < need) need = bf::query_layout(chain, B, S, 0, false, workspace, &w);
   BF_REQUIRE(workspace_bytes >= need, BF_E_WORKSPACE, "bf_chain_crown_query: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
   const int rows = w.both_C ? 2 * S : S;  // of a domain in a sweep
-  bf::refresh_switches(chain);
   bf::CrownWs sweep;
   bf::crown_ws_layout(chain, B, rows, (int)chain->layers.size(), w.sweep, &sweep);
   const std::vector<bf::SmallPack> packs = bf::small_images_packs(chain, &sweep.images);
@@ -897,7 +899,7 @@ extern "C" int bf_chain_crown_intermediate(const bf_chain* chain, const float* i
   BF_REQUIRE(B > 0 && S > 0 && chunk_rows > 0 && (long long)B * S < 2147483647LL && (long long)B * chunk_rows < 2147483647LL, BF_E_INVALID,
              "bf_chain_crown_intermediate: bad sizes");
   bf::QueryWs w;
-  const size_t need = bf::query_layout(chain, B, S, chunk_rows, workspace, &w);
+  const size_t need = bf::query_layout(chain, B, S, chunk_rows, false, workspace, &w);
   BF_REQUIRE(workspace_bytes >= need, BF_E_WORKSPACE, "bf_chain_crown_intermediate: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
   cudaStream_t stream = bf::as_stream(stream_);
   const int R = (int)chain->relu_layers.size();

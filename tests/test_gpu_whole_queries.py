@@ -67,6 +67,36 @@ def test_sides_join_where_no_layer_changes_its_kernel(dev, body, batches):
         assert torch.equal(a.lower, b.lower) and torch.equal(a.upper, b.upper), B
 
 
+# a 100-wide MLP (few rows on the tensor cores by default) and a flatten-first one whose joined sweep would leave the FP32 tiles (by default it does not join)
+@pytest.mark.parametrize("body, batches", [([("fc", 100), ("fc", 10)], (1, 17, 64, 150, 300)), ([("fc", 48), ("fc", 10)], (17, 64, 100))])
+def test_switches_are_read_before_anything_is_decided(dev, monkeypatch, body, batches):
+    """The first query of a chain under BF_B200_FORCE_FFMA=1 is the second one's, and its sides' one by one; a workspace sized before is large enough."""
+    from boundflow_b200 import _lib, crown
+    from boundflow_b200 import workloads as W
+    from boundflow_b200.ir import InputSpec
+    from boundflow_b200.network import compile_chain
+
+    lib = _lib.load()
+    for B in batches:
+        wl = W.make_workload("c2", batch=B, eps=1e-3, net=W.NetSpec((1, 28, 28), body))
+        lo, up, C = wl.lo.to(dev), wl.up.to(dev), wl.C.to(dev)
+        monkeypatch.delenv("BF_B200_FORCE_FFMA", raising=False)
+        chain = compile_chain(wl.module, (1, 28, 28), dev)
+        S, n = int(C.shape[1]), int(lib.bf_chain_query_workspace_bytes(chain.handle, B, int(C.shape[1]), 0))
+        monkeypatch.setenv("BF_B200_FORCE_FFMA", "1")
+        bounds = []
+        for _ in range(2):
+            ws, out = torch.empty(n, dtype=torch.uint8, device=dev), torch.empty((2, B, S), device=dev)
+            launches = _lib.tc_launch_count()
+            _lib.check(lib.bf_chain_crown_query(chain.handle, lo.data_ptr(), up.data_ptr(), 0.0, C.data_ptr(), out[0].data_ptr(), out[1].data_ptr(), ws.data_ptr(), n, B, S, None))
+            assert _lib.tc_launch_count() == launches
+            bounds.append(out)
+        a, b = (crown.run_crown_ibp_mlp(wl.module, InputSpec.box(value_name="input", lower=f(lo), upper=f(up)), linear_spec_C=C) for f in (torch.clone, _wide))
+        torch.cuda.synchronize()
+        for other in (bounds[1], torch.stack((a.lower, a.upper)), torch.stack((b.lower, b.upper))):
+            assert torch.equal(bounds[0], other), B
+
+
 def test_contradictions_are_reported(dev):
     """lower > upper in one input set: both routes raise, and name the same domains."""
     from boundflow_b200 import crown
