@@ -237,14 +237,41 @@ void refresh_switches(const bf_chain* c) {
   c->sw.tc_auto = !(rows && atoi(rows) > 0);
 }
 
-// few rows: crown_small_tc.cu
-static bool small_rows_allowed(const bf_chain* c) { return c->status && !c->sw.force_ffma && c->sw.tc_auto; }
-static bool small_rows(const bf_chain* c, int M, int N, int K, int S, bool adjoint) {
-  return small_rows_allowed(c) && small_tc_supports(M, N, K, S, adjoint);
+static const unsigned char* tc_weights(const bf_chain* c, int layer, bool adjoint, int M, int K, int N) {
+  if (c->pk_bwd.empty() || c->sw.force_ffma) return nullptr;
+  if (M < c->sw.tc_min_rows || K < 32 || N < 32) return nullptr;  // tiny problems stay on the FFMA tiles
+  if (c->sw.tc_auto && ffma_fits_one_wave(M, N)) return nullptr;   // so do layers whose 64 x 64 tiles fit one wave
+  return adjoint ? c->pk_adj[layer] : c->pk_bwd[layer];
+}
+
+// Which Linear layers below `upto` crown_small_tc.cu takes, of those whose sizes suit it, in a sweep of M rows (gradients: in it and its gradient sweep): all,
+// but where another layer of theirs is so large that it stays on the 3xTF32 kernels, only those that would be on these, too.  Both kernels truncate their sums,
+// in the same direction, and beside a TF32 layer FFMA tiles leave the bounds nearer to float64: 784 inputs, three 256-wide layers, 2700 to 4500 rows 2.83e-7
+// (2-norm) and 3.00e-7 with those layers on crown_small_tc.cu, 128-wide, 1440 to 9000 rows 1.96e-7 and 2.05e-7, two 100-wide 2.47e-7 and 2.51e-7.  In the place
+// of TF32 layers it brings 5400 rows of the 256-wide network from 1.80e-6 to 3.01e-7; without any, bounds have 0.67 to 0.94 of the FFMA tiles' error.
+enum FewRows { FEW_ROWS_NONE, FEW_ROWS_FOR_TF32, FEW_ROWS_ALL };
+static FewRows few_rows_call(const bf_chain* c, int M, int S, int upto, bool gradients) {
+  if (!c->status || c->sw.force_ffma || !c->sw.tc_auto) return FEW_ROWS_NONE;
+  for (int i = 0; i < upto; ++i) {
+    const bf_layer_desc& L = c->layers[i];
+    if (L.op != BF_OP_LINEAR) continue;
+    if (!small_tc_supports(M, L.n_in, L.n_out, S, false) && tc_weights(c, i, false, M, L.n_out, L.n_in)) return FEW_ROWS_FOR_TF32;
+    if (gradients && i < c->affine_layers.back() && !small_tc_supports(M, L.n_out, L.n_in, S, true) && tc_weights(c, i, true, M, L.n_in, L.n_out))
+      return FEW_ROWS_FOR_TF32;
+  }
+  return FEW_ROWS_ALL;
+}
+static bool few_rows_layer(const bf_chain* c, FewRows call, int layer, bool adjoint, int M, int S) {
+  const bf_layer_desc& L = c->layers[layer];
+  const int N = adjoint ? L.n_out : L.n_in, K = adjoint ? L.n_in : L.n_out;
+  return call != FEW_ROWS_NONE && small_tc_supports(M, N, K, S, adjoint) && (call == FEW_ROWS_ALL || tc_weights(c, layer, adjoint, M, K, N));
 }
 
 void small_images_layout(const bf_chain* c, int M, int S, int upto, bool adjoint, Carver& cv, SmallImages* images) {
-  if (images) *images = SmallImages{};
+  if (images) {
+    *images = SmallImages{};
+    images->M = M; images->S = S; images->upto = upto; images->gradients = adjoint;
+  }
   for (int i = 0; i < upto; ++i) {
     const bf_layer_desc& L = c->layers[i];
     if (L.op != BF_OP_LINEAR) continue;
@@ -257,18 +284,23 @@ void small_images_layout(const bf_chain* c, int M, int S, int upto, bool adjoint
       to[i] = p + ((0 - reinterpret_cast<uintptr_t>(p)) & 15u);  // the bulk copies' alignment, whatever the workspace's is
     };
     place(L.n_in, L.n_out, false);
-    if (adjoint) place(L.n_out, L.n_in, true);
+    if (adjoint && i < c->affine_layers.back()) place(L.n_out, L.n_in, true);
   }
 }
 
 std::vector<SmallPack> small_images_packs(const bf_chain* c, SmallImages* images) {
-  if (!small_rows_allowed(c)) *images = SmallImages{};
+  const FewRows call = few_rows_call(c, images->M, images->S, images->upto, images->gradients);
   std::vector<SmallPack> packs;
-  for (size_t i = 0; i < c->layers.size(); ++i) {
+  for (int i = 0; i < (int)c->layers.size(); ++i) {
     const bf_layer_desc& L = c->layers[i];
-    if (images->backward(i)) packs.push_back({L.W, L.n_out, L.n_in, 1, images->bwd[i]});
-    if (images->adjoint(i)) packs.push_back({L.W, L.n_out, L.n_in, 0, images->adj[i]});
+    for (int adj = 0; adj < 2; ++adj) {
+      std::vector<unsigned char*>& at = adj ? images->adj : images->bwd;
+      if (at.empty() || !at[i]) continue;
+      if (few_rows_layer(c, call, i, adj, images->M, images->S)) packs.push_back({L.W, L.n_out, L.n_in, adj ? 0 : 1, at[i]});
+      else at[i] = nullptr;
+    }
   }
+  images->any = !packs.empty();
   images->packed = true;
   return packs;
 }
@@ -280,7 +312,7 @@ int small_images_pack(const bf_chain* c, SmallImages* images, cudaStream_t strea
 bool tc_may_run(const bf_chain* c, int M, const SmallImages& images) {
   if (c->status == nullptr || c->sw.force_ffma) return false;
   if (!c->pk_bwd.empty() && M >= c->sw.tc_min_rows) return true;
-  if (!images.bwd.empty() || !images.adj.empty()) return true;
+  if (images.any) return true;
   for (const bf_layer_desc& L : c->layers)
     if (L.op == BF_OP_CONV2D && conv_rows_on_tensor_cores(M, L)) return true;
   return false;
@@ -294,13 +326,6 @@ static bool adjoint_feature_major(const bf_chain* c, int M, int N) {
   // (two feature CTAs per row block: c4 with 384-1024 subdomains 5.95-6.23 against 6.64-6.90 ms per call), the row-major
   // kernel on narrower ones (256 features, 9216-18432 rows: 4.7 against 5.2 ms)
   return ctas >= 128 || N >= 512;
-}
-
-static const unsigned char* tc_weights(const bf_chain* c, int layer, bool adjoint, int M, int K, int N) {
-  if (c->pk_bwd.empty() || c->sw.force_ffma) return nullptr;
-  if (M < c->sw.tc_min_rows || K < 32 || N < 32) return nullptr;  // tiny problems stay on the FFMA tiles
-  if (c->sw.tc_auto && ffma_fits_one_wave(M, N)) return nullptr;   // so do layers whose 64 x 64 tiles fit one wave
-  return adjoint ? c->pk_adj[layer] : c->pk_bwd[layer];
 }
 
 // Backward contraction of linear layer `layer`; *ptiles receives the number of column tiles
@@ -766,13 +791,14 @@ struct QueryWs {
 constexpr size_t JOIN_BYTES = (size_t)1 << 30;
 static bool join_sides(const bf_chain* c, int B, int S) {
   if ((long long)B * S * 2 >= 2147483647LL || crown_ws_layout(c, B, 2 * S, (int)c->layers.size(), nullptr, nullptr) > JOIN_BYTES) return false;
-  const int M = B * S;
-  for (int i = 0; i < (int)c->layers.size(); ++i) {
+  const int M = B * S, nl = (int)c->layers.size();
+  const FewRows few = few_rows_call(c, M, S, nl, false), few2 = few_rows_call(c, 2 * M, 2 * S, nl, false);
+  for (int i = 0; i < nl; ++i) {
     const bf_layer_desc& L = c->layers[i];
     if (L.op == BF_OP_CONV2D && conv_rows_on_tensor_cores(M, L) != conv_rows_on_tensor_cores(2 * M, L)) return false;
     if (L.op != BF_OP_LINEAR) continue;
-    const bool small = small_rows(c, M, L.n_in, L.n_out, S, false);
-    if (small != small_rows(c, 2 * M, L.n_in, L.n_out, 2 * S, false)) return false;
+    const bool small = few_rows_layer(c, few, i, false, M, S);
+    if (small != few_rows_layer(c, few2, i, false, 2 * M, 2 * S)) return false;
     if (small && small_tc_tiles(M, L.n_in, L.n_out) != small_tc_tiles(2 * M, L.n_in, L.n_out)) return false;
     if (small) continue;
     const bool tc = tc_weights(c, i, false, M, L.n_out, L.n_in) != nullptr;

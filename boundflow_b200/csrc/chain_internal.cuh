@@ -54,13 +54,14 @@ struct Carver {
 // (a launch of 3 to 4 us, or part of a query's first), so a call sees the weights as they are when it runs, on whichever stream.
 struct SmallImages {
   std::vector<unsigned char*> bwd, adj;  // per layer; null: another kernel takes the step
-  bool packed = false;
+  int M = 0, S = 0, upto = 0;            // the sweep's rows, rows per domain and layers
+  bool gradients = false, packed = false, any = false;
   const unsigned char* backward(int layer) const { return bwd.empty() ? nullptr : bwd[layer]; }
   const unsigned char* adjoint(int layer) const { return adj.empty() ? nullptr : adj[layer]; }
 };
 // Places for the layers below `upto` of a sweep of M rows, S per domain (adjoint: and of its gradient sweep)
 void small_images_layout(const bf_chain* c, int M, int S, int upto, bool adjoint, Carver& cv, SmallImages* images);
-// Fills them, or drops them all where the switches or an unprepared chain leave the rows to other kernels.  Behind refresh_switches().
+// Fills them, and drops those of layers that a sweep of these sizes leaves to other kernels (few_rows_call).  Behind refresh_switches().
 int small_images_pack(const bf_chain* c, SmallImages* images, cudaStream_t stream);
 std::vector<SmallPack> small_images_packs(const bf_chain* c, SmallImages* images);  // what there is to fill
 

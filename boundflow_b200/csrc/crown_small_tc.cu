@@ -654,7 +654,7 @@ constexpr int PACK_JOBS = 16;
 struct PackJob {
   const float* W;
   unsigned char* out;
-  int ldw, transposed, N, K, nst, first_block;
+  int ldw, transposed, vec, N, K, nst, first_block;  // vec: 128-bit loads along a row of W are legal
 };
 struct PackJobs {
   PackJob job[PACK_JOBS];
@@ -699,6 +699,12 @@ __global__ void __launch_bounds__(256) pack_small_weights_kernel(const __grid_co
   const int f = (int)(i % TF), chunk = (int)(i / TF % (p.nst * 4)), tile = (int)(i / TF / (p.nst * 4));
   const int n = tile * TF + f;
   float v[8];
+  if (!p.transposed && p.vec && n < p.N && chunk * 8 + 8 <= p.K) {
+    const float4* w = reinterpret_cast<const float4*>(p.W + (size_t)n * p.ldw + chunk * 8);
+    const float4 a = w[0], b = w[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int k = chunk * 8 + q;
@@ -740,7 +746,7 @@ static int pack_images(const SmallPack* packs, int count, const stc::QueryStart*
     for (; first < count && jobs.count < stc::PACK_JOBS; ++first) {
       const SmallPack& p = packs[first];
       const int N = p.transposed ? p.cols : p.rows, K = p.transposed ? p.rows : p.cols, nst = ceil_div(K, stc::KS);
-      jobs.job[jobs.count++] = {p.W, p.out, p.cols, p.transposed, N, K, nst, blocks};
+      jobs.job[jobs.count++] = {p.W, p.out, p.cols, p.transposed, p.cols % 4 == 0 && (reinterpret_cast<uintptr_t>(p.W) & 15u) == 0, N, K, nst, blocks};
       blocks += ceil_div(N, stc::TF) * nst * 4 * stc::TF / 256;
     }
     stc::pack_small_weights_kernel<<<blocks + start_blocks, 256, 0, stream>>>(jobs, blocks, start ? *start : stc::QueryStart{});
