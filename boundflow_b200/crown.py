@@ -470,7 +470,7 @@ def crown_from_trace(
         return terms
 
     add_by_side = {_lib.SIDE_LOWER: add_terms(relu_pre_add_coeff_l), _lib.SIDE_UPPER: add_terms(relu_pre_add_coeff_u)}
-    nbytes = int(chain.lib.bf_chain_crown_workspace_bytes(chain.handle, B, S, upto))
+    nbytes = int(chain.lib.bf_chain_crown_workspace_bytes(chain.size_handle, B, S, upto))
     ws = _Workspace.get(device, nbytes)
     outs: List[Optional[torch.Tensor]] = [None, None]
     infl = None
@@ -554,7 +554,7 @@ def _crown_query(chain: CudaChain, plain, linear_spec_C: Optional[torch.Tensor],
     C = _expand_spec(linear_spec_C, B, chain.output_width, device)
     S = int(C.shape[1])
     lower, upper = torch.empty(B, S, dtype=torch.float32, device=device), torch.empty(B, S, dtype=torch.float32, device=device)
-    nbytes = chain.lib.bf_chain_query_workspace_bytes(chain.handle, B, S, 0)
+    nbytes = chain.lib.bf_chain_query_workspace_bytes(chain.size_handle, B, S, 0)
     ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
     a, b, eps = plain
     _lib.check(chain.lib.bf_chain_crown_query(chain.handle, a.data_ptr(), _lib.ptr(b), eps, C.data_ptr(), lower.data_ptr(), upper.data_ptr(), ws.data_ptr(),
@@ -566,7 +566,7 @@ def ibp_query(chain: CudaChain, plain, device: torch.device, B: int) -> Interval
     """Interval bounds of the chain's output in one call of the library."""
     shape = (B,) + tuple(chain.output_shape)
     lower, upper = torch.empty(shape, dtype=torch.float32, device=device), torch.empty(shape, dtype=torch.float32, device=device)
-    nbytes = chain.lib.bf_chain_query_workspace_bytes(chain.interval_handle, B, 0, 0)
+    nbytes = chain.lib.bf_chain_query_workspace_bytes(chain.size_handle, B, 0, 0)
     ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
     a, b, eps = plain
     _lib.check(chain.lib.bf_chain_ibp_query(chain.interval_handle, a.data_ptr(), _lib.ptr(b), eps, lower.data_ptr(), upper.data_ptr(), ws.data_ptr(), nbytes, B,
@@ -699,7 +699,7 @@ def alpha_crown_from_trace(
     best_metric = torch.empty(B, dtype=torch.float32, device=device)
     reduce_code = codes[spec_reduce]
     if beta_splits is None:
-        nbytes = int(chain.lib.bf_chain_alpha_workspace_bytes(chain.handle, B, S))
+        nbytes = int(chain.lib.bf_chain_alpha_workspace_bytes(chain.size_handle, B, S))
         ws = _Workspace.get(device, nbytes)
         _lib.check(
             chain.lib.bf_chain_alpha_beta_crown_reduce(
@@ -726,7 +726,7 @@ def alpha_crown_from_trace(
     else:
         beta = [torch.zeros(B, n, dtype=torch.float32, device=device) for n in chain.relu_widths]
     best_beta = [b.clone() for b in beta]
-    nbytes = int(chain.lib.bf_chain_alpha_beta_workspace_bytes(chain.handle, B, S))
+    nbytes = int(chain.lib.bf_chain_alpha_beta_workspace_bytes(chain.size_handle, B, S))
     ws = _Workspace.get(device, nbytes)
     _lib.check(
         chain.lib.bf_chain_alpha_beta_crown_reduce(
@@ -761,7 +761,7 @@ def _shared_alpha_other(trace, linear_spec_C, alpha0, *, steps, lr, objective, s
     n_rows = 2 * S if paired else S
     best_rows = torch.empty(B, n_rows, dtype=torch.float32, device=device)
     best_upper = None if paired else torch.empty(B, S, dtype=torch.float32, device=device)
-    nbytes = int(chain.lib.bf_chain_alpha_shared_workspace_bytes(chain.handle, B, n_rows, 0))
+    nbytes = int(chain.lib.bf_chain_alpha_shared_workspace_bytes(chain.size_handle, B, n_rows, 0))
     ws = _Workspace.get(device, nbytes)
     obj_code = {"lower": 0, "upper": 0, "gap": _lib.OBJECTIVE_GAP, "both": _lib.OBJECTIVE_BOTH}[objective]
     _lib.check(
@@ -810,7 +810,7 @@ def _alpha_crown_other_objective(trace, linear_spec_C, alpha0, *, steps, lr, spe
     best_rows = torch.empty(B, 2 * S, dtype=torch.float32, device=device)
     best_metric = torch.empty(B, dtype=torch.float32, device=device)
     codes = {"mean": _lib.REDUCE_MEAN, "min": _lib.REDUCE_MIN, "softmin": _lib.REDUCE_SOFTMIN}
-    nbytes = int(chain.lib.bf_chain_alpha_workspace_bytes(chain.handle, B, 2 * S))
+    nbytes = int(chain.lib.bf_chain_alpha_workspace_bytes(chain.size_handle, B, 2 * S))
     ws = _Workspace.get(device, nbytes)
     _lib.check(
         chain.lib.bf_chain_alpha_crown_objective(
@@ -835,7 +835,7 @@ def alpha_grad_from_trace(trace: ForwardTrace, linear_spec_C: torch.Tensor, alph
     alpha = [a.detach().to(device=device, dtype=torch.float32).reshape(-1, n).expand(B, n).contiguous() for a, n in zip(alpha, chain.relu_widths)]
     grads = [torch.empty_like(a) for a in alpha]
     lower = torch.empty(B, S, dtype=torch.float32, device=device)
-    nbytes = int(chain.lib.bf_chain_alpha_workspace_bytes(chain.handle, B, S))
+    nbytes = int(chain.lib.bf_chain_alpha_workspace_bytes(chain.size_handle, B, S))
     ws = _Workspace.get(device, nbytes)
     _lib.check(
         chain.lib.bf_chain_alpha_grad(
@@ -899,7 +899,7 @@ def shared_alpha_crown_from_trace(trace: ForwardTrace, linear_spec_C: Optional[t
         else:
             beta = [torch.zeros(n, dtype=torch.float32, device=device) for n in chain.relu_widths]
         best_beta = [b.clone() for b in beta]
-    nbytes = int(chain.lib.bf_chain_alpha_shared_workspace_bytes(chain.handle, B, S, 1 if with_beta else 0))
+    nbytes = int(chain.lib.bf_chain_alpha_shared_workspace_bytes(chain.size_handle, B, S, 1 if with_beta else 0))
     ws = _Workspace.get(device, nbytes)
     codes = {"mean": _lib.REDUCE_MEAN, "min": _lib.REDUCE_MIN, "softmin": _lib.REDUCE_SOFTMIN}
     _lib.check(
@@ -1319,7 +1319,7 @@ def _crown_intermediate_query(module: Any, spec: Any, plain, linear_spec_C: Opti
            for name, s in zip(chain.relu_input_names, chain.relu_shapes)}
     infeasible = torch.empty(max(R, 1), B, dtype=torch.int32, device=device)
     chunk_rows = min(chunk_rows, max(chain.relu_widths[1:], default=1))  # the workspace holds a chunk
-    nbytes = chain.lib.bf_chain_query_workspace_bytes(chain.handle, B, S, chunk_rows)
+    nbytes = chain.lib.bf_chain_query_workspace_bytes(chain.size_handle, B, S, chunk_rows)
     ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
     a, b, eps = plain
     states = [pre[n] for n in chain.relu_input_names]

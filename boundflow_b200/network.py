@@ -207,19 +207,20 @@ class CudaChain:
         _lib.check(self.lib.bf_chain_create(descs, len(layers), C.byref(handle)))
         self._handle = handle
         # tensor-core path: split + pack the weights (buffer owned here, freed with the chain)
-        self._linear = [l.W for l in layers if l.op == "linear"]
+        self._linear = [l.W for l in layers if l.op == "linear" and not l.W.is_inference()]
         self._lock = threading.Lock()
-        self._packed: Optional[Tuple[int, ...]] = None  # versions of the Linear weights in the images
+        self._packed: Optional[List[int]] = None  # versions of the Linear weights in the images
         self._work: Optional[Tuple[torch.cuda.Event, int]] = None  # behind the copies and images, and the stream that made them
         self._tc_buffer = torch.empty(int(self.lib.bf_chain_tc_bytes(handle)), dtype=torch.uint8, device=self.device)
         self._owned.append(self._tc_buffer)
+        self._device_index = int(self._tc_buffer.device.index)
         self._pack()
 
-    def _versions(self) -> Tuple[int, ...]:
-        return tuple([_version(W) for W in self._linear])
+    def _versions(self) -> List[int]:
+        return [W._version for W in self._linear]
 
     def _raw_stream(self) -> int:
-        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if self.device.index is None else self.device.index)
+        return torch._C._cuda_getCurrentRawStream(self._device_index)
 
     def _pack(self) -> None:
         versions = self._versions()
@@ -253,6 +254,11 @@ class CudaChain:
     def interval_handle(self) -> C.c_void_p:
         """The `bf_chain` for interval passes, which read the weights themselves."""
         self._behind_own_work()
+        return self._handle
+
+    @property
+    def size_handle(self) -> C.c_void_p:
+        """The `bf_chain` for calls that queue no work (workspace sizes)."""
         return self._handle
 
     def copies_current(self, params: Any) -> bool:
