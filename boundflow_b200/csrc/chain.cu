@@ -573,7 +573,7 @@ static size_t crown_ws_layout(const bf_chain* c, int B, int S, int upto, void* b
   float* cacc = cv.take<float>(M);
   float* partial = cv.take<float>(M * (size_t)max_partial_tiles(c->n0));
   char* cs = cv.take<char>(conv_scratch);
-  small_images_layout(c, (int)M, S, upto, false, cv, ws ? &ws->images : nullptr);
+  if (upto == (int)c->layers.size()) small_images_layout(c, (int)M, S, upto, false, cv, ws ? &ws->images : nullptr);  // none for neurons: crown_sweep
   if (ws) {
     ws->buf[0] = b0; ws->buf[1] = b1; ws->cacc = cacc; ws->partial = partial; ws->conv_scratch = cs; ws->bytes = cv.off;
   }
@@ -629,7 +629,11 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
     return rc;
   };
   bf::refresh_switches(chain);
-  if (shared && shared->packed) {
+  // Rows that bound neurons decide which ReLUs are stable and which default slopes are 0 or 1, on the last bit of a sum: they keep sums whose order does not
+  // follow the batch, while crown_small_tc.cu cuts its sums by the number of row tiles.
+  if (C == nullptr || upto_layer < nl) {
+    ws.images = bf::SmallImages{};
+  } else if (shared && shared->packed) {
     ws.images = *shared;
   } else {
     if (int rc = bf::small_images_pack(chain, &ws.images, stream)) return rc;
@@ -948,12 +952,11 @@ extern "C" int bf_chain_crown_intermediate(const bf_chain* chain, const float* i
     if ((rc = bf::query_relax(chain, w, set_l[cur].data(), set_u[cur].data(), r, B, stream)) != BF_OK) return rc;
     for (int s = 0; s < n; s += chunk_rows) {
       const int cnt = std::min(chunk_rows, n - s);
-      bf::SmallImages images;
       for (int side = 0; side < 2; ++side) {
         float* all = side == BF_SIDE_LOWER ? w.new_l[r] : w.new_u[r];
         float* to = cnt == n ? all : (side == BF_SIDE_LOWER ? w.chunk_l : w.chunk_u);
         rc = crown_sweep(chain, upto, side, nullptr, s, w.au.data(), w.bu.data(), w.al.data(), nullptr, w.mid, w.rad, BF_NORM_BOX, 0.f, to, w.sweep,
-                         w.sweep_bytes, B, cnt, stream_, nullptr, &images);
+                         w.sweep_bytes, B, cnt, stream_);
         if (rc != BF_OK) return rc;
       }
       if (cnt < n && (rc = bf::launch_place_columns(w.chunk_l, w.chunk_u, w.new_l[r], w.new_u[r], B, cnt, n, s, stream)) != BF_OK) return rc;

@@ -97,6 +97,30 @@ def test_switches_are_read_before_anything_is_decided(dev, monkeypatch, body, ba
             assert torch.equal(bounds[0], other), B
 
 
+@pytest.mark.parametrize("B", [1, 2, 8])
+def test_neurons_of_linear_layers_keep_the_order_of_their_sums(dev, monkeypatch, B):
+    """Bounds that decide default slopes come from the FP32 tiles at every number of rows: whole query, identity rows and given rows."""
+    from boundflow_b200 import crown
+    from boundflow_b200 import workloads as W
+    from boundflow_b200.ir import InputSpec
+
+    wl = W.make_workload("c1", batch=B, eps=1e-3, net=W.NetSpec((784,), [("fc", 100), ("fc", 128), ("fc", 70), ("fc", 10)]))
+    lo, up, C = wl.lo.to(dev), wl.up.to(dev), wl.C.to(dev)
+    rows = torch.eye(70, device=dev)[None, 20:40].expand(B, -1, -1).contiguous()
+
+    def bounds(f):
+        spec = InputSpec.box(value_name="input", lower=f(lo), upper=f(up))
+        _, pre = crown.run_crown_intermediate_mlp(wl.module, spec, linear_spec_C=C, chunk_rows=50)
+        trace = crown.ibp_trace(wl.module, spec)
+        given = crown.crown_from_trace(trace, rows, output_value=wl.relu_names[2])
+        return [t for s in pre.values() for t in (s.lower, s.upper)] + list(given)
+
+    got = [bounds(f) for f in (torch.clone, _wide)]
+    monkeypatch.setenv("BF_B200_FORCE_FFMA", "1")
+    want = bounds(torch.clone)
+    assert all(torch.equal(a, b) for g in got for a, b in zip(g, want))
+
+
 def test_contradictions_are_reported(dev):
     """lower > upper in one input set: both routes raise, and name the same domains."""
     from boundflow_b200 import crown
