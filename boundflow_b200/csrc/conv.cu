@@ -957,14 +957,17 @@ bool conv_rows_on_tensor_cores(int M, const bf_layer_desc& L) {
 // BF_E_UNSUPPORTED: the caller takes the FP32 kernels.
 static int launch_conv_tc_bwd(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg, const float* add,
                               const float* W, const float* bias, float* A_prev, float* delta, int accumulate, int M, int S,
-                              const bf_layer_desc& L, void* scratch, int* status, cudaStream_t stream) {
+                              const bf_layer_desc& L, void* scratch, int* status, cudaStream_t stream, int sides) {
   const char* ffma = getenv("BF_B200_FORCE_FFMA");
   if ((ffma && ffma[0] == '1') || !A_prev) return BF_E_UNSUPPORTED;
-  ConvTcProblem c = conv_tc_geometry(M, S, L);
+  ConvTcProblem c = conv_tc_geometry(M / sides, S, L);
+  int slots = 0, tiles = 0;
+  double us = 0.0;
+  if (!conv_tc_rule(c, &slots)) return BF_E_UNSUPPORTED;
+  c.M = M;
   c.A = A; c.dpos = dpos; c.dneg = dneg; c.epos = epos; c.eneg = eneg; c.add = dpos ? add : nullptr;
   c.bias = bias; c.W = W; c.out = A_prev; c.status = status;
-  int slots = 0;
-  if (!conv_tc_rule(c, &slots)) return BF_E_UNSUPPORTED;
+  if (!conv_tc_supports(c, &slots, &tiles, &us)) return BF_E_UNSUPPORTED;
   const bool sums = delta && (dpos || bias || !accumulate);
   if (sums) {  // the row sums take the place that the scaled coefficients have on the FP32 path
     if (!scratch || slots > L.Co * L.Ho * L.Wo) return BF_E_UNSUPPORTED;
@@ -998,8 +1001,8 @@ static bool rowseg_keeps(const ConvTArgs& g) {
 
 int launch_crown_bwd_conv2d(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
                             const float* W, const float* bias, float* A_prev, float* delta, int accumulate, int M, int S,
-                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add, bool tensor_cores, int* status) {
-  const int tc = tensor_cores ? launch_conv_tc_bwd(A, dpos, dneg, epos, eneg, add, W, bias, A_prev, delta, accumulate, M, S, L, scratch, status, stream)
+                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add, bool tensor_cores, int* status, int sides) {
+  const int tc = tensor_cores ? launch_conv_tc_bwd(A, dpos, dneg, epos, eneg, add, W, bias, A_prev, delta, accumulate, M, S, L, scratch, status, stream, sides)
                               : BF_E_UNSUPPORTED;
   if (tc != BF_E_UNSUPPORTED) return tc;
   const float* lam = A;
@@ -1410,7 +1413,8 @@ extern "C" size_t bf_crown_relu_conv2d_bwd_scratch_bytes(int B, int S, int Co, i
   return bf::crown_bwd_conv2d_scratch_bytes(B * S, L);
 }
 
-static int conv2d_bwd(bool tensor_cores, const float* A, int side, const float* alpha_u, const float* alpha_l,
+// sides: 0 the FP32 kernels; 1, 2: the kernel that M / sides rows take
+static int conv2d_bwd(int sides, const float* A, int side, const float* alpha_u, const float* alpha_l,
                       const float* beta_u, const float* beta_l, const float* W, const float* bias, float* A_prev, float* delta,
                       int accumulate, void* scratch, size_t scratch_bytes, int B, int S, int Ci, int Hi, int Wi, int Co, int Ho,
                       int Wo, int kh, int kw, int sh, int sw, int ph, int pw, bf_stream_t stream) {
@@ -1437,7 +1441,7 @@ static int conv2d_bwd(bool tensor_cores, const float* A, int side, const float* 
   // (a block then streams a whole coefficient row)
   if (!relu && scratch_bytes < bf_crown_relu_conv2d_bwd_scratch_bytes(B, S, Co, Ho, Wo)) scratch = nullptr;
   return bf::launch_crown_bwd_conv2d(A, dpos, dneg, epos, eneg, W, bias, A_prev, delta, accumulate, B * S, S, L, scratch,
-                                     bf::as_stream(stream), nullptr, tensor_cores, nullptr);
+                                     bf::as_stream(stream), nullptr, sides > 0, nullptr, sides);
 }
 
 extern "C" int bf_crown_relu_conv2d_bwd(const float* A, int side, const float* alpha_u, const float* alpha_l,
@@ -1445,7 +1449,16 @@ extern "C" int bf_crown_relu_conv2d_bwd(const float* A, int side, const float* a
                                         float* A_prev, float* delta, int accumulate, void* scratch, size_t scratch_bytes,
                                         int B, int S, int Ci, int Hi, int Wi, int Co, int Ho, int Wo, int kh, int kw, int sh,
                                         int sw, int ph, int pw, bf_stream_t stream) {
-  return conv2d_bwd(true, A, side, alpha_u, alpha_l, beta_u, beta_l, W, bias, A_prev, delta, accumulate, scratch, scratch_bytes, B, S,
+  return conv2d_bwd(1, A, side, alpha_u, alpha_l, beta_u, beta_l, W, bias, A_prev, delta, accumulate, scratch, scratch_bytes, B, S,
+                    Ci, Hi, Wi, Co, Ho, Wo, kh, kw, sh, sw, ph, pw, stream);
+}
+
+extern "C" int bf_crown_relu_conv2d_bwd_sides(const float* A, int side, const float* alpha_u, const float* alpha_l,
+                                              const float* beta_u, const float* beta_l, const float* W, const float* bias,
+                                              float* A_prev, float* delta, int accumulate, void* scratch, size_t scratch_bytes,
+                                              int B, int S, int Ci, int Hi, int Wi, int Co, int Ho, int Wo, int kh, int kw, int sh,
+                                              int sw, int ph, int pw, bf_stream_t stream) {
+  return conv2d_bwd(2, A, side, alpha_u, alpha_l, beta_u, beta_l, W, bias, A_prev, delta, accumulate, scratch, scratch_bytes, B, S,
                     Ci, Hi, Wi, Co, Ho, Wo, kh, kw, sh, sw, ph, pw, stream);
 }
 
@@ -1454,7 +1467,7 @@ extern "C" int bf_crown_relu_conv2d_bwd_fp32(const float* A, int side, const flo
                                              float* A_prev, float* delta, int accumulate, void* scratch, size_t scratch_bytes,
                                              int B, int S, int Ci, int Hi, int Wi, int Co, int Ho, int Wo, int kh, int kw, int sh,
                                              int sw, int ph, int pw, bf_stream_t stream) {
-  return conv2d_bwd(false, A, side, alpha_u, alpha_l, beta_u, beta_l, W, bias, A_prev, delta, accumulate, scratch, scratch_bytes, B, S,
+  return conv2d_bwd(0, A, side, alpha_u, alpha_l, beta_u, beta_l, W, bias, A_prev, delta, accumulate, scratch, scratch_bytes, B, S,
                     Ci, Hi, Wi, Co, Ho, Wo, kh, kw, sh, sw, ph, pw, stream);
 }
 

@@ -174,10 +174,11 @@ int launch_beta_step(float* beta, float* m, float* v, float* gsum, const int8_t*
 int launch_verdict(const float* lower, float threshold, float tol, const int* infeasible, int8_t* verdict, float* min_lower,
                    int B, int S, cudaStream_t stream);
 // Backward step of a conv2d layer on full rows.  tensor_cores: the tensor-core kernel may take it (conv_rows_on_tensor_cores says
-// whether it takes rows of this number and layer); `status` is raised when one of its waits runs out.
+// whether it takes rows of this number and layer: M / sides of them); `status` is raised when one of its waits runs out.
 int launch_crown_bwd_conv2d(const float* A, const float* dpos, const float* dneg, const float* epos, const float* eneg,
                             const float* W, const float* bias, float* A_prev, float* delta, int accumulate, int M, int S,
-                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add, bool tensor_cores, int* status);
+                            const bf_layer_desc& L, void* scratch, cudaStream_t stream, const float* add, bool tensor_cores, int* status,
+                            int sides = 1);
 bool conv_rows_on_tensor_cores(int M, const bf_layer_desc& L);
 int launch_poison_on_status(const int* status, float* a, long long na, float* b, long long nb, cudaStream_t stream);
 // building blocks for graphs that are not chains

@@ -263,10 +263,11 @@ def _sides_join(module: Any, tr: DagTrace, params: Dict[str, torch.Tensor], S: i
 
 
 def _sweep(lib, module: Any, tr: DagTrace, params: Dict[str, torch.Tensor], relax, C: torch.Tensor, side: int, output_value: str, *,
-           add_l: Optional[Mapping[str, torch.Tensor]] = None, ahat: Optional[Dict[str, torch.Tensor]] = None):
+           add_l: Optional[Mapping[str, torch.Tensor]] = None, ahat: Optional[Dict[str, torch.Tensor]] = None, both: bool = False):
     """One backward sweep of one side.  Returns (bounds [B,S], final coefficients [B,S,n0]).  `add_l[x]` ([B,n], e.g. the
     split term of beta-CROWN on the lower side) is added to this side's coefficients behind ReLU x; `ahat` (a dict) receives the
-    coefficients that arrive at every ReLU's output, which the gradient sweep needs."""
+    coefficients that arrive at every ReLU's output, which the gradient sweep needs; `both`: S is the spec
+    rows and their negations, whose convolutions take the kernels of one side's rows."""
     device, B = tr.mid.device, tr.B
     task = module.get_entry_task()
     S = int(C.shape[1])
@@ -274,7 +275,7 @@ def _sweep(lib, module: Any, tr: DagTrace, params: Dict[str, torch.Tensor], rela
     dynamic = set(tr.lower) - set(params)
     # rows that bound the neurons of a feature map stay on the FP32 convolutions (bf_b200.h)
     neurons = len(tr.shape[output_value]) == 3 and (output_value not in task.output_values or S == _numel(tr.shape[output_value]))
-    conv_bwd = lib.bf_crown_relu_conv2d_bwd_fp32 if neurons else lib.bf_crown_relu_conv2d_bwd
+    conv_bwd = lib.bf_crown_relu_conv2d_bwd_fp32 if neurons else lib.bf_crown_relu_conv2d_bwd_sides if both else lib.bf_crown_relu_conv2d_bwd
     adj: Dict[str, _State] = {output_value: _State(C.clone(), torch.zeros(B, S, device=device))}
     scratch = torch.empty(16, dtype=torch.uint8, device=device)  # of one step at a time, on this stream
 
@@ -406,7 +407,7 @@ def crown_dag(module: Any, input_spec: Any, linear_spec_C: Optional[torch.Tensor
     S = int(C.shape[1])
     if not relu_pre_add_coeff_l and not relu_pre_add_coeff_u and _sides_join(module, tr, params, S, output_value):
         # the upper bound of a row is minus the lower bound of its negation: one sweep, half the launches (residual network, 16 inputs: 778 -> 597 us)
-        both, _ = _sweep(lib, module, tr, params, relax, torch.cat((C, -C), dim=1), _lib.SIDE_LOWER, output_value)
+        both, _ = _sweep(lib, module, tr, params, relax, torch.cat((C, -C), dim=1), _lib.SIDE_LOWER, output_value, both=True)
         return both[:, :S].contiguous(), -both[:, S:], tr
     lo, _ = _sweep(lib, module, tr, params, relax, C, _lib.SIDE_LOWER, output_value, add_l=terms(relu_pre_add_coeff_l))
     up, _ = _sweep(lib, module, tr, params, relax, C, _lib.SIDE_UPPER, output_value, add_l=terms(relu_pre_add_coeff_u))

@@ -195,7 +195,8 @@ int bf_crown_relu_linear_bwd_packed(const float* A, int side,
  * Large row blocks run on the tensor cores (FP32 values as three exact bfloat16 parts).  Every wait of that kernel is
  * bounded; should one run out, the rows it concerns are NaN in A_prev and in delta.
  * bf_crown_relu_conv2d_bwd_fp32: the same on the FP32 kernels at every size, for rows that bound the neurons of a conv layer
- * (a bound within an ulp of zero decides on its ReLU's slope; there are millions of them). */
+ * (a bound within an ulp of zero decides on its ReLU's slope; there are millions of them).
+ * bf_crown_relu_conv2d_bwd_sides: S/2 rows of a domain and their negations, on the kernel that S/2 rows take. */
 size_t bf_crown_relu_conv2d_bwd_scratch_bytes(int B, int S, int Co, int Ho, int Wo);
 int bf_crown_relu_conv2d_bwd(const float* A, int side,
                              const float* alpha_u, const float* alpha_l,
@@ -213,6 +214,14 @@ int bf_crown_relu_conv2d_bwd_fp32(const float* A, int side,
                                   void* scratch, size_t scratch_bytes,
                                   int B, int S, int Ci, int Hi, int Wi, int Co, int Ho, int Wo,
                                   int kh, int kw, int sh, int sw, int ph, int pw, bf_stream_t stream);
+int bf_crown_relu_conv2d_bwd_sides(const float* A, int side,
+                                   const float* alpha_u, const float* alpha_l,
+                                   const float* beta_u, const float* beta_l,
+                                   const float* W, const float* bias,
+                                   float* A_prev, float* delta, int accumulate,
+                                   void* scratch, size_t scratch_bytes,
+                                   int B, int S, int Ci, int Hi, int Wi, int Co, int Ho, int Wo,
+                                   int kh, int kw, int sh, int sw, int ph, int pw, bf_stream_t stream);
 
 /* Building blocks for graphs that are not chains (residual add, fan-out): the reference routes them in
  * _run_crown_backward_from_trace, boundflow/runtime/crown_ibp.py:1748-2030.

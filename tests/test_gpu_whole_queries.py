@@ -200,3 +200,44 @@ def test_graph_sides_in_one_sweep_or_two(dev, B):
     lo2, up2, _ = dag.crown_dag(module, spec, C, relu_pre_add_coeff_l=zero, relu_pre_add_coeff_u=zero)
     scale = torch.maximum(lo2.abs(), up2.abs()).max()
     assert (lo - lo2).abs().max() <= 1e-5 * scale and (up - up2).abs().max() <= 1e-5 * scale and lo.shape == up.shape == (B, 9)
+
+
+# by their number alone, the rows of both sides would change kernels: to the tensor cores (4 to 6 inputs of 16 channels, 1 to 16 of 8) or from them
+@pytest.mark.parametrize("c0, c1, H, batches", [(16, 32, 32, (1, 4, 5, 6, 8, 16)), (8, 8, 32, (2, 4, 10, 16)), (16, 32, 16, (4, 12, 14, 24)), (12, 24, 28, (2, 5, 8))])
+def test_graph_sides_join_on_the_kernels_of_one_side(dev, c0, c1, H, batches):
+    """Same kernels, and same bits on the FP32 ones.  The tensor-core convolution cuts its row sums at tiles that begin elsewhere in the joined block: sums of
+    up to 16384 products in another order, about sqrt(16384) 2^-24 = 8e-6 of their terms' size, and the bias terms are a fraction of the bounds."""
+    from boundflow_b200 import _lib, dag
+    from boundflow_b200.ir import BFTaskModule, BoundTask, InputSpec, TaskKind, TaskOp
+
+    g = torch.Generator().manual_seed(c0 + H)
+    P = {}
+
+    def conv(name, x, y, ci, co, k, s):
+        P["w" + name], P["b" + name] = torch.randn(co, ci, k, k, generator=g) * (2 / (ci * k * k)) ** 0.5, torch.randn(co, generator=g) * 0.1
+        return TaskOp("conv2d", name, [x, "w" + name, "b" + name], [y], {"stride": s, "padding": k // 2, "dilation": 1, "groups": 1})
+
+    ops = [conv("1", "x", "y1", 3, c0, 3, 1), TaskOp("relu", "r1", ["y1"], ["z1"]), conv("2", "z1", "y2", c0, c0, 3, 1), TaskOp("relu", "r2", ["y2"], ["z2"]), conv("3", "z2", "y3", c0, c0, 3, 1),
+           TaskOp("add", "a1", ["y3", "z1"], ["y4"]), TaskOp("relu", "r4", ["y4"], ["z4"]), conv("5", "z4", "y5", c0, c1, 3, 2), TaskOp("relu", "r5", ["y5"], ["z5"]),
+           conv("6", "z5", "y6", c1, c1, 3, 1), conv("7", "z4", "y7", c0, c1, 1, 2), TaskOp("add", "a2", ["y6", "y7"], ["y8"]), TaskOp("relu", "r8", ["y8"], ["z8"]),
+           TaskOp("flatten", "f", ["z8"], ["z9"], {"start_dim": 1, "end_dim": -1}), TaskOp("linear", "l", ["z9", "w9", "b9"], ["out"])]
+    P["w9"], P["b9"] = torch.randn(10, c1 * (H // 2) ** 2, generator=g) * 0.03, torch.randn(10, generator=g)
+    module = BFTaskModule([BoundTask("t", TaskKind.INTERVAL_IBP, ops, ["x"], ["out"])], "t", bindings={"params": {k: v.to(dev) for k, v in P.items()}})
+    for B in batches:
+        x = torch.rand(B, 3, H, H, generator=g).to(dev)
+        spec = InputSpec.box(value_name="x", lower=x - 0.01, upper=x + 0.01)
+        C = torch.randn(B, 9, 10, generator=g).to(dev)
+        count = [_lib.tc_launch_count()]
+        lo, up, tr = dag.crown_dag(module, spec, C)
+        count.append(_lib.tc_launch_count())
+        assert dag._sides_join(module, tr, tr.params, 9, "out")
+        zero = {"y1": torch.zeros(B, c0 * H * H, device=dev)}
+        lo2, up2, _ = dag.crown_dag(module, spec, C, relu_pre_add_coeff_l=zero, relu_pre_add_coeff_u=zero)
+        count.append(_lib.tc_launch_count())
+        on_tensor_cores = count[1] - count[0]
+        assert count[2] - count[1] == 2 * on_tensor_cores
+        scale = torch.maximum(lo2.abs(), up2.abs()).max()
+        print(c0, H, B, on_tensor_cores, float((lo - lo2).abs().max() / scale))
+        if on_tensor_cores == 0:
+            assert torch.equal(lo, lo2) and torch.equal(up, up2), B
+        assert (lo - lo2).abs().max() <= 8e-6 * scale and (up - up2).abs().max() <= 8e-6 * scale
