@@ -588,7 +588,7 @@ extern "C" size_t bf_chain_crown_workspace_bytes(const bf_chain* chain, int B, i
   return bf::crown_ws_layout(chain, B, S, upto_layer, nullptr, nullptr);
 }
 
-// One sweep; `C` dense [B,S,width of the bounded value], or NULL with onehot_first >= 0: the spec rows are rows
+// One sweep, behind refresh_switches(); `C` dense [B,S,width of the bounded value], or NULL with onehot_first >= 0: the spec rows are rows
 // onehot_first .. onehot_first+S-1 of the identity for every domain.  shared: images that sweeps of the same sizes in the same workspace have in common.
 static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const float* C, int onehot_first,
                        const float* const* alpha_u, const float* const* beta_u, const float* const* alpha_l,
@@ -628,7 +628,6 @@ static int crown_sweep(const bf_chain* chain, int upto_layer, int side, const fl
     start = nullptr;
     return rc;
   };
-  bf::refresh_switches(chain);
   // Rows that bound neurons decide which ReLUs are stable and which default slopes are 0 or 1, on the last bit of a sum: they keep sums whose order does not
   // follow the batch, while crown_small_tc.cu cuts its sums by the number of row tiles.
   if (C == nullptr || upto_layer < nl) {
@@ -747,7 +746,8 @@ extern "C" int bf_chain_crown(const bf_chain* chain, int upto_layer, int side, c
                               const float* const* alpha_u, const float* const* beta_u, const float* const* alpha_l,
                               const float* const* add, const float* mid, const float* rad, int norm_p, float eps, float* out,
                               void* workspace, size_t workspace_bytes, int B, int S, bf_stream_t stream) {
-  BF_REQUIRE(C, BF_E_INVALID, "bf_chain_crown: null argument");
+  BF_REQUIRE(chain && C, BF_E_INVALID, "bf_chain_crown: null argument");
+  bf::refresh_switches(chain);
   return crown_sweep(chain, upto_layer, side, C, -1, alpha_u, beta_u, alpha_l, add, mid, rad, norm_p, eps, out, workspace,
                      workspace_bytes, B, S, stream);
 }
@@ -757,7 +757,8 @@ extern "C" int bf_chain_crown_influence(const bf_chain* chain, int upto_layer, i
                                         const float* const* add, const float* mid, const float* rad, int norm_p, float eps,
                                         float* out, float* const* influence, void* workspace, size_t workspace_bytes, int B, int S,
                                         bf_stream_t stream) {
-  BF_REQUIRE(C && influence, BF_E_INVALID, "bf_chain_crown_influence: null argument");
+  BF_REQUIRE(chain && C && influence, BF_E_INVALID, "bf_chain_crown_influence: null argument");
+  bf::refresh_switches(chain);
   return crown_sweep(chain, upto_layer, side, C, -1, alpha_u, beta_u, alpha_l, add, mid, rad, norm_p, eps, out, workspace,
                      workspace_bytes, B, S, stream, influence);
 }
@@ -766,7 +767,9 @@ extern "C" int bf_chain_crown_onehot(const bf_chain* chain, int upto_layer, int 
                                      const float* const* alpha_u, const float* const* beta_u, const float* const* alpha_l,
                                      const float* const* add, const float* mid, const float* rad, int norm_p, float eps,
                                      float* out, void* workspace, size_t workspace_bytes, int B, int S, bf_stream_t stream) {
+  BF_REQUIRE(chain, BF_E_INVALID, "bf_chain_crown_onehot: null argument");
   BF_REQUIRE(first_row >= 0, BF_E_INVALID, "bf_chain_crown_onehot: negative first row");
+  bf::refresh_switches(chain);
   return crown_sweep(chain, upto_layer, side, nullptr, first_row, alpha_u, beta_u, alpha_l, add, mid, rad, norm_p, eps, out,
                      workspace, workspace_bytes, B, S, stream);
 }
@@ -928,6 +931,7 @@ extern "C" int bf_chain_crown_intermediate(const bf_chain* chain, const float* i
   BF_REQUIRE(chain && in_a && C && out_l && out_u && pre_l && pre_u && infeasible && workspace, BF_E_INVALID, "bf_chain_crown_intermediate: null argument");
   BF_REQUIRE(B > 0 && S > 0 && chunk_rows > 0 && (long long)B * S < 2147483647LL && (long long)B * chunk_rows < 2147483647LL, BF_E_INVALID,
              "bf_chain_crown_intermediate: bad sizes");
+  bf::refresh_switches(chain);
   bf::QueryWs w;
   const size_t need = bf::query_layout(chain, B, S, chunk_rows, false, workspace, &w);
   BF_REQUIRE(workspace_bytes >= need, BF_E_WORKSPACE, "bf_chain_crown_intermediate: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
