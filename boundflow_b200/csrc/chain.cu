@@ -244,20 +244,21 @@ static const unsigned char* tc_weights(const bf_chain* c, int layer, bool adjoin
   return adjoint ? c->pk_adj[layer] : c->pk_bwd[layer];
 }
 
-// Which Linear layers below `upto` crown_small_tc.cu takes, of those whose sizes suit it, in a sweep of M rows (gradients: in it and its gradient sweep): all,
-// but where another layer of theirs is so large that it stays on the 3xTF32 kernels, only those that would be on these, too.  Both kernels truncate their sums,
+// Which Linear layers below `upto` crown_small_tc.cu takes, of those whose sizes suit it, in a sweep of M rows (adjoint: a gradient sweep): all, but where
+// another layer is so large that it stays on the 3xTF32 kernels, only those that would be on these, too.  Both kernels truncate their sums,
 // in the same direction, and beside a TF32 layer FFMA tiles leave the bounds nearer to float64: 784 inputs, three 256-wide layers, 2700 to 4500 rows 2.83e-7
 // (2-norm) and 3.00e-7 with those layers on crown_small_tc.cu, 128-wide, 1440 to 9000 rows 1.96e-7 and 2.05e-7, two 100-wide 2.47e-7 and 2.51e-7.  In the place
 // of TF32 layers it brings 5400 rows of the 256-wide network from 1.80e-6 to 3.01e-7; without any, bounds have 0.67 to 0.94 of the FFMA tiles' error.
+// A gradient sweep is asked about apart: its layers of few rows behind such a backward sweep leave gradients with 0.26 to 0.89 of the error that FFMA tiles
+// leave (geometric means of 8 seeds, 20 sizes).
 enum FewRows { FEW_ROWS_NONE, FEW_ROWS_FOR_TF32, FEW_ROWS_ALL };
-static FewRows few_rows_call(const bf_chain* c, int M, int S, int upto, bool gradients) {
+static FewRows few_rows_call(const bf_chain* c, int M, int S, int upto, bool adjoint) {
   if (!c->status || c->sw.force_ffma || !c->sw.tc_auto) return FEW_ROWS_NONE;
   for (int i = 0; i < upto; ++i) {
     const bf_layer_desc& L = c->layers[i];
-    if (L.op != BF_OP_LINEAR) continue;
-    if (!small_tc_supports(M, L.n_in, L.n_out, S, false) && tc_weights(c, i, false, M, L.n_out, L.n_in)) return FEW_ROWS_FOR_TF32;
-    if (gradients && i < c->affine_layers.back() && !small_tc_supports(M, L.n_out, L.n_in, S, true) && tc_weights(c, i, true, M, L.n_in, L.n_out))
-      return FEW_ROWS_FOR_TF32;
+    if (L.op != BF_OP_LINEAR || (adjoint && i == c->affine_layers.back())) continue;
+    const int N = adjoint ? L.n_out : L.n_in, K = adjoint ? L.n_in : L.n_out;
+    if (!small_tc_supports(M, N, K, S, adjoint) && tc_weights(c, i, adjoint, M, K, N)) return FEW_ROWS_FOR_TF32;
   }
   return FEW_ROWS_ALL;
 }
@@ -270,7 +271,7 @@ static bool few_rows_layer(const bf_chain* c, FewRows call, int layer, bool adjo
 void small_images_layout(const bf_chain* c, int M, int S, int upto, bool adjoint, Carver& cv, SmallImages* images) {
   if (images) {
     *images = SmallImages{};
-    images->M = M; images->S = S; images->upto = upto; images->gradients = adjoint;
+    images->M = M; images->S = S; images->upto = upto;
   }
   for (int i = 0; i < upto; ++i) {
     const bf_layer_desc& L = c->layers[i];
@@ -289,14 +290,14 @@ void small_images_layout(const bf_chain* c, int M, int S, int upto, bool adjoint
 }
 
 std::vector<SmallPack> small_images_packs(const bf_chain* c, SmallImages* images) {
-  const FewRows call = few_rows_call(c, images->M, images->S, images->upto, images->gradients);
+  const FewRows call[2] = {few_rows_call(c, images->M, images->S, images->upto, false), few_rows_call(c, images->M, images->S, images->upto, true)};
   std::vector<SmallPack> packs;
   for (int i = 0; i < (int)c->layers.size(); ++i) {
     const bf_layer_desc& L = c->layers[i];
     for (int adj = 0; adj < 2; ++adj) {
       std::vector<unsigned char*>& at = adj ? images->adj : images->bwd;
       if (at.empty() || !at[i]) continue;
-      if (few_rows_layer(c, call, i, adj, images->M, images->S)) packs.push_back({L.W, L.n_out, L.n_in, adj ? 0 : 1, at[i]});
+      if (few_rows_layer(c, call[adj], i, adj, images->M, images->S)) packs.push_back({L.W, L.n_out, L.n_in, adj ? 0 : 1, at[i]});
       else at[i] = nullptr;
     }
   }

@@ -55,7 +55,7 @@ struct Carver {
 struct SmallImages {
   std::vector<unsigned char*> bwd, adj;  // per layer; null: another kernel takes the step
   int M = 0, S = 0, upto = 0;            // the sweep's rows, rows per domain and layers
-  bool gradients = false, packed = false, any = false;
+  bool packed = false, any = false;
   const unsigned char* backward(int layer) const { return bwd.empty() ? nullptr : bwd[layer]; }
   const unsigned char* adjoint(int layer) const { return adj.empty() ? nullptr : adj[layer]; }
 };

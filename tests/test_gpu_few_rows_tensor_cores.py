@@ -116,17 +116,19 @@ def test_gradients_and_bounds_against_float64(dev, D, S, dims):
     assert sharp >= 0.9  # of the entries: the bound is at most a twentieth of the gradients' size
 
 
-# (D, S, widths, steps of the 3xTF32 kernels in the backward and the gradient sweep): 784 columns beyond one wave of FFMA tiles and beyond the rule of few
-# rows (315 tiles of 128 x 32); with 5400 rows the 256-wide layers would be on these kernels, too, and are not; in the last case 512 columns of the gradient sweep of 33 rows per domain
-@pytest.mark.parametrize("D, S, dims, large", [(160, 9, (784, 100, 100, 10), 1), (300, 9, (784, 128, 128, 128, 10), 1), (300, 9, (784, 256, 256, 256, 10), 1), (600, 9, (784, 256, 256, 256, 10), 6), (72, 33, (300, 512, 10), 1)])
-def test_sweeps_with_a_large_layer_keep_the_others_on_fp32_units(dev, D, S, dims, large):
+# (D, S, widths, launches): 784 columns beyond one wave of FFMA tiles and beyond the rule of few rows (315 tiles of 128 x 32) take the 3xTF32 kernel in the
+# backward sweep, whose other layers stay on FFMA tiles; the gradient sweep's layers are all of few rows.  With 5400 rows the 256-wide layers of the
+# backward sweep would be on the 3xTF32 kernel, too, and are not.
+@pytest.mark.parametrize("D, S, dims, launches", [(160, 9, (784, 100, 100, 10), 1 + 2), (300, 9, (784, 128, 128, 128, 10), 1 + 3), (300, 9, (784, 256, 256, 256, 10), 1 + 3),
+                                                  (600, 9, (784, 256, 256, 256, 10), 3 + 3)])
+def test_backward_sweeps_with_a_large_layer_keep_the_others_on_fp32_units(dev, D, S, dims, launches):
     g = torch.Generator().manual_seed(D)
     Ws, bs = [torch.randn((n, k), generator=g) for k, n in zip(dims, dims[1:])], [torch.randn((n,), generator=g) for n in dims[1:]]
     rand = lambda *s: torch.rand(s, generator=g).to(dev)
     chain = _Chain(Ws, bs, dev)
-    _, _, launches = chain.grad(rand(D, S, dims[-1]), [-rand(D, n) for n in dims[1:-1]], [rand(D, n) for n in dims[1:-1]], [rand(D, n) for n in dims[1:-1]], rand(D, dims[0]), rand(D, dims[0]))
+    _, _, counted = chain.grad(rand(D, S, dims[-1]), [-rand(D, n) for n in dims[1:-1]], [rand(D, n) for n in dims[1:-1]], [rand(D, n) for n in dims[1:-1]], rand(D, dims[0]), rand(D, dims[0]))
     chain.close()
-    assert launches == large
+    assert counted == launches
 
 
 @pytest.mark.parametrize("N", (5, 128, 200))
