@@ -794,8 +794,9 @@ struct QueryWs {
 
 // Both sides in one sweep: the upper bound of a row is minus the lower bound of its negation, bit for bit (every kernel of a sweep is symmetric in the sign
 // of a row), so S rows and their negations go down together: half the launches, and fuller waves.  784-100-100-10, 64 inputs: 67 -> 57 us;
-// 784-512x4-10, 500 inputs 557 -> 378, 3000 inputs (three waves of CTAs for four) 1366 -> 1224.  Not where twice the rows would take a layer to another
-// kernel or split of its sums (other bits, or fewer of them right), nor where the rows' workspace grows beyond JOIN_BYTES: sweeps that large fill their waves.
+// 784-512x4-10, 500 inputs 557 -> 378, 3000 inputs (three waves of CTAs for four) 1366 -> 1224.  Only the row sums of tensor-core convolutions are cut at other
+// places of a row (their tiles run on over the rows): bounds of CNNs that have such layers differ by up to 7e-8 of the largest, as far from float64 as before.
+// Not where twice the rows would take a layer to another kernel or split of its sums (other bits, or fewer of them right), nor where the rows' workspace grows beyond JOIN_BYTES: sweeps that large fill their waves.
 constexpr size_t JOIN_BYTES = (size_t)1 << 30;
 static bool join_sides(const bf_chain* c, int B, int S) {
   if ((long long)B * S * 2 >= 2147483647LL || crown_ws_layout(c, B, 2 * S, (int)c->layers.size(), nullptr, nullptr) > JOIN_BYTES) return false;

@@ -10,10 +10,11 @@
 // Where there are fewer tiles than SMs a cluster of two or four CTAs shares a tile: each takes a part of the terms, leaves its sums in shared memory
 // and finishes a part of the features.
 // An FP32 value is split into three bfloat16 parts without a remainder, x = x0 + x1 + x2; all nine
-// products are formed, by four MMAs per 16 terms (an MMA takes max(N / 2, 32 + N / 4) clocks whatever the layout: it reads 4 KB of weights).  Tensor-memory accumulators truncate: the error of a sum grows with its MMA steps, and always towards zero, so the leading
+// products are formed, by four MMAs per 16 terms (an MMA takes max(N / 2, 32 + N / 4) clocks whatever the layout: it reads 4 KB of weights).
+// Tensor-memory accumulators truncate: the error of a sum grows with its MMA steps, and always towards zero, so the leading
 // products of every stage, of short sums of every step, have an accumulator of their own; they are added in FP32.
-// Error against float64 (2-norm) of bounds and gradients of 3 to 6 layers of 64 to 800: 6e-8 to 9e-8 and 8e-8 to 1.6e-7 (FP32 kernels 0.8 to
-// 2e-7 and 2 to 5e-7, TF32 kernels 2e-6), and fewer signs of small coefficients on the wrong side.
+// Error against float64 (2-norm) of bounds and gradients of 3 to 6 layers of 64 to 800 inputs: 6.3e-8 to 9e-8 and 8e-8 to 2.1e-7 (FP32 kernels 9e-8 to
+// 1e-7 and 4e-7 to 1.2e-6, TF32 kernels 1.8e-6 to 3.4e-6 and 8e-6 to 4e-4), and fewer signs of small coefficients on the wrong side.
 // Layouts are K-major; weights without swizzle (8-row x 16-byte core matrices), [16 terms][part][8-term chunk][128 features][16 bytes], rows
 // [part][32 rows][64 bytes] with the 64-byte swizzle: four lanes read 128 bytes of a row and a warp's stores meet different banks.
 // From the end of one launch to the end of the next, FP32 kernels -> here: 1152 x 256 x 256 backward 12.5 -> 6.8 us, adjoint 9.3 -> 6.5; 1152 rows, 256 -> 784
@@ -526,8 +527,8 @@ __global__ void __launch_bounds__(THREADS, 1) crown_small_tc_kernel(const __grid
     __syncwarp();
   }
   // ------------------------------------------------------------------ results
-  // The next launch is placed while these are written.  (Placed at the wait, with its weights' copies next to this launch's loads, the steps of 256-wide
-  // layers take 7.3 us instead of 6.5.)
+  // The next launch is placed while these are written.  (Placed at the wait, with its weights' copies next to this launch's loads, a gradient evaluation of
+  // five 256-wide layers, 128 inputs, takes 144.4 us instead of 141.5, two 512-wide ones, 60 inputs, 75.4 instead of 73.1, four, 37 inputs, 127.0 and 126.8.)
   grid_release();
   tc_fence_before();
   if (CS > 1) cluster_sync_all();
@@ -716,15 +717,15 @@ __global__ void __launch_bounds__(256) pack_small_weights_kernel(const __grid_co
 }  // namespace stc
 
 // CTAs that share the terms of a tile; 0: the problem is not small.
-// Gradient evaluations (one sweep down, one up) of 784-input networks, other kernels -> here, us: up to two tiles an SM three 256-wide layers, 300 inputs
-// 234 -> 161, 500 inputs 242 -> 171, three 128-wide ones, 1000 inputs 195 -> 150; three an SM 256-wide, 530 inputs 218 -> 208, 785 inputs 236 -> 230, five such
-// layers 345 -> 308 and 357 -> 339, 512-wide, 300 inputs 363 -> 291, 800-wide, 200 inputs 456 -> 358, but 128-wide, 1200 inputs 203 -> 210 and 100-wide 204 -> 208;
-// four an SM 256-wide, 900 inputs 250 -> 271.
-// Sums of up to 64 terms are short on the FP32 units, too: three 33-, 48- and 64-wide layers, 1 to 128 inputs 50 to 69 there and 52 to 72 here.
-// Clusters while all CTAs find an SM: four 512-wide layers, 37 inputs 145 us with one CTA a tile, 115 with two, 784-100-100-10, 64 inputs 60 and 52.  Four CTAs
-// share sums above 1024 terms (1568-1568-100-10, 48 inputs: 190 with one CTA a tile, 174); a shorter sum gains little more (500-wide, 9 inputs: 120, 91 and 77 us
-// with one, two and four), and with two the loops of the 784-input network that the tests follow step by step choose their best steps as in FP32 where two
-// steps' objectives are equal up to rounding.
+// Gradient evaluations (one sweep down, one up, images packed) of 784-input networks, other kernels -> here, us: three 256-wide layers, 300 inputs (gradient
+// sweep only, see few_rows_call) 241 -> 187, 500 inputs 245 -> 195, three 128-wide ones, 1000 inputs 201 -> 162; three tiles an SM 256-wide, 530 inputs
+// 227 -> 209, 785 inputs 243 -> 232, five such layers 359 -> 313 and 369 -> 344, 512-wide, 300 inputs 366 -> 283, two 800-wide, 200 inputs 306 -> 250, but
+// (without the packing) 128-wide, 1200 inputs 203 -> 210 and 100-wide 204 -> 208; four an SM 256-wide, 900 inputs 250 -> 271.
+// Sums of up to 64 terms are short on the FP32 units, too: three 33-, 48- and 64-wide layers, 1 to 128 inputs 50 to 69 there and, without the packing, 52 to 72 here.
+// Clusters while all CTAs find an SM: four 512-wide layers, 37 inputs 150 us with one CTA a tile, 121 with two, 784-100-100-10, 64 inputs 63 and 56.  Four CTAs
+// share sums above 1024 terms (1568-1568-100-10, 48 inputs: 199 with one CTA a tile, 182).  Shorter sums would mostly gain from four, too (one, two, four: 500-wide,
+// 9 inputs 118, 89, 77 us, five 256-wide layers, 20 inputs 134, 115, 107, two 784-wide, 16 inputs 107, 77, 87; errors alike), but tests follow loops of a
+// 784-input network step by step, two of whose steps have objectives that are equal up to rounding, and with four such a loop keeps another step.
 static int small_tc_cluster(int M, int N, int K) {
   const long long tiles = (long long)ceil_div(N, stc::TF) * ceil_div(M, stc::NR);
   if (K <= 64 || tiles > (K >= 256 ? 3 : 2) * 148) return 0;
